@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <array>
 #include <cmath>
+#include <climits>
 #include <cstdarg>
 #include <cstdio>
 #include <cstddef>
@@ -437,7 +438,6 @@ int set_smem_attrs() {
     TRY(set_max_dyn_smem(k_fft_mid<1>));
     TRY(set_max_dyn_smem(k_xpass));
     TRY(set_max_dyn_smem(k_plane));
-    TRY(set_max_dyn_smem(k_dist_axis));
     for (int n : {64, 100, 128, 240})
         for (int m = 0; m < 3; ++m) {
             TRY(set_max_dyn_smem(xpass2_for(n, m, false)));
@@ -638,29 +638,30 @@ int inverse3_dev(const Grid3& g, float2* w1, int32_t* out, const MidDesc* d_mid,
 
 int distance_on_device(const int32_t* d_grid, int32_t* d_out, int nx, int ny, int nz, cudaStream_t st,
                        const int* gate = nullptr) {
-    size_t V = (size_t)nx * ny * nz;
-    int far = nx + ny + nz + 10;  // fft3.cu:948
+    const int far = nx + ny + nz + 10;  // fft3.cu:948
     {
-        PROF("k_dist_init", st);
-        pdl(k_dist_init, grid1d(V), 256, 0, st)(d_grid, d_out, V, far, gate);
+        PROF("k_dist_z", st);
+        const long long nlines = (long long)nx * ny;
+        pdl(k_dist_z, (unsigned)((nlines + 7) / 8), 256, 0, st)(d_grid, d_out, (int)nlines, nz, far, gate);
     }
     CKL();
-    for (int axis = 0; axis < 3; ++axis) {
-        int L = axis == 0 ? nx : (axis == 1 ? ny : nz);
-        long long nlines = axis == 0 ? (long long)ny * nz : (axis == 1 ? (long long)nx * nz : (long long)nx * ny);
+    for (int axis = 1; axis >= 0; --axis) {
+        const int L = axis == 0 ? nx : ny;
         if (L <= 1) continue;
-        long long W = std::min<long long>(256, (96 * 1024) / (4LL * L));
-        if (W >= 1) {
-            long long blocks = (nlines + W - 1) / W;
-            {
-                PROF("k_dist_axis", st);
-                pdl(k_dist_axis, (unsigned)blocks, 256, (size_t)W * L * 4, st)(d_out, axis, nx, ny, nz, (int)W, gate);
-            }
+        const long long stride = axis == 0 ? (long long)ny * nz : (long long)nz;
+        const long long inner = stride, outer = axis == 0 ? 1 : nx, ostr = axis == 0 ? 0 : (long long)ny * nz;
+        if (L <= 512 && inner <= INT_MAX && outer <= 65535) {
+            // segments of 8, 16 or 32 cells over at most 16 warps: the
+            // shortest that covers the line, for the most threads in flight
+            const int seg = L <= 128 ? 8 : (L <= 256 ? 16 : 32);
+            auto k = seg == 8 ? k_dist_strided<8> : (seg == 16 ? k_dist_strided<16> : k_dist_strided<32>);
+            PROF("k_dist_axis", st);
+            pdl(k, dim3((unsigned)((inner + 31) / 32), (unsigned)outer), 32 * ((L + seg - 1) / seg), 0, st)(
+                d_out, (int)inner, ostr, L, stride, far, gate);
         } else {
-            {
-                PROF("k_dist_axis_global", st);
-                pdl(k_dist_axis_global, (unsigned)((nlines + 255) / 256), 256, 0, st)(d_out, axis, nx, ny, nz, gate);
-            }
+            PROF("k_dist_axis_global", st);
+            const long long nlines = inner * outer;
+            pdl(k_dist_axis_global, (unsigned)((nlines + 255) / 256), 256, 0, st)(d_out, axis, nx, ny, nz, gate);
         }
         CKL();
     }
@@ -1188,7 +1189,10 @@ struct psb_tray {
         }
         CK(cudaMemcpy(d_pen, pen.data(), sizeof(double) * 3 * nz, cudaMemcpyHostToDevice));
         CK(cudaMemset(d_ls, 0, sizeof(LoopState)));
-        CK(cudaMemset(d_ps, 0, sizeof(PhiStats)));
+        PhiStats ps0;
+        memset(&ps0, 0, sizeof(ps0));
+        ps0.hi = ps0.neglo = INT_MIN;
+        CK(cudaMemcpy(d_ps, &ps0, sizeof(ps0), cudaMemcpyHostToDevice));
         const int* mean_p = (const int*)((const char*)d_ps + offsetof(PhiStats, mean));
         const int* placed_now = (const int*)((const char*)d_ls + offsetof(LoopState, placed_now));
         const int* need_phi = (const int*)((const char*)d_ls + offsetof(LoopState, need_phi));
@@ -1344,22 +1348,8 @@ struct psb_tray {
 
     // mean, norm and max deviation of the distance field, on the device
     int phi_stats(const int* gate) {
-        unsigned long long* raw = (unsigned long long*)((char*)d_ps + offsetof(PhiStats, raw));
-        const int* mean_p = (const int*)((const char*)d_ps + offsetof(PhiStats, mean));
-        CK(cudaMemsetAsync(raw, 0, sizeof(unsigned long long) * 4, st));
-        {
-            PROF("k_stats", st);
-            pdl(k_stats_g, grid1d(V), 256, 0, st)(d_phi, V, nullptr, raw, gate);
-        }
-        CKL();
-        pdl(k_phi_mean, 1, 1, 0, st)(d_ps, (unsigned long long)V, gate);
-        CKL();
-        {
-            PROF("k_stats", st);
-            pdl(k_stats_g, grid1d(V), 256, 0, st)(d_phi, V, mean_p, raw, gate);
-        }
-        CKL();
-        pdl(k_phi_norm, 1, 1, 0, st)(d_ps, gate);
+        PROF("k_stats", st);
+        pdl(k_phi_stats, std::min(grid1d(V), 148 * 4), 256, 0, st)(d_phi, V, d_ps, gate);
         CKL();
         return PSB_OK;
     }

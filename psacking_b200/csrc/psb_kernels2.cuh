@@ -780,64 +780,94 @@ k_ff_reach(const OrientDesc* __restrict__ orients, FloodBufs fb, ScoreParams sp)
 // ---------------------------------------------------------------------------
 // distance field: exact L1 distance to voxels equal to 1 (fft3.cu:887-1004)
 // ---------------------------------------------------------------------------
-__global__ void k_dist_init(const int32_t* __restrict__ g, int32_t* __restrict__ d, size_t V, int far,
-                            const int* gate) {
+// The first axis, straight from the grid: per z line the 0 / far source values
+// and both sweeps in one pass.  d[z] = min over z' of src[z'] + |z - z'| is a
+// running minimum of src[z'] - z' from the left and of src[z'] + z' from the
+// right, each a warp scan; a warp owns a line (32 cells per step, the carry
+// in a register), so every load and store is one contiguous segment and no
+// line waits on another.  A line is read back in the second sweep from the
+// first one's output (L1/L2).
+// grid: ceil(nx*ny / 8), block 256
+__global__ void k_dist_z(const int32_t* __restrict__ g, int32_t* __restrict__ d, int nlines, int nz, int far,
+                         const int* gate) {
     pdl_enter();
     if (gate && !*gate) return;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < V; i += (size_t)gridDim.x * blockDim.x)
-        d[i] = g[i] == 1 ? 0 : far;
+    const int line = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (line >= nlines) return;
+    const int32_t* s = g + (size_t)line * nz;
+    int32_t* o = d + (size_t)line * nz;
+    int carry = far;   // smallest value so far, brought to the previous cell
+    for (int z0 = 0; z0 < nz; z0 += 32) {
+        const int z = z0 + lane;
+        int v = z < nz && s[z] == 1 ? 0 : far;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, k);
+            if (lane >= k) v = min(v, u + k);
+        }
+        v = min(v, carry + lane + 1);
+        if (z < nz) o[z] = v;
+        carry = __shfl_sync(0xffffffffu, v, 31);
+    }
+    __syncwarp();
+    carry = far;
+    for (int z0 = ((nz - 1) / 32) * 32; z0 >= 0; z0 -= 32) {
+        const int z = z0 + lane;
+        int v = z < nz ? o[z] : far;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+            const int u = __shfl_down_sync(0xffffffffu, v, k);
+            if (lane + k < 32) v = min(v, u + k);
+        }
+        v = min(v, carry + 32 - lane);
+        if (z < nz) o[z] = min(v, far);
+        carry = __shfl_sync(0xffffffffu, v, 0);
+    }
 }
 
-// One axis: forward then backward min(d, d_nbr + 1) along lines of length L.
-// Lines are staged in shared memory (W lines per CTA) so both the load and
-// the store are coalesced; element p of line l sits at base(l) + p*stride.
-//   axis x: lines l = y*nz+z,        base = l,                 stride = ny*nz
-//   axis y: lines l = x*nz+z,        base = x*ny*nz + z,       stride = nz
-//   axis z: lines l = x*ny+y,        base = l*nz,              stride = 1
-__global__ void k_dist_axis(int32_t* __restrict__ d, int axis, int nx, int ny, int nz, int W, const int* gate) {
+// One strided axis (y or x): min(d, d_nbr + 1) forward and backward along
+// lines of length L with element stride `stride`.  A CTA takes 32 lines that
+// are neighbours in z (or in y*z), so every row of it is one 128-byte
+// segment; its SEGS warps each hold a segment of SEG cells of all 32 lines in
+// registers, sweep it both ways, hand the segment ends over in shared memory
+// and add what comes in from the other segments: one read and one write of
+// the field, and no sweep longer than SEG cells.  (The form with one thread
+// sweeping a whole line in shared memory took 51 us per axis at 240x123x100
+// and 91 us at 128^3: too few threads, each a chain of L dependent steps.)
+//   line l = a * inner + c starts at a * outer + c, c < inner
+// grid: (ceil(inner / 32), outer lines), block 32 * SEGS, SEG * SEGS >= L
+template <int SEG>
+__global__ void __launch_bounds__(512)
+k_dist_strided(int32_t* __restrict__ d, int inner, long long outer, int L, long long stride, int far,
+                               const int* gate) {
     pdl_enter();
-    extern __shared__ int32_t sd[];
     if (gate && !*gate) return;
-    const int L = axis == 0 ? nx : (axis == 1 ? ny : nz);
-    const long long nlines = axis == 0 ? (long long)ny * nz : (axis == 1 ? (long long)nx * nz : (long long)nx * ny);
-    const long long l0 = (long long)blockIdx.x * W;
-    if (l0 >= nlines) return;
-    const int w = (int)min((long long)W, nlines - l0);
-    const size_t stride = axis == 0 ? (size_t)ny * nz : (axis == 1 ? (size_t)nz : 1);
-    auto base = [&](long long l) -> size_t {
-        if (axis == 0) return (size_t)l;
-        if (axis == 1) return (size_t)(l / nz) * ny * nz + (size_t)(l % nz);
-        return (size_t)l * nz;
-    };
-    const int tid = threadIdx.x, nthr = blockDim.x;
-    if (axis == 2) {
-        for (int idx = tid; idx < w * L; idx += nthr) {
-            int li = idx / L, p = idx - li * L;
-            sd[li * L + p] = d[base(l0 + li) + p];
-        }
-    } else {
-        for (int idx = tid; idx < w * L; idx += nthr) {
-            int p = idx / w, li = idx - p * w;
-            sd[li * L + p] = d[base(l0 + li) + (size_t)p * stride];
-        }
-    }
+    __shared__ int lo[16][32], hi[16][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int c = blockIdx.x * 32 + lane;
+    const int p0 = w * SEG;
+    int32_t* base = d + (size_t)blockIdx.y * outer + c;
+    const bool in = c < inner;
+    int v[SEG];
+#pragma unroll
+    for (int i = 0; i < SEG; ++i) v[i] = in && p0 + i < L ? base[(size_t)(p0 + i) * stride] : far;
+#pragma unroll
+    for (int i = 1; i < SEG; ++i) v[i] = min(v[i], v[i - 1] + 1);
+#pragma unroll
+    for (int i = SEG - 2; i >= 0; --i) v[i] = min(v[i], v[i + 1] + 1);
+    lo[w][lane] = v[0];
+    hi[w][lane] = v[SEG - 1];
     __syncthreads();
-    for (int li = tid; li < w; li += nthr) {
-        int32_t* s = sd + li * L;
-        for (int p = L - 2; p >= 0; --p) s[p] = min(s[p], s[p + 1] + 1);
-        for (int p = 1; p < L; ++p) s[p] = min(s[p], s[p - 1] + 1);
+    // the nearest sources of the other segments, as seen from this one's ends
+    int left = far, right = far;
+    for (int k = 0; k < nw; ++k) {
+        if (k < w) left = min(left, hi[k][lane] + (w - 1 - k) * SEG + 1);
+        if (k > w) right = min(right, lo[k][lane] + (k - 1 - w) * SEG + 1);
     }
-    __syncthreads();
-    if (axis == 2) {
-        for (int idx = tid; idx < w * L; idx += nthr) {
-            int li = idx / L, p = idx - li * L;
-            d[base(l0 + li) + p] = sd[li * L + p];
-        }
-    } else {
-        for (int idx = tid; idx < w * L; idx += nthr) {
-            int p = idx / w, li = idx - p * w;
-            d[base(l0 + li) + (size_t)p * stride] = sd[li * L + p];
-        }
+#pragma unroll
+    for (int i = 0; i < SEG; ++i) {
+        const int r = min(v[i], min(left + i, right + (SEG - 1 - i)));
+        if (in && p0 + i < L) base[(size_t)(p0 + i) * stride] = r;
     }
 }
 
@@ -853,30 +883,6 @@ __global__ void k_dist_axis_global(int32_t* __restrict__ d, int axis, int nx, in
     size_t b = axis == 0 ? (size_t)l : (axis == 1 ? (size_t)(l / nz) * ny * nz + (size_t)(l % nz) : (size_t)l * nz);
     for (int p = L - 2; p >= 0; --p) d[b + p * stride] = min(d[b + p * stride], d[b + (p + 1) * stride] + 1);
     for (int p = 1; p < L; ++p) d[b + p * stride] = min(d[b + p * stride], d[b + (p - 1) * stride] + 1);
-}
-
-// sum and sum of squares (around a shift) for the distance spectrum's mean
-// subtraction; also the max absolute deviation.
-__global__ void k_stats(const int32_t* __restrict__ v, size_t n, int shift, unsigned long long* out) {
-    pdl_enter();
-    long long s = 0, s2 = 0;
-    int mx = 0;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        long long d = (long long)v[i] - shift;
-        s += d;
-        s2 += d * d;
-        mx = max(mx, (int)(d < 0 ? -d : d));
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        s += __shfl_xor_sync(0xffffffffu, s, off);
-        s2 += __shfl_xor_sync(0xffffffffu, s2, off);
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&out[0], (unsigned long long)s);
-        atomicAdd(&out[1], (unsigned long long)s2);
-        atomicMax((unsigned int*)&out[2], (unsigned int)mx);
-    }
 }
 
 // any negative value?

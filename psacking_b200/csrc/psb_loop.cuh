@@ -13,7 +13,9 @@
 #include "psb_kernels2.cuh"
 
 struct PhiStats {
-    unsigned long long raw[4];  // k_stats accumulators (sum, sum of squares, max |.|)
+    unsigned long long raw[2];  // k_phi_stats accumulators: sum, sum of squares,
+    long long hi, neglo;        //   largest value, largest negated value (INT_MIN between calls)
+    unsigned int done;          //   blocks finished
     int mean;                   // rounded mean of phi
     int maxabs;                 // max |phi - mean|
     double norm;                // || phi - mean ||_2
@@ -263,47 +265,60 @@ k_place_item(const OrientDesc* __restrict__ od_item, LoopState* ls, int32_t* __r
     ls->need_phi = (id == 1 && od.nvox > 0) ? 1 : 0;
 }
 
-// distance statistics on the device: mean after the first k_stats pass,
-// norm and max after the second
-__global__ void k_phi_mean(PhiStats* ps, unsigned long long V, const int* gate) {
+// Mean, norm and largest deviation of the distance field in one pass: with
+// S1 = sum v, S2 = sum v^2, lo and hi in exact integers, the rounded mean m
+// gives sum (v - m)^2 = S2 - 2 m S1 + n m^2 and max |v - m| = max(hi - m,
+// m - lo), so no second pass around the mean is needed.  Sums meet in the
+// block before one atomic per block (an atomic per warp of 4,736 blocks on
+// one address took 85 us per pass); the last block finishes the statistics and
+// leaves the accumulators ready for the next call.
+// grid: any, block 256
+__global__ void k_phi_stats(const int32_t* __restrict__ v, size_t n, PhiStats* ps, const int* gate) {
     pdl_enter();
     if (gate && !*gate) return;
-    const long long sum = (long long)ps->raw[0];
-    ps->mean = (int)llround((double)sum / (double)V);
-    ps->raw[0] = ps->raw[1] = ps->raw[2] = ps->raw[3] = 0ULL;
-}
-
-__global__ void k_phi_norm(PhiStats* ps, const int* gate) {
-    pdl_enter();
-    if (gate && !*gate) return;
-    ps->norm = sqrt((double)(long long)ps->raw[1]);
-    ps->maxabs = (int)(unsigned int)(ps->raw[2] & 0xffffffffULL);
-}
-
-// k_stats with a device-side shift and a gate
-__global__ void k_stats_g(const int32_t* __restrict__ v, size_t n, const int* shiftp, unsigned long long* out,
-                          const int* gate) {
-    pdl_enter();
-    if (gate && !*gate) return;
-    const int shift = shiftp ? *shiftp : 0;
     long long s = 0, s2 = 0;
-    int mx = 0;
+    int lo = INT_MAX, hi = INT_MIN;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        long long d = (long long)v[i] - shift;
+        const int d = v[i];
         s += d;
-        s2 += d * d;
-        mx = max(mx, (int)(d < 0 ? -d : d));
+        s2 += (long long)d * d;
+        lo = min(lo, d);
+        hi = max(hi, d);
     }
+    __shared__ long long bs[8], bs2[8];
+    __shared__ int blo[8], bhi[8];
     for (int off = 16; off > 0; off >>= 1) {
         s += __shfl_xor_sync(0xffffffffu, s, off);
         s2 += __shfl_xor_sync(0xffffffffu, s2, off);
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&out[0], (unsigned long long)s);
-        atomicAdd(&out[1], (unsigned long long)s2);
-        atomicMax((unsigned int*)&out[2], (unsigned int)mx);
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) { bs[w] = s; bs2[w] = s2; blo[w] = lo; bhi[w] = hi; }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) {
+        s += bs[k];
+        s2 += bs2[k];
+        lo = min(lo, blo[k]);
+        hi = max(hi, bhi[k]);
     }
+    atomicAdd(&ps->raw[0], (unsigned long long)s);
+    atomicAdd(&ps->raw[1], (unsigned long long)s2);
+    atomicMax(&ps->hi, (long long)hi);
+    atomicMax(&ps->neglo, -(long long)lo);
+    __threadfence();
+    if (atomicAdd(&ps->done, 1u) + 1u != gridDim.x) return;
+    __threadfence();
+    const long long S1 = (long long)atomicAdd(&ps->raw[0], 0ULL), S2 = (long long)atomicAdd(&ps->raw[1], 0ULL);
+    const long long top = atomicMax(&ps->hi, (long long)INT_MIN), low = -atomicMax(&ps->neglo, (long long)INT_MIN);
+    const long long m = llround((double)S1 / (double)n);
+    ps->mean = (int)m;
+    ps->norm = sqrt((double)(S2 - 2 * m * S1 + (long long)n * m * m));
+    ps->maxabs = (int)max(top - m, m - low);
+    ps->raw[0] = ps->raw[1] = 0ULL;
+    ps->hi = ps->neglo = INT_MIN;
+    ps->done = 0u;
 }
 
 // After a placement only the columns under the placed item's box change:
