@@ -1,0 +1,935 @@
+// psb_bound.cuh — the packing search by exact score bounds, without transforms.
+//
+// An item's winner is the free translation with the smallest score
+//   D(t) + penalty(z),   D(t) = sum over item voxels v of w(v) phi(t + v),
+// phi the L1 distance to the tray's sources (the cells equal to 1).  Two
+// lower bounds of D cost a few operations per translation, because phi is at
+// least the L1 distance to any box or half space that holds every source:
+//   * separable: phi(p) >= dx(px) + dy(py) + dz(pz), the distance to the
+//     sources' bounding box, so D(t) >= X(x) + Y(y) + Z(z), each a sum over
+//     one marginal of the item;
+//   * octants: phi(p) >= s.p - h(s) for each sign vector s, h(s) the largest
+//     s.q over the sources q, so D(t) >= W s.t + (s.M - W h(s)) with W the
+//     item's total weight and M its first moment (equality where the whole
+//     item lies beyond the sources in that octant).
+// Both are exact integers, and a score grows with D at fixed z, so a
+// translation whose bounded score exceeds a score already achieved cannot
+// win.  Measured on packing runs (128^3 and 240x123x100 trays, 24
+// orientations, 15-40 million translations per item), between 4 and a few
+// thousand free translations of all orientations together stay below the
+// winner's score; the transforms this replaces evaluated all of them.
+//
+// Per item:
+//   1. k_bound_find (SEED), on a lattice of every fourth column in x and y: the
+//      bit-parallel sample filter (psb_filter.cuh) leaves the translations that
+//      may be free, each warp checks and scores its lowest-bound survivor
+//      exactly, and the item's best score so far comes down;
+//      k_bound_find (LIST), on every column: the z range is cut where the
+//      bounds exceed the best score, the filter runs on what is left, and the
+//      survivors are listed;
+//   2. k_bound_score: the listed translations whose bound still does not
+//      exceed the best score are checked and scored exactly (integer sums), and
+//      the last CTA picks the winner by the reference's tie rules.
+// In the interlocking mode k_bound_ray then looks for a straight free run
+// from the winner to a seed face, which proves it reachable (the reachable
+// translations are a subset of the free ones, so the best free one is then
+// the best reachable one).  Where there is none, k_bound_find (ALL) lists every
+// survivor, k_bound_flood checks them and floods the free ones from the seed
+// faces in one CTA's shared memory (a crowded tray has few), and a second
+// k_bound_score takes the best reachable one.  k_bound_place writes the item.
+// An item this cannot decide (no source, more survivors than the list or
+// free ones than the flood holds) raises BoundState::halt: the launches
+// already queued for later items return at once, and the host runs that item
+// through the transforms and the union-find flood fill.
+#pragma once
+#include "psb_filter.cuh"
+
+#define PSB_BSTEP 4             // seed lattice, in x and y
+#define PSB_BCAP (1 << 16)      // listed translations per item
+#define PSB_BFREE 8192          // free translations the shared-memory flood takes
+#define PSB_BBATCH 16           // sample buckets are padded to whole batches of this many
+#define PSB_BSAMP (PSB_FSAMP + 8 * (PSB_BBATCH - 1))
+#define PSB_BHDR 16             // doubles before a table's X, Y, Z parts
+
+// The distance sources (cells equal to 1): their bounding box and, per sign
+// vector s (bit a of the index set: axis a negative), the largest s.q.
+struct BoundGeom {
+    int lo[3], hi[3];
+    int h[8];
+    int any;                    // a source exists
+    int over;                   // largest excess of the bounds over phi (0 for a distance field)
+};
+
+struct __align__(16) BoundState {
+    unsigned long long best;    // ord_key of the best score so far of the current item
+    int count;                  // listed translations
+    int halt;
+    int need_ray, need_flood;
+    int nwin;                   // translations that were the best when scored
+    unsigned int blocked;       // k_bound_ray: directions with a blocked cell
+    double win_s;
+    int win_o, win_t;
+    unsigned int done, rdone;   // CTAs finished (k_bound_score / k_bound_flood, k_bound_ray)
+    int halt_item;
+    int pad;
+};
+// the part a kernel reads on entry, in two loads (each field on its own would
+// be a dependent round trip to L2 before the work starts)
+struct BoundEntry {
+    double best;
+    int count, halt, need_ray, need_flood, nwin;
+};
+__device__ __forceinline__ BoundEntry bound_entry(const BoundState* st) {
+    const int4 a = __ldcg((const int4*)st), b = __ldcg((const int4*)st + 1);
+    BoundEntry e;
+    const unsigned long long k = (unsigned long long)(unsigned int)a.x | (unsigned long long)(unsigned int)a.y << 32;
+    e.best = k == 0xffffffffffffffffULL ? INFINITY : ord_val(k);
+    e.count = a.z;
+    e.halt = a.w;
+    e.need_ray = b.x;
+    e.need_flood = b.y;
+    e.nwin = b.z;
+    return e;
+}
+
+struct BoundHit {
+    int t, o;
+    double s;                   // the bounded score, then the exact one
+};
+
+__global__ void k_bound_geom_reset(BoundGeom* g) {
+    pdl_enter();
+    if (threadIdx.x != 0) return;
+    for (int a = 0; a < 3; ++a) { g->lo[a] = INT_MAX; g->hi[a] = -1; }
+    for (int k = 0; k < 8; ++k) g->h[k] = INT_MIN;
+    g->any = 0;
+    g->over = 0;
+}
+
+// grid: any, block 256
+__global__ void k_bound_geom(const int32_t* __restrict__ tray, int nx, int ny, int nz, BoundGeom* g) {
+    pdl_enter();
+    const size_t V = (size_t)nx * ny * nz;
+    int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {-1, -1, -1}, h[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) h[k] = INT_MIN;
+    bool any = false;
+    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < V; t += (size_t)gridDim.x * blockDim.x) {
+        if (tray[t] != 1) continue;
+        any = true;
+        const size_t r = t / nz;
+        const int c[3] = {(int)(r / ny), (int)(r % ny), (int)(t % nz)};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) { lo[a] = min(lo[a], c[a]); hi[a] = max(hi[a], c[a]); }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            h[k] = max(h[k], ((k & 1) ? -c[0] : c[0]) + ((k & 2) ? -c[1] : c[1]) + ((k & 4) ? -c[2] : c[2]));
+    }
+    if (!__any_sync(0xffffffffu, any)) return;
+    const bool l0 = (threadIdx.x & 31) == 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = __reduce_min_sync(0xffffffffu, lo[a]);
+        hi[a] = __reduce_max_sync(0xffffffffu, hi[a]);
+        if (l0) { atomicMin(&g->lo[a], lo[a]); atomicMax(&g->hi[a], hi[a]); }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        h[k] = __reduce_max_sync(0xffffffffu, h[k]);
+        if (l0) atomicMax(&g->h[k], h[k]);
+    }
+    if (l0) g->any = 1;
+}
+
+// A distance field handed in by the caller need not be the tray's: the
+// largest excess of the bounds over it, which the tables then subtract.
+// grid: any, block 256
+__global__ void k_bound_over(const int32_t* __restrict__ phi, int nx, int ny, int nz, BoundGeom* g) {
+    pdl_enter();
+    if (!g->any) return;
+    const size_t V = (size_t)nx * ny * nz;
+    long long over = 0;
+    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < V; t += (size_t)gridDim.x * blockDim.x) {
+        const size_t r = t / nz;
+        const int c[3] = {(int)(r / ny), (int)(r % ny), (int)(t % nz)};
+        int b = 0;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) b += max(0, max(g->lo[a] - c[a], c[a] - g->hi[a]));
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            b = max(b, ((k & 1) ? -c[0] : c[0]) + ((k & 2) ? -c[1] : c[1]) + ((k & 4) ? -c[2] : c[2]) - g->h[k]);
+        over = max(over, (long long)b - phi[t]);
+    }
+    const int o = __reduce_max_sync(0xffffffffu, (int)min(over, (long long)INT_MAX));
+    if ((threadIdx.x & 31) == 0 && o > 0) atomicMax(&g->over, o);
+}
+
+// ---------------------------------------------------------------------------
+// bound tables of one orientation of one item
+// ---------------------------------------------------------------------------
+// doubles (every value an integer below 2^53): [0] W, [1..8] s.M - W h(s) per
+// sign vector, [9..11] the numbers of x, y, z translations (x: 0 when the
+// orientation is skipped), then X[nx], Y[ny], Z[nz], and the smallest bounded score at z or
+// above of the separable bound's z part (F0[nz]) and of W z (F1[nz]), which
+// grow with z, so the last z worth testing in a column is a binary search.
+struct BoundTab {
+    const double *X, *Y, *Z, *F0, *F1;
+    const double* c;
+    double W;
+};
+__host__ __device__ inline long long bound_tab_stride(int nx, int ny, int nz) { return PSB_BHDR + nx + ny + 3LL * nz; }
+
+__device__ __forceinline__ BoundTab bound_tab(const double* tab, const ScoreParams& sp) {
+    BoundTab b;
+    b.W = tab[0];
+    b.c = tab + 1;
+    b.X = tab + PSB_BHDR;
+    b.Y = b.X + sp.nx;
+    b.Z = b.Y + sp.ny;
+    b.F0 = b.Z + sp.nz;
+    b.F1 = b.F0 + sp.nz;
+    return b;
+}
+
+// The tables, and the shift-sorted filter samples (as k_cand_prep), of every
+// orientation of the items i0 .. i0 + gridDim.y - 1: they depend on the items
+// and the sources only, so one launch serves a queue of items.
+// grid: (n, items), block 256
+template <int NW>
+__global__ void __launch_bounds__(256)
+k_bound_prep(const OrientDesc* __restrict__ od_all, int n, int i0, const BoundGeom* __restrict__ geom, ScoreParams sp,
+             double* __restrict__ tab, long long tstride, int2* __restrict__ fs, int* __restrict__ fbound) {
+    pdl_enter();
+    // marginals, their prefix sums and the prefix sums of k times them
+    __shared__ unsigned long long hm[3][PSB_MAX_FFT + 1], c0[3][PSB_MAX_FFT + 1], c1[3][PSB_MAX_FFT + 1];
+    __shared__ double sM[3], sW;
+    const int o = blockIdx.x, slot = blockIdx.y * n + o;
+    const OrientDesc& od = od_all[(size_t)(i0 + blockIdx.y) * n + o];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double* T = tab + (size_t)slot * tstride;
+    if (tid < 3) T[9 + tid] = od.skip ? 0.0 : (double)od.valid[tid];
+    if (od.skip) return;
+    // marginals of the oriented item along x, y and z (z by differences)
+    for (int i = tid; i < 3 * (PSB_MAX_FFT + 1); i += 256) (&hm[0][0])[i] = 0ULL;
+    __syncthreads();
+    for (int r = tid; r < od.nruns; r += 256) {
+        const int4 q = __ldg(&od.runs[r]);
+        int a, b, z0, z1;
+        orient_run(od, q, &a, &b, &z0, &z1);
+        const unsigned long long w = (unsigned long long)(long long)q.w, wl = w * (unsigned long long)(z1 - z0 + 1);
+        atomicAdd(&hm[0][a], wl);
+        atomicAdd(&hm[1][b], wl);
+        atomicAdd(&hm[2][z0], w);
+        atomicAdd(&hm[2][z1 + 1], 0ULL - w);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        unsigned long long carry = 0;
+        for (int k0 = 0; k0 < od.e[2]; k0 += 32) {
+            unsigned long long v = k0 + lane < od.e[2] ? hm[2][k0 + lane] : 0ULL;
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned long long u = __shfl_up_sync(0xffffffffu, v, d);
+                if (lane >= d) v += u;
+            }
+            v += carry;
+            if (k0 + lane < od.e[2]) hm[2][k0 + lane] = v;
+            carry = __shfl_sync(0xffffffffu, v, 31);
+        }
+    }
+    __syncthreads();
+    if (warp < 3) {
+        unsigned long long w = 0, m = 0;
+        const int e = od.e[warp];
+        if (lane == 0) c0[warp][0] = c1[warp][0] = 0ULL;
+        for (int k0 = 0; k0 < e; k0 += 32) {
+            unsigned long long v = k0 + lane < e ? hm[warp][k0 + lane] : 0ULL, u = v * (unsigned long long)(k0 + lane);
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned long long v2 = __shfl_up_sync(0xffffffffu, v, d);
+                const unsigned long long u2 = __shfl_up_sync(0xffffffffu, u, d);
+                if (lane >= d) { v += v2; u += u2; }
+            }
+            v += w;
+            u += m;
+            if (k0 + lane < e) { c0[warp][k0 + lane + 1] = v; c1[warp][k0 + lane + 1] = u; }
+            w = __shfl_sync(0xffffffffu, v, 31);
+            m = __shfl_sync(0xffffffffu, u, 31);
+        }
+        if (lane == 0) {
+            sM[warp] = (double)m;
+            if (warp == 0) sW = (double)w;
+        }
+    }
+    __syncthreads();
+    const double W = sW, low = -W * (double)geom->over;
+    if (tid == 0) T[0] = W;
+    if (tid < 8)
+        T[1 + tid] = ((tid & 1) ? -sM[0] : sM[0]) + ((tid & 2) ? -sM[1] : sM[1]) + ((tid & 4) ? -sM[2] : sM[2]) -
+                     W * (double)geom->h[tid] + low;
+    double* part[3] = {T + PSB_BHDR, T + PSB_BHDR + sp.nx, T + PSB_BHDR + sp.nx + sp.ny};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        // sum over k of hm[k] max(0, lo - p - k, p + k - hi): the cells before
+        // the box are k < m1, those behind it k >= m2
+        const long long lo = geom->lo[a], hi = geom->hi[a], e = od.e[a];
+        for (int p = tid; p < od.valid[a]; p += 256) {
+            const long long m1 = min(max(lo - p, 0LL), e), m2 = min(max(hi - p + 1, 0LL), e);
+            const long long v = (lo - p) * (long long)c0[a][m1] - (long long)c1[a][m1] +
+                                (p - hi) * (long long)(c0[a][e] - c0[a][m2]) + (long long)(c1[a][e] - c1[a][m2]);
+            part[a][p] = (double)v + (a == 0 ? low : 0.0);
+        }
+    }
+    __syncthreads();
+    if (warp < 2) {
+        // smallest bounded score at z or above
+        const double* Z = part[2];
+        double* F = part[2] + (warp == 0 ? sp.nz : 2 * sp.nz);
+        double carry = INFINITY;
+        const int Zv = od.valid[2];
+        for (int z0 = ((Zv - 1) / 32) * 32; z0 >= 0 && Zv > 0; z0 -= 32) {
+            const int z = z0 + lane;
+            double v = INFINITY;
+            if (z < Zv) v = (warp == 0 ? Z[z] : W * (double)z) + ref_score(sp, 0.0, z);
+            for (int d = 1; d < 32; d <<= 1) {
+                const double u = __shfl_down_sync(0xffffffffu, v, d);
+                if (lane + d < 32) v = fmin(v, u);
+            }
+            v = fmin(v, carry);
+            if (z < Zv) F[z] = v;
+            carry = __shfl_sync(0xffffffffu, v, 0);
+        }
+    }
+    if (warp == 2) {
+        // the buckets padded to whole batches with copies of their first
+        // sample, so the filter needs no test per sample
+        __shared__ int sb[PSB_FBOUND];
+        __shared__ int2 ss[PSB_FSAMP];
+        sort_samples<NW>(od, sb, lane, [&](int i, int x, int y, int z) {
+            ss[i] = make_int2((x * sp.ny + y) * (NW / 4), z & 31);
+        });
+        __syncwarp();
+        int2* S = fs + (size_t)slot * PSB_BSAMP;
+        int base = 0;
+        for (int k = 0; k < NW; ++k) {
+            const int b0 = sb[k], m = sb[k + 1] - b0, p = (m + PSB_BBATCH - 1) / PSB_BBATCH * PSB_BBATCH;
+            if (lane == 0) fbound[(size_t)slot * PSB_FBOUND + k] = base;
+            for (int i = lane; i < p; i += 32) S[base + i] = ss[b0 + (i < m ? i : 0)];
+            base += p;
+        }
+        if (lane == 0) fbound[(size_t)slot * PSB_FBOUND + NW] = base;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// exact checks of one translation, by one warp over the item's z-runs
+// ---------------------------------------------------------------------------
+// A run meets an occupied cell when one of the free bits of its tray column
+// over its z range is clear (one or two words for most runs).
+__device__ __forceinline__ bool run_blocked(const uint32_t* __restrict__ col, int z0, int z1) {
+    const int w0 = z0 >> 5, w1 = z1 >> 5;
+    const uint32_t m0 = 0xffffffffu << (z0 & 31), m1 = 0xffffffffu >> (31 - (z1 & 31));
+    if (w0 == w1) return (~__ldg(&col[w0]) & m0 & m1) != 0u;
+    uint32_t bad = (~__ldg(&col[w0]) & m0) | (~__ldg(&col[w1]) & m1);
+    for (int w = w0 + 1; w < w1; ++w) bad |= ~__ldg(&col[w]);
+    return bad != 0u;
+}
+
+// The map of an item's runs to tray columns and z ranges at a translation:
+// orient_run, with everything that does not depend on the run taken out.
+struct RunMap {
+    int col, mx, my;            // column = col + mx * q.x + my * q.y
+    int z;                      // z range = z + c0 .. z + c1
+    int ez;                     // flipped: c0 = ez - r1, c1 = ez - r0
+    bool flip;
+};
+__device__ __forceinline__ RunMap run_map(const OrientDesc& d, int ny, int x, int y, int z) {
+    const int lo = d.src_axis[2] == 0 ? 1 : 0;   // q.x runs along this source axis
+    const bool ax = d.src_axis[0] == lo;         // the tray's x comes from q.x
+    const int sa = d.flip[0] ? -ny : ny, sb = d.flip[1] ? -1 : 1;
+    RunMap m;
+    m.mx = ax ? sa : sb;
+    m.my = ax ? sb : sa;
+    m.col = (x + (d.flip[0] ? d.e[0] - 1 : 0)) * ny + y + (d.flip[1] ? d.e[1] - 1 : 0);
+    m.z = z;
+    m.ez = d.e[2] - 1;
+    m.flip = d.flip[2] != 0;
+    return m;
+}
+__device__ __forceinline__ int run_at(const RunMap& m, int4 q, int* z0, int* z1) {
+    const int r0 = q.z & 0xffff, r1 = q.z >> 16;
+    *z0 = m.z + (m.flip ? m.ez - r1 : r0);
+    *z1 = m.z + (m.flip ? m.ez - r0 : r1);
+    return m.col + m.mx * q.x + m.my * q.y;
+}
+
+// Collision-free?  (Item values are positive: negative ones are refused.)
+// Each step checks 128 runs spread over the whole item, so a blocked
+// translation is mostly found out in the first one.
+__device__ __forceinline__ bool bound_free(const OrientDesc& od, const uint32_t* __restrict__ T, int tw, int ny, int x,
+                                           int y, int z) {
+    const int lane = threadIdx.x & 31, nr = od.nruns, steps = (nr + 127) / 128;
+    const int4* runs = od.runs;
+    const RunMap rm = run_map(od, ny, x, y, z);
+    for (int i = 0; i < steps; ++i) {
+        bool hit = false;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int r = i + steps * (32 * u + lane);
+            if (r >= nr) continue;
+            int z0, z1;
+            const int col = run_at(rm, __ldg(&runs[r]), &z0, &z1);
+            hit = run_blocked(T + (size_t)col * tw, z0, z1) || hit;
+        }
+        if (__any_sync(0xffffffffu, hit)) return false;
+    }
+    return true;
+}
+
+// Exact proximity (every lane returns it), from the distance field's prefix
+// sums along z.
+__device__ __forceinline__ long long bound_prox(const OrientDesc& od, const int32_t* __restrict__ pphi, int ny, int nz,
+                                                int x, int y, int z) {
+    const int lane = threadIdx.x & 31, nr = od.nruns;
+    const int4* runs = od.runs;
+    const RunMap rm = run_map(od, ny, x, y, z);
+    long long acc = 0;
+#pragma unroll 4
+    for (int r = lane; r < nr; r += 32) {
+        const int4 q = __ldg(&runs[r]);
+        int z0, z1;
+        const int32_t* P = pphi + (size_t)run_at(rm, q, &z0, &z1) * (nz + 1);
+        acc += (long long)q.w * (__ldg(&P[z1 + 1]) - __ldg(&P[z0]));
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+    return acc;
+}
+
+__device__ __forceinline__ double bound_best(const BoundState* st) {
+    const unsigned long long k = *(const volatile unsigned long long*)&st->best;
+    return k == 0xffffffffffffffffULL ? INFINITY : ord_val(k);
+}
+
+// largest octant bound of a column for z signs + (gp, add W z) and - (gm)
+__device__ __forceinline__ void bound_octants(const BoundTab& b, int x, int y, double* gp, double* gm) {
+    const double dx = b.W * (double)x, dy = b.W * (double)y;
+    *gp = fmax(fmax(dx + dy + b.c[0], -dx + dy + b.c[1]), fmax(dx - dy + b.c[2], -dx - dy + b.c[3]));
+    *gm = fmax(fmax(dx + dy + b.c[4], -dx + dy + b.c[5]), fmax(dx - dy + b.c[6], -dx - dy + b.c[7]));
+}
+
+// the bounded score of cell z of a column (A = X + Y, octant parts gp, gm)
+__device__ __forceinline__ double bound_score(const BoundTab& b, const ScoreParams& sp, double A, double gp, double gm,
+                                              int z) {
+    const double wz = b.W * (double)z;
+    return ref_score(sp, fmax(A + b.Z[z], fmax(gp + wz, gm - wz)), z);
+}
+
+// how many of the nondecreasing F[0..n) are <= lim
+__device__ __forceinline__ int bound_count(const double* __restrict__ F, int n, double lim) {
+    int lo = 0;
+    while (lo < n) {
+        const int mid = (lo + n) >> 1;
+        if (F[mid] <= lim) lo = mid + 1;
+        else n = mid;
+    }
+    return lo;
+}
+
+struct BoundArgs {
+    BoundState* st;
+    const BoundGeom* geom;
+    const double* tab;          // the item's tables (orientation stride tstride)
+    long long tstride;
+    const int2* fs;             // its samples: column offset, bit shift (PSB_BSAMP per orientation)
+    const int* fbound;
+    BoundHit* list;
+    BoundHit* win;
+    const int32_t* pphi;
+};
+
+// The sample filter on 32 columns of translations (lane = one y, col its
+// tray column): c, handed in with the z range to test, is ANDed with the
+// tray's free bits of column (x + s.x, y + s.y) shifted down by s.z for every
+// sample s; the warp stops once no lane holds a survivor.  Only the lowest WA
+// words of c are live: with the z range cut by the bounds that is mostly one
+// or two, and a sample then costs its two loads and two instructions per
+// live word (128 samples by themselves are most of a warp's instructions: with
+// all words, tests per sample and samples handed round by shuffles, 4.3 M per
+// seed pass at 128^3 and 24 orientations, a warp's chain 38k cycles long).
+template <int NQ, int WA, int BATCH>
+__device__ __forceinline__ void bound_filter(const uint4* __restrict__ col, const int2* __restrict__ fs, int fb,
+                                             uint32_t (&c)[4 * NQ]) {
+    constexpr int NW = 4 * NQ;
+#pragma unroll
+    for (int k = 0; k < NW; ++k) {
+        // the quads holding words k .. k + WA of a column
+        constexpr int NQ1 = NQ;
+        const int u0 = k / 4, u1 = (k + WA) / 4 < NQ1 ? (k + WA) / 4 : NQ1 - 1;
+        const int s1 = __shfl_sync(0xffffffffu, fb, k + 1);
+        for (int s0 = __shfl_sync(0xffffffffu, fb, k); s0 < s1; s0 += BATCH) {
+            uint32_t a = 0u;
+#pragma unroll
+            for (int w = 0; w < WA; ++w) a |= c[w];
+            if (!__any_sync(0xffffffffu, a != 0u)) return;
+            uint4 v[BATCH][NQ];
+            int off[BATCH];
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) {
+                const int2 q = __ldg(&fs[s0 + i]);
+                off[i] = q.y;
+#pragma unroll
+                for (int u = 0; u < NQ; ++u)
+                    v[i][u] = u >= u0 && u <= u1 ? __ldg(col + q.x + u) : make_uint4(0u, 0u, 0u, 0u);
+            }
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) {
+                uint32_t T[NW + 1];
+#pragma unroll
+                for (int u = 0; u < NQ; ++u) {
+                    T[4 * u] = v[i][u].x;
+                    T[4 * u + 1] = v[i][u].y;
+                    T[4 * u + 2] = v[i][u].z;
+                    T[4 * u + 3] = v[i][u].w;
+                }
+                T[NW] = 0u;
+#pragma unroll
+                for (int w = 0; w < WA; ++w) {
+                    const uint32_t lo = (w + k < NW) ? T[w + k] : 0u;
+                    const uint32_t hi = (w + k + 1 < NW) ? T[w + k + 1] : 0u;
+                    c[w] &= __funnelshift_r(lo, hi, off[i]);
+                }
+            }
+        }
+    }
+}
+
+// One warp takes 32 columns (x, y0 + STEP * lane) of one orientation at
+// a time; the grid is sized to the chip and strides over the tasks (a CTA per
+// plane and orientation spent its time starting: 5,760 short CTAs per item at
+// 240x123x100).  SEED: the lattice, nothing listed.  ALL: every survivor for the
+// flood, whatever its score (gated).  grid: any, block 128
+enum BoundPass { BOUND_SEED = 0, BOUND_LIST = 1, BOUND_ALL = 2 };
+template <int NQ, int PASS>
+__global__ void __launch_bounds__(128, PASS == BOUND_SEED ? 3 : (NQ == 1 ? 6 : 4))
+k_bound_find(const OrientDesc* __restrict__ orients, int n, int planes, const uint4* __restrict__ tbits, ScoreParams sp,
+             BoundArgs ba) {
+    pdl_enter();
+    BoundState* st = ba.st;
+    const BoundEntry en = bound_entry(st);
+    if (en.halt || (PASS == BOUND_ALL && !en.need_flood)) return;
+    constexpr int NW = 4 * NQ;
+    constexpr int STEP = PASS == BOUND_SEED ? PSB_BSTEP : 1;
+    // the lattice has few warps, each a chain of load latencies: longer batches
+    constexpr int BATCH = PASS == BOUND_SEED ? PSB_BBATCH / NQ : 8 / NQ;
+    const int lane = threadIdx.x & 31, ny = sp.ny;
+    const int yb = (ny + 32 * STEP - 1) / (32 * STEP), tasks = n * planes * yb;
+    const int nwarps = gridDim.x * (blockDim.x >> 5);
+    for (int task = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); task < tasks; task += nwarps) {
+        const int y0 = (task % yb) * 32 * STEP;
+        const int o = (task / yb) % n, x = task / (yb * n) * STEP;
+        const BoundTab bt = bound_tab(ba.tab + (size_t)o * ba.tstride, sp);
+        const double h = bt.c[min(lane, 11) - 1];   // lane l: header entry l
+        const int fb = lane <= NW ? __ldg(&ba.fbound[(size_t)o * PSB_FBOUND + lane]) : 0;
+        const int y = y0 + STEP * lane;
+        const BoundEntry now = bound_entry(st);
+        double best = PASS == BOUND_ALL ? INFINITY : now.best;
+        if (now.count > PSB_BCAP) return;   // the list is lost anyway
+        const int Xv = (int)__shfl_sync(0xffffffffu, h, 9), Yv = (int)__shfl_sync(0xffffffffu, h, 10);
+        const int Zv = (int)__shfl_sync(0xffffffffu, h, 11);
+        if (x >= Xv || y0 >= Yv || Zv <= 0) continue;
+        const bool act = y < Yv;
+        double A = 0.0, gp = 0.0, gm = 0.0;
+        int zc = act ? Zv : 0;
+        if (act) {
+            A = bt.X[x] + bt.Y[y];
+            bound_octants(bt, x, y, &gp, &gm);
+            if (best < INFINITY) {
+                // slack for the roundings of F's sums; the exact test follows
+                const double lim = best + 1e-12 * fabs(best) + 1e-6;
+                zc = bound_count(bt.F0, Zv, lim - A);
+                zc = bound_count(bt.F1, zc, lim - gp);
+            }
+        }
+        uint32_t c[NW];
+        uint32_t some = 0u;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            c[w] = low_bits(zc - 32 * w);
+            some |= c[w];
+        }
+        if (!__any_sync(0xffffffffu, some != 0u)) continue;
+        // (a lane past the last row reads the last one's columns)
+        const uint4* col = tbits + ((size_t)x * ny + min(y, Yv - 1)) * NQ;
+        const int2* fs = ba.fs + (size_t)o * PSB_BSAMP;
+        const int top = __reduce_max_sync(0xffffffffu, zc);
+        if (top <= 32) bound_filter<NQ, 1, BATCH>(col, fs, fb, c);
+        else if (top <= 64) bound_filter<NQ, 2, BATCH>(col, fs, fb, c);
+        else bound_filter<NQ, NW, BATCH>(col, fs, fb, c);
+        some = 0u;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) some |= c[w];
+        if (!__any_sync(0xffffffffu, some != 0u)) continue;
+        if (PASS == BOUND_SEED || (PASS == BOUND_LIST && !(best < INFINITY))) {
+            const OrientDesc& od = orients[o];
+            for (int tries = 0; tries < 3; ++tries) {
+                // the lowest bounded score among the first survivors of each word
+                double lb = INFINITY;
+                int lz = -1;
+#pragma unroll
+                for (int w = 0; w < NW; ++w)
+                    if (c[w]) {
+                        const int z = 32 * w + __ffs(c[w]) - 1;
+                        const double s = bound_score(bt, sp, A, gp, gm, z);
+                        if (s < lb) { lb = s; lz = z; }
+                    }
+                double m = lb;
+                for (int d = 16; d > 0; d >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, d));
+                if (!(m < bound_best(st))) break;   // no survivor, or none that could improve
+                const int src = __ffs(__ballot_sync(0xffffffffu, lz >= 0 && lb == m)) - 1;
+                const int zz = __shfl_sync(0xffffffffu, lz, src);
+                if (bound_free(od, (const uint32_t*)tbits, NW, ny, x, y0 + STEP * src, zz)) {
+                    const long long D = bound_prox(od, ba.pphi, ny, sp.nz, x, y0 + STEP * src, zz);
+                    if (lane == 0) atomicMin(&st->best, ord_key(ref_score(sp, (double)D, zz)));
+                    break;
+                }
+#pragma unroll
+                for (int w = 0; w < NW; ++w)   // blocked: no survivor
+                    if (lane == src && (zz >> 5) == w) c[w] &= ~(1u << (zz & 31));
+            }
+            if (PASS == BOUND_SEED) continue;
+            best = bound_best(st);
+        }
+        int mine = 0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            if (best < INFINITY) {
+                for (uint32_t m = c[w]; m; m &= m - 1u) {
+                    const int z = 32 * w + __ffs(m) - 1;
+                    if (bound_score(bt, sp, A, gp, gm, z) > best) c[w] &= ~(1u << (z & 31));
+                }
+            }
+            mine += __popc(c[w]);
+        }
+        int incl = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += u;
+        }
+        int slot = 0;
+        if (lane == 31 && incl) slot = atomicAdd(&st->count, incl);
+        slot = __shfl_sync(0xffffffffu, slot, 31) + incl - mine;
+#pragma unroll
+        for (int w = 0; w < NW; ++w)
+            for (uint32_t m = c[w]; m && slot < PSB_BCAP; m &= m - 1u, ++slot) {
+                const int z = 32 * w + __ffs(m) - 1;
+                BoundHit h2;
+                h2.t = (x * ny + y) * sp.nz + z;
+                h2.o = o;
+                h2.s = bound_score(bt, sp, A, gp, gm, z);
+                ba.list[slot] = h2;
+            }
+    }
+}
+
+// The item's outcome into the loop state and its decision record
+__device__ __forceinline__ void bound_commit(LoopState* ls, DecisionDev* out, const ScoreParams& sp, int o, int t,
+                                             double s, int ncand) {
+    DecisionDev d;
+    d.diag = 0x800u;   // decided without transforms
+    d.ncand = ncand;
+    d.err_ratio = 0.f;
+    d.found = o >= 0;
+    d.orientation = o;
+    d.score = o >= 0 ? s : 0.0;
+    d.x = o >= 0 ? t / (sp.nz * sp.ny) : -1;
+    d.y = o >= 0 ? (t / sp.nz) % sp.ny : -1;
+    d.z = o >= 0 ? t % sp.nz : -1;
+    *out = d;
+    ls->do_place = d.found;
+    if (!d.found) return;
+    ls->orient = o;
+    ls->px = d.x; ls->py = d.y; ls->pz = d.z;
+    ls->id = ls->id_offset + ls->placed + 1;
+    ls->placed += 1;
+}
+
+// Exact check and score of the listed translations, one warp each, then the
+// winner (in the last CTA to finish): smallest score, on equal scores the
+// lowest orientation, then the tie key within it.  FLOOD: the second pass,
+// over the translations k_bound_flood left (free and reachable, the others
+// carry 1e300).  grid: any, block 256
+template <bool FLOOD>
+__global__ void __launch_bounds__(256)
+k_bound_score(const OrientDesc* __restrict__ orients, const uint4* __restrict__ tbits, int tq, ScoreParams sp,
+              BoundArgs ba, int item, int interlock, LoopState* ls, DecisionDev* out) {
+    pdl_enter();
+    BoundState* st = ba.st;
+    const BoundEntry en = bound_entry(st);
+    if (en.halt || (FLOOD && !en.need_flood)) return;
+    const int count = en.count;
+    const bool fail = count > PSB_BCAP;
+    const int n = fail ? 0 : count;
+    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+    // two entries per warp and step
+    for (int e0 = 2 * (blockIdx.x * wpb + (threadIdx.x >> 5)); e0 < n; e0 += 2 * gridDim.x * wpb) {
+        BoundHit h;
+        h.t = h.o = 0;
+        h.s = 1e300;
+        if (lane < 2 && e0 + lane < n) h = ba.list[e0 + lane];
+        for (unsigned int m = __ballot_sync(0xffffffffu, h.s < 1e299); m; m &= m - 1u) {
+            const int src = __ffs(m) - 1;
+            const int t = __shfl_sync(0xffffffffu, h.t, src), o = __shfl_sync(0xffffffffu, h.o, src);
+            if (__shfl_sync(0xffffffffu, h.s, src) > bound_best(st)) continue;
+            const OrientDesc& od = orients[o];
+            const int z = t % sp.nz, y = (t / sp.nz) % sp.ny, x = t / (sp.nz * sp.ny);
+            if (!FLOOD && !bound_free(od, (const uint32_t*)tbits, 4 * tq, sp.ny, x, y, z)) continue;
+            const double s = ref_score(sp, (double)bound_prox(od, ba.pphi, sp.ny, sp.nz, x, y, z), z);
+            if (lane == 0 && ord_key(s) <= atomicMin(&st->best, ord_key(s))) {
+                // the best so far, or equal to it: a candidate for the tie rules
+                BoundHit w;
+                w.t = t;
+                w.o = o;
+                w.s = s;
+                ba.win[atomicAdd(&st->nwin, 1)] = w;
+            }
+        }
+    }
+    __shared__ bool last;
+    __shared__ unsigned long long red[8];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(&st->done, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const BoundEntry fin = bound_entry(st);
+    const double best = fin.best;
+    unsigned long long win = ~0ULL;
+    for (int e = threadIdx.x; e < fin.nwin; e += blockDim.x) {
+        const volatile BoundHit* h = &ba.win[e];
+        if (h->s == best)
+            win = min(win, ((unsigned long long)(unsigned int)h->o << 32) | tie_key(sp.mode, h->t));
+    }
+    for (int d = 16; d > 0; d >>= 1) win = min(win, __shfl_xor_sync(0xffffffffu, win, d));
+    if (lane == 0) red[threadIdx.x >> 5] = win;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int k = 1; k < wpb; ++k) win = min(win, red[k]);
+    st->count = st->nwin = 0;
+    st->best = 0xffffffffffffffffULL;
+    if (FLOOD) st->need_flood = 0;
+    if (fail) {
+        st->halt = 1;
+        st->halt_item = item;
+        ls->do_place = 0;
+        return;
+    }
+    const bool found = best < (sp.mode == 0 ? 1000000000.0 : 1e29);
+    const int o = found ? (int)(win >> 32) : -1;
+    const int t = found ? untie_key(sp.mode, (unsigned int)win) : -1;
+    if (found && interlock && !FLOOD) {
+        st->need_ray = 1;
+        st->win_o = o;
+        st->win_t = t;
+        st->win_s = best;
+        ls->do_place = 0;
+        out->ncand = count;
+        return;
+    }
+    bound_commit(ls, out, sp, o, t, best, count);
+}
+
+// Interlocking mode: the cells between the winner and the six faces, one
+// warp each (a cell is free when the item fits there, checked exactly); a
+// direction without a blocked cell proves the winner reachable.  The near
+// faces are seeds always, the far ones for a non-empty item (fft3.cu:263-293),
+// which every item here is.  grid: any, block 256
+__global__ void __launch_bounds__(256)
+k_bound_ray(const OrientDesc* __restrict__ orients, const uint4* __restrict__ tbits, int tq, ScoreParams sp,
+            BoundState* st, LoopState* ls, DecisionDev* out) {
+    pdl_enter();
+    const BoundEntry en = bound_entry(st);
+    if (en.halt || !en.need_ray) return;
+    const OrientDesc& od = orients[st->win_o];
+    const int t = st->win_t;
+    const int at[3] = {t / (sp.nz * sp.ny), (t / sp.nz) % sp.ny, t % sp.nz};
+    int len[6], total = 0;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        len[k] = k < 3 ? at[k] : od.valid[k - 3] - 1 - at[k - 3];
+        total += len[k];
+    }
+    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+    for (int e = blockIdx.x * wpb + (threadIdx.x >> 5); e < total; e += gridDim.x * wpb) {
+        int k = 0, i = e, c[3] = {at[0], at[1], at[2]};
+#pragma unroll
+        for (int q = 0; q < 5; ++q)
+            if (k == q && i >= len[q]) { i -= len[q]; k = q + 1; }
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+            if (k % 3 == a) c[a] += k < 3 ? -1 - i : 1 + i;
+        if ((*(volatile unsigned int*)&st->blocked >> k) & 1u) continue;
+        if (!bound_free(od, (const uint32_t*)tbits, 4 * tq, sp.ny, c[0], c[1], c[2]) && lane == 0)
+            atomicOr(&st->blocked, 1u << k);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (atomicInc(&st->rdone, gridDim.x - 1) != gridDim.x - 1) return;
+    __threadfence();
+    const unsigned int blocked = *(volatile unsigned int*)&st->blocked;
+    st->blocked = 0u;
+    st->need_ray = 0;
+    if ((blocked & 63u) == 63u) {
+        st->need_flood = 1;
+        return;
+    }
+    bound_commit(ls, out, sp, st->win_o, t, st->win_s, out->ncand);
+}
+
+// Every listed translation checked exactly (one warp each), then, in the last
+// CTA to finish, the reference's flood fill (fft3.cu:234-455) over the free
+// ones: a breadth-first walk from the seed faces, neighbours along x, y and z
+// within the same orientation looked up in a shared-memory hash of the free
+// translations.  Blocked and unreached ones get the score 1e300.  The walk
+// pushes every translation at most once and a probe visits every slot at most
+// once, so both loops are bounded.  More free translations than the table
+// takes: the item goes to the union-find flood fill (halt).
+// grid: any, block 256, dynamic shared memory bound_flood_smem()
+#define PSB_BSLOTS (2 * PSB_BFREE)
+inline size_t bound_flood_smem() { return (size_t)PSB_BSLOTS * 8 + (size_t)PSB_BFREE * 4; }
+__global__ void __launch_bounds__(256)
+k_bound_flood(const OrientDesc* __restrict__ orients, const uint4* __restrict__ tbits, int tq, ScoreParams sp,
+              BoundArgs ba, int item) {
+    pdl_enter();
+    BoundState* st = ba.st;
+    const BoundEntry en = bound_entry(st);
+    if (en.halt || !en.need_flood) return;
+    const int count = en.count;
+    const int n = count > PSB_BCAP ? 0 : count;   // k_bound_score raises the halt
+    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5, ny = sp.ny, nz = sp.nz;
+    for (int e = blockIdx.x * wpb + (threadIdx.x >> 5); e < n; e += gridDim.x * wpb) {
+        const BoundHit h = ba.list[e];
+        const int z = h.t % nz, y = (h.t / nz) % ny, x = h.t / (nz * ny);
+        if (!bound_free(orients[h.o], (const uint32_t*)tbits, 4 * tq, ny, x, y, z) && lane == 0) ba.list[e].s = 1e300;
+    }
+    __shared__ int head, tail, nfree, last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicInc(&st->done, gridDim.x - 1) == gridDim.x - 1;
+        tail = nfree = 0;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    extern __shared__ unsigned int fsm[];
+    unsigned int* key = fsm;                  // o * V + t, ~0 empty
+    int* val = (int*)(fsm + PSB_BSLOTS);      // list entry, high bit set once reached
+    int* queue = val + PSB_BSLOTS;            // slots in walking order
+    const unsigned int V = (unsigned int)sp.nx * ny * nz;
+    for (int i = threadIdx.x; i < PSB_BSLOTS; i += blockDim.x) key[i] = ~0u;
+    __syncthreads();
+    auto home = [](unsigned int k) { return (int)((k * 2654435761u) >> 16) & (PSB_BSLOTS - 1); };
+    auto find = [&](unsigned int k) {
+        int s = home(k);
+        for (int i = 0; i < PSB_BSLOTS; ++i, s = (s + 1) & (PSB_BSLOTS - 1)) {
+            if (key[s] == k) return s;
+            if (key[s] == ~0u) return -1;
+        }
+        return -1;
+    };
+    for (int e = threadIdx.x; e < n; e += blockDim.x) {
+        const volatile BoundHit* h = &ba.list[e];
+        if (!(h->s < 1e299)) continue;
+        if (atomicAdd(&nfree, 1) >= PSB_BFREE) continue;
+        const unsigned int k = (unsigned int)h->o * V + (unsigned int)h->t;
+        int s = home(k);
+        for (int i = 0; i < PSB_BSLOTS; ++i, s = (s + 1) & (PSB_BSLOTS - 1))
+            if (atomicCAS(&key[s], ~0u, k) == ~0u) {
+                val[s] = e;
+                break;
+            }
+    }
+    __syncthreads();
+    if (nfree > PSB_BFREE) {
+        if (threadIdx.x == 0) {
+            st->count = 0;
+            st->need_flood = 0;
+            st->halt = 1;
+            st->halt_item = item;
+        }
+        return;
+    }
+    for (int s = threadIdx.x; s < PSB_BSLOTS; s += blockDim.x) {
+        if (key[s] == ~0u) continue;
+        const OrientDesc& od = orients[key[s] / V];
+        const int t = (int)(key[s] % V), z = t % nz, y = (t / nz) % ny, x = t / (nz * ny);
+        if (x == 0 || y == 0 || z == 0 || x == od.valid[0] - 1 || y == od.valid[1] - 1 || z == od.valid[2] - 1) {
+            val[s] |= (int)0x80000000u;
+            queue[atomicAdd(&tail, 1)] = s;
+        }
+    }
+    if (threadIdx.x == 0) head = 0;
+    __syncthreads();
+    while (true) {
+        const int h0 = head, h1 = tail;
+        __syncthreads();
+        if (h0 >= h1) break;
+        for (int i = h0 + threadIdx.x; i < h1; i += blockDim.x) {
+            const unsigned int k = key[queue[i]];
+            const int t = (int)(k % V), z = t % nz, y = (t / nz) % ny, x = t / (nz * ny);
+#pragma unroll
+            for (int d = 0; d < 6; ++d) {
+                // a neighbour outside the tray is no listed translation
+                const bool in = d == 0 ? x > 0 : d == 1 ? y > 0 : d == 2 ? z > 0
+                              : d == 3 ? x + 1 < sp.nx : d == 4 ? y + 1 < ny : z + 1 < nz;
+                if (!in) continue;
+                const int step = d % 3 == 0 ? ny * nz : (d % 3 == 1 ? nz : 1);
+                const int s = find(d < 3 ? k - step : k + step);
+                if (s < 0 || (atomicOr(&val[s], (int)0x80000000u) & (int)0x80000000u)) continue;
+                queue[atomicAdd(&tail, 1)] = s;
+            }
+        }
+        if (threadIdx.x == 0) head = h1;
+        __syncthreads();
+    }
+    for (int s = threadIdx.x; s < PSB_BSLOTS; s += blockDim.x)
+        if (key[s] != ~0u && val[s] >= 0) ba.list[val[s]].s = 1e300;
+}
+
+// The first item of an empty tray: every translation is free and the
+// distance field is the far value everywhere, so the score depends on z
+// alone, and the first orientation that fits wins at the origin (the smallest
+// tie key).  o < 0: none fits.  grid: 1, block 1
+__global__ void k_bound_first(int o, double s, ScoreParams sp, LoopState* ls, DecisionDev* out) {
+    pdl_enter();
+    bound_commit(ls, out, sp, o, 0, s, 0);
+}
+
+// The decided placement: each z-run of the item written with its id and
+// cleared from the tray's free bits.  Every cell is empty (the translation
+// was checked exactly against the same bits).  One warp per run.
+// grid: any, block 256
+__global__ void __launch_bounds__(256)
+k_bound_place(const OrientDesc* __restrict__ orients, const LoopState* __restrict__ ls, int32_t* __restrict__ tray,
+              uint32_t* __restrict__ tbits, int tw, int ny, int nz) {
+    pdl_enter();
+    if (!ls->do_place) return;
+    const OrientDesc& od = orients[ls->orient];
+    const int px = ls->px, py = ls->py, pz = ls->pz, id = ls->id;
+    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+    for (int r = blockIdx.x * wpb + (threadIdx.x >> 5); r < od.nruns; r += gridDim.x * wpb) {
+        const int4 q = __ldg(&od.runs[r]);
+        if (q.w <= 0) continue;
+        int a, b, c0, c1;
+        orient_run(od, q, &a, &b, &c0, &c1);
+        const size_t col = (size_t)(px + a) * ny + (py + b);
+        for (int k = pz + c0 + lane; k <= pz + c1; k += 32) tray[col * nz + k] = id;
+        const int w = ((pz + c0) >> 5) + lane;
+        if (w <= (pz + c1) >> 5) {
+            const int z0 = max(pz + c0 - 32 * w, 0), z1 = min(pz + c1 - 32 * w, 31);
+            atomicAnd(&tbits[col * tw + w], ~((0xffffffffu << z0) & (0xffffffffu >> (31 - z1))));
+        }
+    }
+}

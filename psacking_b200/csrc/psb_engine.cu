@@ -32,6 +32,7 @@
 #include "psb_kernels3.cuh"
 #include "psb_kernels4.cuh"
 #include "psb_loop.cuh"
+#include "psb_bound.cuh"
 #include "psb_filter.cuh"
 #include "psb_proposal.cuh"
 #include "psb_voxel.cuh"
@@ -451,6 +452,7 @@ int set_smem_attrs() {
             TRY(set_max_dyn_smem(fwd_plane_for(a, b)));
         }
     for (int n : {64, 100, 128, 240}) TRY(set_max_dyn_smem(xfwd_for(n)));
+    TRY(set_max_dyn_smem(k_bound_flood));
     TRY(set_max_dyn_smem(k_cand_filter_plane<1>));
     TRY(set_max_dyn_smem(k_cand_filter_plane<2>));
     TRY(init_register_twiddles());
@@ -916,13 +918,6 @@ void analyse_item(const int32_t* a, int ex, int ey, int ez, ItemInfo* info, bool
             }
 }
 
-double ulp32(double v) {
-    if (v < 1.0) return 1.19209290e-07;
-    int e;
-    std::frexp(v, &e);  // v = m * 2^e, m in [0.5,1)
-    return std::ldexp(1.0, e - 24);
-}
-
 }  // namespace
 
 // The item's 6 axis permutations as base descriptors (no flips), and each
@@ -998,9 +993,24 @@ struct psb_tray {
     DecisionDev* d_dec = nullptr;
     size_t dec_cap = 0;
 
-    int phi_mean = 0;
-    double phi_norm = 0.0;
-    int phi_maxabs = 0;
+    // what the transforms and the candidate filter read is derived from the
+    // tray and the distance field only when a search needs it: the spectra,
+    // the occupancy prefix sums and the distance statistics (ensure_fft), the
+    // free bits (ensure_bits), the sources' box (ensure_geom)
+    bool occ_stale = true, phi_stale = true, bits_stale = true, geom_stale = true;
+    bool phi_own = true;        // the distance field is the tray's own (not handed in)
+    bool has_source = false;    // the tray holds a cell equal to 1
+
+    // the search by score bounds (psb_bound.cuh): tables and samples of
+    // bcap queued items' orientations, the list of translations, its state
+    BoundGeom* d_bgeom = nullptr;
+    BoundState* d_bstate = nullptr;
+    BoundHit* d_blist = nullptr;   // PSB_BCAP listed translations, then as many winners
+    double* d_btab = nullptr;
+    int2* d_bfs = nullptr;
+    int* d_bfb = nullptr;
+    size_t bcap = 0;
+    BoundState* h_bstate = nullptr;   // pinned
 
     // per-orientation slots
     int cap = 0;
@@ -1119,6 +1129,8 @@ struct psb_tray {
         dfree(d_runs, st); dfree(d_pphi, st); dfree(d_pocc, st);
         dfree(d_ls, st); dfree(d_ps, st); dfree(d_rzd, st); dfree(d_midd, st); dfree(d_od_all, st); dfree(d_base_all, st); dfree(d_dec, st);
         dfree(d_tbits, st); dfree(d_work, st); dfree(d_clist, st);
+        dfree(d_bgeom, st); dfree(d_bstate, st); dfree(d_blist, st); dfree(d_btab, st); dfree(d_bfs, st); dfree(d_bfb, st);
+        bcap = 0;
         for (int p = 0; p < 2; ++p) {
             dfree(d_part[p], st);
             part_cap[p] = 0;
@@ -1149,6 +1161,8 @@ struct psb_tray {
         if (h_desc) cudaFreeHost(h_desc);
         h_desc = nullptr;
         h_desc_cap = 0;
+        if (h_bstate) cudaFreeHost(h_bstate);
+        h_bstate = nullptr;
         if (h_icmeta) cudaFreeHost(h_icmeta);
         h_icmeta = nullptr;
     }
@@ -1354,16 +1368,26 @@ struct psb_tray {
         return PSB_OK;
     }
 
-    // distance spectrum (mean-subtracted) from the device distance field
-    int rebuild_phi_spectrum() {
-        TRY(phi_stats(nullptr));
-        TRY(tray_forward(true, nullptr));
-        PhiStats h;
-        CK(cudaMemcpyAsync(&h, d_ps, sizeof(h), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        phi_mean = h.mean;
-        phi_norm = h.norm;
-        phi_maxabs = h.maxabs;
+    // Everything the transform flow reads, brought up to date with the tray
+    // and the distance field, and its n orientation slots.
+    int ensure_fft(int n) {
+        TRY(ensure_slots(std::max(n, 6)));
+        if (occ_stale) {
+            TRY(prefix_occ());
+            TRY(rebuild_occ());
+            occ_stale = false;
+        }
+        if (phi_stale) {
+            TRY(phi_stats(nullptr));
+            TRY(tray_forward(true, nullptr));   // distance spectrum (mean-subtracted)
+            phi_stale = false;
+        }
+        return PSB_OK;
+    }
+
+    int ensure_bits() {
+        if (bits_stale) TRY(tray_bits());
+        bits_stale = false;
         return PSB_OK;
     }
 
@@ -1380,17 +1404,19 @@ struct psb_tray {
     int set(const int32_t* tray, const int32_t* phi) {
         CK(cudaSetDevice(dev));
         // negative values and occupied cells, one pass over the host cores
-        std::atomic<int> neg(0);
+        std::atomic<int> neg(0), one(0);
         std::atomic<size_t> nocc(0);
         parallel_chunks(V, (size_t)1 << 20, [&](size_t b, size_t e) {
             size_t c = 0;
-            int ng = 0;
+            int ng = 0, n1 = 0;
             for (size_t i = b; i < e; ++i) {
                 c += tray[i] != 0;
                 ng |= tray[i] < 0;
+                n1 |= tray[i] == 1;
             }
             nocc += c;
             if (ng) neg = 1;
+            if (n1) one = 1;
         });
         if (neg) return fail(PSB_ERR_ARG, "tray holds negative values; item ids must be >= 0");
         occ = nocc;
@@ -1400,10 +1426,10 @@ struct psb_tray {
         } else {
             TRY(distance_on_device(d_tray, d_phi, nx, ny, nz, st));
         }
-        TRY(prefix_occ());
         TRY(prefix_phi(nullptr));
-        TRY(rebuild_occ());
-        TRY(rebuild_phi_spectrum());
+        phi_own = phi == nullptr;
+        has_source = one != 0;
+        occ_stale = phi_stale = bits_stale = geom_stale = true;
         CK(cudaStreamSynchronize(st));
         ready = true;
         return PSB_OK;
@@ -1429,12 +1455,10 @@ struct psb_tray {
             od->valid[a] = empty ? n[a] : std::max(0, n[a] - od->hi[a]);
         }
         od->sumI = info.sum;
-        od->base = (double)phi_mean * (double)info.sum;
+        // base, delta and exact depend on the distance statistics: k_prep
+        od->base = od->delta = 0.0;
+        od->exact = 0;
         const long long sabs = info.sabs;  // |D'| <= sum|I| * max|phi - m|
-        double maxD = (double)sabs * (double)phi_maxabs;
-        const double eps = 1.1920928955078125e-07;
-        od->delta = 2.0 * eps * std::sqrt(info.sumsq) * phi_norm + 0.5 * ulp32(maxD) + 1e-3;
-        od->exact = (od->delta >= 0.4 || maxD >= 8388608.0) ? 1 : 0;
         od->item = d_item;
         od->vox = d_vx;
         od->nvox = (int)info.nvox;
@@ -1576,6 +1600,125 @@ struct psb_tray {
         pending_apply = false;
         pdl(k_cand_apply, (n + 127) / 128, 128, 0, st)(d_odb, n, d_vcount, 1, apply_dmax, nullptr, 0LL, 0);
         CKL();
+        return PSB_OK;
+    }
+
+    // ---- search by score bounds (psb_bound.cuh) -------------------------
+    // Usable when the free bits cover the columns (nz <= 256) and there is a
+    // source: without one the distance field is constant, the score depends on
+    // z alone and every free cell of the lowest layer ties.
+    bool bound_usable() const {
+        return g_cand_filter && g_direct_max > 0 && nzw <= 8 && has_source && nx <= PSB_MAX_FFT && ny <= PSB_MAX_FFT;
+    }
+
+    // the search state as a search expects and leaves it (a call that failed
+    // half-way may have left another)
+    int bound_reset() {
+        if (!d_bstate) return PSB_OK;
+        memset(h_bstate, 0, sizeof(BoundState));
+        h_bstate->best = ~0ULL;
+        CK(cudaMemcpyAsync(d_bstate, h_bstate, sizeof(BoundState), cudaMemcpyHostToDevice, st));
+        return PSB_OK;
+    }
+
+    // buffers for `slots` orientations' tables, the sources' geometry and the
+    // free bits
+    int ensure_bound(size_t slots) {
+        if (!d_bstate) {
+            TRY(dalloc(&d_bgeom, 1, st));
+            TRY(dalloc(&d_blist, 2 * (size_t)PSB_BCAP, st));
+            if (!h_bstate) CK(cudaMallocHost(&h_bstate, sizeof(BoundState)));
+            TRY(dalloc(&d_bstate, 1, st));
+            TRY(bound_reset());
+        }
+        if (slots > bcap) {
+            dfree(d_btab, st);
+            dfree(d_bfs, st);
+            dfree(d_bfb, st);
+            bcap = 0;
+            TRY(dalloc(&d_btab, slots * (size_t)bound_tab_stride(nx, ny, nz), st));
+            TRY(dalloc(&d_bfs, slots * PSB_BSAMP, st));
+            TRY(dalloc(&d_bfb, slots * PSB_FBOUND, st));
+            bcap = slots;
+        }
+        TRY(ensure_bits());
+        if (geom_stale) {
+            PROF("k_bound_geom", st);
+            pdl(k_bound_geom_reset, 1, 32, 0, st)(d_bgeom);
+            pdl(k_bound_geom, std::min(grid1d(V), 148 * 4), 256, 0, st)(d_tray, nx, ny, nz, d_bgeom);
+            if (!phi_own) pdl(k_bound_over, std::min(grid1d(V), 148 * 4), 256, 0, st)(d_phi, nx, ny, nz, d_bgeom);
+            CKL();
+            geom_stale = false;
+        }
+        return PSB_OK;
+    }
+
+    // tables and samples of the orientations of `items` items (n each, in a
+    // row from d_odb on) into slots 0 .. items * n - 1
+    int bound_prep(const OrientDesc* d_odb, int n, int items, int mode) {
+        PROF("k_bound_prep", st);
+        auto k = tq == 1 ? k_bound_prep<4> : k_bound_prep<8>;
+        pdl(k, dim3(n, items), 256, 0, st)(d_odb, n, 0, d_bgeom, score_params(mode), d_btab,
+                                           bound_tab_stride(nx, ny, nz), d_bfs, d_bfb);
+        CKL();
+        return PSB_OK;
+    }
+
+    // Queue one item's search: its n orientations at d_odb, tables in the slots
+    // from slot0 on, outcome in *d_out and the loop state.  xmax: the largest
+    // number of x translations.
+    int bound_search(const OrientDesc* d_odb, int n, size_t slot0, int xmax, int mode, bool interlock, int item,
+                     DecisionDev* d_out) {
+        const ScoreParams sp = score_params(mode);
+        const long long ts = bound_tab_stride(nx, ny, nz);
+        const BoundArgs ba{d_bstate, d_bgeom, d_btab + slot0 * ts, ts, d_bfs + slot0 * PSB_BSAMP,
+                           d_bfb + slot0 * PSB_FBOUND, d_blist, d_blist + PSB_BCAP, d_pphi};
+        const int yb = (ny + 31) / 32;
+        auto grid = [&](int tasks) { return (unsigned)std::max(1, std::min(148 * 8, (tasks + 3) / 4)); };
+        const int seedx = (xmax + PSB_BSTEP - 1) / PSB_BSTEP, seedy = (ny + 32 * PSB_BSTEP - 1) / (32 * PSB_BSTEP);
+        {
+            PROF("k_bound_seed", st);
+            auto k = tq == 1 ? k_bound_find<1, BOUND_SEED> : k_bound_find<2, BOUND_SEED>;
+            pdl(k, grid(n * seedx * seedy), 128, 0, st)(d_odb, n, seedx, d_tbits, sp, ba);
+        }
+        CKL();
+        {
+            PROF("k_bound_find", st);
+            auto k = tq == 1 ? k_bound_find<1, BOUND_LIST> : k_bound_find<2, BOUND_LIST>;
+            pdl(k, grid(n * xmax * yb), 128, 0, st)(d_odb, n, xmax, d_tbits, sp, ba);
+        }
+        CKL();
+        {
+            PROF("k_bound_score", st);
+            pdl(k_bound_score<false>, 148 * 6, 256, 0, st)(d_odb, d_tbits, tq, sp, ba, item, interlock ? 1 : 0, d_ls,
+                                                           d_out);
+        }
+        CKL();
+        if (interlock) {
+            {
+                PROF("k_bound_ray", st);
+                pdl(k_bound_ray, 64, 256, 0, st)(d_odb, d_tbits, tq, sp, d_bstate, d_ls, d_out);
+            }
+            CKL();
+            // only for an item whose winner has no straight free run
+            PROF("k_bound_flood", st);
+            auto k = tq == 1 ? k_bound_find<1, BOUND_ALL> : k_bound_find<2, BOUND_ALL>;
+            pdl(k, grid(n * xmax * yb), 128, 0, st)(d_odb, n, xmax, d_tbits, sp, ba);
+            CKL();
+            pdl(k_bound_flood, 148, 256, bound_flood_smem(), st)(d_odb, d_tbits, tq, sp, ba, item);
+            CKL();
+            pdl(k_bound_score<true>, 148, 256, 0, st)(d_odb, d_tbits, tq, sp, ba, item, 1, d_ls, d_out);
+            CKL();
+        }
+        return PSB_OK;
+    }
+
+    // the placement decided by bound_search (or k_bound_first)
+    int bound_place(const OrientDesc* d_odb) {
+        PROF("k_bound_place", st);
+        pdl(k_bound_place, 64, 256, 0, st)(d_odb, d_ls, d_tray, (uint32_t*)d_tbits, 4 * tq, ny, nz);
+        CKL();
+        occ_stale = true;
         return PSB_OK;
     }
 
@@ -1933,11 +2076,13 @@ struct psb_tray {
     int search(const std::vector<OrientDesc>& ods, int mode, bool interlock, std::vector<ResultDev>* res,
                bool lazy = true) {
         const int n = (int)ods.size();
-        TRY(ensure_slots(std::max(n, 6)));
+        TRY(ensure_fft(n));
         std::vector<OrientDesc> od2(ods), bases;
         const bool share = make_bases(&od2, &bases);
         CK(cudaMemcpyAsync(d_od, od2.data(), sizeof(OrientDesc) * n, cudaMemcpyHostToDevice, st));
         if (share) CK(cudaMemcpyAsync(d_bases, bases.data(), sizeof(OrientDesc) * 6, cudaMemcpyHostToDevice, st));
+        pdl(k_prep, (n + 63) / 64, 64, 0, st)(d_od, n, d_ps);
+        CKL();
         const int sst = search_async(d_od, od2, mode, interlock, d_res, lazy, share ? d_bases : nullptr,
                                      share ? &bases : nullptr);
         late_active = false;
@@ -1975,12 +2120,12 @@ struct psb_tray {
         }
         pdl(k_place_write, blocks, 256, 0, st)(d_od, d_tray, nx, ny, nz, px, py, pz, id);
         CKL();
-        TRY(prefix_occ());
-        TRY(rebuild_occ());
+        occ_stale = bits_stale = true;
         if (id == 1 && od.nvox > 0) {  // only voxels equal to 1 are distance sources (fft3.cu:948)
             TRY(distance_on_device(d_tray, d_phi, nx, ny, nz, st));
             TRY(prefix_phi(nullptr));
-            TRY(rebuild_phi_spectrum());
+            phi_stale = geom_stale = true;
+            phi_own = has_source = true;
         }
         CK(cudaStreamSynchronize(st));
         return PSB_OK;
@@ -3014,9 +3159,6 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
         if (final_tray) TRY(psb_tray_get(t, final_tray, nullptr));
         return PSB_OK;
     }
-    // slots for the orientations and the item's 6 permutation bases; reserved
-    // here, before any slot pointer (d_res ...) is handed to a search
-    TRY(t->ensure_slots(std::max(n_orient, 6)));
     // every orientation of every item, described once (bounds, maps, sizes);
     // the error bounds are filled on the device by k_prep from the current
     // distance statistics.  Items [i0, i1) at a time: with a feed (psb_pack)
@@ -3210,7 +3352,8 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
     // queues the gated distance rebuild.  After that ids are >= 2, the
     // distance field is final and the rest of the run is queued without waits.
     bool first_pending = (id_offset == 0);
-    if (filt) TRY(t->tray_bits());
+    if (filt) TRY(t->ensure_bits());
+    TRY(t->bound_reset());
     // The filter rules translations out only where occupied cells block
     // them: while the tray's cells plus every item searched so far (placed
     // or not: an upper bound of the occupancy) fill less than a quarter of
@@ -3218,16 +3361,11 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
     // starts after that.  Its results are exact either way.
     size_t occ_est = t->occ;
     std::vector<OrientDesc> host_ods(n_orient);
-    for (int it = 0; it < n_items; ++it) {
-        if (opt.feed && it == opt.feed_at) {
-            // the rest of the items, staged by the caller while the first
-            // part was searched: uploaded on the copy stream, which the
-            // loop's stream then waits for
-            TRY(opt.feed());
-            TRY(describe_range(opt.feed_at, n_items, t->st_copy));
-            CK(cudaEventRecord(t->ev_copy, t->st_copy));
-            CK(cudaStreamWaitEvent(t->st, t->ev_copy, 0));
-        }
+    // One item through the transforms (and the flood fill), queued.
+    auto transform_item = [&](int it) -> int {
+        // slots for the orientations and the item's 6 permutation bases, before
+        // any slot pointer (d_res ...) is handed to a search
+        TRY(t->ensure_fft(n_orient));
         OrientDesc* d_odb = t->d_od_all + (size_t)it * n_orient;
         for (int o = 0; o < n_orient; ++o) host_ods[o] = all[(size_t)it * n_orient + o];
         // with the filter, k_cand_prep fills the error bounds (k_prep's work)
@@ -3275,7 +3413,6 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
             t->cur_ncol = nullptr;
             TRY(fst);
         }
-        occ_est += (size_t)t->staged[it].nvox;
         ShardRecord* rec = opt.world > 1 || opt.d_local ? (ShardRecord*)opt.d_local : nullptr;
         // the decision below may be fused into the search's last launch
         t->decide = DecideArgs{t->d_ls, t->d_dec + it, t->d_err, rec};
@@ -3331,7 +3468,91 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
             CK(cudaMemcpyAsync(&h, t->d_ls, sizeof(h), cudaMemcpyDeviceToHost, t->st));
             CK(cudaStreamSynchronize(t->st));
             if (h.placed > 0) first_pending = false;
+            if (h.need_phi) {
+                t->geom_stale = true;
+                t->phi_own = t->has_source = true;
+            }
         }
+        if (!filt) t->bits_stale = true;   // k_box_refresh kept no free bits
+        return PSB_OK;
+    };
+    // The plain loop decides items by score bounds (psb_bound.cuh) where it
+    // can: `chunk` items are queued at a time, and when one of them raises the
+    // halt flag the host runs it through the transforms and goes on after it.
+    // The chunk grows while that does not happen (a halt wastes the launches
+    // queued behind it, a chunk costs one wait).
+    const bool plain = filt && g_direct_max > 0 && !opt.prop && !d_hm && !d_per && opt.world == 1 && !opt.d_local &&
+                       (unsigned long long)n_orient * t->V < 0xffffffffULL;   // k_bound_flood's keys
+    const int kChunkMax = 32, kPrepMax = 128;
+    int chunk = 4, prep0 = 0, prep1 = 0;   // items whose bound tables are made: [prep0, prep1)
+    bool fed = !opt.feed;
+    for (int it = 0; it < n_items;) {
+        if (!fed && it >= opt.feed_at) {
+            // the rest of the items, staged by the caller while the first
+            // part was searched: uploaded on the copy stream, which the
+            // loop's stream then waits for
+            TRY(opt.feed());
+            TRY(describe_range(opt.feed_at, n_items, t->st_copy));
+            CK(cudaEventRecord(t->ev_copy, t->st_copy));
+            CK(cudaStreamWaitEvent(t->st, t->ev_copy, 0));
+            fed = true;
+        }
+        OrientDesc* d_odb = t->d_od_all + (size_t)it * n_orient;
+        if (plain && first_pending && t->occ == 0 && t->phi_own && it == 0 && t->staged[it].nvox > 0) {
+            // the first item of an empty tray (k_bound_first)
+            int o = 0;
+            while (o < n_orient && all[o].skip) ++o;
+            const double s = (double)t->staged[0].sum * (double)(t->nx + t->ny + t->nz + 10);
+            const bool found = o < n_orient && s < (mode == PSB_MODE_SCAN ? 1e9 : 1e29);
+            if (found) {
+                pdl(k_bound_first, 1, 1, 0, t->st)(o, s, t->score_params(mode), t->d_ls, t->d_dec);
+                CKL();
+                TRY(t->bound_place(d_odb));
+                TRY(distance_on_device(t->d_tray, t->d_phi, t->nx, t->ny, t->nz, t->st));
+                TRY(t->prefix_phi(nullptr));
+                t->phi_stale = t->geom_stale = true;
+                t->has_source = true;
+                first_pending = false;
+                occ_est += (size_t)t->staged[it].nvox;
+                ++it;
+                continue;
+            }
+        }
+        if (plain && !first_pending && t->bound_usable() && t->staged[it].nvox > 0) {
+            const int lim = fed ? n_items : opt.feed_at;
+            int m = 1;
+            while (m < chunk && it + m < lim && t->staged[it + m].nvox > 0) ++m;
+            TRY(t->ensure_bound((size_t)std::min(kPrepMax, n_items) * n_orient));
+            if (it >= prep1) {
+                prep0 = it;
+                prep1 = std::min(lim, it + kPrepMax);
+                TRY(t->bound_prep(d_odb, n_orient, prep1 - prep0, mode));
+            }
+            m = std::min(m, prep1 - it);
+            for (int k = 0; k < m; ++k) {
+                const OrientDesc* oh = &all[(size_t)(it + k) * n_orient];
+                int xmax = 0;
+                for (int o = 0; o < n_orient; ++o)
+                    if (!oh[o].skip) xmax = std::max(xmax, oh[o].valid[0]);
+                TRY(t->bound_search(d_odb + (size_t)k * n_orient, n_orient, (size_t)(it + k - prep0) * n_orient, xmax, mode,
+                                    interlock != 0, it + k, t->d_dec + it + k));
+                TRY(t->bound_place(d_odb + (size_t)k * n_orient));
+            }
+            CK(cudaMemcpyAsync(t->h_bstate, t->d_bstate, sizeof(BoundState), cudaMemcpyDeviceToHost, t->st));
+            CK(cudaStreamSynchronize(t->st));
+            const bool halted = t->h_bstate->halt != 0;
+            const int stop = halted ? t->h_bstate->halt_item : it + m;
+            for (; it < stop; ++it) occ_est += (size_t)t->staged[it].nvox;
+            if (!halted) {
+                chunk = std::min(2 * chunk, kChunkMax);
+                continue;
+            }
+            chunk = 1;
+            CK(cudaMemsetAsync((char*)t->d_bstate + offsetof(BoundState, halt), 0, sizeof(int), t->st));
+        }
+        TRY(transform_item(it));
+        occ_est += (size_t)t->staged[it].nvox;
+        ++it;
     }
     std::vector<DecisionDev> dec(n_items);
     LoopState h;
@@ -3370,12 +3591,6 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
     if (h.err & 2u) return fail(PSB_ERR_LIMIT, "tie-guard candidates exceeded the capacity %d", kCandCap);
     if (h.err & 4u)
         return fail(PSB_ERR_OVERLAP, "(place_in_tray): a searched position overlapped the tray on exact re-check");
-    // host copies of the distance statistics for later synchronous searches
-    PhiStats ps;
-    CK(cudaMemcpy(&ps, t->d_ps, sizeof(ps), cudaMemcpyDeviceToHost));
-    t->phi_mean = ps.mean;
-    t->phi_norm = ps.norm;
-    t->phi_maxabs = ps.maxabs;
     if (final_tray) TRY(psb_tray_get(t, final_tray, nullptr));
     return PSB_OK;
 }

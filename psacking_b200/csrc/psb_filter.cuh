@@ -46,27 +46,12 @@ __global__ void k_tray_bits(const int32_t* __restrict__ tray, int nx, int ny, in
     }
 }
 
-// The samples of each orientation, oriented and sorted by their word shift
-// s.z / 32 (bucket k holds fs[o][bound[o][k] .. bound[o][k+1])), once per
-// item, so the filter's CTAs only load them.  One warp per orientation.
-// grid: n, block 32
-// It also zeroes the orientation's filter counters (candidates, verified
-// cells, item columns: counts[o], counts[cap + o], counts[2 cap + o]) and,
-// when ps is given, fills its error bound (k_prep's work, one launch less).
-template <int NQ>
-__global__ void k_cand_prep(OrientDesc* __restrict__ orients, int4* __restrict__ fs, int* __restrict__ fbound,
-                            int* __restrict__ counts, int cap, const PhiStats* __restrict__ ps) {
-    pdl_enter();
-    constexpr int NW = 4 * NQ;
-    const int o = blockIdx.x, lane = threadIdx.x;
-    if (lane < 3) counts[(size_t)lane * cap + o] = 0;
-    if (ps && lane == 0) prep_orient(orients[o], ps);
-    __syncwarp();
-    const OrientDesc& od = orients[o];
-    if (od.skip || od.nsamp <= 0) return;
+// The samples of one orientation, oriented and sorted by their word shift
+// s.z / 32 (bucket k holds samples bound[k] .. bound[k+1]), so the filter's
+// warps only load them: store(i, x, y, z) keeps the i-th.  One warp.
+template <int NW, class ST>
+__device__ __forceinline__ void sort_samples(const OrientDesc& od, int* __restrict__ bound, int lane, ST store) {
     const int ns = min(od.nsamp, PSB_FSAMP);
-    int4* S = fs + (size_t)o * PSB_FSAMP;
-    int* bound = fbound + (size_t)o * (PSB_FBOUND);
     int base = 0;
     for (int k = 0; k < NW; ++k) {
         if (lane == 0) bound[k] = base;
@@ -79,11 +64,30 @@ __global__ void k_cand_prep(OrientDesc* __restrict__ orients, int4* __restrict__
             }
             const bool hit = s < ns && (c[2] >> 5) == k;
             const unsigned int b = __ballot_sync(0xffffffffu, hit);
-            if (hit) S[base + __popc(b & ((1u << lane) - 1u))] = make_int4(c[0], c[1], c[2], 0);
+            if (hit) store(base + __popc(b & ((1u << lane) - 1u)), c[0], c[1], c[2]);
             base += __popc(b);
         }
     }
     if (lane == 0) bound[NW] = base;
+}
+
+// sort_samples for every orientation of one item.  It also zeroes the
+// orientation's filter counters (candidates, verified cells, item columns:
+// counts[o], counts[cap + o], counts[2 cap + o]) and, when ps is given, fills
+// its error bound (k_prep's work, one launch less).  grid: n, block 32
+template <int NQ>
+__global__ void k_cand_prep(OrientDesc* __restrict__ orients, int4* __restrict__ fs, int* __restrict__ fbound,
+                            int* __restrict__ counts, int cap, const PhiStats* __restrict__ ps) {
+    pdl_enter();
+    const int o = blockIdx.x, lane = threadIdx.x;
+    if (lane < 3) counts[(size_t)lane * cap + o] = 0;
+    if (ps && lane == 0) prep_orient(orients[o], ps);
+    __syncwarp();
+    const OrientDesc& od = orients[o];
+    if (od.skip || od.nsamp <= 0) return;
+    int4* S = fs + (size_t)o * PSB_FSAMP;
+    sort_samples<4 * NQ>(od, fbound + (size_t)o * PSB_FBOUND, lane,
+                         [&](int i, int x, int y, int z) { S[i] = make_int4(x, y, z, 0); });
 }
 
 __device__ __forceinline__ uint32_t low_bits(int n) { return n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : (1u << n) - 1u); }
