@@ -1,0 +1,427 @@
+// psb_conv.cuh — the proposal network's layers as register-blocked FP32
+// kernels (psb_proposal.cuh holds the network, its inputs, loss and update).
+//
+// Convolutions: kernel 3, stride 2, padding 1, activations [S][C][D^3], BF16
+// weights widened to FP32, FP32 sums.  Written as one FMA chain per thread the
+// layers ran at 2-7 TFLOP/s: every FMA fetched its own input from L1, so they
+// were load-bound.  Here a CTA keeps its inputs and weights in shared memory
+// and a thread a block of results in registers, so that each shared load feeds
+// several FMAs: forward 8 positions x 8 channels (64 FMAs per 8 + 2 loads),
+// backward-data 2 cells x 8 parities x 4 channels (216 per 12 + 28), and
+// backward-weight 4 x 27 weights (108 per 18 + 1).  FP32 throughout: the tensor
+// cores would need the activations split into BF16 parts, and their
+// accumulation truncates.
+#pragma once
+#include <stdint.h>
+
+#include "psb_pdl.cuh"
+
+__device__ __forceinline__ float bf16_up(uint16_t h) { return __uint_as_float((uint32_t)h << 16); }
+
+// ---------------------------------------------------------------------------
+// forward with ReLU
+// ---------------------------------------------------------------------------
+// A CTA computes all CO channels of VPC consecutive output positions (of one
+// sample's SL output slabs, or of NS whole samples), CH input channels at a
+// time.  The staged input has a zero row at index 0 of each axis (the padding;
+// the far side needs none) and each row holds its odd entries behind its even
+// ones, so neighbouring output positions read neighbouring words.
+// Per result the sum runs over channels, then taps, from the bias on.
+template <int CI, int D, int CO, int TV, int CH>
+struct ConvFwd {
+    static constexpr int Do = D / 2, Do2 = Do * Do, Do3 = Do2 * Do;
+    static constexpr int NG = CO / 8, NV = 256 / NG, VPC = NV * TV;
+    static constexpr int SL = VPC < Do3 ? VPC / Do2 : Do;       // output slabs per sample part
+    static constexpr int NS = VPC < Do3 ? 1 : VPC / Do3;        // samples per CTA
+    static constexpr int IS = 2 * SL + 1, P = D + 1, HALF = (P + 1) / 2;   // staged slabs, row length
+    static constexpr int ROW = 2 * HALF, SLAB = P * ROW, CHAN = IS * SLAB;
+    static constexpr size_t smem = sizeof(float) * ((size_t)NS * CH * CHAN + (size_t)CH * 27 * CO);
+    static_assert(VPC % Do2 == 0 && (VPC < Do3 ? Do3 % VPC == 0 : VPC % Do3 == 0) && CI % CH == 0, "tile");
+};
+
+template <int CI, int D, int CO, int TV, int CH>
+__global__ void __launch_bounds__(256)
+k_conv3_fwd(const float* __restrict__ in, int S, const uint16_t* __restrict__ w, const float* __restrict__ bias,
+            float* __restrict__ out) {
+    pdl_enter();
+    using C = ConvFwd<CI, D, CO, TV, CH>;
+    extern __shared__ float4 csm4[];
+    float* ws = (float*)csm4;                    // [CH][27][CO]
+    float* xs = ws + CH * 27 * CO;               // [NS][CH][IS][P][ROW]
+    const int tid = threadIdx.x, vt = tid % C::NV, g = tid / C::NV;
+    const long long v0 = (long long)blockIdx.x * C::VPC;
+    const int s0 = (int)(v0 / C::Do3), od0 = (int)(v0 % C::Do3) / C::Do2;
+    const int ns = min(C::NS, S - s0);
+    float acc[TV][8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const float b = bias[8 * g + c];
+#pragma unroll
+        for (int i = 0; i < TV; ++i) acc[i][c] = b;
+    }
+    int at[TV];   // staged offset of each position's window
+#pragma unroll
+    for (int i = 0; i < TV; ++i) {
+        const int r = vt + i * C::NV, s = r / (C::SL * C::Do2), q = r % (C::SL * C::Do2);
+        at[i] = s * CH * C::CHAN + 2 * (q / C::Do2) * C::SLAB + 2 * (q / C::Do % C::Do) * C::ROW + q % C::Do;
+    }
+    for (int i = tid; i < C::NS * CH * C::CHAN; i += 256) xs[i] = 0.f;   // the padding stays zero
+    __syncthreads();
+    for (int c0 = 0; c0 < CI; c0 += CH) {
+        for (int i = tid; i < CH * 27 * CO; i += 256) {
+            const int co = i % CO, t = i / CO % 27, c = i / (27 * CO);
+            ws[i] = bf16_up(w[((size_t)co * CI + c0 + c) * 27 + t]);
+        }
+        // rows id = 2 od0 - 1 .. of each channel; staged index = id - (2 od0 - 1)
+        constexpr int ROWS = C::IS * D;
+        for (int i = tid; i < ns * CH * ROWS * (D / 4); i += 256) {
+            const int k4 = i % (D / 4), r = i / (D / 4) % ROWS, sc = i / (D / 4 * ROWS);
+            const int sl = r / D, ih = r % D, id = 2 * od0 - 1 + sl;
+            if (id < 0 || id >= D) continue;
+            const int s = sc / CH, c = sc % CH;
+            const float4 v = __ldg((const float4*)(in + (((size_t)(s0 + s) * CI + c0 + c) * D + id) * D * D +
+                                                   (size_t)ih * D) + k4);
+            float* x = xs + (s * CH + c) * C::CHAN + sl * C::SLAB + (ih + 1) * C::ROW;
+            // entry iw sits at padded index iw + 1: odd ones in the second half
+            x[C::HALF + 2 * k4] = v.x;
+            x[2 * k4 + 1] = v.y;
+            x[C::HALF + 2 * k4 + 1] = v.z;
+            x[2 * k4 + 2] = v.w;
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int c = 0; c < CH; ++c) {
+            const float* xc = xs + c * C::CHAN;
+            const float4* wc = (const float4*)(ws + c * 27 * CO + 8 * g);
+#pragma unroll
+            for (int t = 0; t < 27; ++t) {
+                const int kd = t / 9, kh = t / 3 % 3, kw = t % 3;
+                const int off = kd * C::SLAB + kh * C::ROW + (kw == 1 ? C::HALF : kw / 2);
+                const float4 wa = wc[t * (CO / 4)], wb = wc[t * (CO / 4) + 1];
+#pragma unroll
+                for (int i = 0; i < TV; ++i) {
+                    const float x = xc[at[i] + off];
+                    acc[i][0] = fmaf(x, wa.x, acc[i][0]);
+                    acc[i][1] = fmaf(x, wa.y, acc[i][1]);
+                    acc[i][2] = fmaf(x, wa.z, acc[i][2]);
+                    acc[i][3] = fmaf(x, wa.w, acc[i][3]);
+                    acc[i][4] = fmaf(x, wb.x, acc[i][4]);
+                    acc[i][5] = fmaf(x, wb.y, acc[i][5]);
+                    acc[i][6] = fmaf(x, wb.z, acc[i][6]);
+                    acc[i][7] = fmaf(x, wb.w, acc[i][7]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < TV; ++i) {
+        const int r = vt + i * C::NV, s = r / (C::SL * C::Do2), q = r % (C::SL * C::Do2) + od0 * C::Do2;
+        if (s >= ns) continue;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) out[((size_t)(s0 + s) * CO + 8 * g + c) * C::Do3 + q] = fmaxf(acc[i][c], 0.f);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// gradient w.r.t. the input, times the ReLU mask of that input
+// ---------------------------------------------------------------------------
+// Input position (2d + pd, ...) collects, per axis, tap 1 of output d when pd
+// is 0 and taps 2 of d and 0 of d + 1 when it is 1.  A thread owns two
+// neighbouring cells (d, h, w), (d, h, w + 1), all eight parities of each and
+// four input channels: 12 output gradients and 27 weights per output channel
+// feed 54 FMAs per input channel.
+template <int CI, int D, int CO, int CH>
+struct ConvBwd {
+    static constexpr int Do = D / 2, Do2 = Do * Do, Do3 = Do2 * Do;
+    static constexpr int NG = CI / 4, NP = 256 / NG, CELLS = 2 * NP;
+    static constexpr int SL = CELLS < Do3 ? CELLS / Do2 : Do;
+    static constexpr int NS = CELLS < Do3 ? 1 : CELLS / Do3;
+    static constexpr int P = Do + 1, SLAB = P * P, CHAN = (SL + 1) * SLAB;   // zero past the far side
+    static constexpr size_t smem = sizeof(float) * ((size_t)NS * CH * CHAN + (size_t)CH * CI * 28);
+    static_assert(CELLS % Do2 == 0 && (CELLS < Do3 ? Do3 % CELLS == 0 : CELLS % Do3 == 0) && CO % CH == 0, "tile");
+};
+
+template <int CI, int D, int CO, int CH>
+__global__ void __launch_bounds__(256)
+k_conv3_bwd_data(const float* __restrict__ dout, int S, const uint16_t* __restrict__ w, const float* __restrict__ in,
+                 float* __restrict__ din) {
+    pdl_enter();
+    using C = ConvBwd<CI, D, CO, CH>;
+    constexpr int Do = C::Do;
+    extern __shared__ float4 csm4[];
+    float* ws = (float*)csm4;                    // [CH][CI][28]
+    float* gs = ws + CH * CI * 28;               // [NS][CH][SL + 1][P][P]
+    const int tid = threadIdx.x, pt = tid % C::NP, g = tid / C::NP;
+    const long long v0 = (long long)blockIdx.x * C::CELLS;
+    const int s0 = (int)(v0 / C::Do3), d0 = (int)(v0 % C::Do3) / C::Do2;
+    const int ns = min(C::NS, S - s0);
+    // this thread's cell pair
+    const int cell = 2 * pt, cs = cell / (C::SL * C::Do2), q = cell % (C::SL * C::Do2);
+    const int d = q / C::Do2, h = q / Do % Do, cw = q % Do;
+    float acc[4][2][8];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int p = 0; p < 8; ++p) acc[c][e][p] = 0.f;
+    for (int i = tid; i < C::NS * CH * C::CHAN; i += 256) gs[i] = 0.f;
+    __syncthreads();
+    for (int c0 = 0; c0 < CO; c0 += CH) {
+        for (int i = tid; i < CH * CI * 27; i += 256) {
+            const int t = i % 27, ci = i / 27 % CI, c = i / (27 * CI);
+            ws[(c * CI + ci) * 28 + t] = bf16_up(w[((size_t)(c0 + c) * CI + ci) * 27 + t]);
+        }
+        constexpr int NVOX = (C::SL + 1) * C::Do2;
+        for (int i = tid; i < ns * CH * NVOX; i += 256) {
+            const int r = i % NVOX, sc = i / NVOX, s = sc / CH, c = sc % CH;
+            const int od = d0 + r / C::Do2;
+            if (od >= Do) continue;
+            gs[(s * CH + c) * C::CHAN + r / C::Do2 * C::SLAB + r / Do % Do * C::P + r % Do] =
+                __ldg(&dout[((size_t)(s0 + s) * CO + c0 + c) * C::Do3 + (size_t)od * C::Do2 + r % C::Do2]);
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int c = 0; c < CH; ++c) {
+            const float* gc = gs + (cs * CH + c) * C::CHAN + d * C::SLAB + h * C::P + cw;
+            float x[2][2][3];
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int b = 0; b < 2; ++b)
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) x[a][b][e] = gc[a * C::SLAB + b * C::P + e];
+#pragma unroll
+            for (int ci = 0; ci < 4; ++ci) {
+                const float4* w4 = (const float4*)(ws + (c * CI + 4 * g + ci) * 28);
+                float wt[28];
+#pragma unroll
+                for (int k = 0; k < 7; ++k) {
+                    const float4 v = w4[k];
+                    wt[4 * k] = v.x;
+                    wt[4 * k + 1] = v.y;
+                    wt[4 * k + 2] = v.z;
+                    wt[4 * k + 3] = v.w;
+                }
+#pragma unroll
+                for (int t = 0; t < 27; ++t) {
+                    // tap 1: parity 0, output d; tap 2: parity 1, d; tap 0: parity 1, d + 1
+                    const int kd = t / 9, kh = t / 3 % 3, kw = t % 3;
+                    const int p = (kd != 1) * 4 + (kh != 1) * 2 + (kw != 1);
+                    acc[ci][0][p] = fmaf(x[kd == 0][kh == 0][kw == 0], wt[t], acc[ci][0][p]);
+                    acc[ci][1][p] = fmaf(x[kd == 0][kh == 0][1 + (kw == 0)], wt[t], acc[ci][1][p]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (cs >= ns) return;
+#pragma unroll
+    for (int ci = 0; ci < 4; ++ci) {
+        const size_t base = ((size_t)(s0 + cs) * CI + 4 * g + ci) * D * D * D;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const size_t at = base + ((size_t)(2 * (d0 + d) + (r >> 1)) * D + 2 * h + (r & 1)) * D + 2 * cw;
+            const float4 m = __ldg((const float4*)(in + at));
+            float4 v;
+            v.x = !(m.x <= 0.f) ? acc[ci][0][2 * r] : 0.f;
+            v.y = !(m.y <= 0.f) ? acc[ci][0][2 * r + 1] : 0.f;
+            v.z = !(m.z <= 0.f) ? acc[ci][1][2 * r] : 0.f;
+            v.w = !(m.w <= 0.f) ? acc[ci][1][2 * r + 1] : 0.f;
+            *(float4*)(din + at) = v;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// gradient w.r.t. the weights and the bias
+// ---------------------------------------------------------------------------
+// A thread owns four output channels and all 27 taps of one input channel; the
+// CTA's threads cover CG input channels x all CO output channels, NSUB times
+// over, each copy taking its share of the staged rows of output positions.
+// Along a row the window slides by two inputs, so 18 of its 27 values are new
+// per position.  grid.x: input channel groups, grid.y: shares of the samples;
+// the copies meet in shared memory and each CTA adds its sums with one atomic
+// per weight (dw, db zeroed first).
+template <int CI, int D, int CO, int CG, int SL, int NS, int SEG>
+struct ConvBwdW {
+    static constexpr int Do = D / 2, Do2 = Do * Do, Do3 = Do2 * Do;
+    static constexpr int NQ = CO / 4, NSUB = 256 / (CG * NQ);
+    static constexpr int IS = 2 * SL + 1, P = D + 1, SLAB = P * P, CHAN = IS * SLAB;
+    static constexpr int NVOX = SL * Do2, SEGS = NS * NVOX / SEG;
+    static constexpr size_t stage = (size_t)NS * NVOX * CO + (size_t)NS * CG * CHAN;
+    static constexpr size_t red = (size_t)CG * NQ * 108 + CO;
+    static constexpr size_t smem = sizeof(float) * (stage > red ? stage : red);
+    static_assert(256 % (CG * NQ) == 0 && Do % SEG == 0 && Do % SL == 0 && CI % CG == 0, "tile");
+};
+
+template <int CI, int D, int CO, int CG, int SL, int NS, int SEG>
+__global__ void __launch_bounds__(256)
+k_conv3_bwd_weight(const float* __restrict__ dout, const float* __restrict__ in, int S, int chunk,
+                   float* __restrict__ dw, float* __restrict__ db) {
+    pdl_enter();
+    using C = ConvBwdW<CI, D, CO, CG, SL, NS, SEG>;
+    constexpr int Do = C::Do;
+    extern __shared__ float4 csm4[];
+    float* gs = (float*)csm4;                    // [NS][NVOX][CO]
+    float* xs = gs + NS * C::NVOX * CO;          // [NS][CG][IS][P][P]
+    const int tid = threadIdx.x, q = tid % C::NQ, cg = tid / C::NQ % CG, sub = tid / (C::NQ * CG);
+    const int c0 = blockIdx.x * CG, sa = blockIdx.y * chunk, sb = min(S, sa + chunk);
+    const bool bias = blockIdx.x == 0 && cg == 0;
+    float acc[4][27], bacc[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        bacc[k] = 0.f;
+#pragma unroll
+        for (int t = 0; t < 27; ++t) acc[k][t] = 0.f;
+    }
+    for (int i = tid; i < NS * CG * C::CHAN; i += 256) xs[i] = 0.f;
+    __syncthreads();
+    for (int s0 = sa; s0 < sb; s0 += NS) {
+        const int ns = min(NS, sb - s0);
+        for (int od0 = 0; od0 < Do; od0 += SL) {
+            // four positions per load, channels across the lanes: the stores
+            // fall on distinct banks
+            for (int i = tid; i < ns * CO * (C::NVOX / 4); i += 256) {
+                const int c = i % CO, sv = i / CO, s = sv / (C::NVOX / 4), v = sv % (C::NVOX / 4) * 4;
+                const float4 g = __ldg(
+                    (const float4*)(dout + ((size_t)(s0 + s) * CO + c) * C::Do3 + (size_t)od0 * C::Do2 + v));
+                float* d = gs + (s * C::NVOX + v) * CO + c;
+                d[0] = g.x;
+                d[CO] = g.y;
+                d[2 * CO] = g.z;
+                d[3 * CO] = g.w;
+            }
+            constexpr int VIN = C::IS * D * D;
+            for (int i = tid; i < ns * CG * VIN; i += 256) {
+                const int v = i % VIN, sc = i / VIN, s = sc / CG, c = sc % CG;
+                const int sl = v / (D * D), id = 2 * od0 - 1 + sl;
+                float x = 0.f;
+                if (id >= 0) x = __ldg(&in[(((size_t)(s0 + s) * CI + c0 + c) * D + id) * D * D + v % (D * D)]);
+                xs[(s * CG + c) * C::CHAN + sl * C::SLAB + (v / D % D + 1) * C::P + v % D + 1] = x;
+            }
+            __syncthreads();
+            for (int e = sub; e < ns * (C::NVOX / SEG); e += C::NSUB) {
+                const int s = e / (C::NVOX / SEG), v = e % (C::NVOX / SEG) * SEG;
+                const int sl = v / C::Do2, oh = v / Do % Do, ow = v % Do;
+                const float4* gr = (const float4*)(gs + (s * C::NVOX + v) * CO) + q;
+                const float* x = xs + (s * CG + cg) * C::CHAN + 2 * sl * C::SLAB + 2 * oh * C::P + 2 * ow;
+                float win[9][3];
+#pragma unroll
+                for (int r = 0; r < 9; ++r) win[r][2] = x[r / 3 * C::SLAB + r % 3 * C::P];
+#pragma unroll 2
+                for (int i = 0; i < SEG; ++i) {
+#pragma unroll
+                    for (int r = 0; r < 9; ++r) {
+                        win[r][0] = win[r][2];
+                        win[r][1] = x[r / 3 * C::SLAB + r % 3 * C::P + 2 * i + 1];
+                        win[r][2] = x[r / 3 * C::SLAB + r % 3 * C::P + 2 * i + 2];
+                    }
+                    const float4 g = gr[i * (CO / 4)];
+                    const float gv[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+#pragma unroll
+                        for (int t = 0; t < 27; ++t) acc[k][t] = fmaf(gv[k], win[t / 3][t % 3], acc[k][t]);
+                        if (bias) bacc[k] += gv[k];
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    }
+    // the copies' sums, one copy after another
+    float* red = gs;                             // [CG * NQ][108], then [CO]
+    float* rb = red + CG * C::NQ * 108;
+    const int slot = cg * C::NQ + q;
+    for (int k = 0; k < C::NSUB; ++k) {
+        if (sub == k) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                for (int t = 0; t < 27; ++t) {
+                    float* r = red + slot * 108 + j * 27 + t;
+                    *r = k == 0 ? acc[j][t] : *r + acc[j][t];
+                }
+                if (bias) rb[4 * q + j] = k == 0 ? bacc[j] : rb[4 * q + j] + bacc[j];
+            }
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < CG * C::NQ * 108; i += 256) {
+        const int t = i % 27, j = i / 27 % 4, sq = i / 108, co = 4 * (sq % C::NQ) + j, ci = c0 + sq / C::NQ;
+        atomicAdd(&dw[((size_t)co * CI + ci) * 27 + t], red[i]);
+    }
+    if (blockIdx.x == 0)
+        for (int i = tid; i < CO; i += 256) atomicAdd(&db[i], rb[i]);
+}
+
+// ---------------------------------------------------------------------------
+// linear layers: C[M][N] = sum over k of A(m, k) B(k, n)
+// ---------------------------------------------------------------------------
+// 64 x 64 tile per CTA, 4 x 4 results per thread, 16 k at a time in shared
+// memory.  OP 0: y = x W^T + b (A = x [M][K], B = BF16 W [N][K]); OP 1: dx = dy W
+// (A = dy [M][K], B = BF16 W [K][N]), times the ReLU mask of x when xmask is
+// given; OP 2: dW = dy^T x (A = dy [K][M], B = x [K][N]), grid.z shares of k
+// added with atomics (dW zeroed first), with db[m] = sum over k of dy[k][m].
+template <int OP>
+__global__ void __launch_bounds__(256)
+k_linear(const float* __restrict__ a, const void* __restrict__ b, int M, int N, int K, const float* __restrict__ bias,
+         int relu, const float* __restrict__ xmask, float* __restrict__ c, float* __restrict__ db, int kchunk) {
+    pdl_enter();
+    __shared__ float As[16][68], Bs[16][68];
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
+    const int ka = OP == 2 ? blockIdx.z * kchunk : 0, kb = OP == 2 ? min(K, ka + kchunk) : K;
+    float acc[4][4], bsum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = OP == 0 && n0 + 4 * tx + j < N ? bias[n0 + 4 * tx + j] : 0.f;
+    for (int k0 = ka; k0 < kb; k0 += 16) {
+        for (int i = tid; i < 16 * 64; i += 256) {
+            // along the operand's contiguous index
+            const int ak = OP == 2 ? i / 64 : i % 16, am = OP == 2 ? i % 64 : i / 16;
+            float v = 0.f;
+            if (k0 + ak < kb && m0 + am < M)
+                v = OP == 2 ? a[(size_t)(k0 + ak) * M + m0 + am] : a[(size_t)(m0 + am) * K + k0 + ak];
+            As[ak][am] = v;
+            const int bk = OP == 0 ? i % 16 : i / 64, bn = OP == 0 ? i / 16 : i % 64;
+            float u = 0.f;
+            if (k0 + bk < kb && n0 + bn < N)
+                u = OP == 0 ? bf16_up(((const uint16_t*)b)[(size_t)(n0 + bn) * K + k0 + bk])
+                  : OP == 1 ? bf16_up(((const uint16_t*)b)[(size_t)(k0 + bk) * N + n0 + bn])
+                            : ((const float*)b)[(size_t)(k0 + bk) * N + n0 + bn];
+            Bs[bk][bn] = u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const float4 av = *(const float4*)&As[k][4 * ty], bv = *(const float4*)&Bs[k][4 * tx];
+            const float x[4] = {av.x, av.y, av.z, av.w}, y[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+        }
+        if (OP == 2 && blockIdx.x == 0 && tid < 64)
+            for (int k = 0; k < 16; ++k) bsum += As[k][tid];
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int m = m0 + 4 * ty + i;
+        if (m >= M) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int n = n0 + 4 * tx + j;
+            if (n >= N) continue;
+            const size_t at = (size_t)m * N + n;
+            if (OP == 2) atomicAdd(&c[at], acc[i][j]);
+            else if (OP == 1) c[at] = xmask && xmask[at] <= 0.f ? 0.f : acc[i][j];
+            else c[at] = relu ? fmaxf(acc[i][j], 0.f) : acc[i][j];
+        }
+    }
+    if (OP == 2 && blockIdx.x == 0 && tid < 64 && m0 + tid < M) atomicAdd(&db[m0 + tid], bsum);
+}

@@ -2218,21 +2218,35 @@ struct Arena {
     size_t n = 0;
     int dev = -1;
 };
-thread_local Arena g_arena;
+thread_local Arena g_arena, g_arena2;   // the second: sizes known only once the first is in use
 
-int arena(size_t bytes, void** out) {
+int arena(size_t bytes, void** out, Arena* a = nullptr) {
+    if (!a) a = &g_arena;
     int dev = 0;
     CK(cudaGetDevice(&dev));
-    if (g_arena.n < bytes || g_arena.dev != dev) {
-        if (g_arena.p && g_arena.dev == dev) cudaFree(g_arena.p);
-        g_arena.p = nullptr;
-        CK(cudaMalloc(&g_arena.p, bytes));
-        g_arena.n = bytes;
-        g_arena.dev = dev;
+    if (a->n < bytes || a->dev != dev) {
+        if (a->p && a->dev == dev) cudaFree(a->p);
+        a->p = nullptr;
+        a->n = 0;
+        CK(cudaMalloc(&a->p, bytes));
+        a->n = bytes;
+        a->dev = dev;
     }
-    *out = g_arena.p;
+    *out = a->p;
     return PSB_OK;
 }
+
+// Gives an arena above `keep` bytes back when a call ends.
+struct ArenaTrim {
+    Arena* a;
+    size_t keep;
+    ~ArenaTrim() {
+        if (a->n <= keep) return;
+        cudaFree(a->p);
+        a->p = nullptr;
+        a->n = 0;
+    }
+};
 
 // corr (conj_b=1): out[t] = sum_x b[x] a[t+x] ; conv (conj_b=0): linear conv
 int linear_transform_product(const int32_t* a, const int32_t* b, int nx, int ny, int nz, int conj_b, int32_t* out) {
@@ -3839,24 +3853,41 @@ int psb_voxelize_mesh(const float* tris, int ntri, int resolution, int32_t* out,
     if (!tris || !out || !dims_out || ntri <= 0 || resolution <= 0)
         return fail(PSB_ERR_ARG, "voxelize: null pointer, no triangles or bad resolution");
     TRY(ensure_device());
-    // mergeVerticesExact (LibSL Mesh.cpp:350-392): the new index of a vertex
-    // is the rank of its position in lexicographic order
-    const int nv = 3 * ntri;
-    std::vector<std::pair<std::array<float, 3>, int>> all(nv);
-    for (int v = 0; v < nv; ++v) all[v] = {{tris[3 * v], tris[3 * v + 1], tris[3 * v + 2]}, v};
-    std::sort(all.begin(), all.end());
-    std::vector<int> newidx(nv);
-    std::vector<std::array<float, 3>> pos;
-    for (int v = 0; v < nv; ++v) {
-        if (pos.empty() || all[v].first != pos.back()) pos.push_back(all[v].first);
-        newidx[all[v].second] = (int)pos.size() - 1;
+    // the mesh and its bounding box on the device
+    const long long nv = 3LL * ntri;
+    const size_t btris = (sizeof(float) * 3 * nv + 255) / 256 * 256, bchunk = sizeof(int2) * PSB_VCHUNKS;
+    void* base = nullptr;
+    TRY(arena(btris + bchunk + 256, &base));
+    float* d_tris = (float*)base;
+    int2* d_chunks = (int2*)((char*)base + btris);
+    struct Mesh {
+        unsigned long long nchunks;
+        unsigned int key[6];
+        int box[6];
+    } h = {0ULL, {~0u, ~0u, ~0u, 0u, 0u, 0u}, {INT_MAX, INT_MAX, INT_MAX, -1, -1, -1}};
+    Mesh* d_mesh = (Mesh*)((char*)base + btris + bchunk);
+    unsigned int* d_key = (unsigned int*)((char*)d_mesh + offsetof(Mesh, key));
+    int* d_box = (int*)((char*)d_mesh + offsetof(Mesh, box));
+    unsigned long long* d_nchunks = (unsigned long long*)d_mesh;
+    cudaStream_t st = 0;
+    CK(cudaMemcpyAsync(d_tris, tris, sizeof(float) * 3 * nv, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(d_mesh, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+    {
+        PROF("k_voxel_bounds", st);
+        pdl(k_voxel_bounds, std::min(grid1d((size_t)nv), 148 * 2), 256, 0, st)(d_tris, nv, d_key);
     }
+    CKL();
+    CK(cudaMemcpyAsync(&h, d_mesh, sizeof(h), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
     // box transform in float, composed and applied as LibSL's Matrix4x4 does
     // (products accumulated from zero in index order; no fused multiply-add)
     float lo[3], hi[3], ext[3];
     for (int a = 0; a < 3; ++a) {
-        lo[a] = hi[a] = pos[0][a];
-        for (auto& p : pos) { lo[a] = std::min(lo[a], p[a]); hi[a] = std::max(hi[a], p[a]); }
+        for (int e = 0; e < 2; ++e) {
+            const unsigned int k = h.key[3 * e + a];
+            const unsigned int bits = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
+            memcpy(e ? &hi[a] : &lo[a], &bits, sizeof(float));
+        }
         ext[a] = hi[a] - lo[a];
     }
     const float emax = std::max(ext[0], std::max(ext[1], ext[2]));
@@ -3889,20 +3920,10 @@ int psb_voxelize_mesh(const float* tris, int ntri, int resolution, int32_t* out,
     const M4 box = mul(mul(mul(mul(scale((float)resolution * (float)PSB_FP_SCALE), scale(inv)), trans(t1)),
                            scale(factor)),
                        trans(t2));
-    const float top = (float)resolution * (float)PSB_FP_SCALE - 1.f;
-    std::vector<int> pts(3 * pos.size());
-    for (size_t p = 0; p < pos.size(); ++p)
-        for (int i = 0; i < 3; ++i) {
-            volatile float acc = 0.f;
-            for (int k = 0; k < 3; ++k) {
-                volatile float prod = box[i][k] * pos[p][k];
-                acc = acc + prod;
-            }
-            acc = acc + box[i][3];
-            float r = ::roundf(acc);
-            r = std::min(std::max(r, 0.f), top);
-            pts[3 * p + i] = (int)r;
-        }
+    VoxBox vb;
+    for (int i = 0; i < 3; ++i)
+        for (int k = 0; k < 4; ++k) vb.m[i][k] = box[i][k];
+    vb.top = (float)resolution * (float)PSB_FP_SCALE - 1.f;
     int dims[3];
     for (int a = 0; a < 3; ++a) {
         volatile float q = ext[a] / emax;
@@ -3910,50 +3931,45 @@ int psb_voxelize_mesh(const float* tris, int ntri, int resolution, int32_t* out,
         dims[a] = (int)(unsigned int)d;
     }
     const size_t V = (size_t)dims[0] * dims[1] * dims[2];
-    std::vector<int> tri(3 * (size_t)ntri);
-    for (int v = 0; v < nv; ++v) tri[v] = newidx[v];
-    std::vector<unsigned int> hv(V, 0u);
-    if (V > 0) {
-        int *dp = nullptr, *dt = nullptr;
-        unsigned int* dv = nullptr;
-        TRY(dalloc(&dp, pts.size()));
-        TRY(dalloc(&dt, tri.size()));
-        TRY(dalloc(&dv, V));
-        int rc = PSB_OK;
-        if (cudaMemcpy(dp, pts.data(), sizeof(int) * pts.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(dt, tri.data(), sizeof(int) * tri.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemset(dv, 0, sizeof(unsigned int) * V) != cudaSuccess) {
-            rc = fail(PSB_ERR_CUDA, "voxelize: upload failed");
-        } else {
-            const long long warps = 3LL * ntri;
-            PROF("k_voxel_raster", nullptr);
-            k_voxel_raster<<<(unsigned)((warps + 7) / 8), 256>>>(dp, dt, ntri, dims[0], dims[1], dims[2], dv);
-            cudaError_t e = cudaGetLastError();
-            if (e == cudaSuccess) e = cudaMemcpy(hv.data(), dv, sizeof(unsigned int) * V, cudaMemcpyDeviceToHost);
-            if (e != cudaSuccess) rc = fail(PSB_ERR_CUDA, "voxelize: %s", cudaGetErrorString(e));
-        }
-        dfree(dp); dfree(dt); dfree(dv);
-        TRY(rc);
+    dims_out[0] = dims_out[1] = dims_out[2] = 0;
+    if (V == 0) return PSB_OK;
+    // axis bits, then the tight grid
+    const size_t bvox = (sizeof(unsigned int) * V + 255) / 256 * 256;
+    ArenaTrim trim{&g_arena2, (size_t)256 << 20};
+    TRY(arena(2 * bvox, &base, &g_arena2));
+    unsigned int* d_vox = (unsigned int*)base;
+    int32_t* d_out = (int32_t*)((char*)base + bvox);
+    CK(cudaMemsetAsync(d_vox, 0, sizeof(unsigned int) * V, st));
+    {
+        PROF("k_voxel_raster", st);
+        pdl(k_voxel_raster, (unsigned)((24LL * ntri + 255) / 256), 256, 0, st)(d_tris, ntri, vb, dims[0], dims[1],
+                                                                              dims[2], d_vox, d_chunks, d_nchunks);
     }
-    // occupied = any axis bit; then the tight bounding box (make_voxel_grid_tight)
-    int lo3[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, hi3[3] = {-1, -1, -1};
-    for (int i = 0; i < dims[0]; ++i)
-        for (int j = 0; j < dims[1]; ++j)
-            for (int k = 0; k < dims[2]; ++k)
-                if (hv[((size_t)i * dims[1] + j) * dims[2] + k]) {
-                    const int c[3] = {i, j, k};
-                    for (int a = 0; a < 3; ++a) { lo3[a] = std::min(lo3[a], c[a]); hi3[a] = std::max(hi3[a], c[a]); }
-                }
-    if (hi3[0] < 0) {
-        dims_out[0] = dims_out[1] = dims_out[2] = 0;
-        return PSB_OK;
+    CKL();
+    {
+        PROF("k_voxel_chunks", st);
+        pdl(k_voxel_chunks, 148 * 8, 256, 0, st)(d_tris, vb, dims[0], dims[1], dims[2], d_vox, d_chunks, d_nchunks);
     }
-    const int td[3] = {hi3[0] - lo3[0] + 1, hi3[1] - lo3[1] + 1, hi3[2] - lo3[2] + 1};
-    for (int i = 0; i < td[0]; ++i)
-        for (int j = 0; j < td[1]; ++j)
-            for (int k = 0; k < td[2]; ++k)
-                out[((size_t)i * td[1] + j) * td[2] + k] =
-                    hv[((size_t)(i + lo3[0]) * dims[1] + (j + lo3[1])) * dims[2] + (k + lo3[2])] ? 1 : 0;
+    CKL();
+    {
+        PROF("k_voxel_box", st);
+        pdl(k_voxel_box, std::min(grid1d(V, 2048), 148 * 8), 256, 0, st)(d_vox, dims[0], dims[1], dims[2], d_box);
+    }
+    CKL();
+    CK(cudaMemcpyAsync(h.box, d_box, sizeof(h.box), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (h.box[3] < 0) return PSB_OK;   // no occupied voxel
+    int td[3];
+    for (int a = 0; a < 3; ++a) td[a] = h.box[3 + a] - h.box[a] + 1;
+    const size_t T = (size_t)td[0] * td[1] * td[2];
+    {
+        PROF("k_voxel_tight", st);
+        pdl(k_voxel_tight, std::min(grid1d(T, 2048), 148 * 8), 256, 0, st)(d_vox, dims[1], dims[2], h.box[0], h.box[1],
+                                                                          h.box[2], td[0], td[1], td[2], d_out);
+    }
+    CKL();
+    CK(cudaMemcpyAsync(out, d_out, sizeof(int32_t) * T, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
     for (int a = 0; a < 3; ++a) dims_out[a] = td[a];
     return PSB_OK;
 }
