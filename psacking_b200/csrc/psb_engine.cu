@@ -453,6 +453,19 @@ int set_smem_attrs() {
         }
     for (int n : {64, 100, 128, 240}) TRY(set_max_dyn_smem(xfwd_for(n)));
     TRY(set_max_dyn_smem(k_bound_flood));
+    TRY(set_max_dyn_smem(k_conv3_fwd<1, 32, 16, 8, 1>));
+    TRY(set_max_dyn_smem(k_conv3_fwd<16, 16, 32, 8, 4>));
+    TRY(set_max_dyn_smem(k_conv3_fwd<32, 8, 64, 8, 4>));
+    TRY(set_max_dyn_smem(k_conv3_fwd<32, 8, 64, 2, 8>));
+    TRY(set_max_dyn_smem(k_conv3_fwd<64, 4, 64, 2, 8>));
+    TRY(set_max_dyn_smem(k_conv3_fwd<64, 4, 64, 1, 8>));
+    TRY(set_max_dyn_smem(k_conv3_bwd_data<64, 4, 64, 8>));
+    TRY(set_max_dyn_smem(k_conv3_bwd_data<32, 8, 64, 8>));
+    TRY(set_max_dyn_smem(k_conv3_bwd_data<16, 16, 32, 8>));
+    TRY(set_max_dyn_smem(k_conv3_bwd_weight<64, 4, 64, 16, 2, 8, 2>));
+    TRY(set_max_dyn_smem(k_conv3_bwd_weight<32, 8, 64, 8, 4, 2, 4>));
+    TRY(set_max_dyn_smem(k_conv3_bwd_weight<16, 16, 32, 4, 8, 1, 8>));
+    TRY(set_max_dyn_smem(k_conv3_bwd_weight<1, 32, 16, 1, 2, 1, 8>));
     TRY(set_max_dyn_smem(k_cand_filter_plane<1>));
     TRY(set_max_dyn_smem(k_cand_filter_plane<2>));
     TRY(init_register_twiddles());
@@ -2236,6 +2249,28 @@ int arena(size_t bytes, void** out, Arena* a = nullptr) {
     return PSB_OK;
 }
 
+// pinned staging of the calling thread (uploads queued from it end before the
+// call that uses it returns), at most 64 MiB kept; given back with the thread
+struct PinnedBlock {
+    char* p = nullptr;
+    size_t n = 0;
+    ~PinnedBlock() { if (p) cudaFreeHost(p); }
+};
+thread_local PinnedBlock g_pinned;
+
+int pinned(size_t bytes, char** out) {
+    PinnedBlock& b = g_pinned;
+    if (b.n < bytes || b.n > std::max(bytes, (size_t)64 << 20)) {
+        if (b.p) cudaFreeHost(b.p);
+        b.p = nullptr;
+        b.n = 0;
+        CK(cudaMallocHost((void**)&b.p, bytes));
+        b.n = bytes;
+    }
+    *out = b.p;
+    return PSB_OK;
+}
+
 // Gives an arena above `keep` bytes back when a call ends.
 struct ArenaTrim {
     Arena* a;
@@ -2352,6 +2387,7 @@ struct psb_proposal {
         TRY(ensure_device());
         CK(cudaGetDevice(&dev));
         CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        TRY(set_smem_attrs());
         const size_t n = kProp.n;
         TRY(dalloc(&P, n)); TRY(dalloc(&G, n)); TRY(dalloc(&M, n)); TRY(dalloc(&V, n));
         TRY(dalloc(&P16, n)); TRY(dalloc(&isw, n)); TRY(dalloc(&loss, 1)); TRY(dalloc(&stats, 2));
@@ -2385,52 +2421,88 @@ struct psb_proposal {
         return PSB_OK;
     }
 
+    // one convolution layer; the tile that leaves no more than half the chip
+    // idle: 8 positions per thread, fewer where S is small (a batch of 8 items,
+    // S = 192, would be 48 and 24 CTAs in the last two layers)
+    template <int CI, int D, int CO, int TV, int CH>
+    int conv_fwd_tile(const float* in, int S, const PropLayer& L, float* out, cudaStream_t s) {
+        using C = ConvFwd<CI, D, CO, TV, CH>;
+        const long long n = (long long)S * C::Do3;
+        pdl(k_conv3_fwd<CI, D, CO, TV, CH>, (unsigned)((n + C::VPC - 1) / C::VPC), 256, C::smem, s)(
+            in, S, P16 + L.w, P + L.b, out);
+        CKL();
+        return PSB_OK;
+    }
+    // conv stack + f1 (the item branch) over S oriented grids
+    int item_branch(const float* grids, int S, cudaStream_t s) {
+        PROF("k_prop_conv", s);
+        TRY((conv_fwd_tile<1, 32, 16, 8, 1>(grids, S, kProp.c[0], a1, s)));
+        TRY((conv_fwd_tile<16, 16, 32, 8, 4>(a1, S, kProp.c[1], a2, s)));
+        if (S >= 4 * 148) TRY((conv_fwd_tile<32, 8, 64, 8, 4>(a2, S, kProp.c[2], a3, s)));
+        else TRY((conv_fwd_tile<32, 8, 64, 2, 8>(a2, S, kProp.c[2], a3, s)));
+        if (S >= 8 * 148) TRY((conv_fwd_tile<64, 4, 64, 2, 8>(a3, S, kProp.c[3], a4, s)));
+        else TRY((conv_fwd_tile<64, 4, 64, 1, 8>(a3, S, kProp.c[3], a4, s)));
+        return lin_fwd(a4, S, 512, kProp.f1, 64, 1, f1, s);
+    }
+    int lin_fwd(const float* x, int M, int K, const PropLayer& L, int N, int relu, float* y, cudaStream_t s) {
+        pdl(k_linear<0>, dim3((N + 63) / 64, (M + 63) / 64), 256, 0, s)(x, (const void*)(P16 + L.w), M, N, K, P + L.b,
+                                                                      relu, nullptr, y, nullptr, 0);
+        CKL();
+        return PSB_OK;
+    }
+    // dx [M][K] = dy [M][N] W, masked
+    int lin_bwd_data(const float* dy, int M, int N, const PropLayer& L, int K, const float* xmask, float* dx,
+                     cudaStream_t s) {
+        pdl(k_linear<1>, dim3((K + 63) / 64, (M + 63) / 64), 256, 0, s)(dy, (const void*)(P16 + L.w), M, K, N, nullptr,
+                                                                      0, xmask, dx, nullptr, 0);
+        CKL();
+        return PSB_OK;
+    }
+    // dW [N][K] += dy^T x, db += column sums of dy, rows split over up to 32 CTAs per tile
+    int lin_bwd_weight(const float* dy, const float* x, int M, int N, int K, const PropLayer& L, cudaStream_t s) {
+        const int chunk = std::max(64, ((M + 31) / 32 + 15) / 16 * 16);
+        pdl(k_linear<2>, dim3((K + 63) / 64, (N + 63) / 64, (M + chunk - 1) / chunk), 256, 0, s)(
+            dy, (const void*)x, N, K, M, nullptr, 0, nullptr, G + L.w, G + L.b, chunk);
+        CKL();
+        return PSB_OK;
+    }
+
     // forward over B items of no orientations: grids [B*no][32^3], hmaps
     // [B][1024] (device) -> this->logit [B*no]
     int forward(const float* grids, const float* hmaps, int B, int no, cudaStream_t s) {
         const int S = B * no;
         auto g1 = [](long long n) { return (unsigned)((n + 255) / 256); };
-        const int ci[4] = {1, 16, 32, 64}, co[4] = {16, 32, 64, 64}, D[4] = {32, 16, 8, 4};
-        const float* in[4] = {grids, a1, a2, a3};
-        float* out[4] = {a1, a2, a3, a4};
-        for (int i = 0; i < 4; ++i) {
-            const long long n = (long long)S * (D[i] / 2) * (D[i] / 2) * (D[i] / 2);
-            PROF("k_prop_conv", s);
-            pdl(k_conv_fwd, dim3(g1(n), co[i] / PSB_CPT), 256, sizeof(float) * PSB_CPT * ci[i] * 27, s)(
-                in[i], S, ci[i], D[i], P16 + kProp.c[i].w, P + kProp.c[i].b, out[i], co[i]);
-            CKL();
-        }
+        TRY(item_branch(grids, S, s));
         PROF("k_prop_head", s);
-        pdl(k_lin_fwd, g1((long long)S * 64), 256, 0, s)(a4, S, 512, P16 + kProp.f1.w, P + kProp.f1.b, 64, 1, f1);
-        CKL();
-        pdl(k_lin_fwd, g1((long long)B * 64), 256, 0, s)(hmaps, B, PSB_PH * PSB_PH, P16 + kProp.f2.w, P + kProp.f2.b,
-                                                        64, 1, t);
-        CKL();
+        TRY(lin_fwd(hmaps, B, PSB_PH * PSB_PH, kProp.f2, 64, 1, t, s));
         pdl(k_concat, g1((long long)S * 128), 256, 0, s)(f1, t, S, no, hin);
         CKL();
-        pdl(k_lin_fwd, g1((long long)S * 64), 256, 0, s)(hin, S, 128, P16 + kProp.h1.w, P + kProp.h1.b, 64, 1, h1);
-        CKL();
-        pdl(k_lin_fwd, g1(S), 256, 0, s)(h1, S, 64, P16 + kProp.h2.w, P + kProp.h2.b, 1, 0, logit);
-        CKL();
-        return PSB_OK;
+        TRY(lin_fwd(hin, S, 128, kProp.h1, 64, 1, h1, s));
+        return lin_fwd(h1, S, 64, kProp.h2, 1, 0, logit, s);
     }
 
     // item branch only (conv stack + f1) for B items of no orientations
     // whose grids are at `grids`; f1 left in this->f1 [B*no][64]
-    int item_features(const float* grids, int B, int no, cudaStream_t s) {
-        const int S = B * no;
-        auto g1 = [](long long n) { return (unsigned)((n + 255) / 256); };
-        const int ci[4] = {1, 16, 32, 64}, co[4] = {16, 32, 64, 64}, D[4] = {32, 16, 8, 4};
-        const float* in[4] = {grids, a1, a2, a3};
-        float* out[4] = {a1, a2, a3, a4};
-        for (int i = 0; i < 4; ++i) {
-            const long long n = (long long)S * (D[i] / 2) * (D[i] / 2) * (D[i] / 2);
-            PROF("k_prop_conv", s);
-            pdl(k_conv_fwd, dim3(g1(n), co[i] / PSB_CPT), 256, sizeof(float) * PSB_CPT * ci[i] * 27, s)(
-                in[i], S, ci[i], D[i], P16 + kProp.c[i].w, P + kProp.c[i].b, out[i], co[i]);
-            CKL();
-        }
-        pdl(k_lin_fwd, g1((long long)S * 64), 256, 0, s)(a4, S, 512, P16 + kProp.f1.w, P + kProp.f1.b, 64, 1, f1);
+    int item_features(const float* grids, int B, int no, cudaStream_t s) { return item_branch(grids, B * no, s); }
+
+    template <int CI, int D, int CO, int CH>
+    int conv_bwd_data(const float* dout, int S, const PropLayer& L, const float* in, float* din, cudaStream_t s) {
+        using C = ConvBwd<CI, D, CO, CH>;
+        const long long n = (long long)S * C::Do3;
+        PROF("k_prop_bwd_data", s);
+        pdl(k_conv3_bwd_data<CI, D, CO, CH>, (unsigned)((n + C::CELLS - 1) / C::CELLS), 256, C::smem, s)(
+            dout, S, P16 + L.w, in, din);
+        CKL();
+        return PSB_OK;
+    }
+    template <int CI, int D, int CO, int CG, int SL, int NS, int SEG>
+    int conv_bwd_weight(const float* dout, const float* in, int S, const PropLayer& L, cudaStream_t s) {
+        using C = ConvBwdW<CI, D, CO, CG, SL, NS, SEG>;
+        // one CTA per SM: its registers and shared memory fill one
+        const int shares = std::min(S, 148 / (CI / CG)), chunk = (S + shares - 1) / shares;
+        PROF("k_prop_bwd_weight", s);
+        pdl(k_conv3_bwd_weight<CI, D, CO, CG, SL, NS, SEG>, dim3(CI / CG, (S + chunk - 1) / chunk), 256, C::smem, s)(
+            dout, in, S, chunk, G + L.w, G + L.b);
         CKL();
         return PSB_OK;
     }
@@ -2444,47 +2516,24 @@ struct psb_proposal {
         CK(cudaMemsetAsync(loss, 0, sizeof(float), s));
         pdl(k_softmax_ce, (B + 7) / 8, 256, 0, s)(logit, target, mask, B, no, dlogit, loss);
         CKL();
-        pdl(k_lin_bwd_weight, dim3(g1(64), 1), 256, 0, s)(dlogit, h1, S, 1, 64, G + kProp.h2.w, G + kProp.h2.b);
-        CKL();
-        pdl(k_lin_bwd_data, g1((long long)S * 64), 256, 0, s)(dlogit, S, 1, P16 + kProp.h2.w, 64, h1, dh1);
-        CKL();
-        pdl(k_lin_bwd_weight, dim3(g1(128), 64), 256, 0, s)(dh1, hin, S, 64, 128, G + kProp.h1.w, G + kProp.h1.b);
-        CKL();
-        pdl(k_lin_bwd_data, g1((long long)S * 128), 256, 0, s)(dh1, S, 64, P16 + kProp.h1.w, 128, nullptr, dhin);
-        CKL();
+        TRY(lin_bwd_weight(dlogit, h1, S, 1, 64, kProp.h2, s));
+        TRY(lin_bwd_data(dlogit, S, 1, kProp.h2, 64, h1, dh1, s));
+        TRY(lin_bwd_weight(dh1, hin, S, 64, 128, kProp.h1, s));
+        TRY(lin_bwd_data(dh1, S, 64, kProp.h1, 128, nullptr, dhin, s));
         pdl(k_split_item, g1((long long)S * 64), 256, 0, s)(dhin, f1, S, df1);
         CKL();
         pdl(k_split_tray, g1((long long)B * 64), 256, 0, s)(dhin, t, B, no, dt);
         CKL();
-        pdl(k_lin_bwd_weight, dim3(g1(PSB_PH * PSB_PH), 64), 256, 0, s)(dt, hmaps, B, 64, PSB_PH * PSB_PH,
-                                                                       G + kProp.f2.w, G + kProp.f2.b);
-        CKL();
-        pdl(k_lin_bwd_weight, dim3(g1(512), 64), 256, 0, s)(df1, a4, S, 64, 512, G + kProp.f1.w, G + kProp.f1.b);
-        CKL();
-        pdl(k_lin_bwd_data, g1((long long)S * 512), 256, 0, s)(df1, S, 64, P16 + kProp.f1.w, 512, a4, da4);
-        CKL();
-        const int ci[4] = {1, 16, 32, 64}, co[4] = {16, 32, 64, 64}, D[4] = {32, 16, 8, 4};
-        const float* in[4] = {grids, a1, a2, a3};
-        float* dout[4] = {da1, da2, da3, da4};
-        for (int i = 3; i >= 0; --i) {
-            // enough CTAs: about 2048 (ci, co, chunk) triples
-            const int nch_goal = std::max(1, 2048 / (ci[i] * co[i]));
-            const int chunk = std::max(1, (S + nch_goal - 1) / nch_goal);
-            const int nch = (S + chunk - 1) / chunk;
-            {
-                PROF("k_prop_bwd_weight", s);
-                pdl(k_conv_bwd_weight, dim3(ci[i], co[i], nch), 256, 0, s)(dout[i], in[i], S, ci[i], D[i], co[i], chunk,
-                                                                          G + kProp.c[i].w, G + kProp.c[i].b);
-            }
-            CKL();
-            if (i > 0) {
-                const long long n = (long long)S * D[i] * D[i] * D[i];
-                PROF("k_prop_bwd_data", s);
-                pdl(k_conv_bwd_data, dim3(g1(n), ci[i]), 256, sizeof(float) * co[i] * 27, s)(
-                    dout[i], S, ci[i], D[i], P16 + kProp.c[i].w, co[i], in[i], 1, dout[i - 1]);
-                CKL();
-            }
-        }
+        TRY(lin_bwd_weight(dt, hmaps, B, 64, PSB_PH * PSB_PH, kProp.f2, s));
+        TRY(lin_bwd_weight(df1, a4, S, 64, 512, kProp.f1, s));
+        TRY(lin_bwd_data(df1, S, 64, kProp.f1, 512, a4, da4, s));
+        TRY((conv_bwd_weight<64, 4, 64, 16, 2, 8, 2>(da4, a3, S, kProp.c[3], s)));
+        TRY((conv_bwd_data<64, 4, 64, 8>(da4, S, kProp.c[3], a3, da3, s)));
+        TRY((conv_bwd_weight<32, 8, 64, 8, 4, 2, 4>(da3, a2, S, kProp.c[2], s)));
+        TRY((conv_bwd_data<32, 8, 64, 8>(da3, S, kProp.c[2], a2, da2, s)));
+        TRY((conv_bwd_weight<16, 16, 32, 4, 8, 1, 8>(da2, a1, S, kProp.c[1], s)));
+        TRY((conv_bwd_data<16, 16, 32, 8>(da2, S, kProp.c[1], a1, da1, s)));
+        TRY((conv_bwd_weight<1, 32, 16, 1, 2, 1, 8>(da1, grids, S, kProp.c[0], s)));
         return PSB_OK;
     }
 };
@@ -3760,6 +3809,11 @@ int psb_prop_forward_backward(psb_proposal* p, const float* d_grids, const float
     CK(cudaSetDevice(p->dev));
     const int S = n_items * PSB_PNO;
     TRY(p->ensure(S, n_items));
+    if ((uintptr_t)d_grids & 15) {
+        // the first layer reads four values at a time
+        CK(cudaMemcpyAsync(p->a0, d_grids, sizeof(float) * (size_t)S * PSB_PG3, cudaMemcpyDeviceToDevice, p->st));
+        d_grids = p->a0;
+    }
     TRY(p->forward(d_grids, d_hmaps, n_items, PSB_PNO, p->st));
     if (d_target) TRY(p->backward(d_grids, d_hmaps, d_target, d_mask, n_items, PSB_PNO, p->st));
     if (d_logits) CK(cudaMemcpyAsync(d_logits, p->logit, sizeof(float) * S, cudaMemcpyDeviceToDevice, p->st));
@@ -3792,48 +3846,50 @@ int psb_prop_item_grids(const int32_t* const* items, const int32_t* dims, int n_
         return fail(PSB_ERR_ARG, "null pointer or bad count");
     TRY(ensure_device());
     if (n_items == 0) return PSB_OK;
-    std::vector<ItemInfo> infos(n_items);
-    std::vector<int> G(3 * (size_t)n_items), S(n_items);
-    size_t totv = 0;
+    // one block for the upload: the items' table, scaled extents, orientation
+    // maps and values
+    std::vector<GridItem> tab(n_items);
+    size_t cells = 0;
     for (int i = 0; i < n_items; ++i) {
-        const int ex = dims[3 * i], ey = dims[3 * i + 1], ez = dims[3 * i + 2];
-        if (!items[i] || ex <= 0 || ey <= 0 || ez <= 0) return fail(PSB_ERR_ARG, "item %d: bad array", i);
-        analyse_item(items[i], ex, ey, ez, &infos[i]);
-        S[i] = std::max(1, (std::max(ex, std::max(ey, ez)) + PSB_PG - 1) / PSB_PG);
-        for (int a = 0; a < 3; ++a) G[3 * i + a] = (infos[i].dims[a] + S[i] - 1) / S[i];
-        totv += infos[i].vox.size();
+        const int* d = dims + 3 * i;
+        if (!items[i] || d[0] <= 0 || d[1] <= 0 || d[2] <= 0) return fail(PSB_ERR_ARG, "item %d: bad array", i);
+        tab[i].off = (long long)cells;
+        for (int a = 0; a < 3; ++a) tab[i].d[a] = d[a];
+        tab[i].s = std::max(1, (std::max(d[0], std::max(d[1], d[2])) + PSB_PG - 1) / PSB_PG);
+        cells += (size_t)d[0] * d[1] * d[2];
     }
-    float* base = nullptr;
-    int4* vox = nullptr;
-    int *dG = nullptr, *dm = nullptr;
-    TRY(dalloc(&base, (size_t)n_items * PSB_PG3));
-    TRY(dalloc(&vox, std::max<size_t>(totv, 1)));
-    TRY(dalloc(&dG, G.size()));
-    TRY(dalloc(&dm, (size_t)6 * n_orient));
-    int rc = PSB_OK;
-    do {
-        if (cudaMemset(base, 0, sizeof(float) * n_items * PSB_PG3) != cudaSuccess) { rc = fail(PSB_ERR_CUDA, "memset"); break; }
-        size_t off = 0;
-        for (int i = 0; i < n_items && rc == PSB_OK; ++i) {
-            const size_t nv = infos[i].vox.size();
-            if (nv == 0) continue;
-            if (cudaMemcpy(vox + off, infos[i].vox.data(), sizeof(int4) * nv, cudaMemcpyHostToDevice) != cudaSuccess)
-                rc = fail(PSB_ERR_CUDA, "copy");
-            k_base_grid<<<(unsigned)((nv + 255) / 256), 256>>>(vox + off, (int)nv, S[i], base + (size_t)i * PSB_PG3);
-            off += nv;
-        }
-        if (rc != PSB_OK) break;
-        if (cudaMemcpy(dG, G.data(), sizeof(int) * G.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(dm, orient_maps, sizeof(int) * 6 * n_orient, cudaMemcpyHostToDevice) != cudaSuccess) {
-            rc = fail(PSB_ERR_CUDA, "copy");
-            break;
-        }
-        k_orient_grids<<<dim3(PSB_PG3 / 256, n_orient, n_items), 256>>>(base, dG, dm, n_orient, d_out);
-        if (cudaDeviceSynchronize() != cudaSuccess || cudaGetLastError() != cudaSuccess)
-            rc = fail(PSB_ERR_CUDA, "item grids: %s", cudaGetErrorString(cudaGetLastError()));
-    } while (0);
-    dfree(base); dfree(vox); dfree(dG); dfree(dm);
-    return rc;
+    auto up = [](size_t n) { return (n + 255) / 256 * 256; };
+    const size_t oG = up(sizeof(GridItem) * n_items), om = oG + up(sizeof(int) * 3 * n_items);
+    const size_t ov = om + up(sizeof(int) * 6 * n_orient), bytes = ov + up(sizeof(int32_t) * cells);
+    ArenaTrim trim{&g_arena2, (size_t)256 << 20};
+    void* base = nullptr;
+    char* h = nullptr;
+    TRY(arena(bytes + sizeof(float) * (size_t)n_items * PSB_PG3, &base, &g_arena2));
+    TRY(pinned(bytes, &h));
+    char* d = (char*)base;
+    float* grid = (float*)(d + bytes);
+    memcpy(h, tab.data(), sizeof(GridItem) * n_items);
+    int* G = (int*)(h + oG);
+    for (int i = 0; i < n_items; ++i)
+        for (int a = 0; a < 3; ++a) G[3 * i + a] = (tab[i].d[a] + tab[i].s - 1) / tab[i].s;
+    memcpy(h + om, orient_maps, sizeof(int) * 6 * n_orient);
+    for (int i = 0; i < n_items; ++i)
+        memcpy(h + ov + sizeof(int32_t) * tab[i].off, items[i],
+               sizeof(int32_t) * (size_t)tab[i].d[0] * tab[i].d[1] * tab[i].d[2]);
+    cudaStream_t st = 0;
+    CK(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st));
+    for (int i0 = 0; i0 < n_items; i0 += 32768) {   // grid dimensions stay below 65536
+        const int m = std::min(32768, n_items - i0);
+        pdl(k_base_grid_dense, dim3(PSB_PG3 / 256, m), 256, 0, st)((const int32_t*)(d + ov), (const GridItem*)d + i0,
+                                                                 grid + (size_t)i0 * PSB_PG3);
+        CKL();
+        pdl(k_orient_grids, dim3(PSB_PG3 / 256, n_orient, m), 256, 0, st)(
+            grid + (size_t)i0 * PSB_PG3, (const int*)(d + oG) + 3 * i0, (const int*)(d + om), n_orient,
+            d_out + (size_t)i0 * n_orient * PSB_PG3);
+        CKL();
+    }
+    CK(cudaStreamSynchronize(st));
+    return PSB_OK;
 }
 
 int psb_height_map(const int32_t* d_tray, int nx, int ny, int nz, float* d_out) {

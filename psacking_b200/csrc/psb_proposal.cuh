@@ -19,7 +19,7 @@
 #pragma once
 #include <stdint.h>
 
-#include "psb_pdl.cuh"
+#include "psb_conv.cuh"
 
 #define PSB_PG 32          // item grid side
 #define PSB_PG3 (PSB_PG * PSB_PG * PSB_PG)
@@ -37,27 +37,39 @@ __host__ __device__ __forceinline__ uint16_t bf16_bits(float f) {
     u += 0x7fffu + ((u >> 16) & 1u);
     return (uint16_t)(u >> 16);
 }
-__device__ __forceinline__ float bf16_val(uint16_t h) { return __uint_as_float((uint32_t)h << 16); }
+__device__ __forceinline__ float bf16_val(uint16_t h) { return bf16_up(h); }
 
 // ---------------------------------------------------------------------------
 // inputs
 // ---------------------------------------------------------------------------
-// base grid of one item from its voxel list (the synchronous item-grid call;
-// the packing loop uses k_base_grid_runs): cell floor(v / s) gains 1/s^3,
-// s = ceil(max extent / 32).  grid: (ceil(nvox/256)), block 256; out zeroed
-__global__ void k_base_grid(const int4* __restrict__ vox, int nvox, int s, float* __restrict__ out) {
+// base grids of items given as dense arrays (the synchronous item-grid call;
+// the packing loop uses k_base_grid_runs): cell (i, j, k) of an item holds the
+// occupied fraction of its s^3 block, s = ceil(max extent / 32), summed voxel
+// by voxel as the runs form does.  One thread per cell, no atomics.
+// grid: (PSB_PG3 / 256, items), block 256
+struct GridItem {
+    long long off;              // the item's first value in `vals`
+    int d[3], s;
+};
+__global__ void k_base_grid_dense(const int32_t* __restrict__ vals, const GridItem* __restrict__ items,
+                                  float* __restrict__ out) {
     pdl_enter();
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= nvox) return;
-    const int4 q = vox[v];
-    if (q.w <= 0) return;
-    const int i = q.x / s, j = q.y / s, k = q.z / s;
-    atomicAdd(&out[(i * PSB_PG + j) * PSB_PG + k], 1.0f / (float)(s * s * s));
+    const GridItem it = items[blockIdx.y];
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i0 = c / (PSB_PG * PSB_PG) * it.s, j0 = c / PSB_PG % PSB_PG * it.s, k0 = c % PSB_PG * it.s;
+    const float w = 1.0f / (float)(it.s * it.s * it.s);
+    float v = 0.f;
+    const int32_t* a = vals + it.off;
+    for (int i = i0; i < min(i0 + it.s, it.d[0]); ++i)
+        for (int j = j0; j < min(j0 + it.s, it.d[1]); ++j)
+            for (int k = k0; k < min(k0 + it.s, it.d[2]); ++k)
+                if (__ldg(&a[((size_t)i * it.d[1] + j) * it.d[2] + k]) > 0) v += w;
+    out[(size_t)blockIdx.y * PSB_PG3 + c] = v;
 }
 
-// the same base grid from the item's z-runs ({x, y, z0 | z1 << 16, value},
-// one per run of equal nonzero values along z): the cells and weights of the
-// voxel form.  grid: (ceil(nruns/256)), block 256; out zeroed
+// the base grid of one item from its z-runs ({x, y, z0 | z1 << 16, value},
+// one per run of equal nonzero values along z): cell floor(v / s) gains 1/s^3
+// per voxel.  grid: (ceil(nruns/256)), block 256; out zeroed
 __global__ void k_base_grid_runs(const int4* __restrict__ runs, int nruns, int s, float* __restrict__ out) {
     pdl_enter();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -139,205 +151,6 @@ __global__ void k_height_map(const int32_t* __restrict__ tray, int nx, int ny, i
         for (int i = 0; i < nwp; ++i) { s += red[i]; k += cnt[i]; }
         out[cell] = k ? s / (float)k : 0.f;
     }
-}
-
-// ---------------------------------------------------------------------------
-// convolution, kernel 3, stride 2, padding 1 (activations [S][C][D^3])
-// ---------------------------------------------------------------------------
-// forward with ReLU; each thread computes one output voxel for PSB_CPT
-// consecutive output channels, so every input value it loads feeds PSB_CPT
-// multiply-adds.  grid: (ceil(S*Do^3/256), Co/PSB_CPT), block 256;
-// smem PSB_CPT*Ci*27 floats
-#define PSB_CPT 4
-__global__ void k_conv_fwd(const float* __restrict__ in, int S, int Ci, int D, const uint16_t* __restrict__ w,
-                           const float* __restrict__ bias, float* __restrict__ out, int Co) {
-    pdl_enter();
-    extern __shared__ float ws[];   // [PSB_CPT][Ci*27]
-    const int c0 = blockIdx.y * PSB_CPT;
-    for (int i = threadIdx.x; i < PSB_CPT * Ci * 27; i += blockDim.x) {
-        const int c = i / (Ci * 27), r = i % (Ci * 27);
-        ws[i] = bf16_val(w[(size_t)(c0 + c) * Ci * 27 + r]);
-    }
-    __syncthreads();
-    const int Do = D / 2, Do3 = Do * Do * Do, D3 = D * D * D;
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)S * Do3) return;
-    const int s = (int)(idx / Do3), r = (int)(idx % Do3);
-    const int od = r / (Do * Do), oh = (r / Do) % Do, ow = r % Do;
-    float acc[PSB_CPT];
-#pragma unroll
-    for (int c = 0; c < PSB_CPT; ++c) acc[c] = bias[c0 + c];
-    for (int ci = 0; ci < Ci; ++ci) {
-        const float* x = in + ((size_t)s * Ci + ci) * D3;
-        const float* wc = ws + ci * 27;
-#pragma unroll
-        for (int kd = 0; kd < 3; ++kd) {
-            const int id = 2 * od - 1 + kd;
-            if (id < 0 || id >= D) continue;
-#pragma unroll
-            for (int kh = 0; kh < 3; ++kh) {
-                const int ih = 2 * oh - 1 + kh;
-                if (ih < 0 || ih >= D) continue;
-#pragma unroll
-                for (int kw = 0; kw < 3; ++kw) {
-                    const int iw = 2 * ow - 1 + kw;
-                    if (iw < 0 || iw >= D) continue;
-                    const float xv = x[(id * D + ih) * D + iw];
-                    const int t = kd * 9 + kh * 3 + kw;
-#pragma unroll
-                    for (int c = 0; c < PSB_CPT; ++c) acc[c] = fmaf(xv, wc[c * Ci * 27 + t], acc[c]);
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < PSB_CPT; ++c) out[((size_t)s * Co + c0 + c) * Do3 + r] = fmaxf(acc[c], 0.f);
-}
-
-// gradient w.r.t. the input, times the ReLU mask of that input (the previous
-// layer's output; mask_relu = 0 for the network input).
-// grid: (ceil(S*D^3/256), Ci), block 256; smem Co*27 floats
-__global__ void k_conv_bwd_data(const float* __restrict__ dout, int S, int Ci, int D, const uint16_t* __restrict__ w,
-                                int Co, const float* __restrict__ in, int mask_relu, float* __restrict__ din) {
-    pdl_enter();
-    extern __shared__ float ws[];
-    const int ci = blockIdx.y;
-    for (int i = threadIdx.x; i < Co * 27; i += blockDim.x) {
-        const int co = i / 27, t = i % 27;
-        ws[i] = bf16_val(w[((size_t)co * Ci + ci) * 27 + t]);
-    }
-    __syncthreads();
-    const int Do = D / 2, Do3 = Do * Do * Do, D3 = D * D * D;
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)S * D3) return;
-    const int s = (int)(idx / D3), r = (int)(idx % D3);
-    const int id = r / (D * D), ih = (r / D) % D, iw = r % D;
-    float acc = 0.f;
-    // od = (id + 1 - kd) / 2 for the kd of matching parity
-    for (int kd = (id + 1) & 1; kd < 3; kd += 2) {
-        const int od = (id + 1 - kd) >> 1;
-        if (od < 0 || od >= Do) continue;
-        for (int kh = (ih + 1) & 1; kh < 3; kh += 2) {
-            const int oh = (ih + 1 - kh) >> 1;
-            if (oh < 0 || oh >= Do) continue;
-            for (int kw = (iw + 1) & 1; kw < 3; kw += 2) {
-                const int ow = (iw + 1 - kw) >> 1;
-                if (ow < 0 || ow >= Do) continue;
-                const int t = kd * 9 + kh * 3 + kw;
-                const float* g = dout + (size_t)s * Co * Do3 + (od * Do + oh) * Do + ow;
-                for (int co = 0; co < Co; ++co) acc = fmaf(g[(size_t)co * Do3], ws[co * 27 + t], acc);
-            }
-        }
-    }
-    const size_t at = ((size_t)s * Ci + ci) * D3 + r;
-    if (mask_relu && in[at] <= 0.f) acc = 0.f;
-    din[at] = acc;
-}
-
-// gradient w.r.t. the weights and bias: each CTA sums a chunk of samples for
-// one (co, ci) pair and adds its 27 partial sums (and the bias sum when ci ==
-// 0) with atomics.  grid: (Ci, Co, nchunk), block 256; dw, db zeroed first
-__global__ void k_conv_bwd_weight(const float* __restrict__ dout, const float* __restrict__ in, int S, int Ci, int D,
-                                  int Co, int chunk, float* __restrict__ dw, float* __restrict__ db) {
-    pdl_enter();
-    const int ci = blockIdx.x, co = blockIdx.y;
-    const int s0 = blockIdx.z * chunk, s1 = min(S, s0 + chunk);
-    const int Do = D / 2, Do3 = Do * Do * Do, D3 = D * D * D;
-    float acc[27];
-#pragma unroll
-    for (int t = 0; t < 27; ++t) acc[t] = 0.f;
-    float bacc = 0.f;
-    const long long n = (long long)(s1 - s0) * Do3;
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-        const int s = s0 + (int)(i / Do3), r = (int)(i % Do3);
-        const int od = r / (Do * Do), oh = (r / Do) % Do, ow = r % Do;
-        const float g = dout[((size_t)s * Co + co) * Do3 + r];
-        if (g == 0.f) continue;
-        bacc += g;
-        const float* x = in + ((size_t)s * Ci + ci) * D3;
-#pragma unroll
-        for (int kd = 0; kd < 3; ++kd) {
-            const int id = 2 * od - 1 + kd;
-            if (id < 0 || id >= D) continue;
-#pragma unroll
-            for (int kh = 0; kh < 3; ++kh) {
-                const int ih = 2 * oh - 1 + kh;
-                if (ih < 0 || ih >= D) continue;
-#pragma unroll
-                for (int kw = 0; kw < 3; ++kw) {
-                    const int iw = 2 * ow - 1 + kw;
-                    if (iw < 0 || iw >= D) continue;
-                    acc[kd * 9 + kh * 3 + kw] = fmaf(g, x[(id * D + ih) * D + iw], acc[kd * 9 + kh * 3 + kw]);
-                }
-            }
-        }
-    }
-    __shared__ float red[8][28];
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-#pragma unroll
-    for (int t = 0; t < 27; ++t) {
-        float v = acc[t];
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (lane == 0) red[wp][t] = v;
-    }
-    for (int off = 16; off > 0; off >>= 1) bacc += __shfl_xor_sync(0xffffffffu, bacc, off);
-    if (lane == 0) red[wp][27] = bacc;
-    __syncthreads();
-    if (threadIdx.x < 28) {
-        float v = 0.f;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) v += red[k][threadIdx.x];
-        if (threadIdx.x < 27) atomicAdd(&dw[((size_t)co * Ci + ci) * 27 + threadIdx.x], v);
-        else if (ci == 0) atomicAdd(&db[co], v);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// linear layers y[S][N] = x[S][K] W^T + b (W [N][K] BF16)
-// ---------------------------------------------------------------------------
-// forward; relu applied when relu != 0.  grid: ceil(S*N/256)
-__global__ void k_lin_fwd(const float* __restrict__ x, int S, int K, const uint16_t* __restrict__ w,
-                          const float* __restrict__ b, int N, int relu, float* __restrict__ y) {
-    pdl_enter();
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)S * N) return;
-    const int s = (int)(idx / N), n = (int)(idx % N);
-    const float* xr = x + (size_t)s * K;
-    const uint16_t* wr = w + (size_t)n * K;
-    float acc = b[n];
-    for (int k = 0; k < K; ++k) acc = fmaf(xr[k], bf16_val(wr[k]), acc);
-    y[idx] = relu ? fmaxf(acc, 0.f) : acc;
-}
-
-// dx[S][K] = dy[S][N] W, times the ReLU mask of x when xmask != NULL.
-// grid: ceil(S*K/256)
-__global__ void k_lin_bwd_data(const float* __restrict__ dy, int S, int N, const uint16_t* __restrict__ w, int K,
-                               const float* __restrict__ xmask, float* __restrict__ dx) {
-    pdl_enter();
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)S * K) return;
-    const int s = (int)(idx / K), k = (int)(idx % K);
-    float acc = 0.f;
-    for (int n = 0; n < N; ++n) acc = fmaf(dy[(size_t)s * N + n], bf16_val(w[(size_t)n * K + k]), acc);
-    if (xmask && xmask[idx] <= 0.f) acc = 0.f;
-    dx[idx] = acc;
-}
-
-// dW[N][K] = dy^T x, db[N] = sum_s dy.  grid: (ceil(K/256), N); the K == 0
-// column of threads also sums the bias
-__global__ void k_lin_bwd_weight(const float* __restrict__ dy, const float* __restrict__ x, int S, int N, int K,
-                                 float* __restrict__ dw, float* __restrict__ db) {
-    pdl_enter();
-    const int n = blockIdx.y;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= K) return;
-    float acc = 0.f, bacc = 0.f;
-    for (int s = 0; s < S; ++s) {
-        const float g = dy[(size_t)s * N + n];
-        acc = fmaf(g, x[(size_t)s * K + k], acc);
-        bacc += g;
-    }
-    dw[(size_t)n * K + k] = acc;
-    if (k == 0) db[n] = bacc;
 }
 
 // head input: [f1[s] | t[s / no]] (64 + 64).  grid: ceil(S*128/256)
