@@ -34,6 +34,7 @@
 #include "psb_loop.cuh"
 #include "psb_bound.cuh"
 #include "psb_filter.cuh"
+#include "psb_item.cuh"
 #include "psb_proposal.cuh"
 #include "psb_voxel.cuh"
 #include <nvtx3/nvToolsExt.h>
@@ -401,6 +402,27 @@ int init_register_twiddles() {
     return PSB_OK;
 }
 
+// k_item_describe's split cells in farthest-point order from a corner
+int init_cell_order() {
+    unsigned char order[PSB_ICELLS];
+    int dmin[PSB_ICELLS], k = 0;
+    for (int& d : dmin) d = INT_MAX;
+    for (int i = 0; i < PSB_ICELLS; ++i) {
+        order[i] = (unsigned char)k;
+        dmin[k] = -1;
+        int far = -1;
+        for (int c = 0; c < PSB_ICELLS; ++c) {
+            if (dmin[c] < 0) continue;
+            const int dx = c / 25 - k / 25, dy = c / 5 % 5 - k / 5 % 5, dz = c % 5 - k % 5;
+            dmin[c] = std::min(dmin[c], dx * dx + dy * dy + dz * dz);
+            if (far < 0 || dmin[c] > dmin[far]) far = c;
+        }
+        k = far;
+    }
+    CK(cudaMemcpyToSymbol(c_cell_order, order, sizeof(order)));
+    return PSB_OK;
+}
+
 template <class K>
 int set_max_dyn_smem(K func) {
     cudaFuncAttributes fa;
@@ -469,6 +491,7 @@ int set_smem_attrs() {
     TRY(set_max_dyn_smem(k_cand_filter_plane<1>));
     TRY(set_max_dyn_smem(k_cand_filter_plane<2>));
     TRY(init_register_twiddles());
+    TRY(init_cell_order());
     if (dev < 64) done[dev] = true;
     return PSB_OK;
 }
@@ -725,7 +748,6 @@ struct ItemInfo {
     long long sabs = 0;        // sum of |values|
     double sumsq = 0.0;
     long long nvox = 0;        // nonzero voxels
-    std::vector<int4> vox;     // their list (x, y, z, value), when asked for
     std::vector<int4> samp;    // candidate-filter samples (positive voxels, spread out)
     std::vector<int4> runs[3]; // runs of equal nonzero values along each source axis (build_runs)
 };
@@ -877,7 +899,6 @@ void analyse_runs(ItemInfo* info) {
     info->sabs = 0;
     info->sumsq = 0.0;
     info->nvox = 0;
-    info->vox.clear();
     const std::vector<int4>& zr = info->runs[2];
     long long wmax = 0;
     for (const int4& q : zr) wmax = std::max(wmax, std::llabs((long long)q.w));
@@ -903,21 +924,19 @@ void analyse_runs(ItemInfo* info) {
     if (exact) info->sumsq = (double)isq;
 }
 
-void analyse_item(const int32_t* a, int ex, int ey, int ez, ItemInfo* info, bool keep_vox = true) {
+void analyse_item(const int32_t* a, int ex, int ey, int ez, ItemInfo* info) {
     info->dims[0] = ex; info->dims[1] = ey; info->dims[2] = ez;
     for (int k = 0; k < 3; ++k) { info->lo[k] = INT32_MAX; info->hi[k] = -1; }
     info->sum = 0;
     info->sabs = 0;
     info->sumsq = 0.0;
     info->nvox = 0;
-    info->vox.clear();
     for (int i = 0; i < ex; ++i)
         for (int j = 0; j < ey; ++j)
             for (int k = 0; k < ez; ++k) {
                 int v = a[((size_t)i * ey + j) * ez + k];
                 if (v == 0) continue;
                 info->nvox += 1;
-                if (keep_vox) info->vox.push_back(make_int4(i, j, k, v));
                 info->sum += v;
                 info->sabs += std::llabs((long long)v);
                 info->sumsq += (double)v * v;
@@ -1017,13 +1036,13 @@ struct psb_tray {
     // the search by score bounds (psb_bound.cuh): tables and samples of
     // bcap queued items' orientations, the list of translations, its state
     BoundGeom* d_bgeom = nullptr;
-    BoundState* d_bstate = nullptr;
+    BoundState* d_bstate = nullptr;   // in d_reply
     BoundHit* d_blist = nullptr;   // PSB_BCAP listed translations, then as many winners
     double* d_btab = nullptr;
     int2* d_bfs = nullptr;
     int* d_bfb = nullptr;
     size_t bcap = 0;
-    BoundState* h_bstate = nullptr;   // pinned
+    BoundReply* h_reply = nullptr;    // pinned
 
     // per-orientation slots
     int cap = 0;
@@ -1109,13 +1128,14 @@ struct psb_tray {
     cudaStream_t st_copy = nullptr;  // uploads of the second part
     cudaEvent_t ev_copy = nullptr;
 
-    // item staging
-    int32_t* d_items = nullptr;
-    size_t items_cap = 0;
-    int4* d_vox = nullptr;
-    size_t vox_cap = 0;
-    int4* d_runs = nullptr;
-    size_t runs_cap = 0;
+    // the arrays of a synchronous search or placement (stage_arrays): one
+    // block holding their table and values (uploaded), then what the device
+    // makes of them
+    char* d_x = nullptr;
+    size_t x_cap = 0;
+    ItemSums* d_xsums = nullptr;
+    OrientDesc* d_xod = nullptr;
+    BoundReply* d_reply = nullptr;
 
     // per-column prefix sums along z of the distance field and the occupancy
     // (k_col_prefix), for the exact sums over an item's runs
@@ -1138,11 +1158,12 @@ struct psb_tray {
         release_slots();
         dfree(d_tray, st); dfree(d_phi, st); dfree(d_Socc, st); dfree(d_Sphi, st); dfree(d_w1, st); dfree(d_w2, st); dfree(d_wocc, st); dfree(d_pen, st);
         dfree(d_ostat, st);
-        dfree(d_rz, st); dfree(d_mid, st); dfree(d_stats, st); dfree(d_err, st); dfree(d_first, st); dfree(d_needff, st); dfree(d_items, st); dfree(d_vox, st);
-        dfree(d_runs, st); dfree(d_pphi, st); dfree(d_pocc, st);
+        dfree(d_rz, st); dfree(d_mid, st); dfree(d_stats, st); dfree(d_err, st); dfree(d_first, st); dfree(d_needff, st); dfree(d_x, st);
+        x_cap = 0;
+        dfree(d_pphi, st); dfree(d_pocc, st);
         dfree(d_ls, st); dfree(d_ps, st); dfree(d_rzd, st); dfree(d_midd, st); dfree(d_od_all, st); dfree(d_base_all, st); dfree(d_dec, st);
         dfree(d_tbits, st); dfree(d_work, st); dfree(d_clist, st);
-        dfree(d_bgeom, st); dfree(d_bstate, st); dfree(d_blist, st); dfree(d_btab, st); dfree(d_bfs, st); dfree(d_bfb, st);
+        dfree(d_bgeom, st); dfree(d_reply, st); d_bstate = nullptr; dfree(d_blist, st); dfree(d_btab, st); dfree(d_bfs, st); dfree(d_bfb, st);
         bcap = 0;
         for (int p = 0; p < 2; ++p) {
             dfree(d_part[p], st);
@@ -1174,8 +1195,8 @@ struct psb_tray {
         if (h_desc) cudaFreeHost(h_desc);
         h_desc = nullptr;
         h_desc_cap = 0;
-        if (h_bstate) cudaFreeHost(h_bstate);
-        h_bstate = nullptr;
+        if (h_reply) cudaFreeHost(h_reply);
+        h_reply = nullptr;
         if (h_icmeta) cudaFreeHost(h_icmeta);
         h_icmeta = nullptr;
     }
@@ -1289,15 +1310,6 @@ struct psb_tray {
         return PSB_OK;
     }
 
-    int ensure_runs(size_t n) {
-        if (n > runs_cap) {
-            dfree(d_runs, st);
-            runs_cap = std::max(n, (size_t)1 << 14);
-            TRY(dalloc(&d_runs, runs_cap, st));
-        }
-        return PSB_OK;
-    }
-
     // prefix tables of the distance field (gated when gate is set) and of
     // the occupancy
     int prefix_phi(const int* gate) {
@@ -1310,20 +1322,6 @@ struct psb_tray {
         const int ncols = nx * ny;
         pdl(k_col_prefix<1>, (ncols + 7) / 8, 256, 0, st)(d_tray, d_pocc, ncols, nz, nullptr);
         CKL();
-        return PSB_OK;
-    }
-
-    int ensure_staging(size_t n_items, size_t n_vox) {
-        if (n_items > items_cap) {
-            dfree(d_items, st);
-            items_cap = std::max(n_items, (size_t)1 << 16);
-            TRY(dalloc(&d_items, items_cap, st));
-        }
-        if (n_vox > vox_cap) {
-            dfree(d_vox, st);
-            vox_cap = std::max(n_vox, (size_t)1 << 14);
-            TRY(dalloc(&d_vox, vox_cap, st));
-        }
         return PSB_OK;
     }
 
@@ -1443,14 +1441,13 @@ struct psb_tray {
         phi_own = phi == nullptr;
         has_source = one != 0;
         occ_stale = phi_stale = bits_stale = geom_stale = true;
-        CK(cudaStreamSynchronize(st));
         ready = true;
         return PSB_OK;
     }
 
     // Fill an OrientDesc from an item's analysis and a signed permutation.
     void describe(const ItemInfo& info, const int* src_axis, const int* flip, const int32_t* d_item,
-                  const int4* d_vx, const int4* const* d_rn, OrientDesc* od) const {
+                  const int4* const* d_rn, OrientDesc* od) const {
         int n[3] = {nx, ny, nz};
         for (int a = 0; a < 3; ++a) {
             od->src_axis[a] = src_axis[a];
@@ -1473,7 +1470,6 @@ struct psb_tray {
         od->exact = 0;
         const long long sabs = info.sabs;  // |D'| <= sum|I| * max|phi - m|
         od->item = d_item;
-        od->vox = d_vx;
         od->nvox = (int)info.nvox;
         od->perm = -1;
         od->sumsq = info.sumsq;
@@ -1628,21 +1624,26 @@ struct psb_tray {
     // half-way may have left another)
     int bound_reset() {
         if (!d_bstate) return PSB_OK;
-        memset(h_bstate, 0, sizeof(BoundState));
-        h_bstate->best = ~0ULL;
-        CK(cudaMemcpyAsync(d_bstate, h_bstate, sizeof(BoundState), cudaMemcpyHostToDevice, st));
+        memset(h_reply, 0, sizeof(BoundReply));
+        h_reply->st.best = ~0ULL;
+        CK(cudaMemcpyAsync(d_bstate, &h_reply->st, sizeof(BoundState), cudaMemcpyHostToDevice, st));
         return PSB_OK;
+    }
+    int ensure_reply() {
+        if (d_reply) return PSB_OK;
+        if (!h_reply) CK(cudaMallocHost(&h_reply, sizeof(BoundReply)));
+        TRY(dalloc(&d_reply, 1, st));
+        d_bstate = &d_reply->st;
+        return bound_reset();
     }
 
     // buffers for `slots` orientations' tables, the sources' geometry and the
     // free bits
     int ensure_bound(size_t slots) {
-        if (!d_bstate) {
-            TRY(dalloc(&d_bgeom, 1, st));
+        if (!d_blist) {
+            TRY(ensure_reply());
+            if (!d_bgeom) TRY(dalloc(&d_bgeom, 1, st));
             TRY(dalloc(&d_blist, 2 * (size_t)PSB_BCAP, st));
-            if (!h_bstate) CK(cudaMallocHost(&h_bstate, sizeof(BoundState)));
-            TRY(dalloc(&d_bstate, 1, st));
-            TRY(bound_reset());
         }
         if (slots > bcap) {
             dfree(d_btab, st);
@@ -2113,17 +2114,20 @@ struct psb_tray {
         return PSB_OK;
     }
 
-    // device placement of an item described by od (slot 0 of d_od is overwritten)
-    int place(const OrientDesc& od, int px, int py, int pz, int32_t id, int32_t* overlap_ijk) {
-        TRY(ensure_slots(1));
-        CK(cudaMemcpyAsync(d_od, &od, sizeof(OrientDesc), cudaMemcpyHostToDevice, st));
+    // device placement of the staged item (stage_arrays); *nvox: its voxels
+    int place(int px, int py, int pz, int32_t id, int32_t* overlap_ijk, int* nvox) {
         CK(cudaMemsetAsync(d_first, 0xff, sizeof(unsigned long long), st));
-        int blocks = std::max(1, std::min(1024, (od.nvox + 255) / 256));
-        pdl(k_place_check, blocks, 256, 0, st)(d_od, d_tray, nx, ny, nz, px, py, pz, d_first);
+        pdl(k_place_runs_check, 148, 256, 0, st)(d_xod, d_tray, nx, ny, nz, px, py, pz, d_first);
         CKL();
         unsigned long long first = 0;
+        OrientDesc od;
+        int neg = 0;
+        CK(cudaMemcpyAsync(&od, d_xod, sizeof(od), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(&neg, &d_reply->neg, sizeof(neg), cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(&first, d_first, sizeof(first), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        if (neg != INT_MAX) return fail(PSB_ERR_ARG, "orientation %d holds negative values", neg);
+        *nvox = od.nvox;
         if (first != 0xffffffffffffffffULL) {
             int k = (int)(first % nz), j = (int)((first / nz) % ny), i = (int)(first / ((size_t)ny * nz));
             if (overlap_ijk) { overlap_ijk[0] = i; overlap_ijk[1] = j; overlap_ijk[2] = k; }
@@ -2131,7 +2135,7 @@ struct psb_tray {
                         "(place_in_tray): Item to be placed intersects with contents of tray at position (%d, %d, %d)",
                         i, j, k);
         }
-        pdl(k_place_write, blocks, 256, 0, st)(d_od, d_tray, nx, ny, nz, px, py, pz, id);
+        pdl(k_place_runs_write, 148, 256, 0, st)(d_xod, d_tray, nx, ny, nz, px, py, pz, id);
         CKL();
         occ_stale = bits_stale = true;
         if (id == 1 && od.nvox > 0) {  // only voxels equal to 1 are distance sources (fft3.cu:948)
@@ -2147,9 +2151,6 @@ struct psb_tray {
 
 namespace {
 
-const int kIdentity[3] = {0, 1, 2};
-const int kNoFlip[3] = {0, 0, 0};
-
 void to_result(const ResultDev& r, int orient, psb_result* out) {
     out->x = r.found ? r.x : -1;
     out->y = r.found ? r.y : -1;
@@ -2160,69 +2161,6 @@ void to_result(const ResultDev& r, int orient, psb_result* out) {
     out->diag = r.diag;
     out->n_candidates = r.ncand;
     out->err_ratio = r.err_ratio;
-}
-
-// Upload a set of explicit orientation arrays and describe them.
-int stage_arrays(psb_tray* t, const int32_t* const* items, const int32_t* dims, int n, std::vector<OrientDesc>* ods) {
-    std::vector<ItemInfo> infos(n);
-    size_t tot = 0, totv = 0, totr = 0;
-    for (int o = 0; o < n; ++o) {
-        int ex = dims[3 * o], ey = dims[3 * o + 1], ez = dims[3 * o + 2];
-        if (!items[o] || ex <= 0 || ey <= 0 || ez <= 0)
-            return fail(PSB_ERR_ARG, "orientation %d: bad array (dims %d,%d,%d)", o, ex, ey, ez);
-        size_t m = (size_t)ex * ey * ez;
-        if (has_negative(items[o], m)) return fail(PSB_ERR_ARG, "orientation %d holds negative values", o);
-        analyse_item(items[o], ex, ey, ez, &infos[o]);
-        build_runs(items[o], &infos[o], 2);   // identity orientations: z-runs along the item's own z
-        tot += m;
-        totv += infos[o].vox.size();
-        totr += infos[o].runs[2].size();
-    }
-    TRY(t->ensure_staging(tot, totv));
-    TRY(t->ensure_runs(totr));
-    size_t off = 0, offv = 0, offr = 0;
-    ods->resize(n);
-    for (int o = 0; o < n; ++o) {
-        size_t m = (size_t)infos[o].dims[0] * infos[o].dims[1] * infos[o].dims[2];
-        CK(cudaMemcpyAsync(t->d_items + off, items[o], sizeof(int32_t) * m, cudaMemcpyHostToDevice, t->st));
-        if (!infos[o].vox.empty())
-            CK(cudaMemcpyAsync(t->d_vox + offv, infos[o].vox.data(), sizeof(int4) * infos[o].vox.size(),
-                               cudaMemcpyHostToDevice, t->st));
-        if (!infos[o].runs[2].empty())
-            CK(cudaMemcpyAsync(t->d_runs + offr, infos[o].runs[2].data(), sizeof(int4) * infos[o].runs[2].size(),
-                               cudaMemcpyHostToDevice, t->st));
-        const int4* rn[3] = {nullptr, nullptr, t->d_runs + offr};
-        t->describe(infos[o], kIdentity, kNoFlip, t->d_items + off, t->d_vox + offv, rn, &(*ods)[o]);
-        off += m;
-        offv += infos[o].vox.size();
-        offr += infos[o].runs[2].size();
-    }
-    CK(cudaStreamSynchronize(t->st));  // host vectors die at return
-    return PSB_OK;
-}
-
-// cached contexts for the stateless entry points, keyed by dims.  A caller
-// holds g_util_call_mu for its whole call (UtilCall), so a cached context is
-// used by one call at a time and is never dropped while another call uses it.
-std::mutex g_util_mu;
-std::map<std::tuple<int, int, int, int>, std::unique_ptr<psb_tray>> g_util;
-std::recursive_mutex g_util_call_mu;
-typedef std::lock_guard<std::recursive_mutex> UtilCall;
-
-int util_tray(int nx, int ny, int nz, psb_tray** out) {
-    TRY(ensure_device());
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lk(g_util_mu);
-    auto key = std::make_tuple(dev, nx, ny, nz);
-    auto it = g_util.find(key);
-    if (it != g_util.end()) { *out = it->second.get(); return PSB_OK; }
-    if (g_util.size() >= 4) g_util.clear();
-    std::unique_ptr<psb_tray> t(new psb_tray());
-    TRY(t->init(nx, ny, nz));
-    *out = t.get();
-    g_util[key] = std::move(t);
-    return PSB_OK;
 }
 
 // scratch arena for the stateless transforms
@@ -2282,6 +2220,87 @@ struct ArenaTrim {
         a->n = 0;
     }
 };
+
+// Upload explicit orientation arrays and queue their analysis (psb_item.cuh):
+// their descriptors at t->d_xod.  Negative values are found there; the caller
+// reads t->d_reply->neg with its results.
+int stage_arrays(psb_tray* t, const int32_t* const* items, const int32_t* dims, int n) {
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    size_t cells = 0;
+    for (int o = 0; o < n; ++o) {
+        const int32_t* d = dims + 3 * o;
+        if (!items[o] || d[0] <= 0 || d[1] <= 0 || d[2] <= 0)
+            return fail(PSB_ERR_ARG, "orientation %d: bad array (dims %d,%d,%d)", o, d[0], d[1], d[2]);
+        cells += (size_t)d[0] * d[1] * d[2];
+    }
+    const size_t ov = up(sizeof(ItemArr) * n), in = ov + up(sizeof(int32_t) * cells);
+    const size_t os = in, od = os + up(sizeof(ItemSums) * n), op = od + up(sizeof(OrientDesc) * n);
+    const size_t orn = op + up(sizeof(int4) * PSB_FSAMP * n), bytes = orn + sizeof(int4) * cells;
+    if (bytes > t->x_cap) {
+        dfree(t->d_x, t->st);
+        t->x_cap = 0;
+        TRY(dalloc(&t->d_x, std::max(bytes, (size_t)1 << 20), t->st));
+        t->x_cap = std::max(bytes, (size_t)1 << 20);
+    }
+    TRY(t->ensure_reply());
+    char* h = nullptr;
+    TRY(pinned(in, &h));
+    ItemArr* tab = (ItemArr*)h;
+    size_t off = 0;
+    int maxcol = 1;
+    for (int o = 0; o < n; ++o) {
+        const int32_t* d = dims + 3 * o;
+        const size_t m = (size_t)d[0] * d[1] * d[2];
+        tab[o].off = tab[o].roff = (long long)off;
+        for (int a = 0; a < 3; ++a) tab[o].d[a] = d[a];
+        tab[o].skip = d[0] > t->nx || d[1] > t->ny || d[2] > t->nz;
+        memcpy(h + ov + sizeof(int32_t) * off, items[o], sizeof(int32_t) * m);
+        off += m;
+        maxcol = std::max(maxcol, d[0] * d[1]);
+    }
+    CK(cudaMemcpyAsync(t->d_x, h, in, cudaMemcpyHostToDevice, t->st));
+    t->d_xsums = (ItemSums*)(t->d_x + os);
+    t->d_xod = (OrientDesc*)(t->d_x + od);
+    const int32_t* vals = (const int32_t*)(t->d_x + ov);
+    const ItemArr* arrs = (const ItemArr*)t->d_x;
+    int4* runs = (int4*)(t->d_x + orn);
+    PROF("k_item_describe", t->st);
+    pdl(k_item_reset, (n + 127) / 128, 128, 0, t->st)(t->d_xsums, n, &t->d_reply->neg);
+    CKL();
+    for (int o0 = 0; o0 < n; o0 += 65535) {   // grid dimensions
+        pdl(k_item_runs, dim3(std::min(64, (maxcol + 7) / 8), std::min(n - o0, 65535)), 256, 0, t->st)(
+            vals, arrs + o0, runs, t->d_xsums + o0);
+        CKL();
+    }
+    pdl(k_item_describe, n, 256, 0, t->st)(vals, arrs, runs, t->d_xsums, t->nx, t->ny, t->nz,
+                                          (int4*)(t->d_x + op), t->d_xod, &t->d_reply->neg);
+    CKL();
+    return PSB_OK;
+}
+
+// cached contexts for the stateless entry points, keyed by dims.  A caller
+// holds g_util_call_mu for its whole call (UtilCall), so a cached context is
+// used by one call at a time and is never dropped while another call uses it.
+std::mutex g_util_mu;
+std::map<std::tuple<int, int, int, int>, std::unique_ptr<psb_tray>> g_util;
+std::recursive_mutex g_util_call_mu;
+typedef std::lock_guard<std::recursive_mutex> UtilCall;
+
+int util_tray(int nx, int ny, int nz, psb_tray** out) {
+    TRY(ensure_device());
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_util_mu);
+    auto key = std::make_tuple(dev, nx, ny, nz);
+    auto it = g_util.find(key);
+    if (it != g_util.end()) { *out = it->second.get(); return PSB_OK; }
+    if (g_util.size() >= 4) g_util.clear();
+    std::unique_ptr<psb_tray> t(new psb_tray());
+    TRY(t->init(nx, ny, nz));
+    *out = t.get();
+    g_util[key] = std::move(t);
+    return PSB_OK;
+}
 
 // corr (conj_b=1): out[t] = sum_x b[x] a[t+x] ; conv (conj_b=0): linear conv
 int linear_transform_product(const int32_t* a, const int32_t* b, int nx, int ny, int nz, int conj_b, int32_t* out) {
@@ -2846,54 +2865,40 @@ int psb_place_in_tray(const int32_t* item, int ex, int ey, int ez, const int32_t
     if (i0 >= i1 || j0 >= j1 || k0 >= k1) return PSB_OK;
     int bx = i1 - i0, by = j1 - j0, bz = k1 - k0;
     size_t B = (size_t)bx * by * bz;
-    std::vector<int32_t> box(B);
+    // one upload (the box and the item), one kernel, one read-back
+    const size_t I = (size_t)ex * ey * ez;
+    const size_t nb = sizeof(int32_t) * B, ob = (nb + 15) / 16 * 16, oi = 16 + ob;   // [first][box][item]
+    void* base = nullptr;
+    char* h = nullptr;
+    TRY(arena(oi + sizeof(int32_t) * I + 16 + ob + 64, &base));
+    TRY(pinned(oi + sizeof(int32_t) * I, &h));
+    char* d = (char*)base;
+    char* d_out = d + (oi + sizeof(int32_t) * I + 15) / 16 * 16;   // [first][box]
+    *(unsigned long long*)h = 0xffffffffffffffffULL;
+    int32_t* box = (int32_t*)(h + 16);
     for (int i = 0; i < bx; ++i)
         for (int j = 0; j < by; ++j)
             memcpy(&box[((size_t)i * by + j) * bz], &tray[((size_t)(i0 + i) * ny + (j0 + j)) * nz + k0],
                    sizeof(int32_t) * bz);
-    ItemInfo info;
-    analyse_item(item, ex, ey, ez, &info);
-    size_t I = (size_t)ex * ey * ez;
-    void* base = nullptr;
-    size_t need = sizeof(int32_t) * (B + I) + sizeof(int4) * (info.vox.size() + 1) + sizeof(OrientDesc) + 2048;
-    TRY(arena(need, &base));
-    char* p = (char*)base;
-    auto take = [&](size_t n) { char* r = p; p += (n + 255) / 256 * 256; return r; };
-    int32_t* dbox = (int32_t*)take(sizeof(int32_t) * B);
-    int32_t* ditem = (int32_t*)take(sizeof(int32_t) * I);
-    int4* dvox = (int4*)take(sizeof(int4) * (info.vox.size() + 1));
-    OrientDesc* dod = (OrientDesc*)take(sizeof(OrientDesc));
-    unsigned long long* dfirst = (unsigned long long*)take(sizeof(unsigned long long));
-    OrientDesc od;
-    memset(&od, 0, sizeof(od));
-    for (int a = 0; a < 3; ++a) { od.src_axis[a] = a; od.flip[a] = 0; od.e[a] = info.dims[a]; od.b[a] = info.dims[a]; }
-    od.item = ditem;
-    od.vox = dvox;
-    od.nvox = (int)info.vox.size();
-    CK(cudaMemcpy(dbox, box.data(), sizeof(int32_t) * B, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ditem, item, sizeof(int32_t) * I, cudaMemcpyHostToDevice));
-    if (!info.vox.empty()) CK(cudaMemcpy(dvox, info.vox.data(), sizeof(int4) * info.vox.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(dod, &od, sizeof(od), cudaMemcpyHostToDevice));
-    CK(cudaMemset(dfirst, 0xff, sizeof(unsigned long long)));
-    int blocks = std::max(1, std::min(1024, (od.nvox + 255) / 256));
-    // the box is a small tray: position relative to the box origin
-    k_place_check<<<blocks, 256>>>(dod, dbox, bx, by, bz, px - i0, py - j0, pz - k0, dfirst);
+    memcpy(h + oi, item, sizeof(int32_t) * I);
+    cudaStream_t st = 0;
+    CK(cudaMemcpyAsync(d, h, oi + sizeof(int32_t) * I, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(d_out, h, 16, cudaMemcpyHostToDevice, st));
+    pdl(k_place_box, grid1d(B), 256, 0, st)((const int32_t*)(d + 16), bx, by, bz, (const int32_t*)(d + oi), ey, ez,
+                                            i0 - px, j0 - py, k0 - pz, item_id, (int32_t*)(d_out + 16),
+                                            (unsigned long long*)d_out);
     CKL();
-    unsigned long long first = 0;
-    CK(cudaMemcpy(&first, dfirst, sizeof(first), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(h, d_out, 16 + nb, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    const unsigned long long first = *(unsigned long long*)h;
     if (first != 0xffffffffffffffffULL) {
-        int k = (int)(first % bz), j = (int)((first / bz) % by), i = (int)(first / ((size_t)by * bz));
-        i += i0; j += j0; k += k0;
         // row-major order of the box agrees with the tray's row-major order
+        const int k = k0 + (int)(first % bz), j = j0 + (int)((first / bz) % by), i = i0 + (int)(first / ((size_t)by * bz));
         if (overlap_ijk) { overlap_ijk[0] = i; overlap_ijk[1] = j; overlap_ijk[2] = k; }
-        if (out_tray != tray) memcpy(out_tray, tray, sizeof(int32_t) * V);
         return fail(PSB_ERR_OVERLAP,
                     "(place_in_tray): Item to be placed intersects with contents of tray at position (%d, %d, %d)", i,
                     j, k);
     }
-    k_place_write<<<blocks, 256>>>(dod, dbox, bx, by, bz, px - i0, py - j0, pz - k0, item_id);
-    CKL();
-    CK(cudaMemcpy(box.data(), dbox, sizeof(int32_t) * B, cudaMemcpyDeviceToHost));
     for (int i = 0; i < bx; ++i)
         for (int j = 0; j < by; ++j)
             memcpy(&out_tray[((size_t)(i0 + i) * ny + (j0 + j)) * nz + k0], &box[((size_t)i * by + j) * bz],
@@ -2969,12 +2974,56 @@ int psb_tray_search(psb_tray* t, const int32_t* const* items, const int32_t* dim
     psb_result none{-1, -1, -1, 0, 0.0, -1, 0, 0, 0.f};
     *out = none;
     if (n == 0) return PSB_OK;
-    std::vector<OrientDesc> ods;
-    TRY(stage_arrays(t, items, dims, n, &ods));
+    const int mode = mode_flags & 0xf;
+    const bool interlock = (mode_flags & PSB_FLAG_INTERLOCK) != 0;
+    if (!per_orient && t->occ == 0 && t->phi_own) {
+        // an empty tray and its own distance field: every translation is free
+        // and the field constant, so the first array that fits wins at the
+        // origin (see k_bound_first)
+        bool bad = false;
+        for (int o = 0; o < n && !bad; ++o)
+            bad = !items[o] || dims[3 * o] <= 0 || dims[3 * o + 1] <= 0 || dims[3 * o + 2] <= 0 ||
+                  has_negative(items[o], (size_t)dims[3 * o] * dims[3 * o + 1] * dims[3 * o + 2]);
+        for (int o = 0; o < n && !bad; ++o) {
+            const int32_t* d = dims + 3 * o;
+            if (d[0] > t->nx || d[1] > t->ny || d[2] > t->nz) continue;
+            double sum = 0.0;
+            const size_t m = (size_t)d[0] * d[1] * d[2];
+            for (size_t i = 0; i < m; ++i) sum += (double)items[o][i];
+            const double s = sum * (double)(t->nx + t->ny + t->nz + 10);
+            if (!(s < 9007199254740992.0) || s >= (mode == PSB_MODE_SCAN ? 1e9 : 1e29)) break;
+            *out = psb_result{0, 0, 0, 1, s, o, PSB_DIAG_DIRECT, 0, 0.f};
+            return PSB_OK;
+        }
+    }
+    TRY(stage_arrays(t, items, dims, n));
+    if (!per_orient && t->bound_usable() && (unsigned long long)n * t->V < 0xffffffffULL) {
+        TRY(t->ensure_bound(n));
+        TRY(t->bound_prep(t->d_xod, n, 1, mode));
+        TRY(t->bound_search(t->d_xod, n, 0, t->nx, mode, interlock, 0, &t->d_reply->dec));
+        CK(cudaMemcpyAsync(t->h_reply, t->d_reply, sizeof(BoundReply), cudaMemcpyDeviceToHost, t->st));
+        CK(cudaStreamSynchronize(t->st));
+        const BoundReply& r = *t->h_reply;
+        const int neg = r.neg;
+        if (neg != INT_MAX || r.st.halt) {
+            TRY(t->bound_reset());
+            if (neg != INT_MAX) return fail(PSB_ERR_ARG, "orientation %d holds negative values", neg);
+        } else {
+            if (r.dec.found)
+                *out = psb_result{r.dec.x, r.dec.y, r.dec.z, 1, r.dec.score, r.dec.orientation, r.dec.diag, r.dec.ncand,
+                                  r.dec.err_ratio};
+            return PSB_OK;
+        }
+    }
+    std::vector<OrientDesc> ods(n);
+    int neg = INT_MAX;
+    CK(cudaMemcpyAsync(ods.data(), t->d_xod, sizeof(OrientDesc) * n, cudaMemcpyDeviceToHost, t->st));
+    CK(cudaMemcpyAsync(&neg, &t->d_reply->neg, sizeof(neg), cudaMemcpyDeviceToHost, t->st));
+    CK(cudaStreamSynchronize(t->st));
+    if (neg != INT_MAX) return fail(PSB_ERR_ARG, "orientation %d holds negative values", neg);
     std::vector<ResultDev> res;
-    int mode = mode_flags & 0xf;
     // every orientation's own result is exact only without the lazy flood fill
-    TRY(t->search(ods, mode, (mode_flags & PSB_FLAG_INTERLOCK) != 0, &res, per_orient == nullptr));
+    TRY(t->search(ods, mode, interlock, &res, per_orient == nullptr));
     double best = 1e300;
     for (int o = 0; o < n; ++o) {
         psb_result r;
@@ -2993,10 +3042,10 @@ int psb_tray_place(psb_tray* t, const int32_t* item, int ex, int ey, int ez, int
     CK(cudaSetDevice(t->dev));
     const int32_t* items[1] = {item};
     int32_t dims[3] = {ex, ey, ez};
-    std::vector<OrientDesc> ods;
-    TRY(stage_arrays(t, items, dims, 1, &ods));
-    TRY(t->place(ods[0], px, py, pz, item_id, nullptr));
-    t->occ += (size_t)std::max(0, ods[0].nvox);
+    int nvox = 0;
+    TRY(stage_arrays(t, items, dims, 1));
+    TRY(t->place(px, py, pz, item_id, nullptr, &nvox));
+    t->occ += (size_t)nvox;
     return PSB_OK;
 }
 
@@ -3316,7 +3365,7 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
             const psb_tray::StagedDev& sd = t->sdev[it];
             for (int o = 0; o < n_orient; ++o) {
                 OrientDesc& od = all[(size_t)it * n_orient + o];
-                t->describe(t->staged[it], orient_maps + 6 * o, orient_maps + 6 * o + 3, sd.item, nullptr, sd.runs,
+                t->describe(t->staged[it], orient_maps + 6 * o, orient_maps + 6 * o + 3, sd.item, sd.runs,
                             &od);
                 // orientation sharding: the other ranks' orientations are not searched here
                 if (opt.world > 1 && o % opt.world != opt.rank) od.skip = 1;
@@ -3601,10 +3650,10 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
                                     interlock != 0, it + k, t->d_dec + it + k));
                 TRY(t->bound_place(d_odb + (size_t)k * n_orient));
             }
-            CK(cudaMemcpyAsync(t->h_bstate, t->d_bstate, sizeof(BoundState), cudaMemcpyDeviceToHost, t->st));
+            CK(cudaMemcpyAsync(&t->h_reply->st, t->d_bstate, sizeof(BoundState), cudaMemcpyDeviceToHost, t->st));
             CK(cudaStreamSynchronize(t->st));
-            const bool halted = t->h_bstate->halt != 0;
-            const int stop = halted ? t->h_bstate->halt_item : it + m;
+            const bool halted = t->h_reply->st.halt != 0;
+            const int stop = halted ? t->h_reply->st.halt_item : it + m;
             for (; it < stop; ++it) occ_est += (size_t)t->staged[it].nvox;
             if (!halted) {
                 chunk = std::min(2 * chunk, kChunkMax);

@@ -892,42 +892,6 @@ __global__ void k_any_negative(const int32_t* __restrict__ v, size_t n, unsigned
         if (v[i] < 0) { atomicOr(flag, 1u); return; }
 }
 
-// ---------------------------------------------------------------------------
-// placement (packing.cpp:773-788)
-// ---------------------------------------------------------------------------
-// first tray cell (row-major) where an item voxel > 0 meets a tray voxel > 0
-__global__ void k_place_check(const OrientDesc* __restrict__ od_p, const int32_t* __restrict__ tray, int nx, int ny,
-                              int nz, int px, int py, int pz, unsigned long long* first) {
-    pdl_enter();
-    const OrientDesc od = *od_p;
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < od.nvox; v += gridDim.x * blockDim.x) {
-        int4 q = od.vox[v];
-        if (q.w <= 0) continue;
-        int oc[3];
-        orient_voxel(od, q.x, q.y, q.z, oc);
-        int i = px + oc[0], j = py + oc[1], k = pz + oc[2];
-        if (i < 0 || j < 0 || k < 0 || i >= nx || j >= ny || k >= nz) continue;
-        size_t t = ((size_t)i * ny + j) * nz + k;
-        if (tray[t] > 0) atomicMin(first, (unsigned long long)t);
-    }
-}
-
-__global__ void k_place_write(const OrientDesc* __restrict__ od_p, int32_t* __restrict__ tray, int nx, int ny, int nz,
-                              int px, int py, int pz, int32_t id) {
-    pdl_enter();
-    const OrientDesc od = *od_p;
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < od.nvox; v += gridDim.x * blockDim.x) {
-        int4 q = od.vox[v];
-        if (q.w <= 0) continue;
-        int oc[3];
-        orient_voxel(od, q.x, q.y, q.z, oc);
-        int i = px + oc[0], j = py + oc[1], k = pz + oc[2];
-        if (i < 0 || j < 0 || k < 0 || i >= nx || j >= ny || k >= nz) continue;
-        size_t t = ((size_t)i * ny + j) * nz + k;
-        if (tray[t] == 0) tray[t] = id;
-    }
-}
-
 // collision_grid post-pass: out-of-tray positions raised to max(c, 1)
 __global__ void k_oob_raise(int32_t* __restrict__ c, int nx, int ny, int nz, int hx, int hy, int hz) {
     pdl_enter();

@@ -91,3 +91,70 @@ def test_bound_search_trays_at_once(gpu_core):
         one = BinPacker(dims, num_orientations=6, interlocking_free=True).pack_voxels(items)
         assert _key(r) == _key(one)
         np.testing.assert_array_equal(r.tray, one.tray)
+
+
+def _search(core, tray, phi, items, flags):
+    core.gpu_tray_init(tray, phi)
+    try:
+        return core.search_detail(items, flags, per_orientation=False)["best"]
+    finally:
+        core.gpu_tray_cleanup()
+
+
+@pytest.mark.parametrize("flags", [0, 1, 1 | 0x10])   # scan, block, block with interlocking
+@pytest.mark.parametrize("shape", [(9, 7, 8), (33, 31, 32), (40, 65, 33), (36, 40, 129), (64, 64, 64)])
+def test_bound_search_calls(gpu_core, shape, flags):
+    """One synchronous search of explicit arrays, analysed on the device,
+    against the transforms: random trays, sparse and weighted items, an array
+    larger than the tray, distance fields of the tray, of another tray and
+    partly negative ones."""
+    rng = np.random.default_rng(sum(shape) + flags)
+    for trial in range(4):
+        tray = np.zeros(shape, np.int32)
+        for b in range([3, 12, 40, 6][trial]):
+            e = [int(rng.integers(1, max(2, s // 4))) for s in shape]
+            o = [int(rng.integers(0, s - ee + 1)) for s, ee in zip(shape, e)]
+            tray[o[0]:o[0] + e[0], o[1]:o[1] + e[1], o[2]:o[2] + e[2]] = 1 + b % 5
+        items = []
+        for k in range(5):
+            e = [int(rng.integers(1, max(2, s // 3))) for s in shape]
+            it = (rng.random(e) < [1.0, 0.6, 0.1, 0.9, 0.5][k]).astype(np.int32) * int(rng.integers(1, 4))
+            it.flat[0] = 1
+            items.append(it)
+        items.insert(2, np.ones((shape[0] + 1, 2, 2), np.int32))
+        phi = gpu_core.calculate_distance(tray)
+        for p in (phi, gpu_core.calculate_distance(np.roll(tray, 3, 1)), phi // 2 - 4):
+            got = _search(gpu_core, tray, p, items, flags)
+            gpu_core.set_cand_filter(False)
+            try:
+                want = _search(gpu_core, tray, p, items, flags)
+            finally:
+                gpu_core.set_cand_filter(True)
+            assert got == want
+
+
+def test_bound_search_calls_errors_and_empties(gpu_core):
+    tray = np.zeros((20, 18, 16), np.int32)
+    tray[:6, :6, :6] = 1
+    phi = gpu_core.calculate_distance(tray)
+    bad = np.ones((3, 3, 3), np.int32)
+    bad[1, 1, 1] = -2
+    ok = np.ones((2, 3, 4), np.int32)
+    gpu_core.gpu_tray_init(tray, phi)
+    with pytest.raises(RuntimeError, match="orientation 1 holds negative"):
+        gpu_core.search_detail([ok, bad], 1, per_orientation=False)
+    a = gpu_core.search_detail([ok], 1, per_orientation=False)["best"]   # the context stays usable
+    assert a[1]
+    gpu_core.gpu_tray_cleanup()
+    # an empty tray: the first array that fits, at the origin
+    empty = np.zeros((20, 18, 16), np.int32)
+    for items in ([np.ones((30, 2, 2), np.int32), ok], [np.ones((30, 2, 2), np.int32)], [np.zeros((2, 2, 2), np.int32)]):
+        pos, found, score = gpu_core.fft_search_placement(items[-1], empty)
+        gpu_core.set_cand_filter(False)
+        try:
+            gpu_core.gpu_tray_init(empty, gpu_core.calculate_distance(empty))
+            want = gpu_core.search_detail([items[-1]], 0, per_orientation=False)["best"]
+        finally:
+            gpu_core.set_cand_filter(True)
+            gpu_core.gpu_tray_cleanup()
+        assert (tuple(pos), found) == (tuple(want[0]), want[1]) and (not found or score == want[2])
