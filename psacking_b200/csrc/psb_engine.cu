@@ -28,6 +28,7 @@
 #endif
 
 #include "../../include/psb200.h"
+#include "psb_host.cuh"
 #include "psb_kernels2.cuh"
 #include "psb_kernels3.cuh"
 #include "psb_kernels4.cuh"
@@ -717,27 +718,6 @@ bool has_negative(const int32_t* a, size_t n) {
     return false;
 }
 
-// fn(begin, end) over [0, n) in chunks, on up to all host cores (the calling
-// thread takes part); a single chunk runs inline.
-template <typename F>
-void parallel_chunks(size_t n, size_t chunk, F fn) {
-    const size_t nchunks = (n + chunk - 1) / chunk;
-    const int nthr = (int)std::min<size_t>(nchunks, std::max(1u, std::thread::hardware_concurrency()));
-    if (nthr <= 1) {
-        if (n) fn((size_t)0, n);
-        return;
-    }
-    std::atomic<size_t> next(0);
-    auto work = [&]() {
-        for (size_t c = next.fetch_add(1); c < nchunks; c = next.fetch_add(1))
-            fn(c * chunk, std::min(n, (c + 1) * chunk));
-    };
-    std::vector<std::thread> pool;
-    for (int w = 1; w < nthr; ++w) pool.emplace_back(work);
-    work();
-    for (auto& th : pool) th.join();
-}
-
 // ---------------------------------------------------------------------------
 // host-side item analysis
 // ---------------------------------------------------------------------------
@@ -1417,7 +1397,7 @@ struct psb_tray {
         // negative values and occupied cells, one pass over the host cores
         std::atomic<int> neg(0), one(0);
         std::atomic<size_t> nocc(0);
-        parallel_chunks(V, (size_t)1 << 20, [&](size_t b, size_t e) {
+        parallel_chunks(V, (size_t)1 << 19, [&](size_t b, size_t e) {
             size_t c = 0;
             int ng = 0, n1 = 0;
             for (size_t i = b; i < e; ++i) {
@@ -1431,9 +1411,9 @@ struct psb_tray {
         });
         if (neg) return fail(PSB_ERR_ARG, "tray holds negative values; item ids must be >= 0");
         occ = nocc;
-        CK(cudaMemcpyAsync(d_tray, tray, sizeof(int32_t) * V, cudaMemcpyHostToDevice, st));
+        CK(upload_async(d_tray, tray, sizeof(int32_t) * V, st));
         if (phi) {
-            CK(cudaMemcpyAsync(d_phi, phi, sizeof(int32_t) * V, cudaMemcpyHostToDevice, st));
+            CK(upload_async(d_phi, phi, sizeof(int32_t) * V, st));
         } else {
             TRY(distance_on_device(d_tray, d_phi, nx, ny, nz, st));
         }
@@ -2231,7 +2211,7 @@ int stage_arrays(psb_tray* t, const int32_t* const* items, const int32_t* dims, 
         const int32_t* d = dims + 3 * o;
         if (!items[o] || d[0] <= 0 || d[1] <= 0 || d[2] <= 0)
             return fail(PSB_ERR_ARG, "orientation %d: bad array (dims %d,%d,%d)", o, d[0], d[1], d[2]);
-        cells += (size_t)d[0] * d[1] * d[2];
+        cells += ((size_t)d[0] * d[1] * d[2] + 3) / 4 * 4;   // each array on a 16-byte boundary
     }
     const size_t ov = up(sizeof(ItemArr) * n), in = ov + up(sizeof(int32_t) * cells);
     const size_t os = in, od = os + up(sizeof(ItemSums) * n), op = od + up(sizeof(OrientDesc) * n);
@@ -2254,10 +2234,14 @@ int stage_arrays(psb_tray* t, const int32_t* const* items, const int32_t* dims, 
         tab[o].off = tab[o].roff = (long long)off;
         for (int a = 0; a < 3; ++a) tab[o].d[a] = d[a];
         tab[o].skip = d[0] > t->nx || d[1] > t->ny || d[2] > t->nz;
-        memcpy(h + ov + sizeof(int32_t) * off, items[o], sizeof(int32_t) * m);
-        off += m;
+        off += (m + 3) / 4 * 4;
         maxcol = std::max(maxcol, d[0] * d[1]);
     }
+    parallel_chunks((size_t)n, std::max((size_t)1, n * ((size_t)1 << 17) / cells), [&](size_t b, size_t e) {
+        for (size_t o = b; o < e; ++o)
+            stream_copy(h + ov + sizeof(int32_t) * tab[o].off, items[o],
+                        sizeof(int32_t) * (size_t)tab[o].d[0] * tab[o].d[1] * tab[o].d[2]);
+    });
     CK(cudaMemcpyAsync(t->d_x, h, in, cudaMemcpyHostToDevice, t->st));
     t->d_xsums = (ItemSums*)(t->d_x + os);
     t->d_xod = (OrientDesc*)(t->d_x + od);
@@ -2325,8 +2309,8 @@ int linear_transform_product(const int32_t* a, const int32_t* b, int nx, int ny,
     RzDesc* d_rz = (RzDesc*)take(sizeof(RzDesc) * 2);
     MidDesc* d_mid = (MidDesc*)take(sizeof(MidDesc) * 2);
     cudaStream_t st = 0;
-    CK(cudaMemcpyAsync(da, a, sizeof(int32_t) * V, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(db, b, sizeof(int32_t) * V, cudaMemcpyHostToDevice, st));
+    CK(upload_async(da, a, sizeof(int32_t) * V, st));
+    CK(upload_async(db, b, sizeof(int32_t) * V, st));
     RzDesc ra{SRC_GRID_RAW, da, nx, ny, nz, 0, -1, nullptr};
     RzDesc rb{SRC_GRID_RAW, db, nx, ny, nz, 0, -1, nullptr};
     TRY(forward3(g, ra, W1, W2, Sa, d_rz, d_mid, st));
@@ -2339,8 +2323,7 @@ int linear_transform_product(const int32_t* a, const int32_t* b, int nx, int ny,
     CKL();
     CK(cudaStreamSynchronize(st));
     TRY(inverse3_int(g, Sa, W1, W2, da, d_mid, st));
-    CK(cudaMemcpyAsync(out, da, sizeof(int32_t) * V, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    CK(download(out, da, sizeof(int32_t) * V, st));
     return PSB_OK;
 }
 
@@ -2756,9 +2739,9 @@ int psb_calculate_distance(const int32_t* grid, int nx, int ny, int nz, int32_t*
     TRY(arena(sizeof(int32_t) * 2 * V + 512, &base));
     int32_t* dg = (int32_t*)base;
     int32_t* dd = dg + ((V + 63) / 64) * 64;
-    CK(cudaMemcpy(dg, grid, sizeof(int32_t) * V, cudaMemcpyHostToDevice));
+    CK(upload_async(dg, grid, sizeof(int32_t) * V, 0));
     TRY(distance_on_device(dg, dd, nx, ny, nz, 0));
-    CK(cudaMemcpy(out, dd, sizeof(int32_t) * V, cudaMemcpyDeviceToHost));
+    CK(download(out, dd, sizeof(int32_t) * V, 0));
     return PSB_OK;
 }
 
@@ -2858,7 +2841,7 @@ int psb_place_in_tray(const int32_t* item, int ex, int ey, int ez, const int32_t
     if (!out_tray) return fail(PSB_ERR_ARG, "place_in_tray: null output");
     TRY(ensure_device());
     size_t V = (size_t)nx * ny * nz;
-    if (out_tray != tray) memcpy(out_tray, tray, sizeof(int32_t) * V);
+    if (out_tray != tray) parallel_copy(out_tray, tray, sizeof(int32_t) * V);
     // the clipped box of tray cells the item covers
     int i0 = std::max(px, 0), j0 = std::max(py, 0), k0 = std::max(pz, 0);
     int i1 = std::min(nx, px + ex), j1 = std::min(ny, py + ey), k1 = std::min(nz, pz + ez);
@@ -2936,8 +2919,8 @@ int psb_tray_set(psb_tray* t, const int32_t* tray, const int32_t* phi) {
 int psb_tray_get(psb_tray* t, int32_t* tray, int32_t* phi) {
     if (!t) return fail(PSB_ERR_ARG, "null tray");
     CK(cudaSetDevice(t->dev));
-    if (tray) CK(cudaMemcpyAsync(tray, t->d_tray, sizeof(int32_t) * t->V, cudaMemcpyDeviceToHost, t->st));
-    if (phi) CK(cudaMemcpyAsync(phi, t->d_phi, sizeof(int32_t) * t->V, cudaMemcpyDeviceToHost, t->st));
+    if (tray) CK(download(tray, t->d_tray, sizeof(int32_t) * t->V, t->st));
+    if (phi) CK(download(phi, t->d_phi, sizeof(int32_t) * t->V, t->st));
     CK(cudaStreamSynchronize(t->st));
     return PSB_OK;
 }
@@ -3098,7 +3081,7 @@ int stage_upload(psb_tray* t, const int32_t* const* items, int i0, int i1, int p
         const ItemInfo& inf = t->staged[it];
         for (int a = 0; a < 3; ++a) n4 += inf.runs[a].size();
         n4 += inf.samp.size();
-        n1 += (size_t)inf.dims[0] * inf.dims[1] * inf.dims[2];
+        n1 += ((size_t)inf.dims[0] * inf.dims[1] * inf.dims[2] + 3) / 4 * 4;   // 16-byte boundaries
     }
     const size_t bytes = sizeof(int4) * n4 + sizeof(int32_t) * n1;
     if (bytes > t->part_cap[part]) {
@@ -3123,7 +3106,7 @@ int stage_upload(psb_tray* t, const int32_t* const* items, int i0, int i1, int p
         o1[it - i0] = a1;
         for (int a = 0; a < 3; ++a) a4 += inf.runs[a].size();
         a4 += inf.samp.size();
-        a1 += (size_t)inf.dims[0] * inf.dims[1] * inf.dims[2];
+        a1 += ((size_t)inf.dims[0] * inf.dims[1] * inf.dims[2] + 3) / 4 * 4;
     }
     int4* h4 = (int4*)t->h_part[part];
     int32_t* h1 = (int32_t*)(h4 + n4);
@@ -3136,14 +3119,14 @@ int stage_upload(psb_tray* t, const int32_t* const* items, int i0, int i1, int p
             psb_tray::StagedDev& sd = t->sdev[it];
             size_t q = o4[k];
             for (int a = 0; a < 3; ++a) {
-                if (!inf.runs[a].empty()) memcpy(h4 + q, inf.runs[a].data(), sizeof(int4) * inf.runs[a].size());
+                if (!inf.runs[a].empty()) stream_copy(h4 + q, inf.runs[a].data(), sizeof(int4) * inf.runs[a].size());
                 sd.runs[a] = d4 + q;
                 q += inf.runs[a].size();
             }
-            if (!inf.samp.empty()) memcpy(h4 + q, inf.samp.data(), sizeof(int4) * inf.samp.size());
+            if (!inf.samp.empty()) stream_copy(h4 + q, inf.samp.data(), sizeof(int4) * inf.samp.size());
             sd.samp = d4 + q;
             const size_t m = (size_t)inf.dims[0] * inf.dims[1] * inf.dims[2];
-            memcpy(h1 + o1[k], items[it], sizeof(int32_t) * m);
+            stream_copy(h1 + o1[k], items[it], sizeof(int32_t) * m);
             sd.item = d1 + o1[k];
         }
     });
@@ -4073,8 +4056,7 @@ int psb_voxelize_mesh(const float* tris, int ntri, int resolution, int32_t* out,
                                                                           h.box[2], td[0], td[1], td[2], d_out);
     }
     CKL();
-    CK(cudaMemcpyAsync(out, d_out, sizeof(int32_t) * T, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    CK(download(out, d_out, sizeof(int32_t) * T, st));
     for (int a = 0; a < 3; ++a) dims_out[a] = td[a];
     return PSB_OK;
 }
