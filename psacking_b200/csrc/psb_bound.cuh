@@ -20,11 +20,11 @@
 // winner's score; the transforms this replaces evaluated all of them.
 //
 // Per item:
-//   1. k_bound_find (SEED), on a lattice of every fourth column in x and y: the
+//   1. k_bound_seed, on a lattice of every fourth column in x and y: the
 //      bit-parallel sample filter (psb_filter.cuh) leaves the translations that
 //      may be free, each warp checks and scores its lowest-bound survivor
 //      exactly, and the item's best score so far comes down;
-//      k_bound_find (LIST), on every column: the z range is cut where the
+//      k_bound_find, on every column: the z range is cut where the
 //      bounds exceed the best score, the filter runs on what is left, and the
 //      survivors are listed;
 //   2. k_bound_score: the listed translations whose bound still does not
@@ -44,7 +44,7 @@
 #pragma once
 #include "psb_filter.cuh"
 
-#define PSB_BSTEP 4             // seed lattice, in x and y
+#define PSB_BSTEP 4             // seed lattice in x
 #define PSB_BCAP (1 << 16)      // listed translations per item
 #define PSB_BFREE 8192          // free translations the shared-memory flood takes
 #define PSB_BBATCH 16           // sample buckets are padded to whole batches of this many
@@ -169,7 +169,7 @@ __global__ void k_bound_over(const int32_t* __restrict__ phi, int nx, int ny, in
 // ---------------------------------------------------------------------------
 // doubles (every value an integer below 2^53): [0] W, [1..8] s.M - W h(s) per
 // sign vector, [9..11] the numbers of x, y, z translations (x: 0 when the
-// orientation is skipped), then X[nx], Y[ny], Z[nz], and the smallest bounded score at z or
+// orientation is skipped), [12..14] its runs (RunHead), then X[nx], Y[ny], Z[nz], and the smallest bounded score at z or
 // above of the separable bound's z part (F0[nz]) and of W z (F1[nz]), which
 // grow with z, so the last z worth testing in a column is a binary search.
 struct BoundTab {
@@ -191,6 +191,57 @@ __device__ __forceinline__ BoundTab bound_tab(const double* tab, const ScorePara
     return b;
 }
 
+// Orientations that turn the item into the same array as an earlier one: a
+// solid of revolution has 3 different ones of 24, a superellipsoid 6, an
+// extruded profile 6 to 12.  Such an orientation's results equal the earlier
+// one's, which wins the tie, so it is skipped.  The arrays are compared voxel by
+// voxel (a pair that differs mostly does so within the first thousand).
+// grid: (n, items), block 256
+__global__ void __launch_bounds__(256)
+k_bound_dedupe(OrientDesc* __restrict__ od_all, int n) {
+    pdl_enter();
+    OrientDesc* od = od_all + (size_t)blockIdx.y * n;
+    const int o = blockIdx.x;
+    const OrientDesc& d = od[o];
+    if (d.skip) return;
+    const int e0 = d.e[0], e1 = d.e[1], e2 = d.e[2], m = e0 * e1 * e2;
+    // source index of oriented (i, j, k): at + i si + j sj + k sk
+    auto strides = [](const OrientDesc& q, int* st) {
+        const int b[3] = {q.b[1] * q.b[2], q.b[2], 1};
+        st[3] = 0;
+        for (int a = 0; a < 3; ++a) {
+            const int s = q.src_axis[a] == 0 ? b[0] : (q.src_axis[a] == 1 ? b[1] : b[2]);
+            st[a] = q.flip[a] ? -s : s;
+            if (q.flip[a]) st[3] += (q.e[a] - 1) * s;
+        }
+    };
+    int s1[4], s2[4];
+    strides(d, s1);
+    const int32_t* v = d.item;
+    for (int p = 0; p < o; ++p) {
+        const OrientDesc& q = od[p];
+        if (q.e[0] != e0 || q.e[1] != e1 || q.e[2] != e2) continue;
+        strides(q, s2);
+        bool same = true;
+        for (int t0 = 0; t0 < m && same; t0 += 1024) {
+            bool diff = false;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int t = t0 + 256 * u + threadIdx.x;
+                if (t >= m) continue;
+                const int k = t % e2, j = t / e2 % e1, i = t / (e2 * e1);
+                diff |= __ldg(&v[s1[3] + i * s1[0] + j * s1[1] + k * s1[2]]) !=
+                        __ldg(&v[s2[3] + i * s2[0] + j * s2[1] + k * s2[2]]);
+            }
+            same = !__syncthreads_or(diff);
+        }
+        if (same) {
+            if (threadIdx.x == 0) od[o].skip = 1;
+            return;
+        }
+    }
+}
+
 // The tables, and the shift-sorted filter samples (as k_cand_prep), of every
 // orientation of the items i0 .. i0 + gridDim.y - 1: they depend on the items
 // and the sources only, so one launch serves a queue of items.
@@ -209,6 +260,14 @@ k_bound_prep(const OrientDesc* __restrict__ od_all, int n, int i0, const BoundGe
     double* T = tab + (size_t)slot * tstride;
     if (tid < 3) T[9 + tid] = od.skip ? 0.0 : (double)od.valid[tid];
     if (od.skip) return;
+    if (tid == 3) {
+        const bool ax = od.src_axis[0] == (od.src_axis[2] == 0 ? 1 : 0);   // the tray's x comes from a run's q.x
+        T[12] = (double)od.nruns;
+        T[13] = __longlong_as_double((long long)od.runs);
+        T[14] = __longlong_as_double((long long)od.e[0] | (long long)od.e[1] << 12 | (long long)od.e[2] << 24 |
+                                     (long long)(od.flip[0] != 0) << 36 | (long long)(od.flip[1] != 0) << 37 |
+                                     (long long)(od.flip[2] != 0) << 38 | (long long)ax << 39);
+    }
     // marginals of the oriented item along x, y and z (z by differences)
     for (int i = tid; i < 3 * (PSB_MAX_FFT + 1); i += 256) (&hm[0][0])[i] = 0ULL;
     __syncthreads();
@@ -333,6 +392,20 @@ __device__ __forceinline__ bool run_blocked(const uint32_t* __restrict__ col, in
     return bad != 0u;
 }
 
+// An orientation's runs, from its table's header (entry l in lane l), so that
+// a check starts without another round trip for the descriptor.
+struct RunHead {
+    const int4* runs;
+    int nr;
+    long long code;             // extents, flips and the axis of q.x
+};
+__device__ __forceinline__ RunHead run_head(double h) {
+    RunHead r;
+    r.nr = (int)__shfl_sync(0xffffffffu, h, 12);
+    r.runs = (const int4*)__double_as_longlong(__shfl_sync(0xffffffffu, h, 13));
+    r.code = __double_as_longlong(__shfl_sync(0xffffffffu, h, 14));
+    return r;
+}
 // The map of an item's runs to tray columns and z ranges at a translation:
 // orient_run, with everything that does not depend on the run taken out.
 struct RunMap {
@@ -341,17 +414,17 @@ struct RunMap {
     int ez;                     // flipped: c0 = ez - r1, c1 = ez - r0
     bool flip;
 };
-__device__ __forceinline__ RunMap run_map(const OrientDesc& d, int ny, int x, int y, int z) {
-    const int lo = d.src_axis[2] == 0 ? 1 : 0;   // q.x runs along this source axis
-    const bool ax = d.src_axis[0] == lo;         // the tray's x comes from q.x
-    const int sa = d.flip[0] ? -ny : ny, sb = d.flip[1] ? -1 : 1;
+__device__ __forceinline__ RunMap run_map(const RunHead& h, int ny, int x, int y, int z) {
+    const int e0 = (int)(h.code & 4095), e1 = (int)(h.code >> 12 & 4095);
+    const bool f0 = h.code >> 36 & 1, f1 = h.code >> 37 & 1, ax = h.code >> 39 & 1;
+    const int sa = f0 ? -ny : ny, sb = f1 ? -1 : 1;
     RunMap m;
     m.mx = ax ? sa : sb;
     m.my = ax ? sb : sa;
-    m.col = (x + (d.flip[0] ? d.e[0] - 1 : 0)) * ny + y + (d.flip[1] ? d.e[1] - 1 : 0);
+    m.col = (x + (f0 ? e0 - 1 : 0)) * ny + y + (f1 ? e1 - 1 : 0);
     m.z = z;
-    m.ez = d.e[2] - 1;
-    m.flip = d.flip[2] != 0;
+    m.ez = (int)(h.code >> 24 & 4095) - 1;
+    m.flip = h.code >> 38 & 1;
     return m;
 }
 __device__ __forceinline__ int run_at(const RunMap& m, int4 q, int* z0, int* z1) {
@@ -364,31 +437,44 @@ __device__ __forceinline__ int run_at(const RunMap& m, int4 q, int* z0, int* z1)
 // Collision-free?  (Item values are positive: negative ones are refused.)
 // Each step checks 128 runs spread over the whole item, so a blocked
 // translation is mostly found out in the first one.
-__device__ __forceinline__ bool bound_free(const OrientDesc& od, const uint32_t* __restrict__ T, int tw, int ny, int x,
+__device__ __forceinline__ bool bound_free(const RunHead& od, const uint32_t* __restrict__ T, int tw, int ny, int x,
                                            int y, int z) {
-    const int lane = threadIdx.x & 31, nr = od.nruns, steps = (nr + 127) / 128;
+    const int lane = threadIdx.x & 31, nr = od.nr, steps = (nr + 127) / 128;
     const int4* runs = od.runs;
     const RunMap rm = run_map(od, ny, x, y, z);
+    int4 q[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int r = steps * (32 * u + lane);
+        q[u] = r < nr ? __ldg(&runs[r]) : make_int4(0, 0, 0, 0);   // values are positive: w = 0 marks none
+    }
     for (int i = 0; i < steps; ++i) {
+        int4 next[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int r = i + 1 + steps * (32 * u + lane);
+            next[u] = i + 1 < steps && r < nr ? __ldg(&runs[r]) : make_int4(0, 0, 0, 0);
+        }
         bool hit = false;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int r = i + steps * (32 * u + lane);
-            if (r >= nr) continue;
+            if (q[u].w == 0) continue;
             int z0, z1;
-            const int col = run_at(rm, __ldg(&runs[r]), &z0, &z1);
+            const int col = run_at(rm, q[u], &z0, &z1);
             hit = run_blocked(T + (size_t)col * tw, z0, z1) || hit;
         }
         if (__any_sync(0xffffffffu, hit)) return false;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) q[u] = next[u];
     }
     return true;
 }
 
 // Exact proximity (every lane returns it), from the distance field's prefix
 // sums along z.
-__device__ __forceinline__ long long bound_prox(const OrientDesc& od, const int32_t* __restrict__ pphi, int ny, int nz,
+__device__ __forceinline__ long long bound_prox(const RunHead& od, const int32_t* __restrict__ pphi, int ny, int nz,
                                                 int x, int y, int z) {
-    const int lane = threadIdx.x & 31, nr = od.nruns;
+    const int lane = threadIdx.x & 31, nr = od.nr;
     const int4* runs = od.runs;
     const RunMap rm = run_map(od, ny, x, y, z);
     long long acc = 0;
@@ -414,6 +500,11 @@ __device__ __forceinline__ void bound_octants(const BoundTab& b, int x, int y, d
     const double dx = b.W * (double)x, dy = b.W * (double)y;
     *gp = fmax(fmax(dx + dy + b.c[0], -dx + dy + b.c[1]), fmax(dx - dy + b.c[2], -dx - dy + b.c[3]));
     *gm = fmax(fmax(dx + dy + b.c[4], -dx + dy + b.c[5]), fmax(dx - dy + b.c[6], -dx - dy + b.c[7]));
+}
+
+// the runs of orientation o (a warp-wide load of its header)
+__device__ __forceinline__ RunHead run_head_of(const double* __restrict__ tab, long long tstride, int o) {
+    return run_head(tab[(size_t)o * tstride + min((int)(threadIdx.x & 31), 14)]);
 }
 
 // the bounded score of cell z of a column (A = X + Y, octant parts gp, gm)
@@ -455,9 +546,10 @@ struct BoundArgs {
 // live word (128 samples by themselves are most of a warp's instructions: with
 // all words, tests per sample and samples handed round by shuffles, 4.3 M per
 // seed pass at 128^3 and 24 orientations, a warp's chain 38k cycles long).
+// Batches first, first + step, ... of each bucket are taken.
 template <int NQ, int WA, int BATCH>
 __device__ __forceinline__ void bound_filter(const uint4* __restrict__ col, const int2* __restrict__ fs, int fb,
-                                             uint32_t (&c)[4 * NQ]) {
+                                             int first, int step, uint32_t (&c)[4 * NQ]) {
     constexpr int NW = 4 * NQ;
 #pragma unroll
     for (int k = 0; k < NW; ++k) {
@@ -465,7 +557,7 @@ __device__ __forceinline__ void bound_filter(const uint4* __restrict__ col, cons
         constexpr int NQ1 = NQ;
         const int u0 = k / 4, u1 = (k + WA) / 4 < NQ1 ? (k + WA) / 4 : NQ1 - 1;
         const int s1 = __shfl_sync(0xffffffffu, fb, k + 1);
-        for (int s0 = __shfl_sync(0xffffffffu, fb, k); s0 < s1; s0 += BATCH) {
+        for (int s0 = __shfl_sync(0xffffffffu, fb, k) + first * BATCH; s0 < s1; s0 += step * BATCH) {
             uint32_t a = 0u;
 #pragma unroll
             for (int w = 0; w < WA; ++w) a |= c[w];
@@ -502,74 +594,201 @@ __device__ __forceinline__ void bound_filter(const uint4* __restrict__ col, cons
     }
 }
 
-// One warp takes 32 columns (x, y0 + STEP * lane) of one orientation at
-// a time; the grid is sized to the chip and strides over the tasks (a CTA per
-// plane and orientation spent its time starting: 5,760 short CTAs per item at
-// 240x123x100).  SEED: the lattice, nothing listed.  ALL: every survivor for the
-// flood, whatever its score (gated).  grid: any, block 128
-enum BoundPass { BOUND_SEED = 0, BOUND_LIST = 1, BOUND_ALL = 2 };
-template <int NQ, int PASS>
-__global__ void __launch_bounds__(128, PASS == BOUND_SEED ? 3 : (NQ == 1 ? 6 : 4))
-k_bound_find(const OrientDesc* __restrict__ orients, int n, int planes, const uint4* __restrict__ tbits, ScoreParams sp,
+// What a pass needs of 32 columns: the orientation's table, the columns'
+// parts of the bounds (lane = column) and the z range worth testing.
+struct BoundCols {
+    BoundTab bt;
+    int fb;                     // sample bucket bounds, one per lane
+    double h;                   // the table's header, one entry per lane
+    int Yv;
+    bool any;                   // a column has a z range
+    double A, gp, gm;
+    int zc;
+};
+// lane's row y of plane x; best: INFINITY for the whole range
+__device__ __forceinline__ BoundCols bound_cols(const BoundArgs& ba, const ScoreParams& sp, int nw, int o, int x, int y,
+                                                double best) {
+    const int lane = threadIdx.x & 31;
+    BoundCols c;
+    c.bt = bound_tab(ba.tab + (size_t)o * ba.tstride, sp);
+    const double h = c.h = c.bt.c[min(lane, 14) - 1];   // lane l: header entry l
+    c.fb = lane <= nw ? __ldg(&ba.fbound[(size_t)o * PSB_FBOUND + lane]) : 0;
+    const int Xv = (int)__shfl_sync(0xffffffffu, h, 9), Zv = (int)__shfl_sync(0xffffffffu, h, 11);
+    c.Yv = (int)__shfl_sync(0xffffffffu, h, 10);
+    const bool act = x < Xv && y < c.Yv;
+    c.A = c.gp = c.gm = 0.0;
+    c.zc = act ? Zv : 0;
+    if (act) {
+        c.A = c.bt.X[x] + c.bt.Y[y];
+        bound_octants(c.bt, x, y, &c.gp, &c.gm);
+    }
+    if (best < INFINITY) {
+        // slack for the roundings of F's sums; the exact test follows
+        const double lim = best + 1e-12 * fabs(best) + 1e-6;
+        if (!act || c.bt.F0[0] > lim - c.A || c.bt.F1[0] > lim - c.gp) c.zc = 0;
+        if (__any_sync(0xffffffffu, c.zc > 0) && c.zc > 0) {
+            c.zc = bound_count(c.bt.F0, Zv, lim - c.A);
+            c.zc = bound_count(c.bt.F1, c.zc, lim - c.gp);
+        }
+    }
+    c.any = __any_sync(0xffffffffu, c.zc > 0);
+    return c;
+}
+
+// The tasks of a pass: planes x row blocks of the orientations that are searched
+// (of at most 32, those the tables do not mark skipped; a skipped one's tasks
+// would each cost a round trip for its header).
+struct BoundTasks {
+    unsigned int mask;
+    int n, planes, yb, count;
+    __device__ __forceinline__ int orient(int k) const { return n <= 32 ? (int)__fns(mask, 0, k + 1) : k; }
+};
+__device__ __forceinline__ BoundTasks bound_tasks(const BoundArgs& ba, const ScoreParams& sp, int n, int xstep, int rows) {
+    BoundTasks t;
+    t.n = n;
+    const int lane = threadIdx.x & 31;
+    int m = n, X = sp.nx, Y = sp.ny;
+    t.mask = ~0u;
+    if (n <= 32) {
+        const double* h = ba.tab + (size_t)min(lane, n - 1) * ba.tstride;
+        const int xv = lane < n ? (int)h[9] : 0;
+        t.mask = __ballot_sync(0xffffffffu, xv > 0);
+        m = __popc(t.mask);
+        X = __reduce_max_sync(0xffffffffu, xv);
+        Y = __reduce_max_sync(0xffffffffu, xv > 0 ? (int)h[10] : 0);
+    }
+    t.planes = (X + xstep - 1) / xstep;
+    t.yb = (Y + rows - 1) / rows;
+    t.count = m * t.planes * t.yb;
+    return t;
+}
+
+// The first pass: a best score to cut the second one with, from a lattice of
+// columns (every fourth plane, the first four of every 16 rows: rows one by
+// one would touch a cache line each).  There are few tasks and each is a
+// chain of load latencies, so a CTA takes one: its four warps share the
+// samples, meet in shared memory, and then check and score the four survivors
+// of lowest bound, one each.  grid: any, block 128
+template <int NQ>
+__global__ void __launch_bounds__(128, NQ == 1 ? 6 : 3)
+k_bound_seed(int n, const uint4* __restrict__ tbits, ScoreParams sp,
+             BoundArgs ba) {
+    pdl_enter();
+    constexpr int NW = 4 * NQ;
+    __shared__ uint32_t cs[4][NW][32];
+    BoundState* st = ba.st;
+    if (bound_entry(st).halt) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ny = sp.ny;
+    const BoundTasks tm = bound_tasks(ba, sp, n, PSB_BSTEP, 128);
+    for (int task = blockIdx.x; task < tm.count; task += gridDim.x) {
+        const int y0 = task % tm.yb * 128, yl = y0 + lane / 4 * 16 + lane % 4;
+        const int x = task / tm.yb % tm.planes * PSB_BSTEP, o = tm.orient(task / (tm.yb * tm.planes));
+        // (the same in all four warps but for the best score, so no early exit on it)
+        const BoundCols bc = bound_cols(ba, sp, NW, o, x, yl, INFINITY);
+        if (!bc.any) continue;
+        uint32_t c[NW];
+#pragma unroll
+        for (int w = 0; w < NW; ++w) c[w] = low_bits(bc.zc - 32 * w);
+        const uint4* col = tbits + ((size_t)x * ny + min(yl, bc.Yv - 1)) * NQ;
+        bound_filter<NQ, NW, PSB_BBATCH / NQ>(col, ba.fs + (size_t)o * PSB_BSAMP, bc.fb, warp, 4, c);
+        __syncthreads();   // the last task's survivors have been read
+#pragma unroll
+        for (int w = 0; w < NW; ++w) cs[warp][w][lane] = c[w];
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < NW; ++w) c[w] = cs[0][w][lane] & cs[1][w][lane] & cs[2][w][lane] & cs[3][w][lane];
+        // this warp's survivor: the warp-th lowest bounded score among the
+        // first survivors of each word
+        const double now = bound_best(st);
+        double lb[NW];
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            lb[w] = INFINITY;
+            if (c[w]) lb[w] = bound_score(bc.bt, sp, bc.A, bc.gp, bc.gm, 32 * w + __ffs(c[w]) - 1);
+        }
+        double m = INFINITY;
+        int src = 0, zz = -1;
+        for (int k = 0; k <= warp; ++k) {
+            double own = INFINITY;
+            int lw = -1;
+#pragma unroll
+            for (int w = 0; w < NW; ++w)
+                if (lb[w] < own) { own = lb[w]; lw = w; }
+            m = own;
+            for (int d = 16; d > 0; d >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, d));
+            const unsigned int who = __ballot_sync(0xffffffffu, lw >= 0 && own == m);
+            zz = -1;
+            if (!who) break;
+            src = __ffs(who) - 1;
+            int z = -1;
+#pragma unroll
+            for (int w = 0; w < NW; ++w)
+                if (w == lw) {
+                    z = 32 * w + __ffs(c[w]) - 1;
+                    if (lane == src) lb[w] = INFINITY;
+                }
+            zz = __shfl_sync(0xffffffffu, z, src);
+        }
+        if (zz < 0 || !(m < now)) continue;
+        const RunHead od = run_head(bc.h);
+        const int y = y0 + src / 4 * 16 + src % 4;
+        if (!bound_free(od, (const uint32_t*)tbits, NW, ny, x, y, zz)) continue;
+        const long long D = bound_prox(od, ba.pphi, ny, sp.nz, x, y, zz);
+        if (lane == 0) atomicMin(&st->best, ord_key(ref_score(sp, (double)D, zz)));
+    }
+}
+
+// The second pass: one warp takes 32 columns (x, y0 + lane) of one orientation
+// at a time; the grid is sized to the chip and strides over the tasks (a CTA
+// per plane and orientation spent its time starting: 5,760 short CTAs per item
+// at 240x123x100), orientations outermost, so that the warps of an SM share a
+// few tables.  ALL: every survivor for the flood, whatever its score (gated).
+// grid: any, block 128
+template <int NQ, bool ALL>
+__global__ void __launch_bounds__(128, NQ == 1 ? 6 : 4)
+k_bound_find(int n, const uint4* __restrict__ tbits, ScoreParams sp,
              BoundArgs ba) {
     pdl_enter();
     BoundState* st = ba.st;
     const BoundEntry en = bound_entry(st);
-    if (en.halt || (PASS == BOUND_ALL && !en.need_flood)) return;
+    if (en.halt || (ALL && !en.need_flood)) return;
     constexpr int NW = 4 * NQ;
-    constexpr int STEP = PASS == BOUND_SEED ? PSB_BSTEP : 1;
-    // the lattice has few warps, each a chain of load latencies: longer batches
-    constexpr int BATCH = PASS == BOUND_SEED ? PSB_BBATCH / NQ : 8 / NQ;
+    constexpr int BATCH = 8 / NQ;
     const int lane = threadIdx.x & 31, ny = sp.ny;
-    const int yb = (ny + 32 * STEP - 1) / (32 * STEP), tasks = n * planes * yb;
+    const BoundTasks tm = bound_tasks(ba, sp, n, 1, 32);
     const int nwarps = gridDim.x * (blockDim.x >> 5);
-    for (int task = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); task < tasks; task += nwarps) {
-        const int y0 = (task % yb) * 32 * STEP;
-        const int o = (task / yb) % n, x = task / (yb * n) * STEP;
-        const BoundTab bt = bound_tab(ba.tab + (size_t)o * ba.tstride, sp);
-        const double h = bt.c[min(lane, 11) - 1];   // lane l: header entry l
-        const int fb = lane <= NW ? __ldg(&ba.fbound[(size_t)o * PSB_FBOUND + lane]) : 0;
-        const int y = y0 + STEP * lane;
+    for (int task = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); task < tm.count; task += nwarps) {
+        const int y0 = task % tm.yb * 32, x = task / tm.yb % tm.planes, o = tm.orient(task / (tm.yb * tm.planes));
         const BoundEntry now = bound_entry(st);
-        double best = PASS == BOUND_ALL ? INFINITY : now.best;
+        double best = ALL ? INFINITY : now.best;
         if (now.count > PSB_BCAP) return;   // the list is lost anyway
-        const int Xv = (int)__shfl_sync(0xffffffffu, h, 9), Yv = (int)__shfl_sync(0xffffffffu, h, 10);
-        const int Zv = (int)__shfl_sync(0xffffffffu, h, 11);
-        if (x >= Xv || y0 >= Yv || Zv <= 0) continue;
-        const bool act = y < Yv;
-        double A = 0.0, gp = 0.0, gm = 0.0;
-        int zc = act ? Zv : 0;
-        if (act) {
-            A = bt.X[x] + bt.Y[y];
-            bound_octants(bt, x, y, &gp, &gm);
-            if (best < INFINITY) {
-                // slack for the roundings of F's sums; the exact test follows
-                const double lim = best + 1e-12 * fabs(best) + 1e-6;
-                zc = bound_count(bt.F0, Zv, lim - A);
-                zc = bound_count(bt.F1, zc, lim - gp);
-            }
-        }
+        const BoundCols bc = bound_cols(ba, sp, NW, o, x, y0 + lane, best);
+        if (!bc.any) continue;
+        const BoundTab& bt = bc.bt;
+        const double A = bc.A, gp = bc.gp, gm = bc.gm;
+        const int y = y0 + lane;
         uint32_t c[NW];
         uint32_t some = 0u;
 #pragma unroll
-        for (int w = 0; w < NW; ++w) {
-            c[w] = low_bits(zc - 32 * w);
-            some |= c[w];
-        }
-        if (!__any_sync(0xffffffffu, some != 0u)) continue;
+        for (int w = 0; w < NW; ++w) c[w] = low_bits(bc.zc - 32 * w);
         // (a lane past the last row reads the last one's columns)
-        const uint4* col = tbits + ((size_t)x * ny + min(y, Yv - 1)) * NQ;
+        const uint4* col = tbits + ((size_t)x * ny + min(y, bc.Yv - 1)) * NQ;
         const int2* fs = ba.fs + (size_t)o * PSB_BSAMP;
-        const int top = __reduce_max_sync(0xffffffffu, zc);
-        if (top <= 32) bound_filter<NQ, 1, BATCH>(col, fs, fb, c);
-        else if (top <= 64) bound_filter<NQ, 2, BATCH>(col, fs, fb, c);
-        else bound_filter<NQ, NW, BATCH>(col, fs, fb, c);
-        some = 0u;
+        const int top = __reduce_max_sync(0xffffffffu, bc.zc), fb = bc.fb;
+        if (top <= 32) bound_filter<NQ, 1, BATCH>(col, fs, fb, 0, 1, c);
+        else if (top <= 64) bound_filter<NQ, 2, BATCH>(col, fs, fb, 0, 1, c);
+        else bound_filter<NQ, NW, BATCH>(col, fs, fb, 0, 1, c);
 #pragma unroll
         for (int w = 0; w < NW; ++w) some |= c[w];
         if (!__any_sync(0xffffffffu, some != 0u)) continue;
-        if (PASS == BOUND_SEED || (PASS == BOUND_LIST && !(best < INFINITY))) {
-            const OrientDesc& od = orients[o];
+        int held = 0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) held += __popc(c[w]);
+        held = __reduce_add_sync(0xffffffffu, held);
+        if (!ALL && (held > 32 || !(best < INFINITY))) {
+            // no seed found a free translation, or a loose one: try this warp's
+            // best before listing them all
+            const RunHead od = run_head(bc.h);
             for (int tries = 0; tries < 3; ++tries) {
                 // the lowest bounded score among the first survivors of each word
                 double lb = INFINITY;
@@ -586,8 +805,8 @@ k_bound_find(const OrientDesc* __restrict__ orients, int n, int planes, const ui
                 if (!(m < bound_best(st))) break;   // no survivor, or none that could improve
                 const int src = __ffs(__ballot_sync(0xffffffffu, lz >= 0 && lb == m)) - 1;
                 const int zz = __shfl_sync(0xffffffffu, lz, src);
-                if (bound_free(od, (const uint32_t*)tbits, NW, ny, x, y0 + STEP * src, zz)) {
-                    const long long D = bound_prox(od, ba.pphi, ny, sp.nz, x, y0 + STEP * src, zz);
+                if (bound_free(od, (const uint32_t*)tbits, NW, ny, x, y0 + src, zz)) {
+                    const long long D = bound_prox(od, ba.pphi, ny, sp.nz, x, y0 + src, zz);
                     if (lane == 0) atomicMin(&st->best, ord_key(ref_score(sp, (double)D, zz)));
                     break;
                 }
@@ -595,7 +814,6 @@ k_bound_find(const OrientDesc* __restrict__ orients, int n, int planes, const ui
                 for (int w = 0; w < NW; ++w)   // blocked: no survivor
                     if (lane == src && (zz >> 5) == w) c[w] &= ~(1u << (zz & 31));
             }
-            if (PASS == BOUND_SEED) continue;
             best = bound_best(st);
         }
         int mine = 0;
@@ -660,8 +878,8 @@ __device__ __forceinline__ void bound_commit(LoopState* ls, DecisionDev* out, co
 // carry 1e300).  grid: any, block 256
 template <bool FLOOD>
 __global__ void __launch_bounds__(256)
-k_bound_score(const OrientDesc* __restrict__ orients, const uint4* __restrict__ tbits, int tq, ScoreParams sp,
-              BoundArgs ba, int item, int interlock, LoopState* ls, DecisionDev* out) {
+k_bound_score(const uint4* __restrict__ tbits, int tq, ScoreParams sp, BoundArgs ba, int item, int interlock,
+              LoopState* ls, DecisionDev* out) {
     pdl_enter();
     BoundState* st = ba.st;
     const BoundEntry en = bound_entry(st);
@@ -670,8 +888,51 @@ k_bound_score(const OrientDesc* __restrict__ orients, const uint4* __restrict__ 
     const bool fail = count > PSB_BCAP;
     const int n = fail ? 0 : count;
     const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    // two entries per warp and step
-    for (int e0 = 2 * (blockIdx.x * wpb + (threadIdx.x >> 5)); e0 < n; e0 += 2 * gridDim.x * wpb) {
+    __shared__ long long part[8];
+    auto scored = [&](int t, int o, int z, long long D) {
+        const double s = ref_score(sp, (double)D, z);
+        if (ord_key(s) <= atomicMin(&st->best, ord_key(s))) {
+            // the best so far, or equal to it: a candidate for the tie rules
+            BoundHit w;
+            w.t = t;
+            w.o = o;
+            w.s = s;
+            ba.win[atomicAdd(&st->nwin, 1)] = w;
+        }
+    };
+    if (n <= (int)gridDim.x) {
+        // few entries: a CTA each, every run's loads in flight at once
+        for (int e = blockIdx.x; e < n; e += gridDim.x) {
+            const BoundHit h = ba.list[e];
+            if (!(h.s < 1e299)) continue;
+            const RunHead od = run_head_of(ba.tab, ba.tstride, h.o);
+            const int z = h.t % sp.nz, y = (h.t / sp.nz) % sp.ny, x = h.t / (sp.nz * sp.ny);
+            const RunMap rm = run_map(od, sp.ny, x, y, z);
+            const uint32_t* T = (const uint32_t*)tbits;
+            long long acc = 0;
+            bool hit = false;
+#pragma unroll 4
+            for (int r = threadIdx.x; r < od.nr; r += 256) {
+                const int4 q = __ldg(&od.runs[r]);
+                int z0, z1;
+                const int col = run_at(rm, q, &z0, &z1);
+                const int32_t* P = ba.pphi + (size_t)col * (sp.nz + 1);
+                acc += (long long)q.w * (__ldg(&P[z1 + 1]) - __ldg(&P[z0]));
+                if (!FLOOD) hit = run_blocked(T + (size_t)col * 4 * tq, z0, z1) || hit;
+            }
+            for (int d = 16; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+            if (lane == 0) part[threadIdx.x >> 5] = acc;
+            if (__syncthreads_or(hit)) continue;
+            if (threadIdx.x == 0) {
+                for (int k = 1; k < wpb; ++k) acc += part[k];
+                scored(h.t, h.o, z, acc);
+            }
+            __syncthreads();
+        }
+    }
+    // many: two per warp and step, most found blocked by their first 128 runs
+    for (int e0 = n <= (int)gridDim.x ? n : 2 * (blockIdx.x * wpb + (threadIdx.x >> 5)); e0 < n;
+         e0 += 2 * gridDim.x * wpb) {
         BoundHit h;
         h.t = h.o = 0;
         h.s = 1e300;
@@ -680,28 +941,23 @@ k_bound_score(const OrientDesc* __restrict__ orients, const uint4* __restrict__ 
             const int src = __ffs(m) - 1;
             const int t = __shfl_sync(0xffffffffu, h.t, src), o = __shfl_sync(0xffffffffu, h.o, src);
             if (__shfl_sync(0xffffffffu, h.s, src) > bound_best(st)) continue;
-            const OrientDesc& od = orients[o];
+            const RunHead od = run_head_of(ba.tab, ba.tstride, o);
             const int z = t % sp.nz, y = (t / sp.nz) % sp.ny, x = t / (sp.nz * sp.ny);
             if (!FLOOD && !bound_free(od, (const uint32_t*)tbits, 4 * tq, sp.ny, x, y, z)) continue;
-            const double s = ref_score(sp, (double)bound_prox(od, ba.pphi, sp.ny, sp.nz, x, y, z), z);
-            if (lane == 0 && ord_key(s) <= atomicMin(&st->best, ord_key(s))) {
-                // the best so far, or equal to it: a candidate for the tie rules
-                BoundHit w;
-                w.t = t;
-                w.o = o;
-                w.s = s;
-                ba.win[atomicAdd(&st->nwin, 1)] = w;
-            }
+            const long long D = bound_prox(od, ba.pphi, sp.ny, sp.nz, x, y, z);
+            if (lane == 0) scored(t, o, z, D);
         }
     }
     __shared__ bool last;
     __shared__ unsigned long long red[8];
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicInc(&st->done, gridDim.x - 1) == gridDim.x - 1;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicInc(&st->done, gridDim.x - 1) == gridDim.x - 1;
+        __threadfence();
+    }
     __syncthreads();
     if (!last) return;
-    __threadfence();
     const BoundEntry fin = bound_entry(st);
     const double best = fin.best;
     unsigned long long win = ~0ULL;
@@ -745,18 +1001,21 @@ k_bound_score(const OrientDesc* __restrict__ orients, const uint4* __restrict__ 
 // faces are seeds always, the far ones for a non-empty item (fft3.cu:263-293),
 // which every item here is.  grid: any, block 256
 __global__ void __launch_bounds__(256)
-k_bound_ray(const OrientDesc* __restrict__ orients, const uint4* __restrict__ tbits, int tq, ScoreParams sp,
-            BoundState* st, LoopState* ls, DecisionDev* out) {
+k_bound_ray(const uint4* __restrict__ tbits, int tq, ScoreParams sp, BoundArgs ba, LoopState* ls, DecisionDev* out) {
     pdl_enter();
+    BoundState* st = ba.st;
     const BoundEntry en = bound_entry(st);
     if (en.halt || !en.need_ray) return;
-    const OrientDesc& od = orients[st->win_o];
+    const double head = ba.tab[(size_t)st->win_o * ba.tstride + min((int)(threadIdx.x & 31), 14)];
+    const RunHead od = run_head(head);
+    const int valid[3] = {(int)__shfl_sync(0xffffffffu, head, 9), (int)__shfl_sync(0xffffffffu, head, 10),
+                          (int)__shfl_sync(0xffffffffu, head, 11)};
     const int t = st->win_t;
     const int at[3] = {t / (sp.nz * sp.ny), (t / sp.nz) % sp.ny, t % sp.nz};
     int len[6], total = 0;
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-        len[k] = k < 3 ? at[k] : od.valid[k - 3] - 1 - at[k - 3];
+        len[k] = k < 3 ? at[k] : valid[k % 3] - 1 - at[k % 3];
         total += len[k];
     }
     const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
@@ -772,9 +1031,9 @@ k_bound_ray(const OrientDesc* __restrict__ orients, const uint4* __restrict__ tb
         if (!bound_free(od, (const uint32_t*)tbits, 4 * tq, sp.ny, c[0], c[1], c[2]) && lane == 0)
             atomicOr(&st->blocked, 1u << k);
     }
-    __threadfence();
     __syncthreads();
     if (threadIdx.x != 0) return;
+    __threadfence();
     if (atomicInc(&st->rdone, gridDim.x - 1) != gridDim.x - 1) return;
     __threadfence();
     const unsigned int blocked = *(volatile unsigned int*)&st->blocked;
@@ -799,8 +1058,7 @@ k_bound_ray(const OrientDesc* __restrict__ orients, const uint4* __restrict__ tb
 #define PSB_BSLOTS (2 * PSB_BFREE)
 inline size_t bound_flood_smem() { return (size_t)PSB_BSLOTS * 8 + (size_t)PSB_BFREE * 4; }
 __global__ void __launch_bounds__(256)
-k_bound_flood(const OrientDesc* __restrict__ orients, const uint4* __restrict__ tbits, int tq, ScoreParams sp,
-              BoundArgs ba, int item) {
+k_bound_flood(const uint4* __restrict__ tbits, int tq, ScoreParams sp, BoundArgs ba, int item) {
     pdl_enter();
     BoundState* st = ba.st;
     const BoundEntry en = bound_entry(st);
@@ -811,18 +1069,19 @@ k_bound_flood(const OrientDesc* __restrict__ orients, const uint4* __restrict__ 
     for (int e = blockIdx.x * wpb + (threadIdx.x >> 5); e < n; e += gridDim.x * wpb) {
         const BoundHit h = ba.list[e];
         const int z = h.t % nz, y = (h.t / nz) % ny, x = h.t / (nz * ny);
-        if (!bound_free(orients[h.o], (const uint32_t*)tbits, 4 * tq, ny, x, y, z) && lane == 0) ba.list[e].s = 1e300;
+        if (!bound_free(run_head_of(ba.tab, ba.tstride, h.o), (const uint32_t*)tbits, 4 * tq, ny, x, y, z) && lane == 0)
+            ba.list[e].s = 1e300;
     }
     __shared__ int head, tail, nfree, last;
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
+        __threadfence();
         last = atomicInc(&st->done, gridDim.x - 1) == gridDim.x - 1;
+        __threadfence();
         tail = nfree = 0;
     }
     __syncthreads();
     if (!last) return;
-    __threadfence();
     extern __shared__ unsigned int fsm[];
     unsigned int* key = fsm;                  // o * V + t, ~0 empty
     int* val = (int*)(fsm + PSB_BSLOTS);      // list entry, high bit set once reached
@@ -863,9 +1122,9 @@ k_bound_flood(const OrientDesc* __restrict__ orients, const uint4* __restrict__ 
     }
     for (int s = threadIdx.x; s < PSB_BSLOTS; s += blockDim.x) {
         if (key[s] == ~0u) continue;
-        const OrientDesc& od = orients[key[s] / V];
+        const double* v = ba.tab + (size_t)(key[s] / V) * ba.tstride + 9;   // numbers of translations
         const int t = (int)(key[s] % V), z = t % nz, y = (t / nz) % ny, x = t / (nz * ny);
-        if (x == 0 || y == 0 || z == 0 || x == od.valid[0] - 1 || y == od.valid[1] - 1 || z == od.valid[2] - 1) {
+        if (x == 0 || y == 0 || z == 0 || x == (int)v[0] - 1 || y == (int)v[1] - 1 || z == (int)v[2] - 1) {
             val[s] |= (int)0x80000000u;
             queue[atomicAdd(&tail, 1)] = s;
         }

@@ -1658,50 +1658,53 @@ struct psb_tray {
         return PSB_OK;
     }
 
-    // Queue one item's search: its n orientations at d_odb, tables in the slots
-    // from slot0 on, outcome in *d_out and the loop state.  xmax: the largest
+    // Queue one item's search: its n orientations' tables in the slots from
+    // slot0 on, outcome in *d_out and the loop state.  xmax: the largest
     // number of x translations.
-    int bound_search(const OrientDesc* d_odb, int n, size_t slot0, int xmax, int mode, bool interlock, int item,
+    int bound_search(int n, size_t slot0, int xmax, int mode, bool interlock, int item,
                      DecisionDev* d_out) {
         const ScoreParams sp = score_params(mode);
         const long long ts = bound_tab_stride(nx, ny, nz);
         const BoundArgs ba{d_bstate, d_bgeom, d_btab + slot0 * ts, ts, d_bfs + slot0 * PSB_BSAMP,
                            d_bfb + slot0 * PSB_FBOUND, d_blist, d_blist + PSB_BCAP, d_pphi};
         const int yb = (ny + 31) / 32;
-        auto grid = [&](int tasks) { return (unsigned)std::max(1, std::min(148 * 8, (tasks + 3) / 4)); };
-        const int seedx = (xmax + PSB_BSTEP - 1) / PSB_BSTEP, seedy = (ny + 32 * PSB_BSTEP - 1) / (32 * PSB_BSTEP);
+        // at most what the chip holds at once (launch bounds): a second wave
+        // would double a latency-bound kernel
+        auto grid = [&](int tasks) {
+            return (unsigned)std::max(1, std::min(148 * (tq == 1 ? 6 : 4), (tasks + 3) / 4));
+        };
+        const int seedx = (xmax + PSB_BSTEP - 1) / PSB_BSTEP, seedy = (ny + 127) / 128;
         {
             PROF("k_bound_seed", st);
-            auto k = tq == 1 ? k_bound_find<1, BOUND_SEED> : k_bound_find<2, BOUND_SEED>;
-            pdl(k, grid(n * seedx * seedy), 128, 0, st)(d_odb, n, seedx, d_tbits, sp, ba);
+            auto k = tq == 1 ? k_bound_seed<1> : k_bound_seed<2>;
+            pdl(k, (unsigned)std::max(1, std::min(148 * (tq == 1 ? 6 : 3), n * seedx * seedy)), 128, 0, st)(n, d_tbits, sp, ba);
         }
         CKL();
         {
             PROF("k_bound_find", st);
-            auto k = tq == 1 ? k_bound_find<1, BOUND_LIST> : k_bound_find<2, BOUND_LIST>;
-            pdl(k, grid(n * xmax * yb), 128, 0, st)(d_odb, n, xmax, d_tbits, sp, ba);
+            auto k = tq == 1 ? k_bound_find<1, false> : k_bound_find<2, false>;
+            pdl(k, grid(n * xmax * yb), 128, 0, st)(n, d_tbits, sp, ba);
         }
         CKL();
         {
             PROF("k_bound_score", st);
-            pdl(k_bound_score<false>, 148 * 6, 256, 0, st)(d_odb, d_tbits, tq, sp, ba, item, interlock ? 1 : 0, d_ls,
-                                                           d_out);
+            pdl(k_bound_score<false>, 148 * 4, 256, 0, st)(d_tbits, tq, sp, ba, item, interlock ? 1 : 0, d_ls, d_out);
         }
         CKL();
         if (interlock) {
             {
                 PROF("k_bound_ray", st);
-                pdl(k_bound_ray, 64, 256, 0, st)(d_odb, d_tbits, tq, sp, d_bstate, d_ls, d_out);
+                pdl(k_bound_ray, 64, 256, 0, st)(d_tbits, tq, sp, ba, d_ls, d_out);
             }
             CKL();
             // only for an item whose winner has no straight free run
             PROF("k_bound_flood", st);
-            auto k = tq == 1 ? k_bound_find<1, BOUND_ALL> : k_bound_find<2, BOUND_ALL>;
-            pdl(k, grid(n * xmax * yb), 128, 0, st)(d_odb, n, xmax, d_tbits, sp, ba);
+            auto k = tq == 1 ? k_bound_find<1, true> : k_bound_find<2, true>;
+            pdl(k, grid(n * xmax * yb), 128, 0, st)(n, d_tbits, sp, ba);
             CKL();
-            pdl(k_bound_flood, 148, 256, bound_flood_smem(), st)(d_odb, d_tbits, tq, sp, ba, item);
+            pdl(k_bound_flood, 148, 256, bound_flood_smem(), st)(d_tbits, tq, sp, ba, item);
             CKL();
-            pdl(k_bound_score<true>, 148, 256, 0, st)(d_odb, d_tbits, tq, sp, ba, item, 1, d_ls, d_out);
+            pdl(k_bound_score<true>, 148, 256, 0, st)(d_tbits, tq, sp, ba, item, 1, d_ls, d_out);
             CKL();
         }
         return PSB_OK;
@@ -2983,7 +2986,7 @@ int psb_tray_search(psb_tray* t, const int32_t* const* items, const int32_t* dim
     if (!per_orient && t->bound_usable() && (unsigned long long)n * t->V < 0xffffffffULL) {
         TRY(t->ensure_bound(n));
         TRY(t->bound_prep(t->d_xod, n, 1, mode));
-        TRY(t->bound_search(t->d_xod, n, 0, t->nx, mode, interlock, 0, &t->d_reply->dec));
+        TRY(t->bound_search(n, 0, t->nx, mode, interlock, 0, &t->d_reply->dec));
         CK(cudaMemcpyAsync(t->h_reply, t->d_reply, sizeof(BoundReply), cudaMemcpyDeviceToHost, t->st));
         CK(cudaStreamSynchronize(t->st));
         const BoundReply& r = *t->h_reply;
@@ -3343,6 +3346,10 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
         CKL();
         return PSB_OK;
     };
+    // the plain loop: only the best orientation of an item matters
+    const bool plain = filt && g_direct_max > 0 && !opt.prop && !opt.hmaps && !opt.per_orient && opt.world == 1 &&
+                       !opt.d_local &&
+                       (unsigned long long)n_orient * t->V < 0xffffffffULL;   // k_bound_flood's keys
     auto describe_range = [&](int i0, int i1, cudaStream_t s) -> int {
         for (int it = i0; it < i1; ++it) {
             const psb_tray::StagedDev& sd = t->sdev[it];
@@ -3371,6 +3378,12 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
         memcpy(hd_base + b0, allb.data() + b0, sizeof(OrientDesc) * nb);
         CK(cudaMemcpyAsync(t->d_od_all + a0, hd_all + a0, sizeof(OrientDesc) * na, cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(t->d_base_all + b0, hd_base + b0, sizeof(OrientDesc) * nb, cudaMemcpyHostToDevice, s));
+        for (int k = i0; plain && n_orient > 1 && k < i1; k += 32768) {   // grid dimensions
+            PROF("k_bound_dedupe", s);
+            pdl(k_bound_dedupe, dim3(n_orient, std::min(32768, i1 - k)), 256, 0, s)(t->d_od_all + (size_t)k * n_orient,
+                                                                                  n_orient);
+            CKL();
+        }
         if (icols_pre) TRY(item_cols_range(i0, i1, s));
         return PSB_OK;
     };
@@ -3576,8 +3589,6 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
     // halt flag the host runs it through the transforms and goes on after it.
     // The chunk grows while that does not happen (a halt wastes the launches
     // queued behind it, a chunk costs one wait).
-    const bool plain = filt && g_direct_max > 0 && !opt.prop && !d_hm && !d_per && opt.world == 1 && !opt.d_local &&
-                       (unsigned long long)n_orient * t->V < 0xffffffffULL;   // k_bound_flood's keys
     const int kChunkMax = 32, kPrepMax = 128;
     int chunk = 4, prep0 = 0, prep1 = 0;   // items whose bound tables are made: [prep0, prep1)
     bool fed = !opt.feed;
@@ -3629,7 +3640,7 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
                 int xmax = 0;
                 for (int o = 0; o < n_orient; ++o)
                     if (!oh[o].skip) xmax = std::max(xmax, oh[o].valid[0]);
-                TRY(t->bound_search(d_odb + (size_t)k * n_orient, n_orient, (size_t)(it + k - prep0) * n_orient, xmax, mode,
+                TRY(t->bound_search(n_orient, (size_t)(it + k - prep0) * n_orient, xmax, mode,
                                     interlock != 0, it + k, t->d_dec + it + k));
                 TRY(t->bound_place(d_odb + (size_t)k * n_orient));
             }
