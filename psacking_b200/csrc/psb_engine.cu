@@ -461,6 +461,7 @@ int set_smem_attrs() {
     TRY(set_max_dyn_smem(k_fft_mid<-1>));
     TRY(set_max_dyn_smem(k_fft_mid<1>));
     TRY(set_max_dyn_smem(k_xpass));
+    TRY(set_max_dyn_smem(k_corr_x));
     TRY(set_max_dyn_smem(k_plane));
     for (int n : {64, 100, 128, 240})
         for (int m = 0; m < 3; ++m) {
@@ -621,32 +622,6 @@ void forward_mids(const Grid3& g, float2* w1, float2* w2, float2* spec, const in
                    -1, 0, gate};
     // x: [1][n0->F0][F1*H]
     m[1] = MidDesc{w2, spec, 1, g.F[1] * g.H, g.n[0], g.F[0], 0, 0, g.F[1] * g.H, g.F[1] * g.H, -1, 0, gate};
-}
-
-// forward: src grid -> spectrum [F0][F1][H].  w1: [n0][n1][H], w2: [n0][F1][H]
-int forward3(const Grid3& g, const RzDesc& rz_in, float2* w1, float2* w2, float2* spec, RzDesc* d_rz,
-             MidDesc* d_mid, cudaStream_t st) {
-    RzDesc rz = rz_in;
-    rz.out = w1;
-    CK(cudaMemcpyAsync(d_rz, &rz, sizeof(rz), cudaMemcpyHostToDevice, st));
-    MidDesc m[2];
-    forward_mids(g, w1, w2, spec, nullptr, m);
-    CK(cudaMemcpyAsync(d_mid, m, sizeof(m), cudaMemcpyHostToDevice, st));
-    return forward3_dev(g, d_rz, d_mid, st);
-}
-
-int inverse3_dev(const Grid3& g, float2* w1, int32_t* out, const MidDesc* d_mid, cudaStream_t st);
-
-// inverse: spectrum [F0][F1][H] -> int32 grid (rounded, scaled by 1/(F0 F1 F2))
-int inverse3_int(const Grid3& g, float2* spec, float2* w1, float2* w2, int32_t* out, MidDesc* d_mid,
-                 cudaStream_t st) {
-    MidDesc m[2];
-    // x: [1][F0 -> n0][F1*H]   (spec -> w2 [n0][F1][H])
-    m[0] = MidDesc{spec, w2, 1, g.F[1] * g.H, g.F[0], g.n[0], 0, 0, g.F[1] * g.H, g.F[1] * g.H, -1, 0};
-    // y: [n0][F1 -> n1][H]     (w2 -> w1 [n0][n1][H])
-    m[1] = MidDesc{w2, w1, g.n[0], g.H, g.F[1], g.n[1], (long long)g.F[1] * g.H, (long long)g.n[1] * g.H, g.H, g.H, -1, 0};
-    CK(cudaMemcpyAsync(d_mid, m, sizeof(m), cudaMemcpyHostToDevice, st));
-    return inverse3_dev(g, w1, out, d_mid, st);
 }
 
 // inverse with its two MidDescs already on the device (d_mid[0]: x pass
@@ -2289,43 +2264,86 @@ int util_tray(int nx, int ny, int nz, psb_tray** out) {
     return PSB_OK;
 }
 
-// corr (conj_b=1): out[t] = sum_x b[x] a[t+x] ; conv (conj_b=0): linear conv
+// The transforms' descriptors of a product of two grids, passed by value to a
+// kernel that writes them to device memory in stream order (no host-to-device
+// copy, which from pageable memory waits for the stream).
+struct ProductDescs {
+    RzDesc rz[2];          // z passes of a and b
+    MidDesc y[2], yi;      // y passes of a and b; of the inverse
+};
+__global__ void k_product_descs(ProductDescs s, ProductDescs* d) {
+    pdl_enter();
+    if (threadIdx.x == 0) *d = s;
+}
+
+// corr (conj_b=1): out[t] = sum_x b[x] a[t+x] ; conv (conj_b=0): linear conv.
+// z and y passes of both grids in one launch each, the x passes with the
+// product in one (k_corr_x), the inverse y and z passes.
 int linear_transform_product(const int32_t* a, const int32_t* b, int nx, int ny, int nz, int conj_b, int32_t* out) {
     TRY(ensure_device());
     TRY(set_smem_attrs());
     Grid3 g;
     TRY(make_grid3(nx, ny, nz, true, &g));
-    size_t V = (size_t)nx * ny * nz;
-    size_t S = (size_t)g.F[0] * g.F[1] * g.H;
-    size_t w1 = (size_t)nx * ny * g.H, w2 = (size_t)nx * g.F[1] * g.H;
-    size_t bytes = sizeof(float2) * (2 * S + w1 + w2) + sizeof(int32_t) * 2 * V + 4096;
+    const size_t V = (size_t)nx * ny * nz;
+    const size_t w1 = (size_t)nx * ny * g.H, w2 = (size_t)nx * g.F[1] * g.H;
+    const size_t bytes = sizeof(float2) * 2 * (w1 + w2) + sizeof(int32_t) * 2 * V + 8192;
     void* base = nullptr;
     TRY(arena(bytes, &base));
     char* p = (char*)base;
     auto take = [&](size_t n) { char* r = p; p += (n + 255) / 256 * 256; return r; };
-    float2* Sa = (float2*)take(sizeof(float2) * S);
-    float2* Sb = (float2*)take(sizeof(float2) * S);
-    float2* W1 = (float2*)take(sizeof(float2) * w1);
-    float2* W2 = (float2*)take(sizeof(float2) * w2);
+    float2* W1[2] = {(float2*)take(sizeof(float2) * w1), (float2*)take(sizeof(float2) * w1)};
+    float2* W2[2] = {(float2*)take(sizeof(float2) * w2), (float2*)take(sizeof(float2) * w2)};
     int32_t* da = (int32_t*)take(sizeof(int32_t) * V);
     int32_t* db = (int32_t*)take(sizeof(int32_t) * V);
-    RzDesc* d_rz = (RzDesc*)take(sizeof(RzDesc) * 2);
-    MidDesc* d_mid = (MidDesc*)take(sizeof(MidDesc) * 2);
+    ProductDescs* dd = (ProductDescs*)take(sizeof(ProductDescs));
     cudaStream_t st = 0;
     CK(upload_async(da, a, sizeof(int32_t) * V, st));
     CK(upload_async(db, b, sizeof(int32_t) * V, st));
-    RzDesc ra{SRC_GRID_RAW, da, nx, ny, nz, 0, -1, nullptr};
-    RzDesc rb{SRC_GRID_RAW, db, nx, ny, nz, 0, -1, nullptr};
-    TRY(forward3(g, ra, W1, W2, Sa, d_rz, d_mid, st));
-    CK(cudaStreamSynchronize(st));
-    TRY(forward3(g, rb, W1, W2, Sb, d_rz + 1, d_mid, st));
+    ProductDescs pd;
+    for (int k = 0; k < 2; ++k) {
+        pd.rz[k] = RzDesc{SRC_GRID_RAW, k ? db : da, nx, ny, nz, 0, -1, W1[k], nullptr, nullptr};
+        MidDesc m[2];
+        forward_mids(g, W1[k], W2[k], nullptr, nullptr, m);
+        pd.y[k] = m[0];
+    }
+    // y: [n0][F1 -> n1][H]     (W2[0] -> W1[0] [n0][n1][H])
+    pd.yi = MidDesc{W2[0], W1[0], g.n[0], g.H, g.F[1], g.n[1], (long long)g.F[1] * g.H, (long long)g.n[1] * g.H, g.H,
+                    g.H, -1, 0, nullptr};
+    pdl(k_product_descs, 1, 32, 0, st)(pd, dd);
+    CKL();
+    const int npairs = (nx * ny + 1) / 2;
     {
-        PROF("k_spec_mul", st);
-        pdl(k_spec_mul, grid1d(S), 256, 0, st)(Sa, Sb, Sa, S, conj_b);
+        PROF("k_rfft_z", st);
+        pdl(k_rfft_z, dim3((npairs + PSB_PAIRS - 1) / PSB_PAIRS, 2), PSB_THREADS, smem_rz(g.F[2]), st)(
+            dd->rz, nullptr, g.p[2].p, g.p[2].tw);
     }
     CKL();
-    CK(cudaStreamSynchronize(st));
-    TRY(inverse3_int(g, Sa, W1, W2, da, d_mid, st));
+    {
+        PROF("k_fft_mid_fwd", st);
+        pdl(k_fft_mid<-1>, dim3((g.H + PSB_TILE - 1) / PSB_TILE, nx, 2), PSB_THREADS, smem_mid(g.F[1]), st)(
+            dd->y, nullptr, g.p[1].p, g.p[1].tw);
+    }
+    CKL();
+    {
+        PROF("k_corr_x", st);
+        const int C = g.F[1] * g.H;
+        pdl(k_corr_x, (C + PSB_TILE - 1) / PSB_TILE, PSB_THREADS, sizeof(float2) * (g.F[0] + 4 * PSB_TILE * g.F[0]), st)(
+            W2[0], W2[1], nx, C, conj_b, g.p[0].p, g.p[0].tw);
+    }
+    CKL();
+    {
+        PROF("k_fft_mid_inv", st);
+        pdl(k_fft_mid<1>, dim3((g.H + PSB_TILE - 1) / PSB_TILE, nx, 1), PSB_THREADS, smem_mid(g.F[1]), st)(
+            &dd->yi, nullptr, g.p[1].p, g.p[1].tw);
+    }
+    CKL();
+    {
+        PROF("k_irfft_z_int", st);
+        const float scale = (float)(1.0 / ((double)g.F[0] * g.F[1] * g.F[2]));
+        pdl(k_irfft_z_int, (npairs + PSB_PAIRS - 1) / PSB_PAIRS, PSB_THREADS, smem_rz(g.F[2]), st)(
+            W1[0], da, nx * ny, nz, scale, g.p[2].p, g.p[2].tw);
+    }
+    CKL();
     CK(download(out, da, sizeof(int32_t) * V, st));
     return PSB_OK;
 }

@@ -306,6 +306,44 @@ __global__ void k_spec_mul(const float2* __restrict__ a, const float2* __restric
     }
 }
 
+// The x passes of the stateless correlation / convolution in one kernel: per
+// tile of PSB_TILE spectrum columns both grids forward along x, the product
+// above, the inverse along x.  The two spectra (F0 x F1 x H each) stay in shared
+// memory; only the n0 rows of either side of the x axis are read and written.
+// a, b: [n0][C] (z and y transformed); the result goes to a.
+// grid: ceil(C / PSB_TILE), block PSB_THREADS
+__global__ void __launch_bounds__(PSB_THREADS)
+k_corr_x(float2* __restrict__ a, const float2* __restrict__ b, int n0, int C, int conj_b, AxisPlan plan,
+         const float2* __restrict__ g_tw) {
+    pdl_enter();
+    extern __shared__ float2 sm[];
+    const int N = plan.n, T = PSB_TILE, c0 = blockIdx.x * T;
+    float2* tw = sm;
+    float2* A = sm + N;            // 2T lines: a's columns, then b's
+    float2* B = A + 2 * T * N;
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    load_twiddles(tw, g_tw, N, tid, nthr);
+    for (int idx = tid; idx < 2 * T * N; idx += nthr) {
+        const int f = idx / (T * N), r = idx - f * T * N, l = r / T, cl = r - l * T, c = c0 + cl;
+        float2 v = make_float2(0.f, 0.f);
+        if (l < n0 && c < C) v = (f ? b : (const float2*)a)[(size_t)l * C + c];
+        A[(f * T + cl) * N + l] = v;
+    }
+    __syncthreads();
+    float2* R = smem_fft<-1>(A, B, 2 * T, N, plan, tw, tid, nthr);
+    float2* Q = R == A ? B : A;
+    for (int idx = tid; idx < T * N; idx += nthr) {
+        const float2 x = R[idx], y = R[T * N + idx];
+        Q[idx] = conj_b ? c_cmul(y, x) : c_mul(x, y);
+    }
+    __syncthreads();
+    float2* R2 = smem_fft<1>(Q, R, T, N, plan, tw, tid, nthr);
+    for (int idx = tid; idx < T * n0; idx += nthr) {
+        const int l = idx / T, cl = idx - l * T, c = c0 + cl;
+        if (c < C) a[(size_t)l * C + c] = R2[cl * N + l];
+    }
+}
+
 // ---------------------------------------------------------------------------
 // fused x pass of the search: item forward along x, products with the tray's
 // occupancy and distance spectra, inverse along x for both.
