@@ -510,6 +510,33 @@ int set_smem_attrs() {
 std::atomic<int> g_fail_alloc{0};
 std::atomic<long long> g_live_allocs{0};
 
+// The trays' memory pool of the current device.  It keeps up to 1 GiB when
+// trays are freed (the default pool returns everything at the next
+// synchronisation): a tray's dozen buffers otherwise take 2-8 ms to map again
+// for every tray of a many-tray run.
+int tray_pool(cudaMemPool_t* out) {
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(PSB_ERR_ARG, "device index %d out of range", dev);
+    std::lock_guard<std::mutex> lk(mu);
+    if (!pools[dev]) {
+        cudaMemPoolProps props;
+        memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool;
+        CK(cudaMemPoolCreate(&pool, &props));
+        unsigned long long keep = 1ULL << 30;
+        CK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        pools[dev] = pool;
+    }
+    *out = pools[dev];
+    return PSB_OK;
+}
+
 template <class T>
 int dalloc(T** p, size_t n, cudaStream_t s = nullptr) {
     *p = nullptr;
@@ -518,7 +545,9 @@ int dalloc(T** p, size_t n, cudaStream_t s = nullptr) {
         return fail(PSB_ERR_CUDA, "device allocation of %zu B failed (injected by psb_debug_fail_alloc)",
                     sizeof(T) * n);
     if (s) {
-        CK(cudaMallocAsync((void**)p, sizeof(T) * n, s));
+        cudaMemPool_t pool;
+        TRY(tray_pool(&pool));
+        CK(cudaMallocFromPoolAsync((void**)p, sizeof(T) * n, pool, s));
     } else {
         CK(cudaMalloc((void**)p, sizeof(T) * n));
     }
@@ -998,6 +1027,7 @@ struct psb_tray {
     int* d_bfb = nullptr;
     size_t bcap = 0;
     BoundReply* h_reply = nullptr;    // pinned
+    size_t h_reply_cap = 0;
 
     // per-orientation slots
     int cap = 0;
@@ -1074,6 +1104,7 @@ struct psb_tray {
     int* d_icn = nullptr;
     size_t icmeta_cap = 0, icn_cap = 0;
     void* h_icmeta = nullptr;        // pinned staging of the two tables
+    size_t h_icmeta_cap = 0;
     std::vector<long long> icol_off;
     std::vector<int> icol_stride;
     // the current item's precomputed columns for cand_filter (null: compute)
@@ -1143,17 +1174,18 @@ struct psb_tray {
         }
         st = nullptr;
         for (int p = 0; p < 2; ++p) {
-            if (h_part[p]) cudaFreeHost(h_part[p]);
+            PinCache::get().give(h_part[p], h_part_cap[p]);
             h_part[p] = nullptr;
             h_part_cap[p] = 0;
         }
-        if (h_desc) cudaFreeHost(h_desc);
+        PinCache::get().give(h_desc, h_desc_cap);
         h_desc = nullptr;
         h_desc_cap = 0;
-        if (h_reply) cudaFreeHost(h_reply);
+        PinCache::get().give(h_reply, h_reply_cap);
         h_reply = nullptr;
-        if (h_icmeta) cudaFreeHost(h_icmeta);
+        PinCache::get().give(h_icmeta, h_icmeta_cap);
         h_icmeta = nullptr;
+        h_icmeta_cap = 0;
     }
 
     int init(int x, int y, int z) {
@@ -1586,7 +1618,7 @@ struct psb_tray {
     }
     int ensure_reply() {
         if (d_reply) return PSB_OK;
-        if (!h_reply) CK(cudaMallocHost(&h_reply, sizeof(BoundReply)));
+        if (!h_reply) CK(PinCache::get().take((void**)&h_reply, sizeof(BoundReply), &h_reply_cap));
         TRY(dalloc(&d_reply, 1, st));
         d_bstate = &d_reply->st;
         return bound_reset();
@@ -3112,11 +3144,12 @@ int stage_upload(psb_tray* t, const int32_t* const* items, int i0, int i1, int p
         t->part_cap[part] = bytes;
     }
     if (bytes > t->h_part_cap[part]) {
-        if (t->h_part[part]) cudaFreeHost(t->h_part[part]);
+        PinCache::get().give(t->h_part[part], t->h_part_cap[part]);
         t->h_part[part] = nullptr;
         t->h_part_cap[part] = 0;
-        CK(cudaMallocHost(&t->h_part[part], bytes));
-        t->h_part_cap[part] = bytes;
+        size_t got = 0;
+        CK(PinCache::get().take(&t->h_part[part], bytes, &got));
+        t->h_part_cap[part] = got;
     }
     // offsets: every item's runs and samples, then the int32 arrays
     std::vector<size_t> o4(i1 - i0), o1(i1 - i0);
@@ -3302,11 +3335,12 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
     // while the loop runs does not wait for the stream
     const size_t dbytes = sizeof(OrientDesc) * (all.size() + allb.size());
     if (dbytes > t->h_desc_cap) {
-        if (t->h_desc) cudaFreeHost(t->h_desc);
+        PinCache::get().give(t->h_desc, t->h_desc_cap);
         t->h_desc = nullptr;
         t->h_desc_cap = 0;
-        CK(cudaMallocHost(&t->h_desc, dbytes));
-        t->h_desc_cap = dbytes;
+        size_t got = 0;
+        CK(PinCache::get().take(&t->h_desc, dbytes, &got));
+        t->h_desc_cap = got;
     }
     OrientDesc* hd_all = (OrientDesc*)t->h_desc;
     OrientDesc* hd_base = hd_all + all.size();
@@ -3322,9 +3356,12 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
             t->icmeta_cap = 0;
             TRY(dalloc(&t->d_icoff, (size_t)n_items, t->st));
             TRY(dalloc(&t->d_icstr, (size_t)n_items, t->st));
-            if (t->h_icmeta) cudaFreeHost(t->h_icmeta);
+            PinCache::get().give(t->h_icmeta, t->h_icmeta_cap);
             t->h_icmeta = nullptr;
-            CK(cudaMallocHost(&t->h_icmeta, (size_t)n_items * (sizeof(long long) + sizeof(int))));
+            t->h_icmeta_cap = 0;
+            size_t got = 0;
+            CK(PinCache::get().take(&t->h_icmeta, (size_t)n_items * (sizeof(long long) + sizeof(int)), &got));
+            t->h_icmeta_cap = got;
             t->icmeta_cap = n_items;
         }
         if ((size_t)n_items * n_orient > t->icn_cap) {

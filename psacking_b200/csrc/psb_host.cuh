@@ -20,6 +20,7 @@
 #include <cstring>
 #include <deque>
 #include <functional>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <thread>
@@ -139,6 +140,55 @@ inline void parallel_copy(void* dst, const void* src, size_t bytes) {
         memcpy((char*)dst + b, (const char*)src + b, e - b);
     });
 }
+
+// Pinned memory of the trays (staging, descriptors), kept when a tray is
+// destroyed and handed to the next one: cudaMallocHost and cudaFreeHost take
+// 0.5-5 ms each and stop the whole device, and a many-tray run makes a tray's
+// worth of them per tray.  At most kKeep bytes are kept.
+class PinCache {
+  public:
+    static constexpr size_t kKeep = (size_t)256 << 20;
+    static PinCache& get() {
+        static PinCache* p = new PinCache();
+        return *p;
+    }
+    // *got: the bytes it really has
+    cudaError_t take(void** out, size_t bytes, size_t* got) {
+        bytes = std::max(bytes, (size_t)4096);
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            auto it = free_.lower_bound(bytes);
+            if (it != free_.end() && it->first <= std::max(4 * bytes, (size_t)1 << 20)) {
+                *out = it->second;
+                *got = it->first;
+                kept_ -= it->first;
+                free_.erase(it);
+                return cudaSuccess;
+            }
+        }
+        // room to grow: the next user may need a little more
+        *got = (bytes + bytes / 4 + 4095) / 4096 * 4096;
+        return cudaHostAlloc(out, *got, cudaHostAllocPortable);
+    }
+    // nothing queued may use it any more
+    void give(void* p, size_t n) {
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (kept_ + n <= kKeep) {
+                free_.emplace(n, p);
+                kept_ += n;
+                return;
+            }
+        }
+        cudaFreeHost(p);
+    }
+
+  private:
+    std::mutex mu_;
+    std::multimap<size_t, void*> free_;
+    size_t kept_ = 0;
+};
 
 // Pinned blocks, shared by all threads: at most kBlocks per process of at most
 // kBlockMax bytes; a block is free again once the copies queued from it have
