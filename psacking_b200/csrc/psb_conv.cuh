@@ -16,6 +16,13 @@
 
 #include "psb_pdl.cuh"
 
+// one word to shared memory without waiting for it; zero where ok is false
+__device__ __forceinline__ void copy4_async(float* dst, const float* src, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(ok ? 4 : 0)
+                 : "memory");
+}
+
 __device__ __forceinline__ float bf16_up(uint16_t h) { return __uint_as_float((uint32_t)h << 16); }
 
 // ---------------------------------------------------------------------------
@@ -27,6 +34,10 @@ __device__ __forceinline__ float bf16_up(uint16_t h) { return __uint_as_float((u
 // the far side needs none) and each row holds its odd entries behind its even
 // ones, so neighbouring output positions read neighbouring words.
 // Per result the sum runs over channels, then taps, from the bias on.
+// Two CTAs per SM (128 registers): one sums while the other stages.  At 1,536
+// samples, layers 1 to 4: 277, 722, 332 and 237 us against 385, 849, 371 and 316
+// with one CTA of the first two and weights read down their columns (a sector
+// per lane).
 template <int CI, int D, int CO, int TV, int CH>
 struct ConvFwd {
     static constexpr int Do = D / 2, Do2 = Do * Do, Do3 = Do2 * Do;
@@ -35,19 +46,20 @@ struct ConvFwd {
     static constexpr int NS = VPC < Do3 ? 1 : VPC / Do3;        // samples per CTA
     static constexpr int IS = 2 * SL + 1, P = D + 1, HALF = (P + 1) / 2;   // staged slabs, row length
     static constexpr int ROW = 2 * HALF, SLAB = P * ROW, CHAN = IS * SLAB;
-    static constexpr size_t smem = sizeof(float) * ((size_t)NS * CH * CHAN + (size_t)CH * 27 * CO);
+    static constexpr int WR = CO + 4;   // a staged row of weights; padded for the stores, which go down a column
+    static constexpr size_t smem = sizeof(float) * ((size_t)NS * CH * CHAN + (size_t)CH * 27 * WR);
     static_assert(VPC % Do2 == 0 && (VPC < Do3 ? Do3 % VPC == 0 : VPC % Do3 == 0) && CI % CH == 0, "tile");
 };
 
 template <int CI, int D, int CO, int TV, int CH>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 k_conv3_fwd(const float* __restrict__ in, int S, const uint16_t* __restrict__ w, const float* __restrict__ bias,
             float* __restrict__ out) {
     pdl_enter();
     using C = ConvFwd<CI, D, CO, TV, CH>;
     extern __shared__ float4 csm4[];
-    float* ws = (float*)csm4;                    // [CH][27][CO]
-    float* xs = ws + CH * 27 * CO;               // [NS][CH][IS][P][ROW]
+    float* ws = (float*)csm4;                    // [CH][27][WR]
+    float* xs = ws + CH * 27 * C::WR;               // [NS][CH][IS][P][ROW]
     const int tid = threadIdx.x, vt = tid % C::NV, g = tid / C::NV;
     const long long v0 = (long long)blockIdx.x * C::VPC;
     const int s0 = (int)(v0 / C::Do3), od0 = (int)(v0 % C::Do3) / C::Do2;
@@ -68,12 +80,14 @@ k_conv3_fwd(const float* __restrict__ in, int S, const uint16_t* __restrict__ w,
     for (int i = tid; i < C::NS * CH * C::CHAN; i += 256) xs[i] = 0.f;   // the padding stays zero
     __syncthreads();
     for (int c0 = 0; c0 < CI; c0 += CH) {
+#pragma unroll 4
         for (int i = tid; i < CH * 27 * CO; i += 256) {
-            const int co = i % CO, t = i / CO % 27, c = i / (27 * CO);
-            ws[i] = bf16_up(w[((size_t)co * CI + c0 + c) * 27 + t]);
+            const int ct = i % (CH * 27), co = i / (CH * 27);
+            ws[ct * C::WR + co] = bf16_up(w[((size_t)co * CI + c0) * 27 + ct]);
         }
         // rows id = 2 od0 - 1 .. of each channel; staged index = id - (2 od0 - 1)
         constexpr int ROWS = C::IS * D;
+#pragma unroll 4
         for (int i = tid; i < ns * CH * ROWS * (D / 4); i += 256) {
             const int k4 = i % (D / 4), r = i / (D / 4) % ROWS, sc = i / (D / 4 * ROWS);
             const int sl = r / D, ih = r % D, id = 2 * od0 - 1 + sl;
@@ -92,12 +106,12 @@ k_conv3_fwd(const float* __restrict__ in, int S, const uint16_t* __restrict__ w,
 #pragma unroll 1
         for (int c = 0; c < CH; ++c) {
             const float* xc = xs + c * C::CHAN;
-            const float4* wc = (const float4*)(ws + c * 27 * CO + 8 * g);
+            const float4* wc = (const float4*)(ws + c * 27 * C::WR + 8 * g);
 #pragma unroll
             for (int t = 0; t < 27; ++t) {
                 const int kd = t / 9, kh = t / 3 % 3, kw = t % 3;
                 const int off = kd * C::SLAB + kh * C::ROW + (kw == 1 ? C::HALF : kw / 2);
-                const float4 wa = wc[t * (CO / 4)], wb = wc[t * (CO / 4) + 1];
+                const float4 wa = wc[t * (C::WR / 4)], wb = wc[t * (C::WR / 4) + 1];
 #pragma unroll
                 for (int i = 0; i < TV; ++i) {
                     const float x = xc[at[i] + off];
@@ -130,7 +144,9 @@ k_conv3_fwd(const float* __restrict__ in, int S, const uint16_t* __restrict__ w,
 // is 0 and taps 2 of d and 0 of d + 1 when it is 1.  A thread owns two
 // neighbouring cells (d, h, w), (d, h, w + 1), all eight parities of each and
 // four input channels: 12 output gradients and 27 weights per output channel
-// feed 54 FMAs per input channel.
+// feed 54 FMAs per input channel.  Held to 128 registers for two CTAs per SM
+// (with 132 there was one: 1,186 us for 16 <- 32 channels at 1,536 samples,
+// 837 with two).
 template <int CI, int D, int CO, int CH>
 struct ConvBwd {
     static constexpr int Do = D / 2, Do2 = Do * Do, Do3 = Do2 * Do;
@@ -143,7 +159,7 @@ struct ConvBwd {
 };
 
 template <int CI, int D, int CO, int CH>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 k_conv3_bwd_data(const float* __restrict__ dout, int S, const uint16_t* __restrict__ w, const float* __restrict__ in,
                  float* __restrict__ din) {
     pdl_enter();
@@ -169,11 +185,13 @@ k_conv3_bwd_data(const float* __restrict__ dout, int S, const uint16_t* __restri
     for (int i = tid; i < C::NS * CH * C::CHAN; i += 256) gs[i] = 0.f;
     __syncthreads();
     for (int c0 = 0; c0 < CO; c0 += CH) {
+#pragma unroll 4
         for (int i = tid; i < CH * CI * 27; i += 256) {
             const int t = i % 27, ci = i / 27 % CI, c = i / (27 * CI);
             ws[(c * CI + ci) * 28 + t] = bf16_up(w[((size_t)(c0 + c) * CI + ci) * 27 + t]);
         }
         constexpr int NVOX = (C::SL + 1) * C::Do2;
+#pragma unroll 4
         for (int i = tid; i < ns * CH * NVOX; i += 256) {
             const int r = i % NVOX, sc = i / NVOX, s = sc / CH, c = sc % CH;
             const int od = d0 + r / C::Do2;
@@ -241,19 +259,25 @@ k_conv3_bwd_data(const float* __restrict__ dout, int S, const uint16_t* __restri
 // CTA's threads cover CG input channels x all CO output channels, NSUB times
 // over, each copy taking its share of the staged rows of output positions.
 // Along a row the window slides by two inputs, so 18 of its 27 values are new
-// per position.  grid.x: input channel groups, grid.y: shares of the samples;
-// the copies meet in shared memory and each CTA adds its sums with one atomic
-// per weight (dw, db zeroed first).
+// per position.  171 registers a thread allow one CTA per SM, so nothing hides a
+// load's latency but the CTA itself: the next part's inputs and gradients come by
+// asynchronous copies into a second buffer while this part is summed (16 -> 32
+// channels at 1,536 samples: 2.28 ms staged in turn with the sums, 0.98 ms so
+// with 16 loads in flight, 0.77 ms with two buffers).  grid.x: input channel
+// groups, grid.y: shares of the samples; the copies meet in shared memory and
+// each CTA adds its sums with one atomic per weight (dw, db zeroed first).
 template <int CI, int D, int CO, int CG, int SL, int NS, int SEG>
 struct ConvBwdW {
     static constexpr int Do = D / 2, Do2 = Do * Do, Do3 = Do2 * Do;
     static constexpr int NQ = CO / 4, NSUB = 256 / (CG * NQ);
     static constexpr int IS = 2 * SL + 1, P = D + 1, SLAB = P * P, CHAN = IS * SLAB;
     static constexpr int NVOX = SL * Do2, SEGS = NS * NVOX / SEG;
-    static constexpr size_t stage = (size_t)NS * NVOX * CO + (size_t)NS * CG * CHAN;
+    static constexpr int GR = CO + 4;   // a staged position's gradients: 8 positions x 4 channels on 32 banks
+    static constexpr size_t stage = (size_t)NS * NVOX * GR + (size_t)NS * CG * CHAN;
     static constexpr size_t red = (size_t)CG * NQ * 108 + CO;
-    static constexpr size_t smem = sizeof(float) * (stage > red ? stage : red);
+    static constexpr size_t smem = sizeof(float) * (2 * stage > red ? 2 * stage : red);
     static_assert(256 % (CG * NQ) == 0 && Do % SEG == 0 && Do % SL == 0 && CI % CG == 0, "tile");
+    static_assert(NVOX % 8 == 0 && CO % 4 == 0, "staging");
 };
 
 template <int CI, int D, int CO, int CG, int SL, int NS, int SEG>
@@ -264,8 +288,8 @@ k_conv3_bwd_weight(const float* __restrict__ dout, const float* __restrict__ in,
     using C = ConvBwdW<CI, D, CO, CG, SL, NS, SEG>;
     constexpr int Do = C::Do;
     extern __shared__ float4 csm4[];
-    float* gs = (float*)csm4;                    // [NS][NVOX][CO]
-    float* xs = gs + NS * C::NVOX * CO;          // [NS][CG][IS][P][P]
+    float* sm = (float*)csm4;                    // 2 x (gs [NS][NVOX][GR], xs [NS][CG][IS][P][P])
+    constexpr int GS = NS * C::NVOX * C::GR, XS = NS * CG * C::CHAN;
     const int tid = threadIdx.x, q = tid % C::NQ, cg = tid / C::NQ % CG, sub = tid / (C::NQ * CG);
     const int c0 = blockIdx.x * CG, sa = blockIdx.y * chunk, sb = min(S, sa + chunk);
     const bool bias = blockIdx.x == 0 && cg == 0;
@@ -276,63 +300,70 @@ k_conv3_bwd_weight(const float* __restrict__ dout, const float* __restrict__ in,
 #pragma unroll
         for (int t = 0; t < 27; ++t) acc[k][t] = 0.f;
     }
-    for (int i = tid; i < NS * CG * C::CHAN; i += 256) xs[i] = 0.f;
+    for (int i = tid; i < XS; i += 256) sm[2 * GS + i] = sm[2 * GS + XS + i] = 0.f;   // the padding stays zero
     __syncthreads();
-    for (int s0 = sa; s0 < sb; s0 += NS) {
-        const int ns = min(NS, sb - s0);
-        for (int od0 = 0; od0 < Do; od0 += SL) {
-            // four positions per load, channels across the lanes: the stores
-            // fall on distinct banks
-            for (int i = tid; i < ns * CO * (C::NVOX / 4); i += 256) {
-                const int c = i % CO, sv = i / CO, s = sv / (C::NVOX / 4), v = sv % (C::NVOX / 4) * 4;
-                const float4 g = __ldg(
-                    (const float4*)(dout + ((size_t)(s0 + s) * CO + c) * C::Do3 + (size_t)od0 * C::Do2 + v));
-                float* d = gs + (s * C::NVOX + v) * CO + c;
-                d[0] = g.x;
-                d[CO] = g.y;
-                d[2 * CO] = g.z;
-                d[3 * CO] = g.w;
-            }
-            constexpr int VIN = C::IS * D * D;
-            for (int i = tid; i < ns * CG * VIN; i += 256) {
-                const int v = i % VIN, sc = i / VIN, s = sc / CG, c = sc % CG;
-                const int sl = v / (D * D), id = 2 * od0 - 1 + sl;
-                float x = 0.f;
-                if (id >= 0) x = __ldg(&in[(((size_t)(s0 + s) * CI + c0 + c) * D + id) * D * D + v % (D * D)]);
-                xs[(s * CG + c) * C::CHAN + sl * C::SLAB + (v / D % D + 1) * C::P + v % D + 1] = x;
-            }
-            __syncthreads();
-            for (int e = sub; e < ns * (C::NVOX / SEG); e += C::NSUB) {
-                const int s = e / (C::NVOX / SEG), v = e % (C::NVOX / SEG) * SEG;
-                const int sl = v / C::Do2, oh = v / Do % Do, ow = v % Do;
-                const float4* gr = (const float4*)(gs + (s * C::NVOX + v) * CO) + q;
-                const float* x = xs + (s * CG + cg) * C::CHAN + 2 * sl * C::SLAB + 2 * oh * C::P + 2 * ow;
-                float win[9][3];
+    constexpr int PARTS = Do / SL;
+    const int steps = sb > sa ? (sb - sa + NS - 1) / NS * PARTS : 0;
+    auto stage = [&](int step) {
+        const int s0 = sa + step / PARTS * NS, od0 = step % PARTS * SL, ns = min(NS, sb - s0);
+        float* gs = sm + step % 2 * GS;
+        float* xs = sm + 2 * GS + step % 2 * XS;
+        // a warp takes 8 positions x 4 channels: whole sectors, distinct banks
+#pragma unroll 4
+        for (int i = tid; i < ns * C::NVOX * CO; i += 256) {
+            const int v8 = i % 8, c4 = i / 8 % 4, cq = i / 32 % (CO / 4), sv = i / (8 * CO);
+            const int c = 4 * cq + c4, s = sv / (C::NVOX / 8), v = sv % (C::NVOX / 8) * 8 + v8;
+            copy4_async(gs + (s * C::NVOX + v) * C::GR + c,
+                        dout + ((size_t)(s0 + s) * CO + c) * C::Do3 + (size_t)od0 * C::Do2 + v, true);
+        }
+        constexpr int VIN = C::IS * D * D;
+#pragma unroll 4
+        for (int i = tid; i < ns * CG * VIN; i += 256) {
+            const int v = i % VIN, sc = i / VIN, s = sc / CG, c = sc % CG;
+            const int sl = v / (D * D), id = 2 * od0 - 1 + sl;
+            const float* src = in + (((size_t)(s0 + s) * CI + c0 + c) * D + max(id, 0)) * D * D + v % (D * D);
+            copy4_async(xs + (s * CG + c) * C::CHAN + sl * C::SLAB + (v / D % D + 1) * C::P + v % D + 1, src, id >= 0);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (steps) stage(0);
+    for (int step = 0; step < steps; ++step) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();   // this part has landed for all; the other buffer is read by nobody any more
+        if (step + 1 < steps) stage(step + 1);
+        const int ns = min(NS, sb - (sa + step / PARTS * NS));
+        const float* gs = sm + step % 2 * GS;
+        const float* xs = sm + 2 * GS + step % 2 * XS;
+        for (int e = sub; e < ns * (C::NVOX / SEG); e += C::NSUB) {
+            const int s = e / (C::NVOX / SEG), v = e % (C::NVOX / SEG) * SEG;
+            const int sl = v / C::Do2, oh = v / Do % Do, ow = v % Do;
+            const float4* gr = (const float4*)(gs + (s * C::NVOX + v) * C::GR) + q;
+            const float* x = xs + (s * CG + cg) * C::CHAN + 2 * sl * C::SLAB + 2 * oh * C::P + 2 * ow;
+            float win[9][3];
 #pragma unroll
-                for (int r = 0; r < 9; ++r) win[r][2] = x[r / 3 * C::SLAB + r % 3 * C::P];
+            for (int r = 0; r < 9; ++r) win[r][2] = x[r / 3 * C::SLAB + r % 3 * C::P];
 #pragma unroll 2
-                for (int i = 0; i < SEG; ++i) {
+            for (int i = 0; i < SEG; ++i) {
 #pragma unroll
-                    for (int r = 0; r < 9; ++r) {
-                        win[r][0] = win[r][2];
-                        win[r][1] = x[r / 3 * C::SLAB + r % 3 * C::P + 2 * i + 1];
-                        win[r][2] = x[r / 3 * C::SLAB + r % 3 * C::P + 2 * i + 2];
-                    }
-                    const float4 g = gr[i * (CO / 4)];
-                    const float gv[4] = {g.x, g.y, g.z, g.w};
+                for (int r = 0; r < 9; ++r) {
+                    win[r][0] = win[r][2];
+                    win[r][1] = x[r / 3 * C::SLAB + r % 3 * C::P + 2 * i + 1];
+                    win[r][2] = x[r / 3 * C::SLAB + r % 3 * C::P + 2 * i + 2];
+                }
+                const float4 g = gr[i * (C::GR / 4)];
+                const float gv[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
+                for (int k = 0; k < 4; ++k) {
 #pragma unroll
-                        for (int t = 0; t < 27; ++t) acc[k][t] = fmaf(gv[k], win[t / 3][t % 3], acc[k][t]);
-                        if (bias) bacc[k] += gv[k];
-                    }
+                    for (int t = 0; t < 27; ++t) acc[k][t] = fmaf(gv[k], win[t / 3][t % 3], acc[k][t]);
+                    if (bias) bacc[k] += gv[k];
                 }
             }
-            __syncthreads();
         }
     }
+    __syncthreads();   // the buffers become the sums'
     // the copies' sums, one copy after another
-    float* red = gs;                             // [CG * NQ][108], then [CO]
+    float* red = sm;                             // [CG * NQ][108], then [CO]
     float* rb = red + CG * C::NQ * 108;
     const int slot = cg * C::NQ + q;
     for (int k = 0; k < C::NSUB; ++k) {
@@ -360,58 +391,91 @@ k_conv3_bwd_weight(const float* __restrict__ dout, const float* __restrict__ in,
 // ---------------------------------------------------------------------------
 // linear layers: C[M][N] = sum over k of A(m, k) B(k, n)
 // ---------------------------------------------------------------------------
-// 64 x 64 tile per CTA, 4 x 4 results per thread, 16 k at a time in shared
-// memory.  OP 0: y = x W^T + b (A = x [M][K], B = BF16 W [N][K]); OP 1: dx = dy W
-// (A = dy [M][K], B = BF16 W [K][N]), times the ReLU mask of x when xmask is
-// given; OP 2: dW = dy^T x (A = dy [K][M], B = x [K][N]), grid.z shares of k
-// added with atomics (dW zeroed first), with db[m] = sum over k of dy[k][m].
+// 16 R x 64 tile per CTA, R x 4 results per thread, BK terms at a time in
+// shared memory, the next BK on their way to registers meanwhile.  OP 0: y = x
+// W^T + b (A = x [M][K], B = BF16 W [N][K]); OP 1: dx = dy W (A = dy [M][K], B =
+// BF16 W [K][N]), times the ReLU mask of x when xmask is given; OP 2: dW = dy^T
+// x (A = dy [K][M], B = x [K][N]), grid.z shares of k added with atomics (dW
+// zeroed first), with db[m] = sum over k of dy[k][m].
+// The layers are a few MFLOP: what bounds them is the chain of K / BK loads, one
+// memory latency each where nothing is prefetched, on the few CTAs that N = 64
+// leaves.  So the forward layers, whose sum is one chain over K, take R = 1 and
+// BK = 32: 512 -> 64 over 1,536 rows 75 -> 27 us, 1,024 -> 64 over 64 rows 144 ->
+// 54 us (cold caches).
+template <int OP>
+struct LinTile {
+    static constexpr int R = OP == 0 ? 1 : 4, BK = OP == 0 ? 32 : 16, BM = 16 * R;
+};
 template <int OP>
 __global__ void __launch_bounds__(256)
 k_linear(const float* __restrict__ a, const void* __restrict__ b, int M, int N, int K, const float* __restrict__ bias,
          int relu, const float* __restrict__ xmask, float* __restrict__ c, float* __restrict__ db, int kchunk) {
     pdl_enter();
-    __shared__ float As[16][68], Bs[16][68];
+    constexpr int R = LinTile<OP>::R, BK = LinTile<OP>::BK, BM = LinTile<OP>::BM;
+    constexpr int NA = BK * BM / 256, NB = BK * 64 / 256;
+    __shared__ float As[BK][BM + 4], Bs[BK][68];
     const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * 64;
     const int ka = OP == 2 ? blockIdx.z * kchunk : 0, kb = OP == 2 ? min(K, ka + kchunk) : K;
-    float acc[4][4], bsum = 0.f;
+    float acc[R][4], bsum = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = OP == 0 && n0 + 4 * tx + j < N ? bias[n0 + 4 * tx + j] : 0.f;
-    for (int k0 = ka; k0 < kb; k0 += 16) {
-        for (int i = tid; i < 16 * 64; i += 256) {
-            // along the operand's contiguous index
-            const int ak = OP == 2 ? i / 64 : i % 16, am = OP == 2 ? i % 64 : i / 16;
-            float v = 0.f;
+    float pa[NA], pb[NB];
+    // element e of the tiles' loads, along the operand's contiguous index
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int e = 0; e < NA; ++e) {
+            const int i = tid + 256 * e;
+            const int ak = OP == 2 ? i / BM : i % BK, am = OP == 2 ? i % BM : i / BK;
+            pa[e] = 0.f;
             if (k0 + ak < kb && m0 + am < M)
-                v = OP == 2 ? a[(size_t)(k0 + ak) * M + m0 + am] : a[(size_t)(m0 + am) * K + k0 + ak];
-            As[ak][am] = v;
-            const int bk = OP == 0 ? i % 16 : i / 64, bn = OP == 0 ? i / 16 : i % 64;
-            float u = 0.f;
+                pa[e] = OP == 2 ? a[(size_t)(k0 + ak) * M + m0 + am] : a[(size_t)(m0 + am) * K + k0 + ak];
+        }
+#pragma unroll
+        for (int e = 0; e < NB; ++e) {
+            const int i = tid + 256 * e;
+            const int bk = OP == 0 ? i % BK : i / 64, bn = OP == 0 ? i / BK : i % 64;
+            pb[e] = 0.f;
             if (k0 + bk < kb && n0 + bn < N)
-                u = OP == 0 ? bf16_up(((const uint16_t*)b)[(size_t)(n0 + bn) * K + k0 + bk])
-                  : OP == 1 ? bf16_up(((const uint16_t*)b)[(size_t)(k0 + bk) * N + n0 + bn])
-                            : ((const float*)b)[(size_t)(k0 + bk) * N + n0 + bn];
-            Bs[bk][bn] = u;
+                pb[e] = OP == 0 ? bf16_up(((const uint16_t*)b)[(size_t)(n0 + bn) * K + k0 + bk])
+                      : OP == 1 ? bf16_up(((const uint16_t*)b)[(size_t)(k0 + bk) * N + n0 + bn])
+                                : ((const float*)b)[(size_t)(k0 + bk) * N + n0 + bn];
+        }
+    };
+    fetch(ka);
+    for (int k0 = ka; k0 < kb; k0 += BK) {
+#pragma unroll
+        for (int e = 0; e < NA; ++e) {
+            const int i = tid + 256 * e;
+            As[OP == 2 ? i / BM : i % BK][OP == 2 ? i % BM : i / BK] = pa[e];
+        }
+#pragma unroll
+        for (int e = 0; e < NB; ++e) {
+            const int i = tid + 256 * e;
+            Bs[OP == 0 ? i % BK : i / 64][OP == 0 ? i / BK : i % 64] = pb[e];
         }
         __syncthreads();
+        fetch(k0 + BK);   // past kb: zeros, without a load
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            const float4 av = *(const float4*)&As[k][4 * ty], bv = *(const float4*)&Bs[k][4 * tx];
-            const float x[4] = {av.x, av.y, av.z, av.w}, y[4] = {bv.x, bv.y, bv.z, bv.w};
+        for (int k = 0; k < BK; ++k) {
+            const float4 bv = *(const float4*)&Bs[k][4 * tx];
+            const float y[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < R; ++i) {
+                const float x = As[k][R * ty + i];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(x, y[j], acc[i][j]);
+            }
         }
-        if (OP == 2 && blockIdx.x == 0 && tid < 64)
-            for (int k = 0; k < 16; ++k) bsum += As[k][tid];
+        if (OP == 2 && blockIdx.x == 0 && tid < BM)
+            for (int k = 0; k < BK; ++k) bsum += As[k][tid];
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + 4 * ty + i;
+    for (int i = 0; i < R; ++i) {
+        const int m = m0 + R * ty + i;
         if (m >= M) continue;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -423,5 +487,5 @@ k_linear(const float* __restrict__ a, const void* __restrict__ b, int M, int N, 
             else c[at] = relu ? fmaxf(acc[i][j], 0.f) : acc[i][j];
         }
     }
-    if (OP == 2 && blockIdx.x == 0 && tid < 64 && m0 + tid < M) atomicAdd(&db[m0 + tid], bsum);
+    if (OP == 2 && blockIdx.x == 0 && tid < BM && m0 + tid < M) atomicAdd(&db[m0 + tid], bsum);
 }

@@ -488,7 +488,7 @@ int set_smem_attrs() {
     TRY(set_max_dyn_smem(k_conv3_bwd_data<16, 16, 32, 8>));
     TRY(set_max_dyn_smem(k_conv3_bwd_weight<64, 4, 64, 16, 2, 8, 2>));
     TRY(set_max_dyn_smem(k_conv3_bwd_weight<32, 8, 64, 8, 4, 2, 4>));
-    TRY(set_max_dyn_smem(k_conv3_bwd_weight<16, 16, 32, 4, 8, 1, 8>));
+    TRY(set_max_dyn_smem(k_conv3_bwd_weight<16, 16, 32, 4, 4, 1, 8>));
     TRY(set_max_dyn_smem(k_conv3_bwd_weight<1, 32, 16, 1, 2, 1, 8>));
     TRY(set_max_dyn_smem(k_cand_filter_plane<1>));
     TRY(set_max_dyn_smem(k_cand_filter_plane<2>));
@@ -2500,15 +2500,15 @@ struct psb_proposal {
         return lin_fwd(a4, S, 512, kProp.f1, 64, 1, f1, s);
     }
     int lin_fwd(const float* x, int M, int K, const PropLayer& L, int N, int relu, float* y, cudaStream_t s) {
-        pdl(k_linear<0>, dim3((N + 63) / 64, (M + 63) / 64), 256, 0, s)(x, (const void*)(P16 + L.w), M, N, K, P + L.b,
-                                                                      relu, nullptr, y, nullptr, 0);
+        pdl(k_linear<0>, dim3((N + 63) / 64, (M + LinTile<0>::BM - 1) / LinTile<0>::BM), 256, 0, s)(
+            x, (const void*)(P16 + L.w), M, N, K, P + L.b, relu, nullptr, y, nullptr, 0);
         CKL();
         return PSB_OK;
     }
     // dx [M][K] = dy [M][N] W, masked
     int lin_bwd_data(const float* dy, int M, int N, const PropLayer& L, int K, const float* xmask, float* dx,
                      cudaStream_t s) {
-        pdl(k_linear<1>, dim3((K + 63) / 64, (M + 63) / 64), 256, 0, s)(dy, (const void*)(P16 + L.w), M, K, N, nullptr,
+        pdl(k_linear<1>, dim3((K + 63) / 64, (M + LinTile<1>::BM - 1) / LinTile<1>::BM), 256, 0, s)(dy, (const void*)(P16 + L.w), M, K, N, nullptr,
                                                                       0, xmask, dx, nullptr, 0);
         CKL();
         return PSB_OK;
@@ -2586,7 +2586,7 @@ struct psb_proposal {
         TRY((conv_bwd_data<64, 4, 64, 8>(da4, S, kProp.c[3], a3, da3, s)));
         TRY((conv_bwd_weight<32, 8, 64, 8, 4, 2, 4>(da3, a2, S, kProp.c[2], s)));
         TRY((conv_bwd_data<32, 8, 64, 8>(da3, S, kProp.c[2], a2, da2, s)));
-        TRY((conv_bwd_weight<16, 16, 32, 4, 8, 1, 8>(da2, a1, S, kProp.c[1], s)));
+        TRY((conv_bwd_weight<16, 16, 32, 4, 4, 1, 8>(da2, a1, S, kProp.c[1], s)));
         TRY((conv_bwd_data<16, 16, 32, 8>(da2, S, kProp.c[1], a1, da1, s)));
         TRY((conv_bwd_weight<1, 32, 16, 1, 2, 1, 8>(da1, grids, S, kProp.c[0], s)));
         return PSB_OK;
@@ -3500,7 +3500,7 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
             const int m = std::min(kChunk, n_items - i0);
             {
                 PROF("k_prop_inputs", t->st);
-                pdl(k_orient_grids, dim3(PSB_PG3 / 256, n_orient, m), 256, 0, t->st)(
+                pdl(k_orient_grids, dim3(PSB_PG3 / 1024, n_orient, m), 256, 0, t->st)(
                     d_pgrid + (size_t)i0 * PSB_PG3, d_pG + 3 * i0, d_pmaps, n_orient, pr->a0);
             }
             CKL();
@@ -3981,7 +3981,7 @@ int psb_prop_item_grids(const int32_t* const* items, const int32_t* dims, int n_
         pdl(k_base_grid_dense, dim3(PSB_PG3 / 256, m), 256, 0, st)((const int32_t*)(d + ov), (const GridItem*)d + i0,
                                                                  grid + (size_t)i0 * PSB_PG3);
         CKL();
-        pdl(k_orient_grids, dim3(PSB_PG3 / 256, n_orient, m), 256, 0, st)(
+        pdl(k_orient_grids, dim3(PSB_PG3 / 1024, n_orient, m), 256, 0, st)(
             grid + (size_t)i0 * PSB_PG3, (const int*)(d + oG) + 3 * i0, (const int*)(d + om), n_orient,
             d_out + (size_t)i0 * n_orient * PSB_PG3);
         CKL();

@@ -75,3 +75,27 @@ def test_layers_match_float64(gpu_core, B, offset):
         scale = max(np.abs(w).max(), 1e-3 * gmax)
         assert np.abs(got[off:off + w.size] - w).max() <= 2e-3 * scale, name
         off += w.size
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_item_grids_any_destination(gpu_core, offset):
+    """Extents that end inside a group of four cells, and destinations that
+    start 0, 4 and 8 bytes past a 16-byte boundary: equal to the oracle, and
+    nothing written before or behind."""
+    import torch
+    from psacking_b200 import proposal
+    from psacking_b200.rotations import orientation_maps
+    rng = np.random.default_rng(9)
+    maps = np.ascontiguousarray(orientation_maps(24), np.int32)
+    items = [(rng.random(s) < 0.5).astype(np.int32) for s in [(1, 2, 3), (5, 7, 6), (33, 9, 31), (2, 64, 1)]]
+    n = len(items) * 24 * 32 ** 3
+    buf = torch.full((n + 8,), -1.0, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    arr, dims = proposal._ptrs(items)
+    proposal.check(proposal.lib().psb_prop_item_grids(arr, dims.ctypes.data, len(items), maps.ctypes.data, len(maps),
+                                                      buf.data_ptr() + 4 * offset))
+    got = buf.cpu().numpy()
+    assert (got[:offset] == -1).all() and (got[offset + n:] == -1).all()
+    got = got[offset:offset + n].reshape(len(items), 24, 32, 32, 32)
+    for k, it in enumerate(items):
+        assert np.array_equal(got[k], P.oriented_grids(it, maps)), k
