@@ -149,8 +149,9 @@ int psb_tray_destroy(psb_tray* t);
 int psb_tray_dims(const psb_tray* t, int* nx, int* ny, int* nz);
 
 /* gpu_tray_context_init (fft3.cu:1106-1175): upload the tray and its distance
- * field and build both spectra.  phi == NULL computes the distance field on
- * the device from the tray. */
+ * field.  phi == NULL computes the distance field on the device from the tray.
+ * What the searches derive from the two (spectra, free bits, bounds) is built
+ * when a search first needs it. */
 int psb_tray_set(psb_tray* t, const int32_t* tray, const int32_t* phi);
 
 /* Copy the device tray / distance field back to the host. */
@@ -306,13 +307,17 @@ int psb_set_plane_variant(int v);
  * orientations or x planes) blocked; those are skipped, every other cell is
  * decided exactly as before.  It starts once the tray's occupied cells plus
  * the items searched so far reach a quarter of the tray (before that it
- * rarely rules anything out).  Same placements either way; the switch exists
- * for comparisons.  No counterpart in the reference. */
+ * rarely rules anything out).  The score-bound search, which answers most
+ * items of a run and most searches without transforms, is built on the same
+ * test: off, every item and search runs the transforms, unfiltered.  Same
+ * placements either way; the switch exists for comparisons.  No counterpart in
+ * the reference. */
 int psb_set_cand_filter(int on);
 /* Orientations the pre-filter leaves with at most n candidate translations
  * (default 4096; 0 disables) skip the transforms: each candidate is checked
  * exactly against the item's voxel columns and the free ones are scored by
- * exact integer proximity sums.  Same placements either way. */
+ * exact integer proximity sums.  0 also turns the score-bound search off, so
+ * that every item runs the transforms.  Same placements either way. */
 int psb_set_direct_max(int n);
 /* Pre-filter cut-off: a group of 32 translations stops testing samples when,
  * after 32 samples, more than pct % of them still pass (open space, nothing

@@ -989,7 +989,6 @@ struct psb_tray {
     double* d_pen = nullptr;
     RzDesc* d_rz = nullptr;
     MidDesc* d_mid = nullptr;
-    unsigned long long* d_stats = nullptr;
     unsigned int* d_err = nullptr;
     unsigned long long* d_first = nullptr;
 
@@ -1144,7 +1143,7 @@ struct psb_tray {
         release_slots();
         dfree(d_tray, st); dfree(d_phi, st); dfree(d_Socc, st); dfree(d_Sphi, st); dfree(d_w1, st); dfree(d_w2, st); dfree(d_wocc, st); dfree(d_pen, st);
         dfree(d_ostat, st);
-        dfree(d_rz, st); dfree(d_mid, st); dfree(d_stats, st); dfree(d_err, st); dfree(d_first, st); dfree(d_needff, st); dfree(d_x, st);
+        dfree(d_rz, st); dfree(d_mid, st); dfree(d_err, st); dfree(d_first, st); dfree(d_needff, st); dfree(d_x, st);
         x_cap = 0;
         dfree(d_pphi, st); dfree(d_pocc, st);
         dfree(d_ls, st); dfree(d_ps, st); dfree(d_rzd, st); dfree(d_midd, st); dfree(d_od_all, st); dfree(d_base_all, st); dfree(d_dec, st);
@@ -1203,7 +1202,7 @@ struct psb_tray {
         TRY(dalloc(&d_Socc, S, st)); TRY(dalloc(&d_Sphi, S, st));
         TRY(dalloc(&d_w1, (size_t)nx * ny * g.H, st)); TRY(dalloc(&d_w2, (size_t)nx * g.F[1] * g.H, st));
         TRY(dalloc(&d_wocc, (size_t)nx * g.F[1] * g.H, st));
-        TRY(dalloc(&d_pen, 3 * (size_t)nz, st)); TRY(dalloc(&d_rz, 4, st)); TRY(dalloc(&d_mid, 4, st)); TRY(dalloc(&d_stats, 4, st));
+        TRY(dalloc(&d_pen, 3 * (size_t)nz, st)); TRY(dalloc(&d_rz, 4, st)); TRY(dalloc(&d_mid, 4, st));
         TRY(dalloc(&d_work, 8, st));
         CK(cudaMemsetAsync(d_work, 0, sizeof(unsigned long long) * 8, st));
         TRY(dalloc(&d_err, 1, st)); TRY(dalloc(&d_first, 1, st)); TRY(dalloc(&d_needff, 1, st));

@@ -885,13 +885,6 @@ __global__ void k_dist_axis_global(int32_t* __restrict__ d, int axis, int nx, in
     for (int p = 1; p < L; ++p) d[b + p * stride] = min(d[b + p * stride], d[b + (p - 1) * stride] + 1);
 }
 
-// any negative value?
-__global__ void k_any_negative(const int32_t* __restrict__ v, size_t n, unsigned int* flag) {
-    pdl_enter();
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        if (v[i] < 0) { atomicOr(flag, 1u); return; }
-}
-
 // collision_grid post-pass: out-of-tray positions raised to max(c, 1)
 __global__ void k_oob_raise(int32_t* __restrict__ c, int nx, int ny, int nz, int hx, int hy, int hz) {
     pdl_enter();
