@@ -146,7 +146,9 @@ k_conv3_fwd(const float* __restrict__ in, int S, const uint16_t* __restrict__ w,
 // four input channels: 12 output gradients and 27 weights per output channel
 // feed 54 FMAs per input channel.  Held to 128 registers for two CTAs per SM
 // (with 132 there was one: 1,186 us for 16 <- 32 channels at 1,536 samples,
-// 837 with two).
+// 837 with two).  Where the weights of all output channels fit beside the
+// gradients (CH = CO) the CTAs stay and take tile after tile, the weights
+// staged once: 692 us.
 template <int CI, int D, int CO, int CH>
 struct ConvBwd {
     static constexpr int Do = D / 2, Do2 = Do * Do, Do3 = Do2 * Do;
@@ -169,85 +171,90 @@ k_conv3_bwd_data(const float* __restrict__ dout, int S, const uint16_t* __restri
     float* ws = (float*)csm4;                    // [CH][CI][28]
     float* gs = ws + CH * CI * 28;               // [NS][CH][SL + 1][P][P]
     const int tid = threadIdx.x, pt = tid % C::NP, g = tid / C::NP;
-    const long long v0 = (long long)blockIdx.x * C::CELLS;
-    const int s0 = (int)(v0 / C::Do3), d0 = (int)(v0 % C::Do3) / C::Do2;
-    const int ns = min(C::NS, S - s0);
+    const long long ntiles = ((long long)S * C::Do3 + C::CELLS - 1) / C::CELLS;
     // this thread's cell pair
     const int cell = 2 * pt, cs = cell / (C::SL * C::Do2), q = cell % (C::SL * C::Do2);
     const int d = q / C::Do2, h = q / Do % Do, cw = q % Do;
-    float acc[4][2][8];
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-#pragma unroll
-            for (int p = 0; p < 8; ++p) acc[c][e][p] = 0.f;
-    for (int i = tid; i < C::NS * CH * C::CHAN; i += 256) gs[i] = 0.f;
+    for (int i = tid; i < C::NS * CH * C::CHAN; i += 256) gs[i] = 0.f;   // the far side stays zero
     __syncthreads();
-    for (int c0 = 0; c0 < CO; c0 += CH) {
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const long long v0 = tile * C::CELLS;
+        const int s0 = (int)(v0 / C::Do3), d0 = (int)(v0 % C::Do3) / C::Do2;
+        const int ns = min(C::NS, S - s0);
+        float acc[4][2][8];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int p = 0; p < 8; ++p) acc[c][e][p] = 0.f;
+        for (int c0 = 0; c0 < CO; c0 += CH) {
+            if (CH < CO || tile == blockIdx.x) {
 #pragma unroll 4
-        for (int i = tid; i < CH * CI * 27; i += 256) {
-            const int t = i % 27, ci = i / 27 % CI, c = i / (27 * CI);
-            ws[(c * CI + ci) * 28 + t] = bf16_up(w[((size_t)(c0 + c) * CI + ci) * 27 + t]);
-        }
-        constexpr int NVOX = (C::SL + 1) * C::Do2;
-#pragma unroll 4
-        for (int i = tid; i < ns * CH * NVOX; i += 256) {
-            const int r = i % NVOX, sc = i / NVOX, s = sc / CH, c = sc % CH;
-            const int od = d0 + r / C::Do2;
-            if (od >= Do) continue;
-            gs[(s * CH + c) * C::CHAN + r / C::Do2 * C::SLAB + r / Do % Do * C::P + r % Do] =
-                __ldg(&dout[((size_t)(s0 + s) * CO + c0 + c) * C::Do3 + (size_t)od * C::Do2 + r % C::Do2]);
-        }
-        __syncthreads();
-#pragma unroll 1
-        for (int c = 0; c < CH; ++c) {
-            const float* gc = gs + (cs * CH + c) * C::CHAN + d * C::SLAB + h * C::P + cw;
-            float x[2][2][3];
-#pragma unroll
-            for (int a = 0; a < 2; ++a)
-#pragma unroll
-                for (int b = 0; b < 2; ++b)
-#pragma unroll
-                    for (int e = 0; e < 3; ++e) x[a][b][e] = gc[a * C::SLAB + b * C::P + e];
-#pragma unroll
-            for (int ci = 0; ci < 4; ++ci) {
-                const float4* w4 = (const float4*)(ws + (c * CI + 4 * g + ci) * 28);
-                float wt[28];
-#pragma unroll
-                for (int k = 0; k < 7; ++k) {
-                    const float4 v = w4[k];
-                    wt[4 * k] = v.x;
-                    wt[4 * k + 1] = v.y;
-                    wt[4 * k + 2] = v.z;
-                    wt[4 * k + 3] = v.w;
-                }
-#pragma unroll
-                for (int t = 0; t < 27; ++t) {
-                    // tap 1: parity 0, output d; tap 2: parity 1, d; tap 0: parity 1, d + 1
-                    const int kd = t / 9, kh = t / 3 % 3, kw = t % 3;
-                    const int p = (kd != 1) * 4 + (kh != 1) * 2 + (kw != 1);
-                    acc[ci][0][p] = fmaf(x[kd == 0][kh == 0][kw == 0], wt[t], acc[ci][0][p]);
-                    acc[ci][1][p] = fmaf(x[kd == 0][kh == 0][1 + (kw == 0)], wt[t], acc[ci][1][p]);
+                for (int i = tid; i < CH * CI * 27; i += 256) {
+                    const int t = i % 27, ci = i / 27 % CI, c = i / (27 * CI);
+                    ws[(c * CI + ci) * 28 + t] = bf16_up(w[((size_t)(c0 + c) * CI + ci) * 27 + t]);
                 }
             }
+            constexpr int NVOX = (C::SL + 1) * C::Do2;
+#pragma unroll 4
+            for (int i = tid; i < ns * CH * NVOX; i += 256) {
+                const int r = i % NVOX, sc = i / NVOX, s = sc / CH, c = sc % CH;
+                const int od = d0 + r / C::Do2;
+                float x = 0.f;
+                if (od < Do) x = __ldg(&dout[((size_t)(s0 + s) * CO + c0 + c) * C::Do3 + (size_t)od * C::Do2 + r % C::Do2]);
+                gs[(s * CH + c) * C::CHAN + r / C::Do2 * C::SLAB + r / Do % Do * C::P + r % Do] = x;
+            }
+            __syncthreads();
+#pragma unroll 1
+            for (int c = 0; c < CH; ++c) {
+                const float* gc = gs + (cs * CH + c) * C::CHAN + d * C::SLAB + h * C::P + cw;
+                float x[2][2][3];
+#pragma unroll
+                for (int a = 0; a < 2; ++a)
+#pragma unroll
+                    for (int b = 0; b < 2; ++b)
+#pragma unroll
+                        for (int e = 0; e < 3; ++e) x[a][b][e] = gc[a * C::SLAB + b * C::P + e];
+#pragma unroll
+                for (int ci = 0; ci < 4; ++ci) {
+                    const float4* w4 = (const float4*)(ws + (c * CI + 4 * g + ci) * 28);
+                    float wt[28];
+#pragma unroll
+                    for (int k = 0; k < 7; ++k) {
+                        const float4 v = w4[k];
+                        wt[4 * k] = v.x;
+                        wt[4 * k + 1] = v.y;
+                        wt[4 * k + 2] = v.z;
+                        wt[4 * k + 3] = v.w;
+                    }
+#pragma unroll
+                    for (int t = 0; t < 27; ++t) {
+                        // tap 1: parity 0, output d; tap 2: parity 1, d; tap 0: parity 1, d + 1
+                        const int kd = t / 9, kh = t / 3 % 3, kw = t % 3;
+                        const int p = (kd != 1) * 4 + (kh != 1) * 2 + (kw != 1);
+                        acc[ci][0][p] = fmaf(x[kd == 0][kh == 0][kw == 0], wt[t], acc[ci][0][p]);
+                        acc[ci][1][p] = fmaf(x[kd == 0][kh == 0][1 + (kw == 0)], wt[t], acc[ci][1][p]);
+                    }
+                }
+            }
+            __syncthreads();
         }
-        __syncthreads();
-    }
-    if (cs >= ns) return;
+        if (cs >= ns) continue;
 #pragma unroll
-    for (int ci = 0; ci < 4; ++ci) {
-        const size_t base = ((size_t)(s0 + cs) * CI + 4 * g + ci) * D * D * D;
+        for (int ci = 0; ci < 4; ++ci) {
+            const size_t base = ((size_t)(s0 + cs) * CI + 4 * g + ci) * D * D * D;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const size_t at = base + ((size_t)(2 * (d0 + d) + (r >> 1)) * D + 2 * h + (r & 1)) * D + 2 * cw;
-            const float4 m = __ldg((const float4*)(in + at));
-            float4 v;
-            v.x = !(m.x <= 0.f) ? acc[ci][0][2 * r] : 0.f;
-            v.y = !(m.y <= 0.f) ? acc[ci][0][2 * r + 1] : 0.f;
-            v.z = !(m.z <= 0.f) ? acc[ci][1][2 * r] : 0.f;
-            v.w = !(m.w <= 0.f) ? acc[ci][1][2 * r + 1] : 0.f;
-            *(float4*)(din + at) = v;
+            for (int r = 0; r < 4; ++r) {
+                const size_t at = base + ((size_t)(2 * (d0 + d) + (r >> 1)) * D + 2 * h + (r & 1)) * D + 2 * cw;
+                const float4 m = __ldg((const float4*)(in + at));
+                float4 v;
+                v.x = !(m.x <= 0.f) ? acc[ci][0][2 * r] : 0.f;
+                v.y = !(m.y <= 0.f) ? acc[ci][0][2 * r + 1] : 0.f;
+                v.z = !(m.z <= 0.f) ? acc[ci][1][2 * r] : 0.f;
+                v.w = !(m.w <= 0.f) ? acc[ci][1][2 * r + 1] : 0.f;
+                *(float4*)(din + at) = v;
+            }
         }
     }
 }

@@ -484,8 +484,8 @@ int set_smem_attrs() {
     TRY(set_max_dyn_smem(k_conv3_fwd<64, 4, 64, 2, 8>));
     TRY(set_max_dyn_smem(k_conv3_fwd<64, 4, 64, 1, 8>));
     TRY(set_max_dyn_smem(k_conv3_bwd_data<64, 4, 64, 8>));
-    TRY(set_max_dyn_smem(k_conv3_bwd_data<32, 8, 64, 8>));
-    TRY(set_max_dyn_smem(k_conv3_bwd_data<16, 16, 32, 8>));
+    TRY(set_max_dyn_smem(k_conv3_bwd_data<32, 8, 64, 16>));
+    TRY(set_max_dyn_smem(k_conv3_bwd_data<16, 16, 32, 32>));
     TRY(set_max_dyn_smem(k_conv3_bwd_weight<64, 4, 64, 16, 2, 8, 2>));
     TRY(set_max_dyn_smem(k_conv3_bwd_weight<32, 8, 64, 8, 4, 2, 4>));
     TRY(set_max_dyn_smem(k_conv3_bwd_weight<16, 16, 32, 4, 4, 1, 8>));
@@ -2544,7 +2544,8 @@ struct psb_proposal {
         using C = ConvBwd<CI, D, CO, CH>;
         const long long n = (long long)S * C::Do3;
         PROF("k_prop_bwd_data", s);
-        pdl(k_conv3_bwd_data<CI, D, CO, CH>, (unsigned)((n + C::CELLS - 1) / C::CELLS), 256, C::smem, s)(
+        const unsigned tiles = (unsigned)((n + C::CELLS - 1) / C::CELLS);
+        pdl(k_conv3_bwd_data<CI, D, CO, CH>, CH == CO ? std::min(tiles, 2u * 148) : tiles, 256, C::smem, s)(
             dout, S, P16 + L.w, in, din);
         CKL();
         return PSB_OK;
@@ -2584,9 +2585,9 @@ struct psb_proposal {
         TRY((conv_bwd_weight<64, 4, 64, 16, 2, 8, 2>(da4, a3, S, kProp.c[3], s)));
         TRY((conv_bwd_data<64, 4, 64, 8>(da4, S, kProp.c[3], a3, da3, s)));
         TRY((conv_bwd_weight<32, 8, 64, 8, 4, 2, 4>(da3, a2, S, kProp.c[2], s)));
-        TRY((conv_bwd_data<32, 8, 64, 8>(da3, S, kProp.c[2], a2, da2, s)));
+        TRY((conv_bwd_data<32, 8, 64, 16>(da3, S, kProp.c[2], a2, da2, s)));
         TRY((conv_bwd_weight<16, 16, 32, 4, 4, 1, 8>(da2, a1, S, kProp.c[1], s)));
-        TRY((conv_bwd_data<16, 16, 32, 8>(da2, S, kProp.c[1], a1, da1, s)));
+        TRY((conv_bwd_data<16, 16, 32, 32>(da2, S, kProp.c[1], a1, da1, s)));
         TRY((conv_bwd_weight<1, 32, 16, 1, 2, 1, 8>(da1, grids, S, kProp.c[0], s)));
         return PSB_OK;
     }
