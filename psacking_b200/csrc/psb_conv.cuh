@@ -14,6 +14,8 @@
 #pragma once
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "psb_pdl.cuh"
 
 // one word to shared memory without waiting for it; zero where ok is false
@@ -80,7 +82,7 @@ k_conv3_fwd(const float* __restrict__ in, int S, const uint16_t* __restrict__ w,
     for (int i = tid; i < C::NS * CH * C::CHAN; i += 256) xs[i] = 0.f;   // the padding stays zero
     __syncthreads();
     for (int c0 = 0; c0 < CI; c0 += CH) {
-#pragma unroll 4
+#pragma unroll 9
         for (int i = tid; i < CH * 27 * CO; i += 256) {
             const int ct = i % (CH * 27), co = i / (CH * 27);
             ws[ct * C::WR + co] = bf16_up(w[((size_t)co * CI + c0) * 27 + ct]);
@@ -429,7 +431,9 @@ k_linear(const float* __restrict__ a, const void* __restrict__ b, int M, int N, 
     for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = OP == 0 && n0 + 4 * tx + j < N ? bias[n0 + 4 * tx + j] : 0.f;
-    float pa[NA], pb[NB];
+    float pa[NA];
+    using TB = std::conditional_t<OP == 2, float, uint16_t>;
+    TB pb[NB];   // as loaded: widening here would wait for the load
     // element e of the tiles' loads, along the operand's contiguous index
     auto fetch = [&](int k0) {
 #pragma unroll
@@ -444,11 +448,9 @@ k_linear(const float* __restrict__ a, const void* __restrict__ b, int M, int N, 
         for (int e = 0; e < NB; ++e) {
             const int i = tid + 256 * e;
             const int bk = OP == 0 ? i % BK : i / 64, bn = OP == 0 ? i / BK : i % 64;
-            pb[e] = 0.f;
+            pb[e] = 0;
             if (k0 + bk < kb && n0 + bn < N)
-                pb[e] = OP == 0 ? bf16_up(((const uint16_t*)b)[(size_t)(n0 + bn) * K + k0 + bk])
-                      : OP == 1 ? bf16_up(((const uint16_t*)b)[(size_t)(k0 + bk) * N + n0 + bn])
-                                : ((const float*)b)[(size_t)(k0 + bk) * N + n0 + bn];
+                pb[e] = ((const TB*)b)[OP == 0 ? (size_t)(n0 + bn) * K + k0 + bk : (size_t)(k0 + bk) * N + n0 + bn];
         }
     };
     fetch(ka);
@@ -461,7 +463,10 @@ k_linear(const float* __restrict__ a, const void* __restrict__ b, int M, int N, 
 #pragma unroll
         for (int e = 0; e < NB; ++e) {
             const int i = tid + 256 * e;
-            Bs[OP == 0 ? i % BK : i / 64][OP == 0 ? i / BK : i % 64] = pb[e];
+            float u;
+            if constexpr (OP == 2) u = pb[e];
+            else u = bf16_up(pb[e]);
+            Bs[OP == 0 ? i % BK : i / 64][OP == 0 ? i / BK : i % 64] = u;
         }
         __syncthreads();
         fetch(k0 + BK);   // past kb: zeros, without a load

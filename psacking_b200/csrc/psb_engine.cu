@@ -479,6 +479,7 @@ int set_smem_attrs() {
     TRY(set_max_dyn_smem(k_bound_flood));
     TRY(set_max_dyn_smem(k_conv3_fwd<1, 32, 16, 8, 1>));
     TRY(set_max_dyn_smem(k_conv3_fwd<16, 16, 32, 8, 4>));
+    TRY(set_max_dyn_smem(k_conv3_fwd<16, 16, 32, 4, 4>));
     TRY(set_max_dyn_smem(k_conv3_fwd<32, 8, 64, 8, 4>));
     TRY(set_max_dyn_smem(k_conv3_fwd<32, 8, 64, 2, 8>));
     TRY(set_max_dyn_smem(k_conv3_fwd<64, 4, 64, 2, 8>));
@@ -2477,7 +2478,9 @@ struct psb_proposal {
 
     // one convolution layer; the tile that leaves no more than half the chip
     // idle: 8 positions per thread, fewer where S is small (a batch of 8 items,
-    // S = 192, would be 48 and 24 CTAs in the last two layers)
+    // S = 192, would be 48 and 24 CTAs in the last two layers, and 192 CTAs for
+    // 296 places in the second; half tiles there and weights staged nine loads
+    // at a time took the four layers at S = 192 from 421 to 322 us)
     template <int CI, int D, int CO, int TV, int CH>
     int conv_fwd_tile(const float* in, int S, const PropLayer& L, float* out, cudaStream_t s) {
         using C = ConvFwd<CI, D, CO, TV, CH>;
@@ -2491,7 +2494,8 @@ struct psb_proposal {
     int item_branch(const float* grids, int S, cudaStream_t s) {
         PROF("k_prop_conv", s);
         TRY((conv_fwd_tile<1, 32, 16, 8, 1>(grids, S, kProp.c[0], a1, s)));
-        TRY((conv_fwd_tile<16, 16, 32, 8, 4>(a1, S, kProp.c[1], a2, s)));
+        if (S >= 2 * 148) TRY((conv_fwd_tile<16, 16, 32, 8, 4>(a1, S, kProp.c[1], a2, s)));
+        else TRY((conv_fwd_tile<16, 16, 32, 4, 4>(a1, S, kProp.c[1], a2, s)));
         if (S >= 4 * 148) TRY((conv_fwd_tile<32, 8, 64, 8, 4>(a2, S, kProp.c[2], a3, s)));
         else TRY((conv_fwd_tile<32, 8, 64, 2, 8>(a2, S, kProp.c[2], a3, s)));
         if (S >= 8 * 148) TRY((conv_fwd_tile<64, 4, 64, 2, 8>(a3, S, kProp.c[3], a4, s)));

@@ -1,7 +1,7 @@
 """The proposal network's blocked layers at the batch sizes where their tiles
-change or end (24 samples per item; the last two convolutions take smaller
-tiles below 592 and 1184 samples; 592 and 1184 lie between 24 and 25 and
-between 49 and 50 items), against plain torch in float64 with the same BF16
+change or end (24 samples per item; the last three convolutions take smaller
+tiles below 296, 592 and 1184 samples, which lie between 12 and 13, 24 and 25,
+and 49 and 50 items), against plain torch in float64 with the same BF16
 weights.  Tolerances: an FP32 sum of n terms is off by at most about n * 2^-24
 of the sum of magnitudes; the longest forward chain is 1,728 terms and its
 magnitudes stay within 50 times the result's scale, so 1e-4 of the largest
@@ -44,7 +44,7 @@ def _reference(flat, grids, hm, mask, target):
 
 
 @pytest.mark.parametrize("offset", [0, 1])
-@pytest.mark.parametrize("B", [1, 2, 24, 25, 49, 50])
+@pytest.mark.parametrize("B", [1, 2, 12, 13, 24, 25, 49, 50])
 def test_layers_match_float64(gpu_core, B, offset):
     """offset 1: the grids start 4 bytes past an aligned address."""
     import torch
