@@ -3018,21 +3018,27 @@ int psb_tray_search(psb_tray* t, const int32_t* const* items, const int32_t* dim
     const bool interlock = (mode_flags & PSB_FLAG_INTERLOCK) != 0;
     if (!per_orient && t->occ == 0 && t->phi_own) {
         // an empty tray and its own distance field: every translation is free
-        // and the field constant, so the first array that fits wins at the
-        // origin (see k_bound_first)
-        bool bad = false;
-        for (int o = 0; o < n && !bad; ++o)
-            bad = !items[o] || dims[3 * o] <= 0 || dims[3 * o + 1] <= 0 || dims[3 * o + 2] <= 0 ||
-                  has_negative(items[o], (size_t)dims[3 * o] * dims[3 * o + 1] * dims[3 * o + 2]);
-        for (int o = 0; o < n && !bad; ++o) {
+        // and the field constant, so an array's best place is the origin (see
+        // k_bound_first), at its sum times the far value; the arrays may be
+        // different items, so the smallest of them wins, the first on a tie
+        bool general = false;
+        for (int o = 0; o < n && !general; ++o)
+            general = !items[o] || dims[3 * o] <= 0 || dims[3 * o + 1] <= 0 || dims[3 * o + 2] <= 0 ||
+                      has_negative(items[o], (size_t)dims[3 * o] * dims[3 * o + 1] * dims[3 * o + 2]);
+        double best = mode == PSB_MODE_SCAN ? 1e9 : 1e29;
+        int who = -1;
+        for (int o = 0; o < n && !general; ++o) {
             const int32_t* d = dims + 3 * o;
             if (d[0] > t->nx || d[1] > t->ny || d[2] > t->nz) continue;
             double sum = 0.0;
             const size_t m = (size_t)d[0] * d[1] * d[2];
             for (size_t i = 0; i < m; ++i) sum += (double)items[o][i];
             const double s = sum * (double)(t->nx + t->ny + t->nz + 10);
-            if (!(s < 9007199254740992.0) || s >= (mode == PSB_MODE_SCAN ? 1e9 : 1e29)) break;
-            *out = psb_result{0, 0, 0, 1, s, o, PSB_DIAG_DIRECT, 0, 0.f};
+            general = !(s < 9007199254740992.0);   // not exact
+            if (s < best) { best = s; who = o; }
+        }
+        if (!general && who >= 0) {
+            *out = psb_result{0, 0, 0, 1, best, who, PSB_DIAG_DIRECT, 0, 0.f};
             return PSB_OK;
         }
     }

@@ -1,0 +1,105 @@
+"""Tray calls of the C ABI (psb_tray_set, psb_tray_search, psb_tray_place) on
+the inputs where their shortcuts and limits lie, against the transform flow
+(candidate filter off), which every search can fall back to, or against plain
+numpy."""
+import ctypes
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+LIB = Path(__file__).resolve().parent.parent / "psacking_b200" / "libpsb200.so"
+SCAN, BLOCK, INTERLOCK = 0, 1, 0x10
+PSB_ERR_ARG = 1
+
+
+class Res(ctypes.Structure):
+    _fields_ = [("x", ctypes.c_int32), ("y", ctypes.c_int32), ("z", ctypes.c_int32),
+                ("found", ctypes.c_int32), ("score", ctypes.c_double), ("orientation", ctypes.c_int32),
+                ("diag", ctypes.c_uint32), ("n_candidates", ctypes.c_int32), ("err_ratio", ctypes.c_float)]
+
+
+class Tray:
+    """A tray handle; phi None: the tray's own distance field."""
+
+    def __init__(self, tray, phi=None):
+        self.lib = lib = ctypes.CDLL(str(LIB))
+        P, I = ctypes.c_void_p, ctypes.c_int
+        lib.psb_last_error.argtypes = [ctypes.c_char_p, ctypes.c_size_t]
+        lib.psb_tray_create.argtypes = [I, I, I, P]
+        lib.psb_tray_destroy.argtypes = [P]
+        lib.psb_tray_set.argtypes = [P, P, P]
+        lib.psb_tray_get.argtypes = [P, P, P]
+        lib.psb_tray_search.argtypes = [P, P, P, I, I, P, P]
+        lib.psb_tray_place.argtypes = [P, P, I, I, I, I, I, I, ctypes.c_int32]
+        self.shape, self.h = tray.shape, P()
+        self.check(lib.psb_tray_create(*tray.shape, ctypes.byref(self.h)))
+        self.set(tray, phi)
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *a):
+        assert self.lib.psb_tray_destroy(self.h) == 0
+
+    def err(self):
+        buf = ctypes.create_string_buffer(1024)
+        self.lib.psb_last_error(buf, 1024)
+        return buf.value.decode()
+
+    def check(self, st):
+        assert st == 0, self.err()
+
+    def set(self, tray, phi=None):
+        tray = np.ascontiguousarray(tray, np.int32)
+        phi = None if phi is None else np.ascontiguousarray(phi, np.int32)
+        self.check(self.lib.psb_tray_set(self.h, tray.ctypes.data, None if phi is None else phi.ctypes.data))
+
+    def get(self):
+        tray, phi = np.empty(self.shape, np.int32), np.empty(self.shape, np.int32)
+        self.check(self.lib.psb_tray_get(self.h, tray.ctypes.data, phi.ctypes.data))
+        return tray, phi
+
+    def search_status(self, items, flags):
+        items = [np.ascontiguousarray(i, np.int32) for i in items]
+        ptrs = (ctypes.c_void_p * len(items))(*[i.ctypes.data for i in items])
+        dims = np.array([i.shape for i in items], np.int32).ravel()
+        r = Res()
+        return self.lib.psb_tray_search(self.h, ptrs, dims.ctypes.data, len(items), flags, ctypes.byref(r), None), r
+
+    def search(self, items, flags):
+        st, r = self.search_status(items, flags)
+        self.check(st)
+        return (r.found, r.x, r.y, r.z, r.orientation, r.score)
+
+
+def by_transforms(core, tray, phi, items, flags):
+    core.set_cand_filter(False)
+    try:
+        with Tray(tray, phi) as t:
+            # (results per array are asked for: no closed form for an empty tray)
+            per = (Res * len(items))()
+            its = [np.ascontiguousarray(i, np.int32) for i in items]
+            ptrs = (ctypes.c_void_p * len(its))(*[i.ctypes.data for i in its])
+            dims = np.array([i.shape for i in its], np.int32).ravel()
+            r = Res()
+            t.check(t.lib.psb_tray_search(t.h, ptrs, dims.ctypes.data, len(its), flags, ctypes.byref(r),
+                                          ctypes.byref(per)))
+            return (r.found, r.x, r.y, r.z, r.orientation, r.score)
+    finally:
+        core.set_cand_filter(True)
+
+
+@pytest.mark.parametrize("flags", [SCAN, BLOCK, BLOCK | INTERLOCK])
+def test_empty_tray_takes_the_best_array(gpu_core, flags):
+    """Arrays of different sums on an empty tray: the lightest wins wherever it
+    stands, the first of equal ones, and none that does not fit or scores too
+    high for the scan."""
+    empty = np.zeros((20, 18, 16), np.int32)
+    big, one, flat = np.ones((2, 2, 2), np.int32), np.ones((1, 1, 1), np.int32), np.ones((4, 2, 1), np.int32)
+    wide, heavy = np.ones((30, 1, 1), np.int32), np.full((2, 2, 2), 1 << 24, np.int32)
+    for items in ([big, one], [one, big], [big, flat], [wide, big, flat, one, one], [heavy, big], [heavy], [wide]):
+        with Tray(empty) as t:
+            assert t.search(items, flags) == by_transforms(gpu_core, empty, None, items, flags), items
