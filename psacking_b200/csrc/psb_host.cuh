@@ -275,11 +275,26 @@ class PinBlocks {
 // 0.2 ms shorter.
 constexpr size_t kUploadMin = (size_t)3 << 19, kDownloadMin = (size_t)4 << 20;
 
+// Whether the driver takes a copy's bytes before the call returns: of pageable
+// memory only.  Page-locked memory (a pinned tensor's) is read when the copy
+// runs, and memory that CUDA manages may be.
+inline bool host_pageable(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
 // Host array -> device on st.  The source may be reused on return; the copy
-// itself is queued.
+// itself is queued (waited for where it would still be reading the source).
 inline cudaError_t upload_async(void* dst, const void* src, size_t bytes, cudaStream_t st) {
     PinBlock* b = bytes >= kUploadMin ? PinBlocks::get().take(bytes) : nullptr;
-    if (!b) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    if (!b) {
+        const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+        return e != cudaSuccess || host_pageable(src) ? e : cudaStreamSynchronize(st);
+    }
     // the cores copy 512 KiB at a time, the bus takes quarters: every bus copy
     // costs some 20 us besides its bytes
     const size_t chunk = (size_t)512 << 10, n = (bytes + chunk - 1) / chunk, group = (n + 3) / 4;

@@ -1,0 +1,39 @@
+// Runs one case of tests/test_host_copies.py against the stand-in runtime;
+// prints "ok" or what went wrong.
+#include "psb_host.cuh"
+
+#include <cstdio>
+#include <string>
+
+static FakeStream g_stream[2];
+
+// upload_async, the source overwritten as soon as the call has returned
+static bool upload(size_t bytes, bool pinned) {
+    std::vector<char> pageable(pinned ? 0 : bytes), dev(bytes, 0);
+    char* src = pageable.data();
+    if (pinned && cudaHostAlloc((void**)&src, bytes, 0) != cudaSuccess) return false;
+    for (size_t i = 0; i < bytes; ++i) src[i] = (char)(i * 7 + 1);
+    if (upload_async(dev.data(), src, bytes, &g_stream[0]) != cudaSuccess) return false;
+    memset(src, 0x55, bytes);
+    cudaStreamSynchronize(&g_stream[0]);
+    bool same = true;
+    for (size_t i = 0; i < bytes; ++i) same = same && dev[i] == (char)(i * 7 + 1);
+    if (pinned) cudaFreeHost(src);
+    return same;
+}
+
+int main(int argc, char** argv) {
+    const std::string what = argc > 1 ? argv[1] : "";
+    bool ok = false;
+    if (what == "upload") {
+        ok = upload((size_t)atoll(argv[2]), argv[3][0] == 'p');
+    } else if (what == "upload_no_block") {
+        // every staging block in use elsewhere
+        for (int i = 0; i < PinBlocks::kBlocks; ++i)
+            if (!PinBlocks::get().take((size_t)2 << 20)) return 1;
+        ok = upload((size_t)2 << 20, argv[2][0] == 'p');
+    }
+    puts(ok ? "ok" : "wrong");
+    fflush(stdout);
+    _Exit(0);   // the host threads wait for ever
+}

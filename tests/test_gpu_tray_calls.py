@@ -103,3 +103,22 @@ def test_empty_tray_takes_the_best_array(gpu_core, flags):
     for items in ([big, one], [one, big], [big, flat], [wide, big, flat, one, one], [heavy, big], [heavy], [wide]):
         with Tray(empty) as t:
             assert t.search(items, flags) == by_transforms(gpu_core, empty, None, items, flags), items
+
+
+@pytest.mark.parametrize("shape", [(20, 18, 16), (90, 80, 70), (300, 280, 210)])
+def test_tray_set_source_may_be_reused_on_return(gpu_core, shape):
+    """Page-locked arrays, overwritten as soon as psb_tray_set has returned:
+    below the staged sizes, staged, and above a staging block."""
+    import torch
+    rng = np.random.default_rng(5)
+    tray = torch.zeros(shape, dtype=torch.int32).pin_memory().numpy()
+    phi = torch.zeros(shape, dtype=torch.int32).pin_memory().numpy()
+    with Tray(np.zeros(shape, np.int32)) as t:
+        for _ in range(3):
+            want_tray, want_phi = (rng.integers(0, 9, shape, dtype=np.int32) for _ in range(2))
+            tray[...], phi[...] = want_tray, want_phi
+            t.check(t.lib.psb_tray_set(t.h, tray.ctypes.data, phi.ctypes.data))
+            tray[...] = 3
+            phi[...] = -1
+            got_tray, got_phi = t.get()
+            assert np.array_equal(got_tray, want_tray) and np.array_equal(got_phi, want_phi)
