@@ -222,9 +222,9 @@ class PinBlocks {
         if (!best) {
             for (PinBlock& b : blocks_)
                 if (!b.p && !b.held) { best = &b; break; }
-            if (!best)   // every place is in use: replace an idle one that is too small
+            if (!best)   // every place is in use: replace an idle one that is too small or another device's
                 for (PinBlock& b : blocks_)
-                    if (!b.held && b.dev == dev && b.n < bytes &&
+                    if (!b.held && (b.dev != dev || b.n < bytes) &&
                         cudaEventQuery(b.ev[PinBlock::kEvents - 1]) == cudaSuccess) { best = &b; break; }
             if (!best || !make(best, bytes, dev)) return nullptr;
         }
@@ -335,7 +335,10 @@ inline cudaError_t download(void* dst, const void* src, size_t bytes, cudaStream
     if (e == cudaSuccess) {
         std::atomic<int> bad{0};
         HostPool::get().run(n, [&](size_t i) {
-            const cudaError_t w = cudaEventSynchronize(b->ev[i / group]);
+            // the cores' threads start out on device 0, where a call for
+            // another device's event would make a context
+            cudaError_t w = cudaSetDevice(b->dev);
+            if (w == cudaSuccess) w = cudaEventSynchronize(b->ev[i / group]);
             if (w != cudaSuccess) { bad = (int)w; return; }
             const size_t o = i * chunk, m = std::min(chunk, bytes - o);
             memcpy((char*)dst + o, b->p + o, m);

@@ -32,6 +32,23 @@ int main(int argc, char** argv) {
         for (int i = 0; i < PinBlocks::kBlocks; ++i)
             if (!PinBlocks::get().take((size_t)2 << 20)) return 1;
         ok = upload((size_t)2 << 20, argv[2][0] == 'p');
+    } else if (what == "download") {
+        // every byte there on return, no event waited for from another device
+        const size_t bytes = (size_t)atoll(argv[2]);
+        cudaSetDevice(atoi(argv[3]));
+        std::vector<char> dev(bytes), out(bytes, 0);
+        for (size_t i = 0; i < bytes; ++i) dev[i] = (char)(i * 5 + 2);
+        ok = download(out.data(), dev.data(), bytes, &g_stream[0]) == cudaSuccess && out == dev && !fake::wrong_device;
+    } else if (what == "two_devices") {
+        // the first device's idle blocks give way to the second's, and back
+        ok = true;
+        for (int dev : {0, 1, 0}) {
+            cudaSetDevice(dev);
+            PinBlock* b[PinBlocks::kBlocks];
+            for (PinBlock*& x : b) ok = (x = PinBlocks::get().take((size_t)2 << 20)) != nullptr && x->dev == dev && ok;
+            ok = PinBlocks::get().take((size_t)2 << 20) == nullptr && ok;   // none is left while they are held
+            for (PinBlock* x : b) if (x) PinBlocks::get().give(x, &g_stream[dev]);
+        }
     }
     puts(ok ? "ok" : "wrong");
     fflush(stdout);

@@ -34,3 +34,13 @@ def test_upload_source_may_be_reused_on_return(program, size, memory):
 @pytest.mark.parametrize("memory", ["pageable", "locked"])
 def test_upload_without_a_free_block(program, memory):
     _run(program, "upload_no_block", "p" if memory == "locked" else "h")
+
+
+@pytest.mark.parametrize("device", [0, 1])
+@pytest.mark.parametrize("size", [100_000, (4 << 20) + 12, 40 << 20])
+def test_download_waits_on_the_callers_device(program, size, device):
+    _run(program, "download", size, device)
+
+
+def test_staging_blocks_of_several_devices(program):
+    _run(program, "two_devices")
