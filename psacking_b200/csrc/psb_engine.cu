@@ -686,7 +686,7 @@ int distance_on_device(const int32_t* d_grid, int32_t* d_out, int nx, int ny, in
     {
         PROF("k_dist_z", st);
         const long long nlines = (long long)nx * ny;
-        pdl(k_dist_z, (unsigned)((nlines + 7) / 8), 256, 0, st)(d_grid, d_out, (int)nlines, nz, far, gate);
+        pdl(k_dist_z, (unsigned)((nlines + 7) / 8), 256, 0, st)(d_grid, d_out, nlines, nz, far, gate);
     }
     CKL();
     for (int axis = 1; axis >= 0; --axis) {
@@ -694,7 +694,7 @@ int distance_on_device(const int32_t* d_grid, int32_t* d_out, int nx, int ny, in
         if (L <= 1) continue;
         const long long stride = axis == 0 ? (long long)ny * nz : (long long)nz;
         const long long inner = stride, outer = axis == 0 ? 1 : nx, ostr = axis == 0 ? 0 : (long long)ny * nz;
-        if (L <= 512 && inner <= INT_MAX && outer <= 65535) {
+        if (L <= 512 && inner <= INT_MAX - 31 && outer <= 65535) {   // its tiles of 32 lines count in int
             // segments of 8, 16 or 32 cells over at most 16 warps: the
             // shortest that covers the line, for the most threads in flight
             const int seg = L <= 128 ? 8 : (L <= 256 ? 16 : 32);

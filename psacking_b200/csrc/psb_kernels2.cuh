@@ -786,19 +786,21 @@ k_ff_reach(const OrientDesc* __restrict__ orients, FloodBufs fb, ScoreParams sp)
 // right, each a warp scan; a warp owns a line (32 cells per step, the carry
 // in a register), so every load and store is one contiguous segment and no
 // line waits on another.  A line is read back in the second sweep from the
-// first one's output (L1/L2).
+// first one's output (L1/L2).  Lines are counted in 64 bits: a field may have
+// more than 2^27, whose threads are more than 2^32.
 // grid: ceil(nx*ny / 8), block 256
-__global__ void k_dist_z(const int32_t* __restrict__ g, int32_t* __restrict__ d, int nlines, int nz, int far,
+__global__ void k_dist_z(const int32_t* __restrict__ g, int32_t* __restrict__ d, long long nlines, int nz, int far,
                          const int* gate) {
     pdl_enter();
     if (gate && !*gate) return;
-    const int line = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    const long long line = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
     if (line >= nlines) return;
     const int32_t* s = g + (size_t)line * nz;
     int32_t* o = d + (size_t)line * nz;
     int carry = far;   // smallest value so far, brought to the previous cell
-    for (int z0 = 0; z0 < nz; z0 += 32) {
-        const int z = z0 + lane;
+    for (long long z0 = 0; z0 < nz; z0 += 32) {
+        const long long z = z0 + lane;
         int v = z < nz && s[z] == 1 ? 0 : far;
 #pragma unroll
         for (int k = 1; k < 32; k <<= 1) {
@@ -811,8 +813,8 @@ __global__ void k_dist_z(const int32_t* __restrict__ g, int32_t* __restrict__ d,
     }
     __syncwarp();
     carry = far;
-    for (int z0 = ((nz - 1) / 32) * 32; z0 >= 0; z0 -= 32) {
-        const int z = z0 + lane;
+    for (long long z0 = ((nz - 1) / 32) * 32; z0 >= 0; z0 -= 32) {
+        const long long z = z0 + lane;
         int v = z < nz ? o[z] : far;
 #pragma unroll
         for (int k = 1; k < 32; k <<= 1) {
