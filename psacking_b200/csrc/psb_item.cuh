@@ -186,7 +186,10 @@ k_item_describe(const int32_t* __restrict__ vals, const ItemArr* __restrict__ ar
     if (lane != 0) return;
     const int n[3] = {nx, ny, nz};
     OrientDesc d;
-    d.skip = it.skip;
+    // an array with a negative value is an error that the host reads only after
+    // the search: it is not searched, since its numbers of translations come
+    // from its positive voxels and do not keep the negative ones inside
+    d.skip = it.skip || S.neg;
     if (S.neg) atomicMin(neg, o);
     const bool empty = S.hi[0] < 0;
     for (int a = 0; a < 3; ++a) {

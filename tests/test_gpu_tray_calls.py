@@ -122,3 +122,22 @@ def test_tray_set_source_may_be_reused_on_return(gpu_core, shape):
             phi[...] = -1
             got_tray, got_phi = t.get()
             assert np.array_equal(got_tray, want_tray) and np.array_equal(got_phi, want_phi)
+
+
+@pytest.mark.parametrize("flags", [SCAN, BLOCK, BLOCK | INTERLOCK])
+def test_negative_values_anywhere_are_refused(gpu_core, flags):
+    """Negative voxels beyond the positive ones, or no positive ones at all:
+    an error that names the first such array, and the tray stays usable."""
+    tray = np.zeros((20, 18, 16), np.int32)
+    tray[:6, :6, :6] = 1
+    ok = np.ones((2, 3, 4), np.int32)
+    only = np.full((12, 12, 12), -1, np.int32)
+    beyond = np.zeros((12, 11, 10), np.int32)
+    beyond[0, 0, 0] = 2
+    beyond[11, 10, 9] = -3
+    with Tray(tray) as t:
+        want = t.search([ok], flags)
+        for items, bad in (([only], 0), ([ok, beyond], 1), ([ok, ok, only, beyond], 2)):
+            st, _ = t.search_status(items, flags)
+            assert st == PSB_ERR_ARG and "orientation %d holds negative" % bad in t.err()
+            assert t.search([ok], flags) == want
