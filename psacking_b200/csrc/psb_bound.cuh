@@ -37,10 +37,11 @@
 // survivor, k_bound_flood checks them and floods the free ones from the seed
 // faces in one CTA's shared memory (a crowded tray has few), and a second
 // k_bound_score takes the best reachable one.  k_bound_place writes the item.
-// An item this cannot decide (no source, more survivors than the list or
-// free ones than the flood holds) raises BoundState::halt: the launches
-// already queued for later items return at once, and the host runs that item
-// through the transforms and the union-find flood fill.
+// An item this cannot decide (no source, weights or distances too large for
+// exact scores, more survivors than the list or free ones than the flood holds)
+// raises BoundState::halt: the launches already queued for later items return at
+// once, and the host runs that item through the transforms and the union-find
+// flood fill.
 #pragma once
 #include "psb_filter.cuh"
 
@@ -58,6 +59,7 @@ struct BoundGeom {
     int h[8];
     int any;                    // a source exists
     int over;                   // largest excess of the bounds over phi (0 for a distance field)
+    int pmax;                   // no value of phi is larger, or smaller than -pmax - 1
 };
 
 struct __align__(16) BoundState {
@@ -97,13 +99,15 @@ struct BoundHit {
     double s;                   // the bounded score, then the exact one
 };
 
-__global__ void k_bound_geom_reset(BoundGeom* g) {
+// pmax: 0 where k_bound_over follows
+__global__ void k_bound_geom_reset(BoundGeom* g, int pmax) {
     pdl_enter();
     if (threadIdx.x != 0) return;
     for (int a = 0; a < 3; ++a) { g->lo[a] = INT_MAX; g->hi[a] = -1; }
     for (int k = 0; k < 8; ++k) g->h[k] = INT_MIN;
     g->any = 0;
     g->over = 0;
+    g->pmax = pmax;
 }
 
 // grid: any, block 256
@@ -142,13 +146,15 @@ __global__ void k_bound_geom(const int32_t* __restrict__ tray, int nx, int ny, i
 }
 
 // A distance field handed in by the caller need not be the tray's: the
-// largest excess of the bounds over it, which the tables then subtract.
+// largest excess of the bounds over it, which the tables then subtract, and the
+// range of its values.
 // grid: any, block 256
 __global__ void k_bound_over(const int32_t* __restrict__ phi, int nx, int ny, int nz, BoundGeom* g) {
     pdl_enter();
     if (!g->any) return;
     const size_t V = (size_t)nx * ny * nz;
     long long over = 0;
+    int pmax = 0;
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < V; t += (size_t)gridDim.x * blockDim.x) {
         const size_t r = t / nz;
         const int c[3] = {(int)(r / ny), (int)(r % ny), (int)(t % nz)};
@@ -158,20 +164,31 @@ __global__ void k_bound_over(const int32_t* __restrict__ phi, int nx, int ny, in
 #pragma unroll
         for (int k = 0; k < 8; ++k)
             b = max(b, ((k & 1) ? -c[0] : c[0]) + ((k & 2) ? -c[1] : c[1]) + ((k & 4) ? -c[2] : c[2]) - g->h[k]);
-        over = max(over, (long long)b - phi[t]);
+        const int p = phi[t];
+        over = max(over, (long long)b - p);
+        pmax = max(pmax, p < 0 ? -1 - p : p);
     }
     const int o = __reduce_max_sync(0xffffffffu, (int)min(over, (long long)INT_MAX));
-    if ((threadIdx.x & 31) == 0 && o > 0) atomicMax(&g->over, o);
+    pmax = __reduce_max_sync(0xffffffffu, pmax);
+    if ((threadIdx.x & 31) != 0) return;
+    if (o > 0) atomicMax(&g->over, o);
+    atomicMax(&g->pmax, pmax);
 }
 
 // ---------------------------------------------------------------------------
 // bound tables of one orientation of one item
 // ---------------------------------------------------------------------------
-// doubles (every value an integer below 2^53): [0] W, [1..8] s.M - W h(s) per
-// sign vector, [9..11] the numbers of x, y, z translations (x: 0 when the
-// orientation is skipped), [12..14] its runs (RunHead), then X[nx], Y[ny], Z[nz], and the smallest bounded score at z or
-// above of the separable bound's z part (F0[nz]) and of W z (F1[nz]), which
-// grow with z, so the last z worth testing in a column is a binary search.
+// doubles: [0] W, [1..8] s.M - W h(s) per sign vector, [9..11] the numbers of
+// x, y, z translations (x: 0 when the orientation is skipped), [12..14] its runs
+// (RunHead), [15] the slack of the z cut, infinite where the exact scores
+// themselves do not fit (the search then goes to the transforms), then X[nx],
+// Y[ny], Z[nz], and the smallest bounded score at z or above of the separable
+// bound's z part (F0[nz]) and of W z (F1[nz]), which grow with z, so the last z
+// worth testing in a column is a binary search.
+// The bounds are integers, exact while they stay below 2^53.  Heavier items
+// (values in the millions) pass that: [1..8] and X are then lowered by more than
+// every rounding of the sums made of them, so that no bound rounds above its
+// score.
 struct BoundTab {
     const double *X, *Y, *Z, *F0, *F1;
     const double* c;
@@ -319,8 +336,17 @@ k_bound_prep(const OrientDesc* __restrict__ od_all, int n, int i0, const BoundGe
         }
     }
     __syncthreads();
-    const double W = sW, low = -W * (double)geom->over;
-    if (tid == 0) T[0] = W;
+    // no part or sum of a bound exceeds top; a sum is a dozen operations at
+    // most, each off by 2^-53 of that
+    const double W = sW, top = W * ((double)geom->over + 8.0 * (sp.nx + sp.ny + sp.nz));
+    const double low = -W * (double)geom->over - (top < 9007199254740992.0 ? 0.0 : 0x1p-49 * top);
+    if (tid == 0) {
+        T[0] = W;
+        // a run's proximity (up to 256 cells) is a 32-bit sum, an item's and its
+        // moments (k times the weights) 64-bit ones
+        const double pmax = geom->pmax;
+        T[15] = pmax < 8388608.0 && W * fmax(pmax + 1.0, 1024.0) < 0x1p62 ? 1e-6 + 1e-15 * top : INFINITY;
+    }
     if (tid < 8)
         T[1 + tid] = ((tid & 1) ? -sM[0] : sM[0]) + ((tid & 2) ? -sM[1] : sM[1]) + ((tid & 4) ? -sM[2] : sM[2]) -
                      W * (double)geom->h[tid] + low;
@@ -611,7 +637,7 @@ __device__ __forceinline__ BoundCols bound_cols(const BoundArgs& ba, const Score
     const int lane = threadIdx.x & 31;
     BoundCols c;
     c.bt = bound_tab(ba.tab + (size_t)o * ba.tstride, sp);
-    const double h = c.h = c.bt.c[min(lane, 14) - 1];   // lane l: header entry l
+    const double h = c.h = c.bt.c[min(lane, 15) - 1];   // lane l: header entry l
     c.fb = lane <= nw ? __ldg(&ba.fbound[(size_t)o * PSB_FBOUND + lane]) : 0;
     const int Xv = (int)__shfl_sync(0xffffffffu, h, 9), Zv = (int)__shfl_sync(0xffffffffu, h, 11);
     c.Yv = (int)__shfl_sync(0xffffffffu, h, 10);
@@ -624,7 +650,7 @@ __device__ __forceinline__ BoundCols bound_cols(const BoundArgs& ba, const Score
     }
     if (best < INFINITY) {
         // slack for the roundings of F's sums; the exact test follows
-        const double lim = best + 1e-12 * fabs(best) + 1e-6;
+        const double lim = best + 1e-12 * fabs(best) + __shfl_sync(0xffffffffu, h, 15);
         if (!act || c.bt.F0[0] > lim - c.A || c.bt.F1[0] > lim - c.gp) c.zc = 0;
         if (__any_sync(0xffffffffu, c.zc > 0) && c.zc > 0) {
             c.zc = bound_count(c.bt.F0, Zv, lim - c.A);
@@ -763,6 +789,10 @@ k_bound_find(int n, const uint4* __restrict__ tbits, ScoreParams sp,
         double best = ALL ? INFINITY : now.best;
         if (now.count > PSB_BCAP) return;   // the list is lost anyway
         const BoundCols bc = bound_cols(ba, sp, NW, o, x, y0 + lane, best);
+        if (!(__shfl_sync(0xffffffffu, bc.h, 15) < INFINITY)) {   // not scored here: the list counts as lost
+            if (lane == 0) atomicMax(&st->count, PSB_BCAP + 1);
+            return;
+        }
         if (!bc.any) continue;
         const BoundTab& bt = bc.bt;
         const double A = bc.A, gp = bc.gp, gm = bc.gm;
@@ -974,13 +1004,13 @@ k_bound_score(const uint4* __restrict__ tbits, int tq, ScoreParams sp, BoundArgs
     st->count = st->nwin = 0;
     st->best = 0xffffffffffffffffULL;
     if (FLOOD) st->need_flood = 0;
-    if (fail) {
+    const bool found = best < (sp.mode == 0 ? 1000000000.0 : 1e29);
+    if (fail || (found && win == ~0ULL)) {   // (the second cannot be: a score has its translation)
         st->halt = 1;
         st->halt_item = item;
         ls->do_place = 0;
         return;
     }
-    const bool found = best < (sp.mode == 0 ? 1000000000.0 : 1e29);
     const int o = found ? (int)(win >> 32) : -1;
     const int t = found ? untie_key(sp.mode, (unsigned int)win) : -1;
     if (found && interlock && !FLOOD) {

@@ -1645,7 +1645,7 @@ struct psb_tray {
         TRY(ensure_bits());
         if (geom_stale) {
             PROF("k_bound_geom", st);
-            pdl(k_bound_geom_reset, 1, 32, 0, st)(d_bgeom);
+            pdl(k_bound_geom_reset, 1, 32, 0, st)(d_bgeom, phi_own ? nx + ny + nz + 10 : 0);
             pdl(k_bound_geom, std::min(grid1d(V), 148 * 4), 256, 0, st)(d_tray, nx, ny, nz, d_bgeom);
             if (!phi_own) pdl(k_bound_over, std::min(grid1d(V), 148 * 4), 256, 0, st)(d_phi, nx, ny, nz, d_bgeom);
             CKL();

@@ -8,6 +8,8 @@ from pathlib import Path
 import numpy as np
 import pytest
 
+from oracle import psb_oracle as O
+
 pytestmark = pytest.mark.gpu
 
 LIB = Path(__file__).resolve().parent.parent / "psacking_b200" / "libpsb200.so"
@@ -141,3 +143,73 @@ def test_negative_values_anywhere_are_refused(gpu_core, flags):
             st, _ = t.search_status(items, flags)
             assert st == PSB_ERR_ARG and "orientation %d holds negative" % bad in t.err()
             assert t.search([ok], flags) == want
+
+
+def _boxes(rng, shape, n):
+    tray = np.zeros(shape, np.int32)
+    for k in range(n):
+        e = [int(rng.integers(2, s // 3)) for s in shape]
+        o = [int(rng.integers(0, s - ee + 1)) for s, ee in zip(shape, e)]
+        tray[o[0]:o[0] + e[0], o[1]:o[1] + e[1], o[2]:o[2] + e[2]] = 1 + k % 3
+    return tray
+
+
+@pytest.mark.parametrize("flags", [BLOCK, BLOCK | INTERLOCK])
+@pytest.mark.parametrize("top", [1, 1 << 20, 1 << 26, (1 << 31) - 1])
+def test_search_with_heavy_items(gpu_core, monkeypatch, top, flags):
+    """Item values whose bounds stay below 2^53 and such that pass it, against
+    the oracle's exact sums (not the transforms: in FP32 their collision counts
+    are not exact at such weights).  The oracle's FP64 correlations are exact up
+    to about 2^30, so they take the values' halves one by one."""
+    corr = O.corr_exact
+    monkeypatch.setattr(O, "corr_exact", lambda t, i, linear=True:
+                        (corr(t, np.asarray(i) >> 16, linear) << 16) + corr(t, np.asarray(i) & 0xffff, linear))
+    rng = np.random.default_rng(top % 1000 + flags)
+    shape = (60, 50, 44)
+    for trial in range(4):
+        tray = _boxes(rng, shape, 3 + 4 * trial)
+        items = []
+        for e in ((14, 12, 10), (18, 18, 18), (9, 21, 11)):
+            it = rng.integers(top - top // 3, top, e, endpoint=True, dtype=np.int64).astype(np.int32)
+            it[rng.random(e) < 0.2] = 0
+            items.append(it)
+        phi = O.calculate_distance(tray)
+        pos, found, score, o = O.fft_search_batch(items, tray, phi, 1, interlock=flags != BLOCK)
+        for handed_in in (None, phi):
+            with Tray(tray, handed_in) as t:
+                assert t.search(items, flags) == (int(found),) + tuple(pos) + (o, score)
+
+
+def test_heavy_items_far_from_a_corner_source(gpu_core):
+    """One source in the tray's corner, where a bound equals the proximity it
+    bounds, and proximities of 2^53 and more: a bound that is rounded up must
+    not rule its own translation out.  The free space takes an item in twelve
+    places at the far end, the lowest of which (a column of the seed lattice)
+    wins."""
+    rng = np.random.default_rng(1)
+    i, j, k = np.indices((32, 32, 32))
+    for trial in range(40):
+        tray = np.full((300, 40, 40), 2, np.int32)
+        tray[0, 0, 0] = 1
+        at = (260, trial % 4, 3 + trial % 5)
+        tray[at[0]:at[0] + 34, at[1]:at[1] + 33, at[2]:at[2] + 33] = 0
+        item = rng.integers((1 << 31) - (1 << 22), 1 << 31, (32, 32, 32), dtype=np.int64)
+        prox = int((item * (i + j + k)).sum()) + int(item.sum()) * sum(at)
+        assert prox > 1 << 53
+        with Tray(tray) as t:
+            assert t.search([item], BLOCK) == (1,) + at + (0, O.score_block(float(prox), at[2], 40)), trial
+
+
+@pytest.mark.parametrize("flags", [BLOCK, BLOCK | INTERLOCK])
+@pytest.mark.parametrize("shift", [-(1 << 30), -(1 << 23) + 200, -5000, 5000, (1 << 23) - 200, 1 << 23, 1 << 30])
+def test_search_with_shifted_distances(gpu_core, shift, flags):
+    """A distance field handed in whose values are far from the tray's, up to
+    where a run's sum passes 32 bits."""
+    rng = np.random.default_rng(abs(shift) % 1000 + flags)
+    shape = (36, 40, 70)
+    for trial in range(4):
+        tray = _boxes(rng, shape, 2 + 3 * trial)
+        phi = gpu_core.calculate_distance(tray) + np.int32(shift)
+        items = [np.ones((3, 4, 30), np.int32), np.ones((5, 6, 7), np.int32)]
+        with Tray(tray, phi) as t:
+            assert t.search(items, flags) == by_transforms(gpu_core, tray, phi, items, flags)
