@@ -516,8 +516,22 @@ __device__ __forceinline__ long long bound_prox(const RunHead& od, const int32_t
     return acc;
 }
 
+// The best score and the count as they are now.  Other warps are changing them,
+// so one lane reads for the warp: lanes that each read for themselves could see
+// different values and part ways around a warp-wide vote.  (Called by whole warps.)
 __device__ __forceinline__ double bound_best(const BoundState* st) {
-    const unsigned long long k = *(const volatile unsigned long long*)&st->best;
+    unsigned long long k = 0ULL;
+    if ((threadIdx.x & 31) == 0) k = *(const volatile unsigned long long*)&st->best;
+    k = __shfl_sync(0xffffffffu, k, 0);
+    return k == 0xffffffffffffffffULL ? INFINITY : ord_val(k);
+}
+// both in one load; returns the best score
+__device__ __forceinline__ double bound_now(const BoundState* st, int* listed) {
+    int4 a = make_int4(0, 0, 0, 0);
+    if ((threadIdx.x & 31) == 0) a = __ldcg((const int4*)st);
+    *listed = __shfl_sync(0xffffffffu, a.z, 0);
+    const unsigned int lo = __shfl_sync(0xffffffffu, a.x, 0), hi = __shfl_sync(0xffffffffu, a.y, 0);
+    const unsigned long long k = lo | (unsigned long long)hi << 32;
     return k == 0xffffffffffffffffULL ? INFINITY : ord_val(k);
 }
 
@@ -785,9 +799,10 @@ k_bound_find(int n, const uint4* __restrict__ tbits, ScoreParams sp,
     const int nwarps = gridDim.x * (blockDim.x >> 5);
     for (int task = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); task < tm.count; task += nwarps) {
         const int y0 = task % tm.yb * 32, x = task / tm.yb % tm.planes, o = tm.orient(task / (tm.yb * tm.planes));
-        const BoundEntry now = bound_entry(st);
-        double best = ALL ? INFINITY : now.best;
-        if (now.count > PSB_BCAP) return;   // the list is lost anyway
+        int listed;
+        double best = bound_now(st, &listed);
+        if (ALL) best = INFINITY;
+        if (listed > PSB_BCAP) return;   // the list is lost anyway
         const BoundCols bc = bound_cols(ba, sp, NW, o, x, y0 + lane, best);
         if (!(__shfl_sync(0xffffffffu, bc.h, 15) < INFINITY)) {   // not scored here: the list counts as lost
             if (lane == 0) atomicMax(&st->count, PSB_BCAP + 1);
@@ -1057,7 +1072,9 @@ k_bound_ray(const uint4* __restrict__ tbits, int tq, ScoreParams sp, BoundArgs b
 #pragma unroll
         for (int a = 0; a < 3; ++a)
             if (k % 3 == a) c[a] += k < 3 ? -1 - i : 1 + i;
-        if ((*(volatile unsigned int*)&st->blocked >> k) & 1u) continue;
+        unsigned int blocked = 0u;   // as one lane sees it: other warps are adding to it
+        if (lane == 0) blocked = *(volatile unsigned int*)&st->blocked;
+        if (__shfl_sync(0xffffffffu, blocked, 0) >> k & 1u) continue;
         if (!bound_free(od, (const uint32_t*)tbits, 4 * tq, sp.ny, c[0], c[1], c[2]) && lane == 0)
             atomicOr(&st->blocked, 1u << k);
     }
