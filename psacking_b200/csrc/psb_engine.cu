@@ -1121,6 +1121,7 @@ struct psb_tray {
     size_t x_cap = 0;
     ItemSums* d_xsums = nullptr;
     OrientDesc* d_xod = nullptr;
+    const int32_t* d_xitem = nullptr;   // the first array's values
     BoundReply* d_reply = nullptr;
 
     // per-column prefix sums along z of the distance field and the occupancy
@@ -2104,11 +2105,23 @@ struct psb_tray {
         return PSB_OK;
     }
 
-    // device placement of the staged item (stage_arrays); *nvox: its voxels
-    int place(int px, int py, int pz, int32_t id, int32_t* overlap_ijk, int* nvox) {
+    // device placement of the staged item (stage_arrays) of extent e; *nvox: its voxels
+    int place(const int32_t* e, int px, int py, int pz, int32_t id, int32_t* overlap_ijk, int* nvox) {
+        const long long at[3] = {px, py, pz}, n[3] = {nx, ny, nz};
+        PlaceBox box;
+        size_t cells = 1;   // of the item inside the tray
+        for (int a = 0; a < 3; ++a) {
+            const long long lo = std::max(0LL, at[a]), hi = std::min(n[a], at[a] + e[a]);
+            box.lo[a] = (int)lo;
+            box.n[a] = (int)std::max(0LL, hi - lo);
+            box.off[a] = (int)(lo - at[a]);
+            cells *= (size_t)box.n[a];
+        }
         CK(cudaMemsetAsync(d_first, 0xff, sizeof(unsigned long long), st));
-        pdl(k_place_runs_check, 148, 256, 0, st)(d_xod, d_tray, nx, ny, nz, px, py, pz, d_first);
-        CKL();
+        if (cells) {
+            pdl(k_place_dense<false>, grid1d(cells), 256, 0, st)(d_xitem, e[1], e[2], d_tray, ny, nz, box, id, d_first);
+            CKL();
+        }
         unsigned long long first = 0;
         OrientDesc od;
         int neg = 0;
@@ -2125,8 +2138,10 @@ struct psb_tray {
                         "(place_in_tray): Item to be placed intersects with contents of tray at position (%d, %d, %d)",
                         i, j, k);
         }
-        pdl(k_place_runs_write, 148, 256, 0, st)(d_xod, d_tray, nx, ny, nz, px, py, pz, id);
-        CKL();
+        if (cells) {
+            pdl(k_place_dense<true>, grid1d(cells), 256, 0, st)(d_xitem, e[1], e[2], d_tray, ny, nz, box, id, d_first);
+            CKL();
+        }
         occ_stale = bits_stale = true;
         if (id == 1 && od.nvox > 0) {  // only voxels equal to 1 are distance sources (fft3.cu:948)
             TRY(distance_on_device(d_tray, d_phi, nx, ny, nz, st));
@@ -2255,7 +2270,7 @@ int stage_arrays(psb_tray* t, const int32_t* const* items, const int32_t* dims, 
     CK(cudaMemcpyAsync(t->d_x, h, in, cudaMemcpyHostToDevice, t->st));
     t->d_xsums = (ItemSums*)(t->d_x + os);
     t->d_xod = (OrientDesc*)(t->d_x + od);
-    const int32_t* vals = (const int32_t*)(t->d_x + ov);
+    const int32_t* vals = t->d_xitem = (const int32_t*)(t->d_x + ov);
     const ItemArr* arrs = (const ItemArr*)t->d_x;
     int4* runs = (int4*)(t->d_x + orn);
     PROF("k_item_describe", t->st);
@@ -3090,7 +3105,7 @@ int psb_tray_place(psb_tray* t, const int32_t* item, int ex, int ey, int ez, int
     int32_t dims[3] = {ex, ey, ez};
     int nvox = 0;
     TRY(stage_arrays(t, items, dims, 1));
-    TRY(t->place(px, py, pz, item_id, nullptr, &nvox));
+    TRY(t->place(dims, px, py, pz, item_id, nullptr, &nvox));
     t->occ += (size_t)nvox;
     return PSB_OK;
 }

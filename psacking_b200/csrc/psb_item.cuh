@@ -214,38 +214,29 @@ k_item_describe(const int32_t* __restrict__ vals, const ItemArr* __restrict__ ar
     out[o] = d;
 }
 
-// Placement of a described item by its runs: the first tray cell (row-major)
-// where it meets an occupied one, then, when there is none, the cells written
-// (packing.cpp:773-788; parts outside the tray are left out).  One warp per
-// run.  grid: any, block 256
-__global__ void k_place_runs_check(const OrientDesc* __restrict__ od_p, const int32_t* __restrict__ tray, int nx, int ny,
-                                   int nz, int px, int py, int pz, unsigned long long* first) {
+// Placement of an item in a resident tray: the first tray cell (row-major)
+// where it meets an occupied one (WRITE false), then, when there is none, the
+// cells written (packing.cpp:773-788).  Over the dense item, since a run's ends
+// are 16 bits wide and the item may be longer than the tray (parts outside are
+// left out): tray box of n cells from lo on, which lies at off in the item.
+// grid: any, block 256
+struct PlaceBox {
+    int lo[3], n[3], off[3];
+};
+template <bool WRITE>
+__global__ void k_place_dense(const int32_t* __restrict__ item, int ey, int ez, int32_t* __restrict__ tray, int ny, int nz,
+                              PlaceBox b, int32_t id, unsigned long long* first) {
     pdl_enter();
-    const OrientDesc& od = *od_p;
-    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    for (int r = blockIdx.x * wpb + (threadIdx.x >> 5); r < od.nruns; r += gridDim.x * wpb) {
-        const int4 q = od.runs[r];
-        const int i = px + q.x, j = py + q.y;
-        if (q.w <= 0 || i < 0 || j < 0 || i >= nx || j >= ny) continue;
-        const size_t col = ((size_t)i * ny + j) * nz;
-        const int z1 = min(nz - 1, pz + (q.z >> 16));
-        for (int z = max(0, pz + (q.z & 0xffff)) + lane; z <= z1; z += 32)
-            if (tray[col + z] > 0) atomicMin(first, (unsigned long long)(col + z));
-    }
-}
-__global__ void k_place_runs_write(const OrientDesc* __restrict__ od_p, int32_t* __restrict__ tray, int nx, int ny, int nz,
-                                   int px, int py, int pz, int32_t id) {
-    pdl_enter();
-    const OrientDesc& od = *od_p;
-    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    for (int r = blockIdx.x * wpb + (threadIdx.x >> 5); r < od.nruns; r += gridDim.x * wpb) {
-        const int4 q = od.runs[r];
-        const int i = px + q.x, j = py + q.y;
-        if (q.w <= 0 || i < 0 || j < 0 || i >= nx || j >= ny) continue;
-        const size_t col = ((size_t)i * ny + j) * nz;
-        const int z1 = min(nz - 1, pz + (q.z >> 16));
-        for (int z = max(0, pz + (q.z & 0xffff)) + lane; z <= z1; z += 32)
-            if (tray[col + z] == 0) tray[col + z] = id;
+    const size_t m = (size_t)b.n[0] * b.n[1] * b.n[2];
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < m; t += (size_t)gridDim.x * blockDim.x) {
+        const int k = (int)(t % b.n[2]), j = (int)(t / b.n[2] % b.n[1]), i = (int)(t / ((size_t)b.n[2] * b.n[1]));
+        if (__ldg(&item[((size_t)(i + b.off[0]) * ey + (j + b.off[1])) * ez + k + b.off[2]]) <= 0) continue;
+        const size_t c = ((size_t)(i + b.lo[0]) * ny + (j + b.lo[1])) * nz + k + b.lo[2];
+        if (WRITE) {
+            if (tray[c] == 0) tray[c] = id;
+        } else if (tray[c] > 0) {
+            atomicMin(first, (unsigned long long)c);
+        }
     }
 }
 

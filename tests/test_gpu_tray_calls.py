@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 LIB = Path(__file__).resolve().parent.parent / "psacking_b200" / "libpsb200.so"
 SCAN, BLOCK, INTERLOCK = 0, 1, 0x10
-PSB_ERR_ARG = 1
+PSB_ERR_ARG, PSB_ERR_OVERLAP = 1, 4
 
 
 class Res(ctypes.Structure):
@@ -213,3 +213,32 @@ def test_search_with_shifted_distances(gpu_core, shift, flags):
         items = [np.ones((3, 4, 30), np.int32), np.ones((5, 6, 7), np.int32)]
         with Tray(tray, phi) as t:
             assert t.search(items, flags) == by_transforms(gpu_core, tray, phi, items, flags)
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("length", [30, 32767, 32768, 65536, 100_001])
+def test_place_arrays_longer_than_the_tray(gpu_core, length, axis):
+    """Long arrays whose last cells reach into the tray, and such that meet a
+    filled cell there: the tray's part is written, or nothing is."""
+    rng = np.random.default_rng(length)
+    shape = (20, 18, 16)
+    tray = np.zeros(shape, np.int32)
+    tray[tuple(slice(8, 10) if a == axis else slice(None) for a in range(3))] = 3   # met by the longer reach only
+    e = [3, 4, 5]
+    e[axis] = length
+    item = (rng.random(e) < 0.7).astype(np.int32)
+    at = [1, 2, 3]
+    for inside in (6, 15):
+        at[axis] = inside - length
+        want = tray.copy()
+        lo = [max(0, a) for a in at]
+        hi = [min(s, a + m) for s, a, m in zip(shape, at, e)]
+        box = tuple(slice(p, q) for p, q in zip(lo, hi))
+        part = item[tuple(slice(p - a, q - a) for p, q, a in zip(lo, hi, at))] > 0
+        overlap = bool((want[box][part] > 0).any())
+        if not overlap:
+            want[box][part] = 7
+        with Tray(tray) as t:
+            st = t.lib.psb_tray_place(t.h, item.ctypes.data, *e, *at, 7)
+            assert st == (PSB_ERR_OVERLAP if overlap else 0), t.err()
+            np.testing.assert_array_equal(t.get()[0], want)
