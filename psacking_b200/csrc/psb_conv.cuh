@@ -27,9 +27,33 @@ __device__ __forceinline__ void copy4_async(float* dst, const float* src, bool o
 
 __device__ __forceinline__ float bf16_up(uint16_t h) { return __uint_as_float((uint32_t)h << 16); }
 
+// The kernels below multiply the zeros around an input, and zero gradients,
+// where the layer's definition has no term.  That gives the same sums as long as
+// the other factor is finite; a term it is not for makes the sum infinite or NaN.
+// So results that are not finite are summed once more, term by term, without
+// the terms that do not exist (the functions named _terms, out of line: the
+// check is the only cost for ordinary values).
+__device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) < INFINITY); }
+
 // ---------------------------------------------------------------------------
 // forward with ReLU
 // ---------------------------------------------------------------------------
+// one result before the ReLU: sample s, channel co, output position r
+template <int CI, int D>
+__device__ __noinline__ float conv3_fwd_terms(const float* __restrict__ in, int s, const uint16_t* __restrict__ w,
+                                              const float* __restrict__ bias, int co, int r) {
+    constexpr int Do = D / 2;
+    const int od = r / (Do * Do), oh = r / Do % Do, ow = r % Do;
+    float acc = bias[co];
+#pragma unroll 1
+    for (int ct = 0; ct < CI * 27; ++ct) {
+        const int t = ct % 27, id = 2 * od - 1 + t / 9, ih = 2 * oh - 1 + t / 3 % 3, iw = 2 * ow - 1 + t % 3;
+        if (id < 0 || ih < 0 || iw < 0) continue;
+        acc = fmaf(in[((((size_t)s * CI + ct / 27) * D + id) * D + ih) * D + iw], bf16_up(w[(size_t)co * CI * 27 + ct]), acc);
+    }
+    return acc;
+}
+
 // A CTA computes all CO channels of VPC consecutive output positions (of one
 // sample's SL output slabs, or of NS whole samples), CH input channels at a
 // time.  The staged input has a zero row at index 0 of each axis (the padding;
@@ -130,12 +154,24 @@ k_conv3_fwd(const float* __restrict__ in, int S, const uint16_t* __restrict__ w,
         }
         __syncthreads();
     }
+    bool again = false;
 #pragma unroll
     for (int i = 0; i < TV; ++i) {
         const int r = vt + i * C::NV, s = r / (C::SL * C::Do2), q = r % (C::SL * C::Do2) + od0 * C::Do2;
         if (s >= ns) continue;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) out[((size_t)(s0 + s) * CO + 8 * g + c) * C::Do3 + q] = fmaxf(acc[i][c], 0.f);
+        for (int c = 0; c < 8; ++c) {
+            again = again || not_finite(acc[i][c]);
+            out[((size_t)(s0 + s) * CO + 8 * g + c) * C::Do3 + q] = fmaxf(acc[i][c], 0.f);
+        }
+    }
+    if (!again) return;
+#pragma unroll 1
+    for (int e = 0; e < 8 * TV; ++e) {
+        const int r = vt + e / 8 * C::NV, s = r / (C::SL * C::Do2), q = r % (C::SL * C::Do2) + od0 * C::Do2;
+        const int co = 8 * g + e % 8;
+        if (s < ns)
+            out[((size_t)(s0 + s) * CO + co) * C::Do3 + q] = fmaxf(conv3_fwd_terms<CI, D>(in, s0 + s, w, bias, co, q), 0.f);
     }
 }
 
@@ -161,6 +197,23 @@ struct ConvBwd {
     static constexpr size_t smem = sizeof(float) * ((size_t)NS * CH * CHAN + (size_t)CH * CI * 28);
     static_assert(CELLS % Do2 == 0 && (CELLS < Do3 ? Do3 % CELLS == 0 : CELLS % Do3 == 0) && CO % CH == 0, "tile");
 };
+
+// one result before the mask: sample s, channel ci, input position (id, ih, iw)
+template <int CI, int D, int CO>
+__device__ __noinline__ float conv3_bwd_data_terms(const float* __restrict__ dout, int s, const uint16_t* __restrict__ w,
+                                                   int ci, int id, int ih, int iw) {
+    constexpr int Do = D / 2, Do3 = Do * Do * Do;
+    float acc = 0.f;
+#pragma unroll 1
+    for (int t = 0; t < 27; ++t) {
+        const int ed = id + 1 - t / 9, eh = ih + 1 - t / 3 % 3, ew = iw + 1 - t % 3;   // twice the output position
+        if ((ed | eh | ew) & 1 || ed / 2 >= Do || eh / 2 >= Do || ew / 2 >= Do || ed < 0 || eh < 0 || ew < 0) continue;
+        const float* g = dout + (size_t)s * CO * Do3 + (ed / 2 * Do + eh / 2) * Do + ew / 2;
+#pragma unroll 1
+        for (int co = 0; co < CO; ++co) acc = fmaf(g[(size_t)co * Do3], bf16_up(w[((size_t)co * CI + ci) * 27 + t]), acc);
+    }
+    return acc;
+}
 
 template <int CI, int D, int CO, int CH>
 __global__ void __launch_bounds__(256, 2)
@@ -243,11 +296,14 @@ k_conv3_bwd_data(const float* __restrict__ dout, int S, const uint16_t* __restri
             __syncthreads();
         }
         if (cs >= ns) continue;
+        bool again = false;
 #pragma unroll
         for (int ci = 0; ci < 4; ++ci) {
             const size_t base = ((size_t)(s0 + cs) * CI + 4 * g + ci) * D * D * D;
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
+#pragma unroll
+                for (int p = 0; p < 4; ++p) again = again || not_finite(acc[ci][p >> 1][2 * r + (p & 1)]);
                 const size_t at = base + ((size_t)(2 * (d0 + d) + (r >> 1)) * D + 2 * h + (r & 1)) * D + 2 * cw;
                 const float4 m = __ldg((const float4*)(in + at));
                 float4 v;
@@ -257,6 +313,13 @@ k_conv3_bwd_data(const float* __restrict__ dout, int S, const uint16_t* __restri
                 v.w = !(m.w <= 0.f) ? acc[ci][1][2 * r + 1] : 0.f;
                 *(float4*)(din + at) = v;
             }
+        }
+        if (!again) continue;
+#pragma unroll 1
+        for (int e = 0; e < 64; ++e) {
+            const int ci = 4 * g + e / 16, id = 2 * (d0 + d) + (e >> 3 & 1), ih = 2 * h + (e >> 2 & 1), iw = 2 * cw + (e & 3);
+            const size_t at = ((((size_t)(s0 + cs) * CI + ci) * D + id) * D + ih) * D + iw;
+            din[at] = in[at] <= 0.f ? 0.f : conv3_bwd_data_terms<CI, D, CO>(dout, s0 + cs, w, ci, id, ih, iw);
         }
     }
 }
@@ -288,6 +351,30 @@ struct ConvBwdW {
     static_assert(256 % (CG * NQ) == 0 && Do % SEG == 0 && Do % SL == 0 && CI % CG == 0, "tile");
     static_assert(NVOX % 8 == 0 && CO % 4 == 0, "staging");
 };
+
+// one thread's 27 sums for input channel ci and output channel co over the
+// samples [sa, sb); returns the bias sum
+template <int CI, int D, int CO>
+__device__ __noinline__ float conv3_bwd_weight_terms(const float* __restrict__ dout, const float* __restrict__ in, int sa,
+                                                     int sb, int ci, int co, float* __restrict__ sums) {
+    constexpr int Do = D / 2, Do3 = Do * Do * Do;
+    float b = 0.f;
+    for (int t = 0; t < 27; ++t) sums[t] = 0.f;
+    for (int s = sa; s < sb; ++s)
+        for (int r = 0; r < Do3; ++r) {
+            const float g = dout[((size_t)s * CO + co) * Do3 + r];
+            if (g == 0.f) continue;
+            b += g;
+            const int od = r / (Do * Do), oh = r / Do % Do, ow = r % Do;
+#pragma unroll 1
+            for (int t = 0; t < 27; ++t) {
+                const int id = 2 * od - 1 + t / 9, ih = 2 * oh - 1 + t / 3 % 3, iw = 2 * ow - 1 + t % 3;
+                if (id < 0 || ih < 0 || iw < 0) continue;
+                sums[t] = fmaf(g, in[((((size_t)s * CI + ci) * D + id) * D + ih) * D + iw], sums[t]);
+            }
+        }
+    return b;
+}
 
 template <int CI, int D, int CO, int CG, int SL, int NS, int SEG>
 __global__ void __launch_bounds__(256)
@@ -370,12 +457,28 @@ k_conv3_bwd_weight(const float* __restrict__ dout, const float* __restrict__ in,
             }
         }
     }
-    __syncthreads();   // the buffers become the sums'
+    bool again = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+#pragma unroll
+        for (int t = 0; t < 27; ++t) again = again || not_finite(acc[k][t]);
+        again = again || not_finite(bacc[k]);
+    }
+    again = __syncthreads_or(again);   // the buffers become the sums'
     // the copies' sums, one copy after another
     float* red = sm;                             // [CG * NQ][108], then [CO]
     float* rb = red + CG * C::NQ * 108;
     const int slot = cg * C::NQ + q;
-    for (int k = 0; k < C::NSUB; ++k) {
+    if (again) {
+        for (int p = tid; p < CG * CO; p += 256) {
+            const int co = p % CO, ci = p / CO;
+            const float b = conv3_bwd_weight_terms<CI, D, CO>(dout, in, sa, sb, c0 + ci, co,
+                                                              red + (ci * C::NQ + co / 4) * 108 + co % 4 * 27);
+            if (blockIdx.x == 0 && ci == 0) rb[co] = b;
+        }
+        __syncthreads();
+    }
+    for (int k = 0; k < (again ? 0 : C::NSUB); ++k) {
         if (sub == k) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
