@@ -2193,20 +2193,28 @@ int arena(size_t bytes, void** out, Arena* a = nullptr) {
 }
 
 // pinned staging of the calling thread (uploads queued from it end before the
-// call that uses it returns), at most 64 MiB kept; given back with the thread
+// call that uses it returns), at most kPinnedKeep kept (PinnedTrim); given back
+// with the thread
+constexpr size_t kPinnedKeep = (size_t)64 << 20;
 struct PinnedBlock {
     char* p = nullptr;
     size_t n = 0;
-    ~PinnedBlock() { if (p) cudaFreeHost(p); }
+    void drop() {
+        if (p) cudaFreeHost(p);
+        p = nullptr;
+        n = 0;
+    }
+    ~PinnedBlock() { drop(); }
 };
 thread_local PinnedBlock g_pinned;
+struct PinnedTrim {
+    ~PinnedTrim() { if (g_pinned.n > kPinnedKeep) g_pinned.drop(); }
+};
 
 int pinned(size_t bytes, char** out) {
     PinnedBlock& b = g_pinned;
-    if (b.n < bytes || b.n > std::max(bytes, (size_t)64 << 20)) {
-        if (b.p) cudaFreeHost(b.p);
-        b.p = nullptr;
-        b.n = 0;
+    if (b.n < bytes) {
+        b.drop();
         CK(cudaMallocHost((void**)&b.p, bytes));
         b.n = bytes;
     }
@@ -2226,9 +2234,34 @@ struct ArenaTrim {
     }
 };
 
+// Gives a tray's block of staged arrays back when a call ends, where it is larger
+// than what a packing program's searches need.
+struct StageTrim {
+    psb_tray* t;
+    ~StageTrim() {
+        if (t->x_cap <= (size_t)256 << 20) return;
+        dfree(t->d_x, t->st);
+        t->x_cap = 0;
+    }
+};
+
+// number of runs of equal nonzero values along z (k_item_runs)
+size_t count_runs(const int32_t* a, size_t cols, size_t ez) {
+    size_t r = 0;
+    for (size_t c = 0; c < cols; ++c, a += ez) {
+        r += a[0] != 0;
+        for (size_t z = 1; z < ez; ++z) r += a[z] != 0 && a[z] != a[z - 1];
+    }
+    return r;
+}
+
 // Upload explicit orientation arrays and queue their analysis (psb_item.cuh):
 // their descriptors at t->d_xod.  Negative values are found there; the caller
 // reads t->d_reply->neg with its results.
+// There is room for a run per cell, four times the arrays' own size, up to
+// 2^24 cells (256 MiB of runs); above that the host counts the runs first, so
+// that large sparse arrays take what they fill.  Arrays of more than
+// kPinnedKeep are not copied into pinned memory as a whole.
 int stage_arrays(psb_tray* t, const int32_t* const* items, const int32_t* dims, int n) {
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
     size_t cells = 0;
@@ -2240,7 +2273,18 @@ int stage_arrays(psb_tray* t, const int32_t* const* items, const int32_t* dims, 
     }
     const size_t ov = up(sizeof(ItemArr) * n), in = ov + up(sizeof(int32_t) * cells);
     const size_t os = in, od = os + up(sizeof(ItemSums) * n), op = od + up(sizeof(OrientDesc) * n);
-    const size_t orn = op + up(sizeof(int4) * PSB_FSAMP * n), bytes = orn + sizeof(int4) * cells;
+    const bool counted = cells > (size_t)1 << 24;
+    std::vector<size_t> nruns(counted ? n : 0);
+    size_t room = cells;
+    if (counted) {
+        parallel_chunks((size_t)n, 1, [&](size_t b, size_t e) {
+            for (size_t o = b; o < e; ++o)
+                nruns[o] = count_runs(items[o], (size_t)dims[3 * o] * dims[3 * o + 1], dims[3 * o + 2]);
+        });
+        room = 0;
+        for (size_t r : nruns) room += r;
+    }
+    const size_t orn = op + up(sizeof(int4) * PSB_FSAMP * n), bytes = orn + sizeof(int4) * room;
     if (bytes > t->x_cap) {
         dfree(t->d_x, t->st);
         t->x_cap = 0;
@@ -2249,25 +2293,31 @@ int stage_arrays(psb_tray* t, const int32_t* const* items, const int32_t* dims, 
     }
     TRY(t->ensure_reply());
     char* h = nullptr;
-    TRY(pinned(in, &h));
+    const bool whole = in <= kPinnedKeep;
+    TRY(pinned(whole ? in : ov, &h));
     ItemArr* tab = (ItemArr*)h;
-    size_t off = 0;
-    int maxcol = 1;
+    size_t off = 0, roff = 0;
+    long long maxcol = 1;
     for (int o = 0; o < n; ++o) {
         const int32_t* d = dims + 3 * o;
         const size_t m = (size_t)d[0] * d[1] * d[2];
-        tab[o].off = tab[o].roff = (long long)off;
+        tab[o].off = (long long)off;
+        tab[o].roff = (long long)(counted ? roff : off);
+        tab[o].room = (long long)(counted ? nruns[o] : m);
+        if (counted) roff += nruns[o];
         for (int a = 0; a < 3; ++a) tab[o].d[a] = d[a];
         tab[o].skip = d[0] > t->nx || d[1] > t->ny || d[2] > t->nz;
         off += (m + 3) / 4 * 4;
-        maxcol = std::max(maxcol, d[0] * d[1]);
+        maxcol = std::max(maxcol, (long long)d[0] * d[1]);
     }
-    parallel_chunks((size_t)n, std::max((size_t)1, n * ((size_t)1 << 17) / cells), [&](size_t b, size_t e) {
-        for (size_t o = b; o < e; ++o)
-            stream_copy(h + ov + sizeof(int32_t) * tab[o].off, items[o],
-                        sizeof(int32_t) * (size_t)tab[o].d[0] * tab[o].d[1] * tab[o].d[2]);
-    });
-    CK(cudaMemcpyAsync(t->d_x, h, in, cudaMemcpyHostToDevice, t->st));
+    auto size = [&](size_t o) { return sizeof(int32_t) * (size_t)tab[o].d[0] * tab[o].d[1] * tab[o].d[2]; };
+    if (whole)
+        parallel_chunks((size_t)n, std::max((size_t)1, n * ((size_t)1 << 17) / cells), [&](size_t b, size_t e) {
+            for (size_t o = b; o < e; ++o) stream_copy(h + ov + sizeof(int32_t) * tab[o].off, items[o], size(o));
+        });
+    CK(cudaMemcpyAsync(t->d_x, h, whole ? in : ov, cudaMemcpyHostToDevice, t->st));
+    for (int o = 0; o < n && !whole; ++o)
+        CK(upload_async(t->d_x + ov + sizeof(int32_t) * tab[o].off, items[o], size(o), t->st));
     t->d_xsums = (ItemSums*)(t->d_x + os);
     t->d_xod = (OrientDesc*)(t->d_x + od);
     const int32_t* vals = t->d_xitem = (const int32_t*)(t->d_x + ov);
@@ -2277,7 +2327,7 @@ int stage_arrays(psb_tray* t, const int32_t* const* items, const int32_t* dims, 
     pdl(k_item_reset, (n + 127) / 128, 128, 0, t->st)(t->d_xsums, n, &t->d_reply->neg);
     CKL();
     for (int o0 = 0; o0 < n; o0 += 65535) {   // grid dimensions
-        pdl(k_item_runs, dim3(std::min(64, (maxcol + 7) / 8), std::min(n - o0, 65535)), 256, 0, t->st)(
+        pdl(k_item_runs, dim3((unsigned)std::min(64LL, (maxcol + 7) / 8), std::min(n - o0, 65535)), 256, 0, t->st)(
             vals, arrs + o0, runs, t->d_xsums + o0);
         CKL();
     }
@@ -2926,6 +2976,7 @@ int psb_place_in_tray(const int32_t* item, int ex, int ey, int ez, const int32_t
     void* base = nullptr;
     char* h = nullptr;
     TRY(arena(oi + sizeof(int32_t) * I + 16 + ob + 64, &base));
+    PinnedTrim ptrim;
     TRY(pinned(oi + sizeof(int32_t) * I, &h));
     char* d = (char*)base;
     char* d_out = d + (oi + sizeof(int32_t) * I + 15) / 16 * 16;   // [first][box]
@@ -3057,6 +3108,8 @@ int psb_tray_search(psb_tray* t, const int32_t* const* items, const int32_t* dim
             return PSB_OK;
         }
     }
+    PinnedTrim ptrim;
+    StageTrim strim{t};
     TRY(stage_arrays(t, items, dims, n));
     if (!per_orient && t->bound_usable() && (unsigned long long)n * t->V < 0xffffffffULL) {
         TRY(t->ensure_bound(n));
@@ -3104,6 +3157,8 @@ int psb_tray_place(psb_tray* t, const int32_t* item, int ex, int ey, int ez, int
     const int32_t* items[1] = {item};
     int32_t dims[3] = {ex, ey, ez};
     int nvox = 0;
+    PinnedTrim ptrim;
+    StageTrim strim{t};
     TRY(stage_arrays(t, items, dims, 1));
     TRY(t->place(dims, px, py, pz, item_id, nullptr, &nvox));
     t->occ += (size_t)nvox;
@@ -3988,6 +4043,7 @@ int psb_prop_item_grids(const int32_t* const* items, const int32_t* dims, int n_
     void* base = nullptr;
     char* h = nullptr;
     TRY(arena(bytes + sizeof(float) * (size_t)n_items * PSB_PG3, &base, &g_arena2));
+    PinnedTrim ptrim;
     TRY(pinned(bytes, &h));
     char* d = (char*)base;
     float* grid = (float*)(d + bytes);

@@ -10,7 +10,7 @@
 // One array: its values, the room for its runs and its dims.
 struct ItemArr {
     long long off;              // first value in `vals`
-    long long roff;             // first entry in `runs` (room for every cell)
+    long long roff, room;       // first entry in `runs`, entries there
     int d[3];
     int skip;                   // larger than the tray
 };
@@ -56,7 +56,8 @@ k_item_runs(const int32_t* __restrict__ vals, const ItemArr* __restrict__ arrs, 
     pdl_enter();
     const ItemArr it = arrs[blockIdx.y];
     const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    const int ncol = it.d[0] * it.d[1], ez = it.d[2];
+    const long long ncol = (long long)it.d[0] * it.d[1];
+    const int ez = it.d[2];
     const unsigned int below = (1u << lane) - 1u;
     ItemSums* S = sums + blockIdx.y;
     int4* R = runs + it.roff;
@@ -64,9 +65,9 @@ k_item_runs(const int32_t* __restrict__ vals, const ItemArr* __restrict__ arrs, 
     long long sum = 0;
     int nvox = 0, neg = 0;
     int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {-1, -1, -1};
-    for (int c = blockIdx.x * wpb + (threadIdx.x >> 5); c < ncol; c += gridDim.x * wpb) {
+    for (long long c = blockIdx.x * wpb + (threadIdx.x >> 5); c < ncol; c += gridDim.x * wpb) {
         const int32_t* col = vals + it.off + (size_t)c * ez;
-        const int i = c / it.d[1], j = c % it.d[1];
+        const int i = c >> 31 ? (int)(c / it.d[1]) : (int)c / it.d[1], j = (int)(c - (long long)i * it.d[1]);
         int cnt = 0;
         for (int z0 = 0; z0 < ez; z0 += 32) {
             const int z = z0 + lane;
@@ -88,6 +89,7 @@ k_item_runs(const int32_t* __restrict__ vals, const ItemArr* __restrict__ arrs, 
         int base = 0;
         if (lane == 0) base = atomicAdd(&S->nruns, cnt);
         base = __shfl_sync(0xffffffffu, base, 0);
+        if (base + cnt > it.room) continue;   // cannot be, unless the array changed while it was counted
         int s = base, e = base;
         for (int z0 = 0; z0 < ez; z0 += 32) {
             const int z = z0 + lane;
@@ -148,7 +150,8 @@ k_item_describe(const int32_t* __restrict__ vals, const ItemArr* __restrict__ ar
     __shared__ unsigned long long best[PSB_ICELLS];
     const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const ItemArr it = arrs[o];
-    const ItemSums S = sums[o];
+    ItemSums S = sums[o];
+    S.nruns = (int)min((long long)S.nruns, it.room);
     const int4* R = runs + it.roff;
     for (int i = tid; i < PSB_ICELLS; i += 256) best[i] = 0ULL;
     __syncthreads();

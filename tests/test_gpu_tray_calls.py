@@ -242,3 +242,32 @@ def test_place_arrays_longer_than_the_tray(gpu_core, length, axis):
             st = t.lib.psb_tray_place(t.h, item.ctypes.data, *e, *at, 7)
             assert st == (PSB_ERR_OVERLAP if overlap else 0), t.err()
             np.testing.assert_array_equal(t.get()[0], want)
+
+
+def test_search_of_many_large_arrays(gpu_core):
+    """Arrays that are counted before they are staged (above 2^24 cells, and too
+    large to be pinned as a whole) find what each finds on its own, and the tray
+    does not keep the memory they took (20 bytes per cell with room for a run
+    per cell; the tray's pool keeps 1 GiB)."""
+    import torch
+    rng = np.random.default_rng(8)
+    shape = (190, 185, 181)
+    tray = np.zeros(shape, np.int32)
+    tray[100:110, 5:25, 5:25] = 1
+    tray[60:90, 40:90, 30:60] = 2
+    items = []
+    for k in range(24):
+        it = np.zeros((180, 180, 180 - k), np.int32)
+        for _ in range(8):
+            it[tuple(slice(int(v), int(v) + 4) for v in rng.integers(0, 150, 3))] = 1 + k % 2
+        it[0, 0, 0] = it[-1, -1, -1] = 1
+        items.append(it)
+    with Tray(tray) as t:
+        alone = [t.search([i], BLOCK) for i in items]
+        free0 = torch.cuda.mem_get_info()[0]
+        got = t.search(items, BLOCK)
+        assert free0 - torch.cuda.mem_get_info()[0] < 3 << 29
+    found = [(r[5], o) for o, r in enumerate(alone) if r[0]]
+    assert found
+    score, o = min(found)
+    assert got == alone[o][:4] + (o, score)
