@@ -1067,7 +1067,9 @@ struct psb_tray {
     uint4* d_tbits = nullptr;               // free bits of the tray (k_tray_bits), tq uint4 per column
     int tq = 0;
     unsigned long long* d_work = nullptr;   // collision-kernel work counters (SearchBufs::work)
-    size_t occ = 0;                         // occupied cells of the tray, kept on the host
+    // occupied cells of the tray, kept on the host; inexact after a call that
+    // failed half-way, but 0 only when the tray is empty
+    size_t occ = 0;
     OrientDesc* d_bases = nullptr;          // their descriptors (synchronous searches)
     unsigned int* d_diag = nullptr;
     unsigned int* d_errmax = nullptr;
@@ -1419,6 +1421,7 @@ struct psb_tray {
         });
         if (neg) return fail(PSB_ERR_ARG, "tray holds negative values; item ids must be >= 0");
         occ = nocc;
+        ready = false;   // until the upload has been queued
         CK(upload_async(d_tray, tray, sizeof(int32_t) * V, st));
         if (phi) {
             CK(upload_async(d_phi, phi, sizeof(int32_t) * V, st));
@@ -2105,8 +2108,8 @@ struct psb_tray {
         return PSB_OK;
     }
 
-    // device placement of the staged item (stage_arrays) of extent e; *nvox: its voxels
-    int place(const int32_t* e, int px, int py, int pz, int32_t id, int32_t* overlap_ijk, int* nvox) {
+    // device placement of the staged item (stage_arrays) of extent e
+    int place(const int32_t* e, int px, int py, int pz, int32_t id, int32_t* overlap_ijk) {
         const long long at[3] = {px, py, pz}, n[3] = {nx, ny, nz};
         PlaceBox box;
         size_t cells = 1;   // of the item inside the tray
@@ -2130,7 +2133,6 @@ struct psb_tray {
         CK(cudaMemcpyAsync(&first, d_first, sizeof(first), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         if (neg != INT_MAX) return fail(PSB_ERR_ARG, "orientation %d holds negative values", neg);
-        *nvox = od.nvox;
         if (first != 0xffffffffffffffffULL) {
             int k = (int)(first % nz), j = (int)((first / nz) % ny), i = (int)(first / ((size_t)ny * nz));
             if (overlap_ijk) { overlap_ijk[0] = i; overlap_ijk[1] = j; overlap_ijk[2] = k; }
@@ -2138,6 +2140,7 @@ struct psb_tray {
                         "(place_in_tray): Item to be placed intersects with contents of tray at position (%d, %d, %d)",
                         i, j, k);
         }
+        occ += (size_t)od.nvox;
         if (cells) {
             pdl(k_place_dense<true>, grid1d(cells), 256, 0, st)(d_xitem, e[1], e[2], d_tray, ny, nz, box, id, d_first);
             CKL();
@@ -3156,12 +3159,10 @@ int psb_tray_place(psb_tray* t, const int32_t* item, int ex, int ey, int ez, int
     CK(cudaSetDevice(t->dev));
     const int32_t* items[1] = {item};
     int32_t dims[3] = {ex, ey, ez};
-    int nvox = 0;
     PinnedTrim ptrim;
     StageTrim strim{t};
     TRY(stage_arrays(t, items, dims, 1));
-    TRY(t->place(dims, px, py, pz, item_id, nullptr, &nvox));
-    t->occ += (size_t)nvox;
+    TRY(t->place(dims, px, py, pz, item_id, nullptr));
     return PSB_OK;
 }
 
@@ -3602,7 +3603,9 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
     // or not: an upper bound of the occupancy) fill less than a quarter of
     // the tray it rarely skips anything and only costs its kernels, so it
     // starts after that.  Its results are exact either way.
-    size_t occ_est = t->occ;
+    const size_t occ0 = t->occ;
+    t->occ = std::max(occ0, (size_t)1);   // not empty any more, should the run fail half-way
+    size_t occ_est = occ0;
     std::vector<OrientDesc> host_ods(n_orient);
     // One item through the transforms (and the flood fill), queued.
     auto transform_item = [&](int it) -> int {
@@ -3739,7 +3742,7 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
             fed = true;
         }
         OrientDesc* d_odb = t->d_od_all + (size_t)it * n_orient;
-        if (plain && first_pending && t->occ == 0 && t->phi_own && it == 0 && t->staged[it].nvox > 0) {
+        if (plain && first_pending && occ0 == 0 && t->phi_own && it == 0 && t->staged[it].nvox > 0) {
             // the first item of an empty tray (k_bound_first)
             int o = 0;
             while (o < n_orient && all[o].skip) ++o;
@@ -3816,6 +3819,7 @@ int pack_staged_impl(psb_tray* t, const int32_t* orient_maps, int n_orient, int 
         to_result(per[i], o, &opt.per_orient[i]);
         if (all[i].skip) opt.per_orient[i].diag |= 0x200u;
     }
+    t->occ = occ0;
     for (int it = 0; it < n_items; ++it) {
         psb_result r;
         r.x = dec[it].x; r.y = dec[it].y; r.z = dec[it].z;

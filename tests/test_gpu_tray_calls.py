@@ -271,3 +271,33 @@ def test_search_of_many_large_arrays(gpu_core):
     assert found
     score, o = min(found)
     assert got == alone[o][:4] + (o, score)
+
+
+def test_search_after_a_run_that_failed(gpu_core):
+    """Packing runs on an empty tray that fail at one of their allocations: a
+    search then answers for what the tray holds, be it empty or not."""
+    from psacking_b200 import workloads
+    from psacking_b200.rotations import orientation_maps
+    items = [np.ascontiguousarray(i, np.int32) for i in workloads.config1_items(5)[:6]]
+    ptrs = (ctypes.c_void_p * len(items))(*[i.ctypes.data for i in items])
+    dims = np.array([i.shape for i in items], np.int32).ravel()
+    maps = np.ascontiguousarray(orientation_maps(4), np.int32)
+    small = np.ones((2, 3, 2), np.int32)
+    filled = failed = 0
+    for k in range(1, 64):
+        with Tray(np.zeros((40, 36, 30), np.int32)) as t:
+            t.lib.psb_pack.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_int, ctypes.c_void_p, ctypes.c_int, ctypes.c_int,
+                                                               ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p]
+            t.lib.psb_debug_fail_alloc(k)
+            st = t.lib.psb_pack(t.h, ptrs, dims.ctypes.data, len(items), maps.ctypes.data, 4, 0, 0, (Res * len(items))(),
+                                None)
+            t.lib.psb_debug_fail_alloc(0)
+            tray, _ = t.get()
+            got = t.search([small], BLOCK)
+            pos = tuple(slice(p, p + e) for p, e in zip(got[1:4], small.shape))
+            assert got[0] and not tray[pos].any(), (k, st, got)
+            if st == 0:
+                break
+            failed += 1
+            filled += bool(tray.any())
+    assert failed >= 3 and filled >= 1
