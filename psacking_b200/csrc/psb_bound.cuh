@@ -896,9 +896,10 @@ k_bound_find(int n, const uint4* __restrict__ tbits, ScoreParams sp,
 
 // The item's outcome into the loop state and its decision record
 __device__ __forceinline__ void bound_commit(LoopState* ls, DecisionDev* out, const ScoreParams& sp, int o, int t,
-                                             double s, int ncand) {
+                                             double s, int ncand, bool flood = false) {
     DecisionDev d;
-    d.diag = 0x800u;   // decided without transforms
+    // decided without transforms; by a second selection after the flood fill
+    d.diag = flood ? 0xc00u : 0x800u;
     d.ncand = ncand;
     d.err_ratio = 0.f;
     d.found = o >= 0;
@@ -1037,7 +1038,7 @@ k_bound_score(const uint4* __restrict__ tbits, int tq, ScoreParams sp, BoundArgs
         out->ncand = count;
         return;
     }
-    bound_commit(ls, out, sp, o, t, best, count);
+    bound_commit(ls, out, sp, o, t, best, count, FLOOD);
 }
 
 // Interlocking mode: the cells between the winner and the six faces, one

@@ -301,3 +301,31 @@ def test_search_after_a_run_that_failed(gpu_core):
             failed += 1
             filled += bool(tray.any())
     assert failed >= 3 and filled >= 1
+
+
+@pytest.mark.parametrize("hole", ["sealed", "bent", "straight"])
+def test_search_reports_its_flood_fill(gpu_core, hole):
+    """A crowded tray whose best free place lies in a cavity: the flood-fill bit
+    of the result is set when that place has no straight way out, by the search
+    without transforms as by the transforms' form that floods only then."""
+    tray = np.full((24, 24, 100), 2, np.int32)   # tall: the height penalty is small at z = 1
+    tray[16:, 16:, :] = 0
+    tray[4:14, 4:14, 1:12] = 0
+    tray[8, 8, 1] = 1
+    if hole == "bent":
+        tray[4:9, 9:14, 12:] = 0
+    elif hole == "straight":
+        tray[4:14, 4:14, 12:] = 0
+    item = np.ones((4, 4, 5), np.int32)
+    FLOOD, DIRECT = 0x400, 0x800
+    with Tray(tray) as t:
+        got, r = t.search([item], BLOCK | INTERLOCK), t.search_status([item], BLOCK | INTERLOCK)[1]
+        assert r.diag & DIRECT and bool(r.diag & FLOOD) == (hole != "straight")
+        gpu_core.set_cand_filter(False)
+        gpu_core.set_plane_variant(2)
+        try:
+            assert t.search([item], BLOCK | INTERLOCK) == got
+            assert t.search_status([item], BLOCK | INTERLOCK)[1].diag & FLOOD == r.diag & FLOOD
+        finally:
+            gpu_core.set_plane_variant(3)
+            gpu_core.set_cand_filter(True)
