@@ -23,6 +23,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -76,8 +77,12 @@ class HostPool {
 
   private:
     HostPool() : pid_(getpid()) {
-        workers_ = (int)std::min(11u, std::max(1u, std::thread::hardware_concurrency()) - 1u);
-        for (int i = 0; i < workers_; ++i) std::thread([this] { loop(); }).detach();
+        const int want = (int)std::min(11u, std::max(1u, std::thread::hardware_concurrency()) - 1u);
+        try {
+            for (; workers_ < want; ++workers_) std::thread([this] { loop(); }).detach();
+        } catch (const std::system_error&) {
+            // no more threads to be had: the callers do the rest themselves
+        }
     }
     void loop() {
         std::unique_lock<std::mutex> lk(mu_);

@@ -5,6 +5,18 @@
 #include <cstdio>
 #include <string>
 
+#ifdef THREADS
+// a process that may have no more than THREADS threads of its own
+#include <cerrno>
+#include <dlfcn.h>
+#include <pthread.h>
+extern "C" int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* x) noexcept {
+    static int made = 0;
+    if (made++ >= THREADS) return EAGAIN;
+    return ((decltype(&pthread_create))dlsym(RTLD_NEXT, "pthread_create"))(t, a, f, x);
+}
+#endif
+
 static FakeStream g_stream[2];
 
 // upload_async, the source overwritten as soon as the call has returned
@@ -49,6 +61,14 @@ int main(int argc, char** argv) {
             ok = PinBlocks::get().take((size_t)2 << 20) == nullptr && ok;   // none is left while they are held
             for (PinBlock* x : b) if (x) PinBlocks::get().give(x, &g_stream[dev]);
         }
+    } else if (what == "chunks") {
+        const size_t n = (size_t)atoll(argv[2]);
+        std::vector<std::atomic<int>> seen(n);
+        parallel_chunks(n, 10, [&](size_t b, size_t e) {
+            for (size_t i = b; i < e; ++i) ++seen[i];
+        });
+        ok = true;
+        for (auto& c : seen) ok = ok && c == 1;
     }
     puts(ok ? "ok" : "wrong");
     fflush(stdout);

@@ -11,12 +11,16 @@ HERE = Path(__file__).resolve().parent / "host_copies"
 CSRC = HERE.parent.parent / "psacking_b200" / "csrc"
 
 
-@pytest.fixture(scope="module")
-def program(tmp_path_factory):
+def _build(tmp_path_factory, *flags):
     out = tmp_path_factory.mktemp("host_copies") / "main"
-    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", f"-I{HERE}", f"-I{CSRC}", "-x", "c++",
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", f"-I{HERE}", f"-I{CSRC}", *flags, "-x", "c++",
                     str(HERE / "main.cpp"), "-o", str(out)], check=True, capture_output=True, text=True)
     return str(out)
+
+
+@pytest.fixture(scope="module")
+def program(tmp_path_factory):
+    return _build(tmp_path_factory)
 
 
 def _run(program, *args):
@@ -44,3 +48,12 @@ def test_download_waits_on_the_callers_device(program, size, device):
 
 def test_staging_blocks_of_several_devices(program):
     _run(program, "two_devices")
+
+
+@pytest.mark.parametrize("threads", [0, 2])
+def test_without_threads_the_caller_does_the_work(tmp_path_factory, threads):
+    few = _build(tmp_path_factory, f"-DTHREADS={threads}")
+    for n in (1, 10, 11, 5000):
+        _run(few, "chunks", n)
+    _run(few, "upload", 5 << 20, "h")
+    _run(few, "download", 5 << 20, 0)
