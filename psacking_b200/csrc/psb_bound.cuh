@@ -260,19 +260,19 @@ k_bound_dedupe(OrientDesc* __restrict__ od_all, int n) {
 }
 
 // The tables, and the shift-sorted filter samples (as k_cand_prep), of every
-// orientation of the items i0 .. i0 + gridDim.y - 1: they depend on the items
-// and the sources only, so one launch serves a queue of items.
+// orientation of the items of a queue: they depend on the items and the sources
+// only, so one launch serves them all.
 // grid: (n, items), block 256
 template <int NW>
 __global__ void __launch_bounds__(256)
-k_bound_prep(const OrientDesc* __restrict__ od_all, int n, int i0, const BoundGeom* __restrict__ geom, ScoreParams sp,
+k_bound_prep(const OrientDesc* __restrict__ od_all, int n, const BoundGeom* __restrict__ geom, ScoreParams sp,
              double* __restrict__ tab, long long tstride, int2* __restrict__ fs, int* __restrict__ fbound) {
     pdl_enter();
     // marginals, their prefix sums and the prefix sums of k times them
     __shared__ unsigned long long hm[3][PSB_MAX_FFT + 1], c0[3][PSB_MAX_FFT + 1], c1[3][PSB_MAX_FFT + 1];
     __shared__ double sM[3], sW;
-    const int o = blockIdx.x, slot = blockIdx.y * n + o;
-    const OrientDesc& od = od_all[(size_t)(i0 + blockIdx.y) * n + o];
+    const int slot = blockIdx.y * n + blockIdx.x;
+    const OrientDesc& od = od_all[slot];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double* T = tab + (size_t)slot * tstride;
     if (tid < 3) T[9 + tid] = od.skip ? 0.0 : (double)od.valid[tid];
@@ -567,7 +567,6 @@ __device__ __forceinline__ int bound_count(const double* __restrict__ F, int n, 
 
 struct BoundArgs {
     BoundState* st;
-    const BoundGeom* geom;
     const double* tab;          // the item's tables (orientation stride tstride)
     long long tstride;
     const int2* fs;             // its samples: column offset, bit shift (PSB_BSAMP per orientation)

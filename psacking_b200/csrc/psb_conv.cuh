@@ -8,9 +8,10 @@
 // and a thread a block of results in registers, so that each shared load feeds
 // several FMAs: forward 8 positions x 8 channels (64 FMAs per 8 + 2 loads),
 // backward-data 2 cells x 8 parities x 4 channels (216 per 12 + 28), and
-// backward-weight 4 x 27 weights (108 per 18 + 1).  FP32 throughout: the tensor
-// cores would need the activations split into BF16 parts, and their
-// accumulation truncates.
+// backward-weight 4 x 27 weights (108 per 18 + 1).  FP32 throughout.  On the
+// tensor cores the FP32 activations would have to be split into three BF16 parts
+// (the weights are BF16 already); whether that keeps the present error has not
+// been tried.
 #pragma once
 #include <stdint.h>
 

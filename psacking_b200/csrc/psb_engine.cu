@@ -1663,7 +1663,7 @@ struct psb_tray {
     int bound_prep(const OrientDesc* d_odb, int n, int items, int mode) {
         PROF("k_bound_prep", st);
         auto k = tq == 1 ? k_bound_prep<4> : k_bound_prep<8>;
-        pdl(k, dim3(n, items), 256, 0, st)(d_odb, n, 0, d_bgeom, score_params(mode), d_btab,
+        pdl(k, dim3(n, items), 256, 0, st)(d_odb, n, d_bgeom, score_params(mode), d_btab,
                                            bound_tab_stride(nx, ny, nz), d_bfs, d_bfb);
         CKL();
         return PSB_OK;
@@ -1676,7 +1676,7 @@ struct psb_tray {
                      DecisionDev* d_out) {
         const ScoreParams sp = score_params(mode);
         const long long ts = bound_tab_stride(nx, ny, nz);
-        const BoundArgs ba{d_bstate, d_bgeom, d_btab + slot0 * ts, ts, d_bfs + slot0 * PSB_BSAMP,
+        const BoundArgs ba{d_bstate, d_btab + slot0 * ts, ts, d_bfs + slot0 * PSB_BSAMP,
                            d_bfb + slot0 * PSB_FBOUND, d_blist, d_blist + PSB_BCAP, d_pphi};
         const int yb = (ny + 31) / 32;
         // at most what the chip holds at once (launch bounds): a second wave

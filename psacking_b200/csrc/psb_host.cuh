@@ -5,7 +5,7 @@
 // one thread, and a fresh result array takes its page faults there as well:
 // 0.4-0.6 ms per copy at 240x123x100, several copies per call.  Here they go
 // through pinned blocks in chunks, the host cores copying one chunk while the
-// next is on the bus.  The cores' threads are made once per process (one
+// next is on the bus.  The threads that do so are made once per process (one
 // std::thread per core and call cost 0.2-0.4 ms per use).
 #pragma once
 #include <cuda_runtime.h>
