@@ -2171,11 +2171,20 @@ void to_result(const ResultDev& r, int orient, psb_result* out) {
     out->err_ratio = r.err_ratio;
 }
 
-// scratch arena for the stateless transforms
+// scratch arena of the stateless calls, kept by the calling thread and given
+// back with it
 struct Arena {
     void* p = nullptr;
     size_t n = 0;
     int dev = -1;
+    void drop() {
+        if (p) cudaFree(p);
+        p = nullptr;
+        n = 0;
+    }
+    ~Arena() {
+        if (p && cudaSetDevice(dev) == cudaSuccess) drop();
+    }
 };
 thread_local Arena g_arena, g_arena2;   // the second: sizes known only once the first is in use
 
@@ -2184,9 +2193,7 @@ int arena(size_t bytes, void** out, Arena* a = nullptr) {
     int dev = 0;
     CK(cudaGetDevice(&dev));
     if (a->n < bytes || a->dev != dev) {
-        if (a->p && a->dev == dev) cudaFree(a->p);
-        a->p = nullptr;
-        a->n = 0;
+        a->drop();
         CK(cudaMalloc(&a->p, bytes));
         a->n = bytes;
         a->dev = dev;
@@ -2230,10 +2237,7 @@ struct ArenaTrim {
     Arena* a;
     size_t keep;
     ~ArenaTrim() {
-        if (a->n <= keep) return;
-        cudaFree(a->p);
-        a->p = nullptr;
-        a->n = 0;
+        if (a->n > keep) a->drop();
     }
 };
 
