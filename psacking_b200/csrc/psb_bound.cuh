@@ -707,7 +707,13 @@ __device__ __forceinline__ BoundTasks bound_tasks(const BoundArgs& ba, const Sco
 // one would touch a cache line each).  There are few tasks and each is a
 // chain of load latencies, so a CTA takes one: its four warps share the
 // samples, meet in shared memory, and then check and score the four survivors
-// of lowest bound, one each.  grid: any, block 128
+// of lowest bound, one each.  Bound by those latencies: 13 % of the cycles issue,
+// 8.6 of 14.2 cycles per instruction wait for a load (a 128^3 tray, 24
+// orientations: 744 CTAs, 20 us).  So the CTAs per SM matter little: 6 (80
+// registers, 100 bytes spilled) and 4 (128 registers, 12 bytes) give 1.44 and
+// 1.45 ms for 20 boxes at 64^3, 7.9 and 8.1 ms for 100 items at 128^3, 42.2 and
+// 41.5 ms for 350 at 240x123x100, where runs of one side differ by up to 8 %.
+// grid: any, block 128
 template <int NQ>
 __global__ void __launch_bounds__(128, NQ == 1 ? 6 : 3)
 k_bound_seed(int n, const uint4* __restrict__ tbits, ScoreParams sp,
