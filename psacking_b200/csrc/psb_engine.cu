@@ -3883,7 +3883,12 @@ int psb_pack(psb_tray* t, const int32_t* const* items, const int32_t* dims, int 
         rest.join();
         return stage_upload(t, items, first, n_items, 1, t->st_copy);
     };
-    return pack_staged_impl(t, orient_maps, n_orient, interlock, id_offset, out_placements, final_tray, o);
+    const int rc = pack_staged_impl(t, orient_maps, n_orient, interlock, id_offset, out_placements, final_tray, o);
+    // a run that failed after the second part was queued has not waited for it,
+    // and that part's blocks are freed on the tray's own stream, into a pool
+    // that other trays take from
+    if (rc != PSB_OK) cudaStreamSynchronize(t->st_copy);
+    return rc;
 }
 
 int psb_pack_many(int n_trays, const int32_t* tray_dims, const int32_t* const* items, const int32_t* item_dims,

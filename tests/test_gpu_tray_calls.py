@@ -329,3 +329,31 @@ def test_search_reports_its_flood_fill(gpu_core, hole):
         finally:
             gpu_core.set_plane_variant(3)
             gpu_core.set_cand_filter(True)
+
+
+def test_failed_streamed_runs_leave_other_trays_alone(gpu_core):
+    """Runs staged in two parts that fail at each of their allocations, their
+    trays destroyed at once: the next tray, whose buffers come from the same
+    pool, packs as it does on its own."""
+    from psacking_b200 import BinPacker, workloads
+    from psacking_b200.rotations import orientation_maps
+    items = [np.ascontiguousarray(i, np.int32) for s in range(4) for i in workloads.config1_items(s)][:70]
+    ptrs = (ctypes.c_void_p * len(items))(*[i.ctypes.data for i in items])
+    dims = np.array([i.shape for i in items], np.int32).ravel()
+    maps = np.ascontiguousarray(orientation_maps(4), np.int32)
+    packer = BinPacker((50, 44, 60), num_orientations=4, interlocking_free=True)
+    want = packer.pack_voxels(items[:30]).tray
+    failed = 0
+    for k in range(1, 100):
+        with Tray(np.zeros((64, 64, 40), np.int32)) as t:
+            t.lib.psb_pack.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_int, ctypes.c_void_p, ctypes.c_int, ctypes.c_int,
+                                                               ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p]
+            t.lib.psb_debug_fail_alloc(k)
+            st = t.lib.psb_pack(t.h, ptrs, dims.ctypes.data, len(items), maps.ctypes.data, 4, 1, 0, (Res * len(items))(),
+                                None)
+            t.lib.psb_debug_fail_alloc(0)
+        np.testing.assert_array_equal(packer.pack_voxels(items[:30]).tray, want)
+        if st == 0:
+            break
+        failed += 1
+    assert failed >= 3
